@@ -480,10 +480,11 @@ __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src,
 #ifndef FSR_SMOOTH_MIN_BLOCKS
 #define FSR_SMOOTH_MIN_BLOCKS 4  // 64 registers: 4 blocks of 256 threads per SM (measured best of 1, 4, 5, 6)
 #endif
+template <bool kFast>
 __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(const float4* __restrict__ sorted, uint32_t n,
                                                      const uint2* __restrict__ ranges, Grid sp, float R,
-                                                     float R_rcp, float R_lt2, int coop_ok, float one_minus_lambda,
-                                                     float lambda, float mass, float4* __restrict__ mean,
+                                                     float R_rcp, float R_lt2, float tiny, int coop_ok,
+                                                     float one_minus_lambda, float lambda, float mass, float4* __restrict__ mean,
                                                      float4* __restrict__ mean32, float4* __restrict__ smoothed)
 {
     __shared__ float4 s_q[kThreads];  // 32 staged candidates per warp
@@ -506,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
         const float dx = __fsub_rn(p.x, q.x), dy = __fsub_rn(p.y, q.y), dz = __fsub_rn(p.z, q.z);
         const float d2 = dot3_rn(dx, dy, dz);
         if (!(d2 < R_lt2)) return;  // d >= R: weight 0, and +0 terms leave the sums unchanged
-        const float s = div_exact(__fsqrt_rn(d2), R, R_rcp);
+        const float s = dist_over<kFast>(d2, R, R_rcp, tiny);
         const float wt = __fsub_rn(1.0f, __fmul_rn(__fmul_rn(s, s), s));
         ws = __fadd_rn(ws, wt);
         mx = __fadd_rn(mx, __fmul_rn(q.x, wt));
@@ -625,7 +626,7 @@ constexpr uint32_t kCovSplitBelow = 1u << 17;  // particles below which P = 4
 #define FSR_COV_MIN_BLOCKS 16
 #endif
 
-template <int P>
+template <int P, bool kFast>
 __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs a, Counters* ctr)
 {
     __shared__ float4 s_q[kCovThreads];  // 32 staged candidates per warp
@@ -677,7 +678,7 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
             const float4 m32 = a.mean32[t];
             if (dot3_rn(__fsub_rn(q.x, m32.x), __fsub_rn(q.y, m32.y), __fsub_rn(q.z, m32.z)) < a.R_le2) ++nn;
         }
-        if (d2 < a.R_lt2) acc.add(vx, vy, vz, div_exact(__fsqrt_rn(d2), a.R, a.R_rcp));
+        if (d2 < a.R_lt2) acc.add(vx, vy, vz, dist_over<kFast>(d2, a.R, a.R_rcp, a.tiny));
     };
     auto near = [&](const float4& q) {
         return dot3_rn(__fsub_rn(q.x, m.x), __fsub_rn(q.y, m.y), __fsub_rn(q.z, m.z)) < pre2;
@@ -1290,9 +1291,9 @@ void launch_smooth(const KernelCtx& c, const float4* sorted, uint32_t n, const u
     // warps may walk the union of their windows when the cull radius stays
     // below two cells (see k_smooth)
     const int coop_ok = (R * 1.0001f + 1e-4f * sp.cs) < 2.0f * sp.cs * 0.9999f ? 1 : 0;
-    k_smooth<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R, sqrt_threshold(R, false),
-                                                       coop_ok, oml, lambda, mass, mean, mean32,
-                                                       smoothed);
+    const auto kernel = fast_radius(R) ? k_smooth<true> : k_smooth<false>;
+    kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R, sqrt_threshold(R, false),
+                                                         tiny_d2(R), coop_ok, oml, lambda, mass, mean, mean32, smoothed);
     ++g_launches;
 }
 
@@ -1304,10 +1305,15 @@ void launch_cov(const KernelCtx& c, const CovArgs& a0, Counters* ctr)
     a.R_rcp = 1.0f / a.R;
     a.R_le2 = sqrt_threshold(a.R, true);
     a.coop_ok = (a.R + a.R * 1.0001f + 1e-4f * a.sp.cs) < 2.0f * a.sp.cs * 0.9999f ? 1 : 0;
-    if (a.n < kCovSplitBelow)
-        k_cov<4><<<blocks_for((uint64_t)a.n * 4, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
-    else
-        k_cov<1><<<blocks_for(a.n, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+    a.tiny = tiny_d2(a.R);
+    const bool fast = fast_radius(a.R);
+    if (a.n < kCovSplitBelow) {
+        const auto kernel = fast ? k_cov<4, true> : k_cov<4, false>;
+        kernel<<<blocks_for((uint64_t)a.n * 4, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+    } else {
+        const auto kernel = fast ? k_cov<1, true> : k_cov<1, false>;
+        kernel<<<blocks_for(a.n, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+    }
     ++g_launches;
 }
 

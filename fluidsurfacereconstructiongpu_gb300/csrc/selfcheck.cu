@@ -29,6 +29,35 @@ __global__ void k_check_division(uint32_t hi_bits, float b, float rb, unsigned l
     if (local) atomicAdd(bad, local);
 }
 
+// Every float x in [2^-100, 2^100]: root_exact must equal __fsqrt_rn.  And
+// every float d2 in [0, R^2]: the weight 1 - (d/R)^3 formed through
+// dist_over<true> must equal the one through __fsqrt_rn and __fdiv_rn.
+__global__ void k_check_root(uint32_t lo_bits, uint32_t hi_bits, float R, float rR, float tiny, uint32_t r2_bits,
+                             unsigned long long* bad, unsigned long long* first_bad)
+{
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const uint64_t start = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long local = 0;
+    for (uint64_t i = lo_bits + start; i <= hi_bits; i += stride) {
+        const float x = __uint_as_float((uint32_t)i);
+        if (__float_as_uint(fsr::root_exact(x)) != __float_as_uint(__fsqrt_rn(x))) {
+            ++local;
+            atomicMin(first_bad, (unsigned long long)i);
+        }
+    }
+    auto weight = [](float s) { return __fsub_rn(1.0f, __fmul_rn(__fmul_rn(s, s), s)); };
+    for (uint64_t i = start; i <= r2_bits; i += stride) {
+        const float d2 = __uint_as_float((uint32_t)i);
+        const float a = weight(fsr::dist_over<true>(d2, R, rR, tiny));
+        const float b = weight(__fdiv_rn(__fsqrt_rn(d2), R));
+        if (__float_as_uint(a) != __float_as_uint(b)) {
+            ++local;
+            atomicMin(first_bad, (unsigned long long)i);
+        }
+    }
+    if (local) atomicAdd(bad, local);
+}
+
 // Every float x in (0, 1]: spiky_grad must equal float(k x x) in double.
 __global__ void k_check_spiky(double k, float khi, float klo, unsigned long long* bad, unsigned long long* first_bad)
 {
@@ -97,6 +126,34 @@ extern "C" fsr_status fsr_check_division(float b, uint64_t* n_checked, uint64_t*
     cudaFree(d);
     if (e != cudaSuccess) return FSR_ERR_CUDA;
     *n_checked = (uint64_t)hi_bits + 1;
+    *n_mismatch = out[0];
+    return FSR_OK;
+}
+
+extern "C" fsr_status fsr_check_root(float R, uint64_t* n_checked, uint64_t* n_mismatch)
+{
+    if (!fsr::fast_radius(R) || !n_checked || !n_mismatch) return FSR_ERR_INVALID_ARGUMENT;
+    const float lo = 0x1p-100f, hi = 0x1p100f, r2 = R * R;
+    uint32_t lo_bits, hi_bits, r2_bits;
+    std::memcpy(&lo_bits, &lo, 4);
+    std::memcpy(&hi_bits, &hi, 4);
+    std::memcpy(&r2_bits, &r2, 4);
+    unsigned long long* d = nullptr;
+    if (cudaMalloc(&d, 16) != cudaSuccess) return FSR_ERR_CUDA;
+    const unsigned long long init[2] = {0ull, ~0ull};
+    cudaError_t e = cudaMemcpy(d, init, 16, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        int dev = 0, sms = 1;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        k_check_root<<<sms * 8, 256>>>(lo_bits, hi_bits, R, 1.0f / R, fsr::tiny_d2(R), r2_bits, d, d + 1);
+        e = cudaGetLastError();
+    }
+    unsigned long long out[2] = {0, 0};
+    if (e == cudaSuccess) e = cudaMemcpy(out, d, 16, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    if (e != cudaSuccess) return FSR_ERR_CUDA;
+    *n_checked = (uint64_t)hi_bits - lo_bits + 1 + r2_bits + 1;
     *n_mismatch = out[0];
     return FSR_OK;
 }

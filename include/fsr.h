@@ -382,6 +382,13 @@ fsr_status fsr_batch_copy_mesh(const fsr_batch* b, uint32_t frame, float* pos, f
  * counts the results that differ (0 expected). */
 fsr_status fsr_check_division(float R, uint64_t* n_checked, uint64_t* n_mismatch);
 
+/* Self-check of the square root the same kernels use (an FMA correction of an
+ * approximate root, Markstein) for R in [2^-20, 2^40]: the root of every
+ * float in [2^-100, 2^100] against the correctly rounded one, and the weight
+ * 1 - (d/R)^3 of every squared distance in [0, R^2]; counts the results that
+ * differ (0 expected). */
+fsr_status fsr_check_root(float R, uint64_t* n_checked, uint64_t* n_mismatch);
+
 /* Self-check of the FP32 form of the colour field's gradient float(k x x)
  * (evaluated in double by the reference; k < 0, |k| in [1e-20, 1e30]): runs
  * it and the double expression for every float x in (0, 1] and counts the

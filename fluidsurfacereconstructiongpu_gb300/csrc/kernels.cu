@@ -461,6 +461,24 @@ __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src,
     return __popc(m);
 }
 
+// Lanes whose windows span few cells together walk their union together
+// (below); a warp whose windows lie further apart (its particles run over the
+// end of a row of cells) is cut into such sets of lanes, each walked on its own.
+// The lanes of `left` that form a set with its first lane: together with that
+// lane's window theirs spans at most span + 1 cells per axis.
+constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
+__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
+{
+    const int lead = __ffs((int)left) - 1;
+    bool ok = (left >> lane) & 1u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
+        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
+    }
+    return __ballot_sync(0xffffffffu, ok || lane == lead);
+}
+
 // ------------------------------------------------------------ anisotropic path
 // calculationOfMeanAndSmoothParticles (cu:598-658).  Two means per particle:
 // * mean32: the reference's FP32 sum sum(w x) / sum(w) in its order with its
@@ -480,10 +498,10 @@ __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src,
 #ifndef FSR_SMOOTH_MIN_BLOCKS
 #define FSR_SMOOTH_MIN_BLOCKS 4  // 64 registers: 4 blocks of 256 threads per SM (measured best of 1, 4, 5, 6)
 #endif
-template <bool kFast>
+template <bool kFast, bool kSets>
 __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(const float4* __restrict__ sorted, uint32_t n,
                                                      const uint2* __restrict__ ranges, Grid sp, float R,
-                                                     float R_rcp, float R_lt2, float tiny, int coop_ok,
+                                                     float R_rcp, float R_lt2, float tiny, int span,
                                                      float one_minus_lambda, float lambda, float mass, float4* __restrict__ mean,
                                                      float4* __restrict__ mean32, float4* __restrict__ smoothed)
 {
@@ -541,25 +559,30 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
             }
         }
     };
-    // A warp whose windows span at most 4 cells per axis walks their union
-    // together: each chunk of 32 candidates is loaded once (one per lane)
-    // and every lane tests all of them, so no lane idles on a window of its
-    // own.  Exact: a candidate outside a lane's window lies beyond the cull
-    // radius of its particle on some axis (coop_ok: that radius is below 2
-    // cells, so the +-2 cell window never cuts a lane's narrowed window),
-    // and the lane's own candidates keep their window order.
-    int ulo[3], uhi[3];
-    bool compact = coop_ok != 0;
+    // Lanes whose windows span few cells per axis walk their union together:
+    // each chunk of 32 candidates is loaded once (one per lane) and every lane
+    // tests all of them, so no lane idles on a window of its own.  Exact: a
+    // candidate outside a lane's window lies beyond the cull radius of its
+    // particle on some axis (span >= 0: that radius is below 2 cells, so the
+    // +-2 cell window never cuts a lane's narrowed window), and the lane's own
+    // candidates keep their window order.
+    // kSets (R above a cell: windows of up to 5 x 5 x 5 cells, which a lane on
+    // its own would take thousands of steps for): a warp whose windows lie
+    // apart walks them set by set.  Else the whole warp is one set or none
+    // (measured at R = 0.8 cells: in sets, smoothing 0.81 -> 0.87 ms at 1M).
+    auto walk = [&](bool in_set) {
+        int ulo[3], uhi[3];
+        bool compact = true;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        ulo[a] = (int)__reduce_min_sync(0xffffffffu, active ? (unsigned)w.lo[a] : 0x7fffffffu);
-        uhi[a] = (int)__reduce_max_sync(0xffffffffu, active ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
-        compact = compact && uhi[a] - ulo[a] <= 3;
-    }
-    if (compact) {
+        for (int a = 0; a < 3; ++a) {
+            ulo[a] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)w.lo[a] : 0x7fffffffu);
+            uhi[a] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
+            compact = compact && uhi[a] - ulo[a] <= span;
+        }
+        if (!kSets && !compact) return false;
         // candidates beyond R of every lane's particle are dropped at staging
         // (their weights are 0: the sums are unchanged)
-        const WarpBox box = warp_box(active, p.x, p.y, p.z, cull_radius(R, sp.cs));
+        const WarpBox box = warp_box(in_set, p.x, p.y, p.z, cull_radius(R, sp.cs));
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 uint32_t beg, end;
@@ -568,14 +591,27 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
                     uint32_t nbox;
                     const uint32_t cnt = stage_in_box(sorted, base, end, box, sq, lane, nbox);
                     __syncwarp();
-                    for (uint32_t k = 0; k < cnt; ++k) add(sq[k]);
-                    since += nbox;
-                    if (since >= 32) fold();
+                    if (!kSets || in_set) {
+                        for (uint32_t k = 0; k < cnt; ++k) add(sq[k]);
+                        since += nbox;
+                        if (since >= 32) fold();
+                    }
                     __syncwarp();
                 }
             }
-    } else {
-        if (!active) return;
+        return true;
+    };
+    uint32_t left = __ballot_sync(0xffffffffu, active);
+    if (kSets) {
+        for (int sets = 0; left != 0u && span >= 0 && sets < kMaxSets; ++sets) {
+            const uint32_t set = window_mates(left, w, span, lane);
+            left &= ~set;
+            walk((set >> lane) & 1u);
+        }
+    } else if (walk(active)) {
+        left = 0u;
+    }
+    if ((left >> lane) & 1u) {
         for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
             for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
                 uint32_t beg, end;
@@ -602,6 +638,239 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
                               __fadd_rn(__fmul_rn(one_minus_lambda, p.y), __fmul_rn(lambda, ay)),
                               __fadd_rn(__fmul_rn(one_minus_lambda, p.z), __fmul_rn(lambda, az)),
                               __fdiv_rn(mass, p.w));
+}
+
+//
+// Four lanes per particle; a block of four warps takes 32 consecutive sorted
+// particles, a warp eight of them.  The sums must run in candidate order, but
+// the weights need not: the candidates that reach the warp's box are staged,
+// the four lanes of a particle compute the weights of every fourth group of
+// four of them, and then each lane adds one component of the sums (the
+// weight, x, y or z) over all of them in order.
+constexpr int kQuadThreads = 128;
+constexpr uint32_t kQuadCap = 96;               // staged candidates of a warp (multiple of 4)
+constexpr uint32_t kQuadRow = kQuadCap + 4;   // row pitch in words: rows 4 banks apart
+constexpr uint32_t kQuadGroups = 8;             // chunk sums in flight
+
+struct QuadSlice {
+    float q[4][kQuadRow];  // 1, x, y, z of the staged candidates
+    float w[8][kQuadRow];  // per particle: their weights (0 at and beyond R)
+    uint32_t gend[kQuadGroups];  // ends of the closed chunk sums
+};
+
+template <bool kFast>
+__global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* __restrict__ sorted, uint32_t n,
+                                                     const uint2* __restrict__ ranges, Grid sp, float R,
+                                                     float R_rcp, float R_lt2, float tiny, int max_span,
+                                                     float one_minus_lambda, float lambda, float mass, float4* __restrict__ mean,
+                                                     float4* __restrict__ mean32, float4* __restrict__ smoothed)
+{
+    __shared__ __align__(16) QuadSlice slices[kQuadThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    QuadSlice& S = slices[warp];
+    const uint32_t first = blockIdx.x * 32u;
+    if (first + 8u * warp >= n) return;
+    // the block's 32 particles, one per lane: their windows and box decide the
+    // walk and the chunk sums (the same for the four warps)
+    const bool there = first + lane < n;
+    const float4 pl = there ? sorted[first + lane] : make_float4(0.f, 0.f, 0.f, 1.f);
+    // cells beyond R on some axis only hold zero-weight particles, whose +0
+    // terms leave the exact sums unchanged: skip them
+    const Window wl = narrow(window(cell1(pl.x, sp.min[0], sp.cs), cell1(pl.y, sp.min[1], sp.cs),
+                                    cell1(pl.z, sp.min[2], sp.cs), 2, sp),
+                             pl.x, pl.y, pl.z, cull_radius(R, sp.cs), sp);
+    // this lane's particle and component
+    const int src = 8 * warp + (lane >> 2), comp = lane & 3, part = lane >> 2;
+    const uint32_t t = first + src;
+    const bool active = t < n;
+    float4 p;
+    p.x = __shfl_sync(0xffffffffu, pl.x, src);
+    p.y = __shfl_sync(0xffffffffu, pl.y, src);
+    p.z = __shfl_sync(0xffffffffu, pl.z, src);
+    p.w = __shfl_sync(0xffffffffu, pl.w, src);
+    const float pc = comp == 0 ? 0.f : comp == 1 ? p.x : comp == 2 ? p.y : p.z;
+    // the reference's FP32 sum of this component, the chunk sum, its
+    // compensated total; component 0 sums the weights (q = 1, dx = -1)
+    float ref = 0.f, chunk = 0.f;
+    Kahan tot;
+    auto fold = [&]() {
+        tot.add(chunk);
+        chunk = 0.f;
+    };
+    auto weight = [&](float qx, float qy, float qz) {
+        const float d2 = dot3_rn(__fsub_rn(p.x, qx), __fsub_rn(p.y, qy), __fsub_rn(p.z, qz));
+        // d >= R: weight 0, and +0 terms leave the sums unchanged
+        const float s = dist_over<kFast>(d2, R, R_rcp, tiny);
+        return d2 < R_lt2 ? __fsub_rn(1.0f, __fmul_rn(__fmul_rn(s, s), s)) : 0.f;
+    };
+    auto sum = [&](float q, float wt) {
+        ref = __fadd_rn(ref, __fmul_rn(q, wt));
+        chunk = __fmaf_rn(-wt, __fsub_rn(pc, q), chunk);
+    };
+    // weights of the staged candidates [0, fill), then this component's sums over [s, e)
+    auto weights = [&](uint32_t fill, bool on) {
+        __syncwarp();
+        for (uint32_t k = 4u * comp; k < fill; k += 16u) {
+            const float4 X = *reinterpret_cast<const float4*>(&S.q[1][k]);
+            const float4 Y = *reinterpret_cast<const float4*>(&S.q[2][k]);
+            const float4 Z = *reinterpret_cast<const float4*>(&S.q[3][k]);
+            float4 W;
+            W.x = weight(X.x, Y.x, Z.x);
+            W.y = weight(X.y, Y.y, Z.y);
+            W.z = weight(X.z, Y.z, Z.z);
+            W.w = weight(X.w, Y.w, Z.w);
+            *reinterpret_cast<float4*>(&S.w[part][k]) = on ? W : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        __syncwarp();
+    };
+    auto sums = [&](uint32_t s, uint32_t e) {
+        for (uint32_t k = s; k < e; k += 4) {
+            const float4 Q = *reinterpret_cast<const float4*>(&S.q[comp][k]);
+            const float4 W = *reinterpret_cast<const float4*>(&S.w[part][k]);
+            sum(Q.x, W.x);
+            sum(Q.y, W.y);
+            sum(Q.z, W.z);
+            sum(Q.w, W.w);
+        }
+    };
+    auto row_range = [&](int x0, int x1, int yy, int zz, uint32_t& beg, uint32_t& end) {
+        const uint32_t c0 = lin3(x0, yy, zz, sp);
+        beg = kEmpty;
+        end = 0;
+        for (int xx = 0; xx <= x1 - x0; ++xx) {
+            const uint2 r = __ldg(&ranges[c0 + xx]);
+            if (r.x != kEmpty) {
+                beg = min(beg, r.x);
+                end = max(end, r.y);
+            }
+        }
+    };
+    // Particles whose windows span few cells per axis walk their union
+    // together (window_mates), as in k_smooth; the sets are the block's.
+    for (uint32_t k = lane; k < kQuadRow; k += 32) S.q[0][k] = 1.0f;
+    const float r = cull_radius(R, sp.cs);
+    uint32_t left = __ballot_sync(0xffffffffu, there);
+    uint32_t since = 0;  // candidates taken since the chunk sums last joined the totals
+    for (int sets = 0; left != 0u && max_span >= 0 && sets < kMaxSets; ++sets) {
+        const uint32_t set = window_mates(left, wl, max_span, lane);
+        left &= ~set;
+        if (((set >> (8 * warp)) & 0xffu) == 0u) continue;  // none of this warp's particles
+        const bool in_set = (set >> lane) & 1u;
+        const bool mine_in = (set >> src) & 1u;
+        int ulo[3], uhi[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            ulo[a] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)wl.lo[a] : 0x7fffffffu);
+            uhi[a] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(wl.hi[a] + 1) : 0u) - 1;
+        }
+        // candidates beyond R of every particle of the warp are dropped at
+        // staging; the chunk sums join the totals once at least 32 candidates
+        // of the set's box have passed since the last time
+        const WarpBox box = warp_box(in_set, pl.x, pl.y, pl.z, r);
+        const WarpBox mine = warp_box(mine_in, p.x, p.y, p.z, r);
+        uint32_t fill = 0, ngr = 0;
+        since = 0;
+        // pads the staged candidates to a multiple of 4 with ones of weight 0
+        auto pad = [&]() {
+            const uint32_t m = (0u - fill) & 3u;
+            if ((uint32_t)lane < m) S.q[1][fill + lane] = S.q[2][fill + lane] = S.q[3][fill + lane] = 1.0e18f;
+            fill += m;
+        };
+        auto flush = [&]() {
+            pad();
+            weights(fill, mine_in);
+            uint32_t s = 0;
+            for (uint32_t g = 0; g < ngr; ++g) {
+                const uint32_t e = S.gend[g];
+                sums(s, e);
+                fold();
+                s = e;
+            }
+            sums(s, fill);
+            fill = ngr = 0;
+            __syncwarp();
+        };
+        for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
+            for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
+                uint32_t beg, end;
+                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                float4 next = beg + lane < end ? __ldg(&sorted[beg + lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
+                for (uint32_t base = beg; base < end; base += 32) {
+                    const float4 q = next;
+                    if (base + 32 + lane < end) next = __ldg(&sorted[base + 32 + lane]);
+                    const bool in = base + lane < end && box.holds(q);
+                    const uint32_t nbox = __popc(__ballot_sync(0xffffffffu, in));
+                    if (nbox == 0u) continue;
+                    const bool keep = in && mine.reaches(q);
+                    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        const uint32_t k = fill + __popc(m & ((1u << lane) - 1u));
+                        S.q[1][k] = q.x;
+                        S.q[2][k] = q.y;
+                        S.q[3][k] = q.z;
+                    }
+                    fill += __popc(m);
+                    since += nbox;
+                    if (since >= 32) {
+                        since = 0;
+                        pad();
+                        if (lane == 0) S.gend[ngr] = fill;
+                        ++ngr;
+                    }
+                    if (fill + 35u > kQuadCap || ngr == kQuadGroups) flush();
+                }
+            }
+        flush();
+    }
+    if (left != 0u) {
+        // each particle walks its own window, 32 candidates at a time
+        Window w;
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            w.lo[a] = __shfl_sync(0xffffffffu, wl.lo[a], src);
+            w.hi[a] = __shfl_sync(0xffffffffu, wl.hi[a], src);
+        }
+        since = 0;
+        if ((left >> src) & 1u)
+            for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
+                for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
+                    uint32_t beg, end;
+                    row_range(w.lo[0], w.hi[0], yy, zz, beg, end);
+                    const uint32_t quad = 0xfu << (lane & 28);
+                    for (uint32_t base = beg; base < end; base += 32) {
+                        const uint32_t lim = min(end, base + 32u);
+                        for (uint32_t i = base + comp; i < lim; i += 4) {
+                            const float4 q = __ldg(&sorted[i]);
+                            S.w[part][i - base] = weight(q.x, q.y, q.z);
+                        }
+                        __syncwarp(quad);
+                        for (uint32_t i = base; i < lim; ++i) {
+                            const float wt = S.w[part][i - base];
+                            if (wt != 0.f)
+                                sum(comp == 0 ? 1.0f : __ldg(reinterpret_cast<const float*>(sorted + i) + comp - 1), wt);
+                        }
+                        __syncwarp(quad);
+                        since += lim - base;
+                        if (since >= 32) {
+                            fold();
+                            since = 0;
+                        }
+                    }
+                }
+        __syncwarp();
+    }
+    fold();
+    const int lead = lane & 28;  // component 0 holds the weight sums (>= 1: the particle itself has weight 1)
+    const float ws = __shfl_sync(0xffffffffu, ref, lead);
+    const float val = tot.s - tot.c;
+    const float W = __shfl_sync(0xffffffffu, val, lead);
+    if (!active) return;
+    const uint32_t o = 4u * t + ((comp + 3) & 3);  // x, y, z, weight sum (mean.w: the adjoint divides by it)
+    reinterpret_cast<float*>(mean32)[o] = comp == 0 ? ws : __fdiv_rn(ref, ws);
+    const float ax = pc + val / W;
+    reinterpret_cast<float*>(mean)[o] = comp == 0 ? W : ax;
+    reinterpret_cast<float*>(smoothed)[o] =
+        comp == 0 ? __fdiv_rn(mass, p.w) : __fadd_rn(__fmul_rn(one_minus_lambda, pc), __fmul_rn(lambda, ax));
 }
 
 // calculationOfTransformMatricesForParticles (cu:689-827) for every
@@ -1288,12 +1557,30 @@ void launch_smooth(const KernelCtx& c, const float4* sorted, uint32_t n, const u
     if (!n) return;
     // (1.0 - lambda) is evaluated in double and rounded (cu:656)
     const float oml = (float)(1.0 - (double)lambda);
-    // warps may walk the union of their windows when the cull radius stays
-    // below two cells (see k_smooth)
-    const int coop_ok = (R * 1.0001f + 1e-4f * sp.cs) < 2.0f * sp.cs * 0.9999f ? 1 : 0;
-    const auto kernel = fast_radius(R) ? k_smooth<true> : k_smooth<false>;
-    kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R, sqrt_threshold(R, false),
-                                                         tiny_d2(R), coop_ok, oml, lambda, mass, mean, mean32, smoothed);
+    // lanes may walk the union of their windows when the cull radius stays
+    // below two cells (see k_smooth); it spans up to one cell more per axis than
+    // the windows of particles of one cell
+    const bool coop_ok = (R * 1.0001f + 1e-4f * sp.cs) < 2.0f * sp.cs * 0.9999f;
+    const int max_span = coop_ok ? 2 * (int)std::ceil(std::max(1.0f, R * 1.0001f / sp.cs)) + 1 : -1;
+    // Four lanes per particle while one would leave the SMs with two or three
+    // warps per scheduler; more lanes cost more instructions per particle once
+    // the GPU is full.  Measured, one lane / four (ms): R = 0.8 cells: 20k
+    // particles 0.19 / 0.07, 32k 0.12 / 0.09, 64k 0.11-0.23 / 0.14-0.18, 120k
+    // 0.28 / 0.31; R = 1.54 cells: 20k 0.62 / 0.25, 40k 0.80 / 0.46, 100k 0.87 /
+    // 1.03.
+    const bool wide = max_span > 3, fast = fast_radius(R);
+    if (n < (wide ? 81920u : 49152u)) {
+        const auto kernel = fast ? k_smooth_quads<true> : k_smooth_quads<false>;
+        kernel<<<blocks_for(n, 32), kQuadThreads, 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R,
+                                                                sqrt_threshold(R, false), tiny_d2(R), max_span, oml,
+                                                                lambda, mass, mean, mean32, smoothed);
+    } else {
+        const auto kernel = wide ? (fast ? k_smooth<true, true> : k_smooth<false, true>)
+                                 : (fast ? k_smooth<true, false> : k_smooth<false, false>);
+        kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R,
+                                                             sqrt_threshold(R, false), tiny_d2(R), max_span, oml, lambda,
+                                                             mass, mean, mean32, smoothed);
+    }
     ++g_launches;
 }
 

@@ -1,0 +1,59 @@
+"""The neighbour walks of the anisotropic path, against the oracles, where
+their choices change: a warp's lanes in one set of windows, in several (rows of
+cells that end inside the warp) and scattered over the grid; neighbour radii
+below and above a cell; the sizes on both sides of the lines between the kernels
+(four lanes per particle or one); the smallest frames.  The bars are those of
+the parity tests (FP32 means and counts exact, G and the field against FP64)."""
+import numpy as np
+import pytest
+
+from tests.test_gpu_parity import _run
+
+pytestmark = pytest.mark.gpu
+
+# neighbour radius / cell: 0.8 (the benchmark's), 1.54 (the defaults'), 0.38 and 1.05 (multiples of h that
+# the library and the oracle round alike)
+SETTINGS = {
+    "fine": dict(smoothing_lambda=0.9, aniso_radius_over_h=1.0, cell_size_scale=1.25, grid_ratio=4, iso=0.0),
+    "default": {},
+    "short": dict(smoothing_lambda=0.9, aniso_radius_over_h=0.5, cell_size_scale=1.3, grid_ratio=3),
+    "over": dict(smoothing_lambda=0.5, aniso_radius_over_h=1.365, cell_size_scale=1.3, grid_ratio=3),
+}
+
+
+def _frame(n, h, spread, seed):
+    """n particles uniform in a box of the given fraction of the unit cube."""
+    from fluidsurfacereconstructiongpu_gb300 import synthetic
+    rng = np.random.default_rng(seed)
+    pos = (0.5 + spread * (rng.random((n, 3)) - 0.5)).astype(np.float32)
+    return synthetic.ParticleFrame(bbox_min=np.zeros(3, np.float32), bbox_max=np.ones(3, np.float32), h=h,
+                                   particle_radius=h / 4, mass=1000.0 * (h / 4) ** 3, pos=pos,
+                                   density=np.full(n, 1000.0, np.float32))
+
+
+@pytest.mark.parametrize("settings", sorted(SETTINGS))
+@pytest.mark.parametrize("n", [1, 7, 33, 1000])
+def test_few_particles(n, settings):
+    _run("yu13", _frame(n, 0.08, 0.3, n), **SETTINGS[settings])
+
+
+@pytest.mark.parametrize("settings", ["fine", "default", "over"])
+def test_scattered_particles(settings):
+    """About one particle to two cells: every lane a window of its own."""
+    _run("yu13", _frame(3000, 0.05, 0.95, 5), **SETTINGS[settings])
+
+
+@pytest.mark.parametrize("settings", ["fine", "default", "over"])
+def test_rows_of_few_cells(settings):
+    """A slab two cells wide: most warps run over the ends of several rows."""
+    fr = _frame(4000, 0.04, 0.9, 6)
+    fr.pos[:, 0] = 0.5 + (fr.pos[:, 0] - 0.5) * 0.1
+    _run("yu13", fr, **SETTINGS[settings])
+
+
+@pytest.mark.parametrize("n_side,settings", [(36, "fine"), (37, "fine"), (43, "default"), (44, "default")])
+def test_both_sides_of_the_lanes_per_particle_rule(n_side, settings):
+    """46,656 / 50,653 and 79,507 / 85,184 particles."""
+    from fluidsurfacereconstructiongpu_gb300 import synthetic
+    fr = synthetic.lattice_cube(n_side, 0.008, seed=n_side, jitter_frac=0.3, origin=(0.2, 0.2, 0.2))
+    _run("yu13", fr, **SETTINGS[settings])

@@ -445,6 +445,8 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
 // number inside the grown box itself, which the callers count towards their
 // chunk sums exactly as before the reach test was added, so that the sums
 // join their totals at the same points.
+// kIndexed: with their sorted index in w.
+template <bool kIndexed = false>
 __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src, uint32_t base, uint32_t end,
                                                  const WarpBox& box, float4* sq, int lane, uint32_t& nbox)
 {
@@ -454,6 +456,7 @@ __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src,
         q = __ldg(&src[base + lane]);
         in = box.holds(q);
         keep = in && box.reaches(q);
+        if (kIndexed) q.w = __uint_as_float(base + lane);
     }
     nbox = __popc(__ballot_sync(0xffffffffu, in));
     const uint32_t m = __ballot_sync(0xffffffffu, keep);
@@ -888,14 +891,19 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
 // walk and the lanes' sums and counts are joined at the end (the covariance
 // sums may be taken in any order, the count is an integer).  P = 4 for
 // small frames, whose particles alone are too few warps to fill the GPU; P
-// = 1 otherwise (four lanes measured slower once the GPU is full).
+// = 1 otherwise (four lanes measured slower once the GPU is full).  P = 16
+// for the smallest frames with wide windows (kSets: thousands of candidates
+// per particle; measured with P = 4 / 16 at R = 1.54 cells: 5k particles 0.21 /
+// 0.12 ms, 10k 0.29 / 0.21, 20k 0.42 / 0.38, 40k 0.56 / 0.76).  kSets itself, P =
+// 4: 40k particles 1.07 -> 0.56 ms, 200k 4.3 -> 2.3 ms.
 constexpr int kCovThreads = 64;
 constexpr uint32_t kCovSplitBelow = 1u << 17;  // particles below which P = 4
+constexpr uint32_t kCovWideBelow = 12288;      // and P = 16 with kSets
 #ifndef FSR_COV_MIN_BLOCKS
 #define FSR_COV_MIN_BLOCKS 16
 #endif
 
-template <int P, bool kFast>
+template <int P, bool kFast, bool kSets>
 __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs a, Counters* ctr)
 {
     __shared__ float4 s_q[kCovThreads];  // 32 staged candidates per warp
@@ -968,44 +976,70 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
     // as in k_smooth.  Exact when the +-2 cell window never cuts a lane's
     // window narrowed about its mean (the mean lies within R of the particle:
     // launch_cov checks R + cull radius < 2 cells), so every candidate the
-    // union adds lies beyond R of that lane's mean.
-    int ulo[3], uhi[3];
-    bool compact = a.coop_ok != 0;
+    // union adds lies beyond R of that lane's mean.  kSets (that check fails,
+    // R near or above a cell): a lane takes only the staged candidates of its
+    // own window, whose cells of a row are one run of the sorted particles,
+    // and windows that lie apart are walked set by set.
+    auto walk = [&](bool in_set) {
+        int ulo[3], uhi[3];
+        bool compact = a.coop_ok != 0;
 #pragma unroll
-    for (int ax = 0; ax < 3; ++ax) {
-        ulo[ax] = (int)__reduce_min_sync(0xffffffffu, act ? (unsigned)w.lo[ax] : 0x7fffffffu);
-        uhi[ax] = (int)__reduce_max_sync(0xffffffffu, act ? (unsigned)(w.hi[ax] + 1) : 0u) - 1;
-        compact = compact && uhi[ax] - ulo[ax] <= 3;
-    }
-    if (compact) {
+        for (int ax = 0; ax < 3; ++ax) {
+            ulo[ax] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)w.lo[ax] : 0x7fffffffu);
+            uhi[ax] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(w.hi[ax] + 1) : 0u) - 1;
+            compact = compact && uhi[ax] - ulo[ax] <= 3;
+        }
+        if (!kSets && !compact) return false;
         // candidates beyond R of every lane's mean are dropped at staging
-        const WarpBox box = warp_box(act, m.x, m.y, m.z, cr);
+        const WarpBox box = warp_box(in_set, m.x, m.y, m.z, cr);
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
-                uint32_t beg, end;
+                uint32_t beg, end, own = 0, len = 0;
                 row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                if (kSets && in_set && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
+                    row_range(w.lo[0], w.hi[0], yy, zz, own, len);
+                    len = len > own ? len - own : 0u;
+                }
+                auto mine = [&](const float4& q) { return !kSets || __float_as_uint(q.w) - own < len; };
                 for (uint32_t base = beg; base < end; base += 32) {
                     uint32_t nbox;
-                    const uint32_t cnt = stage_in_box(a.sorted, base, end, box, sq, lane, nbox);
+                    const uint32_t cnt = stage_in_box<kSets>(a.sorted, base, end, box, sq, lane, nbox);
                     __syncwarp();
-                    if (act) {
+                    if (in_set) {
                         uint32_t k = sub;
                         for (; k + 3 * P < cnt; k += 4 * P) {
                             const float4 q0 = sq[k], q1 = sq[k + P], q2 = sq[k + 2 * P], q3 = sq[k + 3 * P];
-                            const bool n0 = near(q0), n1 = near(q1), n2 = near(q2), n3 = near(q3);
+                            const bool n0 = near(q0) && mine(q0), n1 = near(q1) && mine(q1);
+                            const bool n2 = near(q2) && mine(q2), n3 = near(q3) && mine(q3);
                             if (n0) take(q0);
                             if (n1) take(q1);
                             if (n2) take(q2);
                             if (n3) take(q3);
                         }
-                        for (; k < cnt; k += P) take(sq[k]);
-                        since += nbox / P;
+                        for (; k < cnt; k += P) {
+                            const float4 q = sq[k];
+                            if (mine(q)) take(q);
+                        }
+                        since += kSets ? (nbox + P - 1) / P : nbox / P;
                         if (since >= 32) fold();
                     }
                     __syncwarp();
                 }
             }
-    } else if (act && P > 1) {
+        return true;
+    };
+    uint32_t left = __ballot_sync(0xffffffffu, act);
+    if (kSets) {
+        for (int sets = 0; left != 0u && sets < kMaxSets; ++sets) {
+            const uint32_t set = window_mates(left, w, 5, lane);
+            left &= ~set;
+            walk((set >> lane) & 1u);
+        }
+    } else if (walk(act)) {
+        left = 0u;
+    }
+    const bool alone = (left >> lane) & 1u;
+    if (alone && P > 1) {
         for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
             for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
                 uint32_t beg, end;
@@ -1016,7 +1050,7 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
                     if (++since >= 32) fold();
                 }
             }
-    } else if (act) {
+    } else if (alone) {
         for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
             for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
                 uint32_t beg, end;
@@ -1594,12 +1628,18 @@ void launch_cov(const KernelCtx& c, const CovArgs& a0, Counters* ctr)
     a.coop_ok = (a.R + a.R * 1.0001f + 1e-4f * a.sp.cs) < 2.0f * a.sp.cs * 0.9999f ? 1 : 0;
     a.tiny = tiny_d2(a.R);
     const bool fast = fast_radius(a.R);
-    if (a.n < kCovSplitBelow) {
-        const auto kernel = fast ? k_cov<4, true> : k_cov<4, false>;
-        kernel<<<blocks_for((uint64_t)a.n * 4, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+    const bool sets = a.coop_ok == 0;
+    auto launch = [&](auto kernel, uint32_t lanes) {
+        kernel<<<blocks_for((uint64_t)a.n * lanes, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+    };
+    if (sets && a.n < kCovWideBelow) {
+        launch(fast ? k_cov<16, true, true> : k_cov<16, false, true>, 16);
+    } else if (a.n < kCovSplitBelow) {
+        if (sets) launch(fast ? k_cov<4, true, true> : k_cov<4, false, true>, 4);
+        else launch(fast ? k_cov<4, true, false> : k_cov<4, false, false>, 4);
     } else {
-        const auto kernel = fast ? k_cov<1, true> : k_cov<1, false>;
-        kernel<<<blocks_for(a.n, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+        if (sets) launch(fast ? k_cov<1, true, true> : k_cov<1, false, true>, 1);
+        else launch(fast ? k_cov<1, true, false> : k_cov<1, false, false>, 1);
     }
     ++g_launches;
 }

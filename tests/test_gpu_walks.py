@@ -51,9 +51,10 @@ def test_rows_of_few_cells(settings):
     _run("yu13", fr, **SETTINGS[settings])
 
 
-@pytest.mark.parametrize("n_side,settings", [(36, "fine"), (37, "fine"), (43, "default"), (44, "default")])
+@pytest.mark.parametrize("n_side,settings", [(36, "fine"), (37, "fine"), (43, "default"), (44, "default"),
+                                             (23, "default"), (24, "default"), (50, "over"), (51, "over")])
 def test_both_sides_of_the_lanes_per_particle_rule(n_side, settings):
-    """46,656 / 50,653 and 79,507 / 85,184 particles."""
+    """46,656 / 50,653, 79,507 / 85,184, 12,167 / 13,824 and 125,000 / 132,651 particles."""
     from fluidsurfacereconstructiongpu_gb300 import synthetic
     fr = synthetic.lattice_cube(n_side, 0.008, seed=n_side, jitter_frac=0.3, origin=(0.2, 0.2, 0.2))
     _run("yu13", fr, **SETTINGS[settings])

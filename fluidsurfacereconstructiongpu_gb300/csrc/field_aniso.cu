@@ -59,7 +59,7 @@ struct CandTables {
 };
 
 // Group g (a key of the (res + 1)^3 window-centre grid): its cell and its
-// vertex index box [x0, x1) x [y0, y1) x [z0, z1).
+// vertex index box [x0, x1) x [y0, y1) x [z0, z1).  Every lane of the warp calls it.
 __device__ __forceinline__ bool group_box(uint32_t g, const Grid& sp, const Grid& sc, uint32_t ratio, int c[3],
                                           int lo[3], int hi[3])
 {
@@ -67,12 +67,18 @@ __device__ __forceinline__ bool group_box(uint32_t g, const Grid& sp, const Grid
     c[0] = (int)(g % kx);
     c[1] = (int)((g / kx) % ky);
     c[2] = (int)(g / (kx * ky));
-    lo[0] = first_vertex<0>(c[0], sc, sp, ratio);
-    hi[0] = first_vertex<0>(c[0] + 1, sc, sp, ratio);
-    lo[1] = first_vertex<1>(c[1], sc, sp, ratio);
-    hi[1] = first_vertex<1>(c[1] + 1, sc, sp, ratio);
-    lo[2] = first_vertex<2>(c[2], sc, sp, ratio);
-    hi[2] = first_vertex<2>(c[2] + 1, sc, sp, ratio);
+    // the six ends, one per lane (lane 2 a: lo of axis a, 2 a + 1: hi)
+    const int lane = threadIdx.x & 31, axis = min(lane >> 1, 2);
+    const int ca = (axis == 0 ? c[0] : axis == 1 ? c[1] : c[2]) + (lane & 1);
+    const int nres = (int)(axis == 0 ? sc.res[0] : axis == 1 ? sc.res[1] : sc.res[2]);
+    const float vmin = axis == 0 ? sc.min[0] : axis == 1 ? sc.min[1] : sc.min[2];
+    const float cmin = axis == 0 ? sp.min[0] : axis == 1 ? sp.min[1] : sp.min[2];
+    const int end = first_vertex(ca, ratio, nres, vmin, sc.cs, cmin, sp.cs);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        lo[a] = __shfl_sync(0xffffffffu, end, 2 * a);
+        hi[a] = __shfl_sync(0xffffffffu, end, 2 * a + 1);
+    }
     return hi[0] > lo[0] && hi[1] > lo[1] && hi[2] > lo[2];
 }
 
@@ -422,56 +428,101 @@ __device__ __forceinline__ float4 vert_pos(uint32_t loc, const int lo[3], const 
 // candidates reaching it; a counting sort by brick, the order within a brick
 // is that of the atomics, which changes no result since a vertex's sum does
 // not depend on its tile and culling only skips exact zeros), and the box of
-// each 32-vertex tile.  hist: kPassVerts words of scratch.
-__device__ __forceinline__ void pass_layout(const uint32_t* vloc, const int lo[3], const Grid& sc, uint16_t* order,
-                                            uint32_t* hist, float4* box, uint32_t nv, float inv, int lane, float4& pl,
-                                            float4& ph)
+// each 32-vertex tile.  Boxes are formed from the vertices' indices by warp
+// reductions (positions do not decrease with the index); frames of many small
+// groups spent a fifth of their field time on the float boxes this replaces.
+// hist: kPassVerts words of scratch.
+struct IndexBox {
+    uint32_t lo[3], hi[3];
+    __device__ __forceinline__ void clear()
+    {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = 1023u;
+            hi[a] = 0u;
+        }
+    }
+    __device__ __forceinline__ void add(uint32_t loc)
+    {
+        const uint32_t i[3] = {loc & 1023u, (loc >> 10) & 1023u, loc >> 20};
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = min(lo[a], i[a]);
+            hi[a] = max(hi[a], i[a]);
+        }
+    }
+    // the box of all lanes' boxes
+    __device__ __forceinline__ void join()
+    {
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            lo[a] = __reduce_min_sync(0xffffffffu, lo[a]);
+            hi[a] = __reduce_max_sync(0xffffffffu, hi[a]);
+        }
+    }
+    __device__ __forceinline__ float4 low(const int o[3], const Grid& sc) const
+    {
+        return make_float4(vpos1(o[0] + (int)lo[0], sc.min[0], sc.cs), vpos1(o[1] + (int)lo[1], sc.min[1], sc.cs),
+                           vpos1(o[2] + (int)lo[2], sc.min[2], sc.cs), 0.f);
+    }
+    __device__ __forceinline__ float4 high(const int o[3], const Grid& sc) const
+    {
+        return make_float4(vpos1(o[0] + (int)hi[0], sc.min[0], sc.cs), vpos1(o[1] + (int)hi[1], sc.min[1], sc.cs),
+                           vpos1(o[2] + (int)hi[2], sc.min[2], sc.cs), 0.f);
+    }
+};
+
+// kInPlace: vloc and vrank are reordered (order is not used); else order[v] is
+// the place of the v-th vertex.
+template <bool kInPlace>
+__device__ __forceinline__ void pass_layout(uint32_t* vloc, uint32_t* vrank, const int lo[3], const Grid& sc,
+                                            uint16_t* order, uint32_t* hist, float4* box, uint32_t nv, int lane,
+                                            float4& pl, float4& ph)
 {
     const uint32_t ntiles = (nv + 31) / 32;
-    pl = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f);
-    ph = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.f);
-    for (uint32_t q = lane; q < nv; q += 32) {
-        const float4 v = vert_pos(vloc[q], lo, sc);
-        pl.x = fminf(pl.x, v.x); pl.y = fminf(pl.y, v.y); pl.z = fminf(pl.z, v.z);
-        ph.x = fmaxf(ph.x, v.x); ph.y = fmaxf(ph.y, v.y); ph.z = fmaxf(ph.z, v.z);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        pl.x = fminf(pl.x, __shfl_xor_sync(0xffffffffu, pl.x, o));
-        pl.y = fminf(pl.y, __shfl_xor_sync(0xffffffffu, pl.y, o));
-        pl.z = fminf(pl.z, __shfl_xor_sync(0xffffffffu, pl.z, o));
-        ph.x = fmaxf(ph.x, __shfl_xor_sync(0xffffffffu, ph.x, o));
-        ph.y = fmaxf(ph.y, __shfl_xor_sync(0xffffffffu, ph.y, o));
-        ph.z = fmaxf(ph.z, __shfl_xor_sync(0xffffffffu, ph.z, o));
-    }
-    const int gx = (__float2int_rn((ph.x - pl.x) * inv) >> 2) + 1;
-    const int gy = (__float2int_rn((ph.y - pl.y) * inv) >> 2) + 1;
-    const int gz = (__float2int_rn((ph.z - pl.z) * inv) >> 1) + 1;
-    const int nbins = gx * gy * gz;
-    if (nbins <= kPassVerts) {
-        for (int b = lane; b < nbins; b += 32) hist[b] = 0u;
+    IndexBox pass;
+    pass.clear();
+    for (uint32_t q = lane; q < nv; q += 32) pass.add(vloc[q]);
+    pass.join();
+    pl = pass.low(lo, sc);
+    ph = pass.high(lo, sc);
+    if (ntiles == 1u) {  // one tile: any order, the pass's box
+        if (!kInPlace && (uint32_t)lane < nv) order[lane] = (uint16_t)lane;
+        if (lane == 0) {
+            box[0] = pl;
+            box[1] = ph;
+        }
         __syncwarp();
-        int key[kPassVerts / 32];
-        uint32_t slot[kPassVerts / 32];
+        return;
+    }
+    const uint32_t gx = ((pass.hi[0] - pass.lo[0]) >> 2) + 1u;
+    const uint32_t gy = ((pass.hi[1] - pass.lo[1]) >> 2) + 1u;
+    const uint32_t gz = ((pass.hi[2] - pass.lo[2]) >> 1) + 1u;
+    const uint32_t nbins = gx * gy * gz;
+    if (nbins <= (uint32_t)kPassVerts) {
+        for (uint32_t b = lane; b < nbins; b += 32) hist[b] = 0u;
+        __syncwarp();
+        uint32_t at[kPassVerts / 32];  // brick | place in it << 16
+        uint32_t loc[kPassVerts / 32], rank[kPassVerts / 32];
 #pragma unroll
         for (int k = 0; k < kPassVerts / 32; ++k) {
             const uint32_t q = lane + 32 * k;
-            key[k] = 0;
-            slot[k] = 0;
+            at[k] = 0;
             if (q < nv) {
-                const float4 v = vert_pos(vloc[q], lo, sc);
-                const int ix = __float2int_rn((v.x - pl.x) * inv) >> 2;
-                const int iy = __float2int_rn((v.y - pl.y) * inv) >> 2;
-                const int iz = __float2int_rn((v.z - pl.z) * inv) >> 1;
-                key[k] = min(ix, gx - 1) + gx * (min(iy, gy - 1) + gy * min(iz, gz - 1));
-                slot[k] = atomicAdd(hist + key[k], 1u);
+                const uint32_t l = vloc[q];
+                loc[k] = l;
+                if (kInPlace) rank[k] = vrank[q];
+                const uint32_t ix = ((l & 1023u) - pass.lo[0]) >> 2, iy = (((l >> 10) & 1023u) - pass.lo[1]) >> 2;
+                const uint32_t iz = ((l >> 20) - pass.lo[2]) >> 1;
+                const uint32_t key = ix + gx * (iy + gy * iz);
+                at[k] = key | (atomicAdd(hist + key, 1u) << 16);
             }
         }
         __syncwarp();
         // exclusive scan of the bins, lane by lane in blocks of nbins / 32
-        const int per = (nbins + 31) / 32;
+        const uint32_t per = (nbins + 31u) / 32u, b0 = lane * per, b1 = min(nbins, b0 + per);
         uint32_t tot = 0;
-        for (int b = lane * per; b < min(nbins, lane * per + per); ++b) tot += hist[b];
+        for (uint32_t b = b0; b < b1; ++b) tot += hist[b];
         uint32_t x = tot;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -479,8 +530,7 @@ __device__ __forceinline__ void pass_layout(const uint32_t* vloc, const int lo[3
             if (lane >= o) x += y;
         }
         uint32_t run = x - tot;
-        __syncwarp();
-        for (int b = lane * per; b < min(nbins, lane * per + per); ++b) {
+        for (uint32_t b = b0; b < b1; ++b) {
             const uint32_t hcount = hist[b];
             hist[b] = run;
             run += hcount;
@@ -489,21 +539,29 @@ __device__ __forceinline__ void pass_layout(const uint32_t* vloc, const int lo[3
 #pragma unroll
         for (int k = 0; k < kPassVerts / 32; ++k) {
             const uint32_t q = lane + 32 * k;
-            if (q < nv) order[hist[key[k]] + slot[k]] = (uint16_t)q;
+            if (q < nv) {
+                const uint32_t to = hist[at[k] & 0xffffu] + (at[k] >> 16);
+                if (kInPlace) {
+                    vloc[to] = loc[k];
+                    vrank[to] = rank[k];
+                } else {
+                    order[to] = (uint16_t)q;
+                }
+            }
         }
-    } else {
+    } else if (!kInPlace) {
         for (uint32_t q = lane; q < nv; q += 32) order[q] = (uint16_t)q;
     }
     __syncwarp();
-    if ((uint32_t)lane < ntiles) {
-        float4 tl = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f), th = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.f);
-        for (uint32_t q = 32 * lane; q < min(nv, 32 * lane + 32); ++q) {
-            const float4 v = vert_pos(vloc[order[q]], lo, sc);
-            tl.x = fminf(tl.x, v.x); tl.y = fminf(tl.y, v.y); tl.z = fminf(tl.z, v.z);
-            th.x = fmaxf(th.x, v.x); th.y = fmaxf(th.y, v.y); th.z = fmaxf(th.z, v.z);
-        }
-        box[2 * lane] = tl;
-        box[2 * lane + 1] = th;
+#pragma unroll 1
+    for (uint32_t t = 0; t < ntiles; ++t) {
+        IndexBox tile;
+        tile.clear();
+        const uint32_t q = 32u * t + (uint32_t)lane;
+        if (q < nv) tile.add(vloc[kInPlace ? q : (uint32_t)order[q]]);
+        tile.join();
+        if (lane == 0) box[2 * t] = tile.low(lo, sc);
+        if (lane == 1) box[2 * t + 1] = tile.high(lo, sc);
     }
     __syncwarp();
 }
@@ -705,8 +763,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
             const uint32_t ntiles = (nv + 31) / 32;
             // the pass's box, brick order and tile boxes
             float4 pl, ph;
-            pass_layout(w.vloc, lo, a.sc, w.order, reinterpret_cast<uint32_t*>(&w.psum[0][0]), w.box, nv,
-                        1.0f / a.sc.cs, lane, pl, ph);  // psum is zeroed below
+            pass_layout<false>(w.vloc, w.vrank, lo, a.sc, w.order, reinterpret_cast<uint32_t*>(&w.psum[0][0]), w.box, nv, lane, pl, ph);  // psum is zeroed below
             // two sums per vertex: the involved particles' terms, then the
             // non-involved particles' (the unscaled kernel: about 1e-7 each,
             // thousands of them) and the rounding errors of the first sum,
@@ -715,7 +772,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
             // the sums live in the warp's shared slice, so that the tile loops
             // need not be unrolled (the kernel's code stays small enough for
             // the instruction cache)
-            for (int t = 0; t < kPassTiles; ++t) w.psum[t][lane] = w.usum[t][lane] = 0.f;
+            for (uint32_t t = 0; t < ntiles; ++t) w.psum[t][lane] = w.usum[t][lane] = 0.f;
             const uint32_t total_inv = w.total_inv;
             // involved candidates: staged with their G, culled per tile by
             // their support sphere, evaluated two at a time
@@ -867,18 +924,28 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
 // updateScalarFieldValueZB05 (cu:230-289) and updateScalarFieldValueTC01
 // (cu:178-227) grouped like the anisotropic field: a band vertex's
 // candidates are the particles of the +-1 cells around its cell, the same for
-// every vertex of the cell, so one warp streams them once per pass of up to
-// 256 vertices and, per brick tile, evaluates only those within h of the
-// tile's box.  Each vertex sums its terms in window order (cells z, y, x,
+// every vertex of the cell.  One warp streams them once per pass of up to 256
+// vertices, stages up to kIsoSeg of those within h of the pass's box and then
+// goes through the brick tiles: the ones within h of the tile are listed two to
+// a pair and every lane evaluates one pair per step.  (Issue-bound: 29.8 of 32
+// threads per instruction, 70 % of the issue slots.  Tiles inside the chunk of
+// 32 candidates, as before, cost each tile its vertices' positions and sums, a
+// list and a half-empty pair per chunk: 910 -> 637 M instructions and 1.07 ->
+// 0.81 ms on the 256k Akinci12 frame; 1.10 -> 0.85 ms on the 1M ZB05 frame.)  Each vertex sums its terms in window order (cells z, y, x,
 // particles in sorted order); candidates of the window cells the per-vertex
 // walk narrows away lie beyond h and add nothing.
+// Candidates staged at a time: with 120 six blocks fit an SM (64: 1.07 -> 0.88
+// ms instead of 0.81 on the 256k Akinci12 frame; 128, five blocks: 0.81, but
+// 0.88 instead of 0.85 on the 1M ZB05 frame, of small groups).
+constexpr uint32_t kIsoSeg = 120;
 struct IsoSlice {
-    float4 lst[32];                // one tile's candidates in lane order, two to a pair block (list_iso_pair)
-    uint32_t vloc[kPassVerts];     // the pass's band vertices: index in the group's box (vert_loc)
+    float4 lxy[kIsoSeg / 2];       // one tile's candidates in order, two to a pair: (x, x', y, y')
+    float2 lz[kIsoSeg / 2];        // and (z, z')
+    float cx[kIsoSeg], cy[kIsoSeg], cz[kIsoSeg];  // the staged candidates
+    uint32_t vloc[kPassVerts];     // the pass's band vertices in brick order: index in the group's box (vert_loc)
     uint32_t vrank[kPassVerts];    // and band rank
     float4 box[2 * kPassTiles];    // per tile: lo, hi
     float sum[4][kPassTiles][32];  // per vertex: weight sum, then (ZB05) sum w (x - v)
-    uint16_t order[kPassVerts];    // the pass's vertices in brick order
     uint32_t rb[9], rp[10];        // the window's rows: first particle, prefix of lengths
 };
 
@@ -890,21 +957,8 @@ __device__ __forceinline__ bool within(float4 q, float4 lo, float4 hi, float r2)
     return fmaf(gx, gx, fmaf(gy, gy, gz * gz)) < r2;
 }
 
-// A tile's candidates listed two to a pair block of 2 float4: entry pos in
-// the x and z components, entry pos + 1 in y and w,
-//   (x, x') (y, y') | (z, z') (unused)
-// so that the offsets and squared distances of both are formed by packed
-// FP32x2 operations.
-__device__ __forceinline__ void list_iso_pair(float4 q, float* lst, uint32_t pos)
-{
-    float* d = lst + (pos >> 1) * 8 + (pos & 1u);
-    d[0] = q.x;
-    d[2] = q.y;
-    d[4] = q.z;
-}
-
 template <bool TC01>
-__global__ void __launch_bounds__(kFT) k_field_iso_grouped(IsoFieldArgs a, BandView band, uint32_t ratio, Counters* ctr)
+__global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, BandView band, uint32_t ratio, Counters* ctr)
 {
     __shared__ IsoSlice slices[kFWarps];
     const int lane = threadIdx.x & 31;
@@ -958,102 +1012,144 @@ __global__ void __launch_bounds__(kFT) k_field_iso_grouped(IsoFieldArgs a, BandV
 
         auto pass = [&](uint32_t nv) {
             float4 pl, ph;
-            pass_layout(w.vloc, lo, a.sc, w.order, reinterpret_cast<uint32_t*>(&w.sum[0][0][0]), w.box, nv,
-                        1.0f / a.sc.cs, lane, pl, ph);  // the sums are zeroed next
+            pass_layout<true>(w.vloc, w.vrank, lo, a.sc, nullptr, reinterpret_cast<uint32_t*>(&w.sum[0][0][0]), w.box, nv, lane, pl, ph);  // the sums are zeroed next
             const uint32_t ntiles = (nv + 31) / 32;
             for (int k = 0; k < kSums; ++k)
-                for (int t = 0; t < kPassTiles; ++t) w.sum[k][t][lane] = 0.f;
+                for (uint32_t t = 0; t < ntiles; ++t) w.sum[k][t][lane] = 0.f;
             __syncwarp();
+            // a candidate's place in the list: two to a pair
+            auto list = [&](const float4& q, uint32_t pos) {
+                float* d = reinterpret_cast<float*>(w.lxy + (pos >> 1)) + (pos & 1u);
+                d[0] = q.x;
+                d[2] = q.y;
+                reinterpret_cast<float*>(w.lz)[pos] = q.z;
+            };
+            // the listed candidates [0, cnt) for tile t: each lane takes one pair
+            // per step for its vertex, in order
+            auto evaluate = [&](uint32_t t, uint32_t cnt) {
+                if ((cnt & 1u) && lane == 0) {  // the last pair's other half: beyond h of everything
+                    float* d = reinterpret_cast<float*>(w.lxy + (cnt >> 1)) + 1;
+                    d[0] = d[2] = reinterpret_cast<float*>(w.lz)[cnt] = 1.0e18f;
+                }
+                __syncwarp();
+                const uint32_t v = 32 * t + lane;
+                if (v < nv) {
+                    const float4 vp = vert_pos(w.vloc[v], lo, a.sc);
+                    float ws = w.sum[0][t][lane];
+                    float ax = 0.f, ay = 0.f, az = 0.f;
+                    if (!TC01) {
+                        ax = w.sum[1][t][lane];
+                        ay = w.sum[2][t][lane];
+                        az = w.sum[3][t][lane];
+                    }
+                    const float2 nvx = make_float2(-vp.x, -vp.x), nvy = make_float2(-vp.y, -vp.y),
+                                 nvz = make_float2(-vp.z, -vp.z);
+                    const float2 ninv = make_float2(-a.inv_h2, -a.inv_h2), one = make_float2(1.0f, 1.0f);
+                    const uint32_t pairs = (cnt + 1) >> 1;
+                    // (two copies: 0.90 -> 0.82 ms on the 256k Akinci12 frame;
+                    // four crowd the instruction cache: 0.90)
+#pragma unroll 2
+                    for (uint32_t j = 0; j < pairs; ++j) {
+                        const float4 A = w.lxy[j];
+                        const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nvx);
+                        const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nvy);
+                        const float2 dz = __fadd2_rn(w.lz[j], nvz);
+                        const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                        if (TC01) {
+                            const float ua = d2.x * a.inv_h2 * 0.5f, ub = d2.y * a.inv_h2 * 0.5f;
+                            const float ta = ua * ua - ua + 0.25f, tb = ub * ub - ub + 0.25f;
+                            if (d2.x <= a.h2) ws += ta;
+                            if (d2.y <= a.h2) ws += tb;
+                        } else {
+                            const float2 u = __ffma2_rn(d2, ninv, one);
+                            const float2 u2 = __fmul2_rn(u, u);
+                            const float2 wt = __fmul2_rn(u2, u);
+                            if (d2.x < a.h2) {
+                                ws = ws + wt.x;
+                                ax = fmaf(dx.x, wt.x, ax);
+                                ay = fmaf(dy.x, wt.x, ay);
+                                az = fmaf(dz.x, wt.x, az);
+                            }
+                            if (d2.y < a.h2) {
+                                ws = ws + wt.y;
+                                ax = fmaf(dx.y, wt.y, ax);
+                                ay = fmaf(dy.y, wt.y, ay);
+                                az = fmaf(dz.y, wt.y, az);
+                            }
+                        }
+                    }
+                    w.sum[0][t][lane] = ws;
+                    if (!TC01) {
+                        w.sum[1][t][lane] = ax;
+                        w.sum[2][t][lane] = ay;
+                        w.sum[3][t][lane] = az;
+                    }
+                }
+                __syncwarp();  // the list is rewritten next
+            };
+            // the staged candidates [0, fill) against every tile: the ones within
+            // h of the tile are listed and evaluated; with one tile, whose box is
+            // the pass's, the candidates are listed as they are staged
+            uint32_t fill = 0;
+            const bool one_tile = ntiles == 1u;
+            auto tiles = [&]() {
+                if (one_tile) {
+                    evaluate(0, fill);
+                    fill = 0;
+                    return;
+                }
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t t = 0; t < ntiles; ++t) {
+                    const float4 tl = w.box[2 * t], th = w.box[2 * t + 1];
+                    uint32_t cnt = 0;
+                    for (uint32_t b = 0; b < fill; b += 32) {
+                        const uint32_t i = b + (uint32_t)lane;
+                        float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (i < fill) {
+                            q.x = w.cx[i];
+                            q.y = w.cy[i];
+                            q.z = w.cz[i];
+                        }
+                        const bool in = i < fill && within(q, tl, th, cr2);
+                        const uint32_t m = __ballot_sync(0xffffffffu, in);
+                        if (in) list(q, cnt + __popc(m & ((1u << lane) - 1u)));
+                        cnt += __popc(m);
+                    }
+                    if (cnt != 0u) evaluate(t, cnt);
+                }
+                fill = 0;
+            };
+            int row = 0;
             for (uint32_t cb = 0; cb < total; cb += 32) {
                 const uint32_t j = cb + lane;
                 bool keep = false;
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (j < total) {
-                    int r = 0;
-                    while (r < 8 && w.rp[r + 1] <= j) ++r;
-                    q = __ldg(&a.sorted[w.rb[r] + (j - w.rp[r])]);
+                    while (row < 8 && w.rp[row + 1] <= j) ++row;
+                    q = __ldg(&a.sorted[w.rb[row] + (j - w.rp[row])]);
                     keep = within(q, pl, ph, cr2);
                 }
-                const uint32_t any = __ballot_sync(0xffffffffu, keep);
-                __syncwarp();
-                if (any) {
-#pragma unroll 1
-                    for (int t = 0; t < kPassTiles; ++t) {
-                        if ((uint32_t)t >= ntiles) break;
-                        const uint32_t m = __ballot_sync(0xffffffffu, keep && within(q, w.box[2 * t], w.box[2 * t + 1], cr2));
-                        if (!m) continue;
-                        // the candidates within h of the tile, listed in lane
-                        // order two to a pair block
-                        if ((m >> lane) & 1u)
-                            list_iso_pair(q, reinterpret_cast<float*>(w.lst), __popc(m & ((1u << lane) - 1u)));
-                        __syncwarp();
-                        const uint32_t v = 32 * t + lane;
-                        if (v < nv) {
-                            const float4 vp = vert_pos(w.vloc[w.order[v]], lo, a.sc);
-                            float ws = w.sum[0][t][lane];
-                            float ax = 0.f, ay = 0.f, az = 0.f;
-                            if (!TC01) {
-                                ax = w.sum[1][t][lane];
-                                ay = w.sum[2][t][lane];
-                                az = w.sum[3][t][lane];
-                            }
-                            const float2 nvx = make_float2(-vp.x, -vp.x), nvy = make_float2(-vp.y, -vp.y),
-                                         nvz = make_float2(-vp.z, -vp.z);
-                            const uint32_t cnt = __popc(m);
-                            // one pair block per step: offsets and squared
-                            // distances of both by packed operations (the
-                            // roundings of the scalar forms), the rest per
-                            // candidate; terms added in list (lane) order.  Not
-                            // unrolled: copies of the body crowd the
-                            // instruction cache
-#pragma unroll 1
-                            for (uint32_t j = 0; j < cnt; j += 2) {
-                                const bool two = j + 1 < cnt;
-                                const float4 A = w.lst[j], B = w.lst[j + 1];  // pair block j / 2
-                                const float2 dx = __fadd2_rn(make_float2(A.x, A.y), nvx);
-                                const float2 dy = __fadd2_rn(make_float2(A.z, A.w), nvy);
-                                const float2 dz = __fadd2_rn(make_float2(B.x, B.y), nvz);
-                                const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
-                                const float dxa = dx.x, dya = dy.x, dza = dz.x, d2a = d2.x;
-                                const float dxb = dx.y, dyb = dy.y, dzb = dz.y, d2b = d2.y;
-                                if (TC01) {
-                                    const float ua = d2a * a.inv_h2 * 0.5f, ub = d2b * a.inv_h2 * 0.5f;
-                                    const float ta = ua * ua - ua + 0.25f, tb = ub * ub - ub + 0.25f;
-                                    if (d2a <= a.h2) ws += ta;
-                                    if (two && d2b <= a.h2) ws += tb;
-                                } else {
-                                    const float ua = 1.0f - d2a * a.inv_h2, ub = 1.0f - d2b * a.inv_h2;
-                                    const float wa = ua * ua * ua, wb = ub * ub * ub;
-                                    if (d2a < a.h2) {
-                                        ws += wa;
-                                        ax = fmaf(dxa, wa, ax);
-                                        ay = fmaf(dya, wa, ay);
-                                        az = fmaf(dza, wa, az);
-                                    }
-                                    if (two && d2b < a.h2) {
-                                        ws += wb;
-                                        ax = fmaf(dxb, wb, ax);
-                                        ay = fmaf(dyb, wb, ay);
-                                        az = fmaf(dzb, wb, az);
-                                    }
-                                }
-                            }
-                            w.sum[0][t][lane] = ws;
-                            if (!TC01) {
-                                w.sum[1][t][lane] = ax;
-                                w.sum[2][t][lane] = ay;
-                                w.sum[3][t][lane] = az;
-                            }
-                        }
-                        __syncwarp();  // the list is rewritten for the next tile
+                const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const uint32_t pos = fill + __popc(m & ((1u << lane) - 1u));
+                    if (one_tile) {
+                        list(q, pos);
+                    } else {
+                        w.cx[pos] = q.x;
+                        w.cy[pos] = q.y;
+                        w.cz[pos] = q.z;
                     }
                 }
-                __syncwarp();
+                fill += __popc(m);
+                if (fill > kIsoSeg - 32) tiles();
             }
+            if (fill) tiles();
+            __syncwarp();
             for (int t = 0; t < (int)ntiles; ++t) {
                 const uint32_t v = 32 * t + lane;
                 if (v < nv) {
-                    const uint32_t rank = w.vrank[w.order[v]];
+                    const uint32_t rank = w.vrank[v];
                     if (rank < nb) {
                         const float ws = w.sum[0][t][lane];
                         if (TC01) {

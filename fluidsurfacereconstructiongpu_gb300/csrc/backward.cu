@@ -212,16 +212,28 @@ __global__ void k_field_backward_iso(BwdArgs a)
     a.gx[j] = make_float4(gx, gy, gz, 0.f);
 }
 
-// dL/d(particle radius) of ZB05: -sum of dL/dphi over vertices with weight
-__global__ void k_radius_grad(BwdArgs a, const Counters* ctr, float* out)
+// dL/d(particle radius) of ZB05: -sum of dL/dphi over vertices with weight.
+// Summed in FP64: millions of terms of both signs, and FP32 partial sums added
+// in the order of the atomics were off by up to 2e-6 of the result, differently
+// in each run.  Bound by the read of dL/dphi; the weight sums are read only
+// where it is not zero (500k-particle frame: 50 -> 35 us).
+__global__ void k_radius_grad(BwdArgs a, const Counters* ctr, double* out)
 {
     const uint32_t nb = min(ctr->n_band, a.cap_band);
-    float s = 0.f;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x)
-        if (a.mv[t].w > 0.f) s -= a.gphi[t];
+    double s = 0.0;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x) {
+        const float g = a.gphi[t];
+        if (g != 0.f && a.mv[t].w > 0.f) s -= (double)g;
+    }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0 && s != 0.f) atomicAdd(out, s);
+    __shared__ double warps[kT / 32];
+    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kT / 32; ++w) s += warps[w];
+        if (s != 0.0) atomicAdd(out, s);
+    }
 }
 
 // ---------------------------------------------------------------- anisotropic field
@@ -642,7 +654,7 @@ inline unsigned nblk(uint64_t n) { return (unsigned)std::max<uint64_t>(1, (n + k
 }  // namespace
 
 void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, const Counters* ctr, int method,
-                     float lambda, float R, float* radius_grad_dev, float* out_grad_xyz)
+                     float lambda, float R, double* radius_grad_dev, float* out_grad_xyz)
 {
     const unsigned pb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_valid + kT - 1) / kT,
                                                                           (uint64_t)c.num_sms * 16));

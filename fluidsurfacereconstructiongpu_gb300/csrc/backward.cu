@@ -164,54 +164,7 @@ __device__ __forceinline__ void window_box(const BwdArgs& a, const int c[3], int
     }
 }
 
-// ---------------------------------------------------------------- ZB05 / TC01 field
-template <bool TC01>
-__global__ void k_field_backward_iso(BwdArgs a)
-{
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= a.n) return;
-    const float4 q = a.sorted[j];
-    const int c[3] = {cell1(q.x, a.sp.min[0], a.sp.cs), cell1(q.y, a.sp.min[1], a.sp.cs),
-                      cell1(q.z, a.sp.min[2], a.sp.cs)};
-    float gx = 0.f, gy = 0.f, gz = 0.f;
-    if (near_gradient(a, c[0], c[1], c[2], 1)) {
-        const float p[3] = {q.x, q.y, q.z};
-        int lo[3], hi[3];
-        window_box(a, c, 1, p, cull_radius(a.h, a.sp.cs), lo, hi);
-        const float h2 = a.h * a.h, inv_h2 = 1.0f / h2;
-        for_band_vertices(a, lo, hi, [&](uint32_t rank, float g, float vx, float vy, float vz) {
-            const float dx = q.x - vx, dy = q.y - vy, dz = q.z - vz;
-            const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            if (TC01) {
-                if (d2 > h2) return;
-                const float tt = d2 * inv_h2 * 0.5f;
-                const float s = g * (2.f * tt - 1.f) * inv_h2;
-                gx = fmaf(s, dx, gx);
-                gy = fmaf(s, dy, gy);
-                gz = fmaf(s, dz, gz);
-            } else {
-                if (d2 >= h2) return;
-                const float4 m = a.mv[rank];  // mean - v, weight sum
-                if (!(m.w > 0.f)) return;
-                const float ml = sqrtf(fmaf(m.x, m.x, fmaf(m.y, m.y, m.z * m.z)));
-                if (!(ml > 0.f)) return;
-                const float u = 1.0f - d2 * inv_h2;
-                const float wt = u * u * u;
-                // d phi / d xbar = (xbar - v) / |xbar - v|
-                const float ex = g * m.x / ml, ey = g * m.y / ml, ez = g * m.z / ml;
-                // d xbar / d x_j = (w I + (x_j - xbar) (dw/dx_j)^T) / W, dw/dx_j = -6 u^2 (x_j - v) / h^2
-                const float proj = ex * (dx - m.x) + ey * (dy - m.y) + ez * (dz - m.z);
-                const float k2 = proj * (-6.0f * u * u * inv_h2);
-                const float iw = 1.0f / m.w;
-                gx += (wt * ex + k2 * dx) * iw;
-                gy += (wt * ey + k2 * dy) * iw;
-                gz += (wt * ez + k2 * dz) * iw;
-            }
-        });
-    }
-    a.gx[j] = make_float4(gx, gy, gz, 0.f);
-}
-
+// ---------------------------------------------------------------- ZB05 radius
 // dL/d(particle radius) of ZB05: -sum of dL/dphi over vertices with weight.
 // Summed in FP64: millions of terms of both signs, and FP32 partial sums added
 // in the order of the atomics were off by up to 2e-6 of the result, differently
@@ -691,16 +644,8 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
         k_smooth_backward<<<nblk(a.n), kT, 0, c.stream>>>(a, cov->sorted, cov->mean, cov->ranges, cov->sp, a.n, R,
                                                            cov->R_lt2, smooth_coop, lambda);
         g_launches += 3;
-    } else if (method == FSR_METHOD_TC01) {
-        if (!launch_field_iso_backward_grouped(c, a, true, ctr)) {
-            k_field_backward_iso<true><<<nblk(a.n), kT, 0, c.stream>>>(a);
-            ++g_launches;
-        }
     } else {
-        if (!launch_field_iso_backward_grouped(c, a, false, ctr)) {
-            k_field_backward_iso<false><<<nblk(a.n), kT, 0, c.stream>>>(a);
-            ++g_launches;
-        }
+        launch_field_iso_backward(c, a, method == FSR_METHOD_TC01, ctr);
         if (radius_grad_dev) {
             k_radius_grad<<<bb, kT, 0, c.stream>>>(a, ctr, radius_grad_dev);
             ++g_launches;

@@ -428,10 +428,10 @@ __device__ __forceinline__ float4 vert_pos(uint32_t loc, const int lo[3], const 
 // candidates reaching it; a counting sort by brick, the order within a brick
 // is that of the atomics, which changes no result since a vertex's sum does
 // not depend on its tile and culling only skips exact zeros), and the box of
-// each 32-vertex tile.  Boxes are formed from the vertices' indices by warp
+// each 32-vertex tile (kVerts: the most vertices of a pass).  Boxes are formed from the vertices' indices by warp
 // reductions (positions do not decrease with the index); frames of many small
 // groups spent a fifth of their field time on the float boxes this replaces.
-// hist: kPassVerts words of scratch.
+// hist: kVerts words of scratch.
 struct IndexBox {
     uint32_t lo[3], hi[3];
     __device__ __forceinline__ void clear()
@@ -474,7 +474,7 @@ struct IndexBox {
 
 // kInPlace: vloc and vrank are reordered (order is not used); else order[v] is
 // the place of the v-th vertex.
-template <bool kInPlace>
+template <bool kInPlace, int kVerts = kPassVerts>
 __device__ __forceinline__ void pass_layout(uint32_t* vloc, uint32_t* vrank, const int lo[3], const Grid& sc,
                                             uint16_t* order, uint32_t* hist, float4* box, uint32_t nv, int lane,
                                             float4& pl, float4& ph)
@@ -499,13 +499,13 @@ __device__ __forceinline__ void pass_layout(uint32_t* vloc, uint32_t* vrank, con
     const uint32_t gy = ((pass.hi[1] - pass.lo[1]) >> 2) + 1u;
     const uint32_t gz = ((pass.hi[2] - pass.lo[2]) >> 1) + 1u;
     const uint32_t nbins = gx * gy * gz;
-    if (nbins <= (uint32_t)kPassVerts) {
+    if (nbins <= (uint32_t)kVerts) {
         for (uint32_t b = lane; b < nbins; b += 32) hist[b] = 0u;
         __syncwarp();
-        uint32_t at[kPassVerts / 32];  // brick | place in it << 16
-        uint32_t loc[kPassVerts / 32], rank[kPassVerts / 32];
+        uint32_t at[kVerts / 32];  // brick | place in it << 16
+        uint32_t loc[kVerts / 32], rank[kVerts / 32];
 #pragma unroll
-        for (int k = 0; k < kPassVerts / 32; ++k) {
+        for (int k = 0; k < kVerts / 32; ++k) {
             const uint32_t q = lane + 32 * k;
             at[k] = 0;
             if (q < nv) {
@@ -537,7 +537,7 @@ __device__ __forceinline__ void pass_layout(uint32_t* vloc, uint32_t* vrank, con
         }
         __syncwarp();
 #pragma unroll
-        for (int k = 0; k < kPassVerts / 32; ++k) {
+        for (int k = 0; k < kVerts / 32; ++k) {
             const uint32_t q = lane + 32 * k;
             if (q < nv) {
                 const uint32_t to = hist[at[k] & 0xffffu] + (at[k] >> 16);
@@ -568,18 +568,19 @@ __device__ __forceinline__ void pass_layout(uint32_t* vloc, uint32_t* vrank, con
 
 // The band vertices of a group's index box [lo, hi), listed into (vloc,
 // vrank) by row segments of at most 32 vertices (two bitset
-// words), `per` segments per step so that one step adds at most kPassVerts
+// words), `per` segments per step so that one step adds at most kVerts
 // vertices; pass(count) runs whenever the next step would not fit, and at
-// the end.
-template <class PassFn>
+// the end.  keep(bits, r0): which of a segment's vertices (the first set bit
+// of rank r0) are wanted.
+template <int kVerts, class KeepFn, class PassFn>
 __device__ __forceinline__ void list_band_vertices(const Grid& sc, const BandView& band, const int lo[3],
                                                    const int hi[3], uint32_t* vloc, uint32_t* vrank, int lane,
-                                                   PassFn&& pass)
+                                                   KeepFn&& keep, PassFn&& pass)
 {
     const int nx = hi[0] - lo[0], ny = hi[1] - lo[1], nz = hi[2] - lo[2];
     const int nseg = (nx + 31) / 32;
     const int units = ny * nz * nseg;
-    const int per = max(1, min(32, kPassVerts / min(nx, 32)));
+    const int per = max(1, min(32, kVerts / min(nx, 32)));
     int ub = 0;
     while (ub < units) {
         uint32_t count = 0;
@@ -602,6 +603,8 @@ __device__ __forceinline__ void list_band_vertices(const Grid& sc, const BandVie
                 // rm is vertex v0 + b, so its rank adds the set bits below b
                 r0 = __ldg(band.prefix + w0) + __popc((uint32_t)bits & ((1u << sh) - 1u));
             }
+            const uint32_t all = rm;
+            rm = keep(rm, r0);
             const uint32_t n = __popc(rm);
             uint32_t x = n;
 #pragma unroll
@@ -610,13 +613,13 @@ __device__ __forceinline__ void list_band_vertices(const Grid& sc, const BandVie
                 if (lane >= o) x += y;
             }
             const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
-            // (tot <= kPassVerts by the choice of `per`: an empty pass always takes the step)
-            if (count > 0 && count + tot > (uint32_t)kPassVerts) break;  // run the pass, then this step again
+            // (tot <= kVerts by the choice of `per`: an empty pass always takes the step)
+            if (count > 0 && count + tot > (uint32_t)kVerts) break;  // run the pass, then this step again
             uint32_t slot = count + x - n;
             for (uint32_t m = rm; m; m &= m - 1u) {
                 const int bx = __ffs(m) - 1;
                 vloc[slot] = vert_loc(x0 + bx - lo[0], ry - lo[1], rz - lo[2]);
-                vrank[slot++] = r0 + __popc(rm & ((1u << bx) - 1u));
+                vrank[slot++] = r0 + __popc(all & ((1u << bx) - 1u));
             }
             count += tot;
         }
@@ -624,6 +627,8 @@ __device__ __forceinline__ void list_band_vertices(const Grid& sc, const BandVie
         if (count > 0) pass(count);
     }
 }
+
+__device__ __forceinline__ uint32_t keep_all(uint32_t bits, uint32_t) { return bits; }
 
 // The unscaled kernel's part of the field at vertex v, sum_j c_j (1 - |x_j -
 // v|^2)^3 over the group's non-involved candidates j, is one polynomial in
@@ -915,7 +920,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
             __syncwarp();
         };
 
-        list_band_vertices(a.sc, a.band, lo, hi, w.vloc, w.vrank, lane, pass);
+        list_band_vertices<kPassVerts>(a.sc, a.band, lo, hi, w.vloc, w.vrank, lane, keep_all, pass);
         __syncwarp();
     }
 }
@@ -949,6 +954,45 @@ struct IsoSlice {
     uint32_t rb[9], rp[10];        // the window's rows: first particle, prefix of lengths
 };
 
+// The rows of the +-1 window around cell c (clamped as window() clamps), z then
+// y: first particles rb[9] and the prefix of their lengths rp[10]; returns the
+// number of particles.  Every lane of the warp calls it.
+__device__ __forceinline__ uint32_t window_rows(const Grid& sp, const uint2* __restrict__ ranges, const int c[3],
+                                                uint32_t* rb, uint32_t* rp, int lane)
+{
+    uint32_t beg = kEmpty, end = 0;
+    if (lane < 9) {
+        const int x0 = clampi(c[0] - 1, 0, (int)sp.res[0] - 1), x1 = clampi(c[0] + 1, 0, (int)sp.res[0] - 1);
+        const int y0 = clampi(c[1] - 1, 0, (int)sp.res[1] - 1), y1 = clampi(c[1] + 1, 0, (int)sp.res[1] - 1);
+        const int z0 = clampi(c[2] - 1, 0, (int)sp.res[2] - 1), z1 = clampi(c[2] + 1, 0, (int)sp.res[2] - 1);
+        const int yy = y0 + lane % 3, zz = z0 + lane / 3;
+        if (yy <= y1 && zz <= z1) {
+            const uint32_t c0 = lin3(x0, yy, zz, sp);
+            for (int xx = 0; xx <= x1 - x0; ++xx) {
+                const uint2 r = __ldg(&ranges[c0 + xx]);
+                if (r.x != kEmpty) {
+                    beg = min(beg, r.x);
+                    end = max(end, r.y);
+                }
+            }
+        }
+    }
+    const uint32_t len = end > beg ? end - beg : 0u;
+    uint32_t x = len;
+#pragma unroll
+    for (int o = 1; o < 16; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane < 9) {
+        rb[lane] = beg;
+        rp[lane] = x - len;
+    }
+    if (lane == 8) rp[9] = x;
+    __syncwarp();
+    return __shfl_sync(0xffffffffu, x, 8);
+}
+
 __device__ __forceinline__ bool within(float4 q, float4 lo, float4 hi, float r2)
 {
     const float gx = fmaxf(0.f, fmaxf(lo.x - q.x, q.x - hi.x));
@@ -977,38 +1021,7 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, Ba
         const uint32_t g = a.glist[k / nslab];
         int c[3], lo[3], hi[3];
         if (!group_box(g, a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi)) continue;
-        // rows of the +-1 window (clamped as window() clamps), z then y
-        if (lane < 9) {
-            const int x0 = clampi(c[0] - 1, 0, (int)a.sp.res[0] - 1), x1 = clampi(c[0] + 1, 0, (int)a.sp.res[0] - 1);
-            const int y0 = clampi(c[1] - 1, 0, (int)a.sp.res[1] - 1), y1 = clampi(c[1] + 1, 0, (int)a.sp.res[1] - 1);
-            const int z0 = clampi(c[2] - 1, 0, (int)a.sp.res[2] - 1), z1 = clampi(c[2] + 1, 0, (int)a.sp.res[2] - 1);
-            const int yy = y0 + lane % 3, zz = z0 + lane / 3;
-            uint32_t beg = kEmpty, end = 0;
-            if (yy <= y1 && zz <= z1) {
-                const uint32_t c0 = lin3(x0, yy, zz, a.sp);
-                for (int xx = 0; xx <= x1 - x0; ++xx) {
-                    const uint2 r = __ldg(&a.ranges[c0 + xx]);
-                    if (r.x != kEmpty) {
-                        beg = min(beg, r.x);
-                        end = max(end, r.y);
-                    }
-                }
-            }
-            w.rb[lane] = beg;
-            w.rp[lane + 1] = beg == kEmpty ? 0u : end - beg;  // lengths for now
-        }
-        __syncwarp();
-        if (lane == 0) {
-            uint32_t acc = 0;
-            for (int r = 0; r < 9; ++r) {
-                const uint32_t len = w.rp[r + 1];
-                w.rp[r] = acc;
-                acc += len;
-            }
-            w.rp[9] = acc;
-        }
-        __syncwarp();
-        const uint32_t total = w.rp[9];
+        const uint32_t total = window_rows(a.sp, a.ranges, c, w.rb, w.rp, lane);
 
         auto pass = [&](uint32_t nv) {
             float4 pl, ph;
@@ -1169,76 +1182,9 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, Ba
             }
             __syncwarp();
         };
-        list_band_vertices(a.sc, band, lo, hi, w.vloc, w.vrank, lane, pass);
+        list_band_vertices<kPassVerts>(a.sc, band, lo, hi, w.vloc, w.vrank, lane, keep_all, pass);
         __syncwarp();
     }
-}
-
-// The group box's vertices with a non-zero dL/dphi, listed in 4 x 4 x 2
-// bricks of the box, so that each 32 consecutive ones (which share one
-// culling box in the ZB05/TC01 adjoint) lie close together: a count per brick, a scan,
-// then a scatter (the order inside a brick is that of the atomics; it changes
-// no sum but the float atomics' order, which is not fixed anyway).
-// emit(slot, lx, ly, lz, rank, gv) stores one vertex (slots below `cap` only);
-// hist holds `cap` words.  Every thread of the block calls it; returns the
-// number of such vertices.
-template <class Emit>
-__device__ uint32_t list_grad_vertices(const BandView& band, const float* __restrict__ gphi, uint32_t nb,
-                                       const Grid& sc, const int lo[3], const int hi[3], uint32_t* hist, uint32_t cap,
-                                       uint32_t* s_tot, Emit&& emit)
-{
-    const int tid = threadIdx.x, lane = tid & 31;
-    const int nx = hi[0] - lo[0], ny = hi[1] - lo[1], nz = hi[2] - lo[2];
-    const int nbox = nx * ny * nz;
-    const int bx = (nx + 3) / 4, by = (ny + 3) / 4, bz = (nz + 1) / 2;
-    const bool bricks = (uint32_t)(bx * by * bz) <= cap;  // (always, for boxes within the capacity)
-    const int nbins = bricks ? bx * by * bz : 1;
-    auto key = [&](int lx, int ly, int lz) { return bricks ? (lx >> 2) + bx * ((ly >> 2) + by * (lz >> 1)) : 0; };
-    auto grad = [&](int i, int& lx, int& ly, int& lz, uint32_t& rank) -> float {
-        lx = i % nx;
-        ly = (i / nx) % ny;
-        lz = i / (nx * ny);
-        const uint32_t v = lin3(lo[0] + lx, lo[1] + ly, lo[2] + lz, sc);
-        if (!band_has(band, v)) return 0.f;
-        rank = band_rank(band, v);
-        return rank < nb ? __ldg(gphi + rank) : 0.f;
-    };
-    for (int b = tid; b < nbins; b += blockDim.x) hist[b] = 0u;
-    __syncthreads();
-    for (int i = tid; i < nbox; i += blockDim.x) {
-        int lx, ly, lz;
-        uint32_t rank = 0;
-        if (grad(i, lx, ly, lz, rank) != 0.f) atomicAdd(&hist[key(lx, ly, lz)], 1u);
-    }
-    __syncthreads();
-    if (tid < 32) {  // exclusive scan of the counts
-        uint32_t run = 0;
-        for (int b0 = 0; b0 < nbins; b0 += 32) {
-            const int b = b0 + lane;
-            const uint32_t cnt = b < nbins ? hist[b] : 0u;
-            uint32_t x = cnt;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (b < nbins) hist[b] = run + x - cnt;
-            run += __shfl_sync(0xffffffffu, x, 31);
-        }
-        if (lane == 0) *s_tot = run;
-    }
-    __syncthreads();
-    for (int i = tid; i < nbox; i += blockDim.x) {
-        int lx, ly, lz;
-        uint32_t rank = 0;
-        const float gv = grad(i, lx, ly, lz, rank);
-        if (gv != 0.f) {
-            const uint32_t slot = atomicAdd(&hist[key(lx, ly, lz)], 1u);
-            if (slot < cap) emit(slot, lx, ly, lz, rank, gv);
-        }
-    }
-    __syncthreads();
-    return *s_tot;
 }
 
 // ---------------------------------------------------------------- adjoint
@@ -1468,148 +1414,206 @@ __global__ void k_field_aniso_backward_grouped(BwdGroupArgs a, uint32_t ratio, c
 }
 
 // Adjoint of the ZB05 / TC01 fields (updateScalarFieldValueZB05 cu:230-289,
-// TC01 cu:178-227), grouped like the anisotropic adjoint: a group's vertices
-// with dL/dphi != 0 (and, for ZB05, their (mean - v, weight sum) from the
-// forward) sit in shared memory with one box per 32; the candidates are the
-// particles of the +-1 cell window around the group's cell (the forward's
-// window for each of those vertices), one per thread, and each adds its
-// dL/dx over the active vertices within h with one float4 atomic.
+// TC01 cu:178-227), grouped like the forward field with the roles swapped: a
+// warp takes a group (or a z slab of it), lists the vertices with dL/dphi != 0 in
+// brick tiles, stages the window's particles within h of their box, and per tile
+// gives the particles within h of the tile one lane each; a lane walks the
+// tile's vertices two at a time with packed FP32x2 operations (the clamp of 1 -
+// d^2/h^2 at 0 drops the ones beyond h) and adds its sums to the particle's in
+// shared memory; one float4 atomic per particle and segment ends it.
+//   ZB05: phi = |xbar - v| - r_p; with e = (xbar - v) dL/dphi / (|xbar - v| W) per
+//   vertex, dL/dx_j += w e + (e.d - e.(xbar - v)) (-6 u^2 / h^2) d, d = x_j - v,
+//   u = 1 - d^2/h^2, w = u^3
+//   TC01: phi = sum t^2 - t + 1/4, t = d^2 / 2h^2: dL/dx_j += dL/dphi (2t - 1) / h^2 d
+// (A block per group, whose eight warps met at five barriers per group, spent
+// most of its time waiting there; 500k-particle ZB05 frame: 0.67 -> @IB@ ms.)
+constexpr int kBwdVerts = 128;        // vertices of a pass
+constexpr uint32_t kBwdSeg = 96;      // particles staged at a time
 template <bool TC01>
-__global__ void __launch_bounds__(kBT) k_field_iso_backward_grouped(BwdArgs a, uint32_t vlist_cap, const Counters* ctr)
+struct IsoBwdSlice {
+    float4 vxy[kBwdVerts / 2];                // the pass's vertices two to a pair: (x, x', y, y')
+    float2 vz[kBwdVerts / 2];                 // (z, z')
+    float4 exy[TC01 ? 1 : kBwdVerts / 2];     // ZB05: e of the two, (ex, ex', ey, ey')
+    float4 ezw[TC01 ? 1 : kBwdVerts / 2];     // (ez, ez', e.(xbar - v), ...')
+    float2 g[TC01 ? kBwdVerts / 2 : 1];       // TC01: dL/dphi of the two
+    uint32_t vloc[kBwdVerts], vrank[kBwdVerts];
+    uint32_t hist[kBwdVerts];
+    float4 box[2 * (kBwdVerts / 32)];
+    float cx[kBwdSeg], cy[kBwdSeg], cz[kBwdSeg];  // the staged particles
+    float gx[kBwdSeg], gy[kBwdSeg], gz[kBwdSeg];  // their dL/dx
+    uint32_t cj[kBwdSeg];                         // their sorted index
+    uint32_t list[kBwdSeg];                       // those within h of the tile
+    uint32_t rb[9], rp[10];
+};
+
+template <bool TC01>
+__global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const Counters* ctr)
 {
-    extern __shared__ __align__(16) unsigned char smem[];
-    float4* av = reinterpret_cast<float4*>(smem);  // active vertices: (v, dL/dphi)
-    // ZB05, per active vertex: e = (mean - v) dL/dphi / (|mean - v| W) and e.(mean - v), so that a pair
-    // needs no square root or division (W: the weight sum; vertices without weight get 0)
-    float4* am = av + vlist_cap;
-    float4* cbox = am + (TC01 ? 0 : vlist_cap);     // per 32 of them: lo, hi
-    uint32_t* hist = reinterpret_cast<uint32_t*>(cbox + 2 * ((vlist_cap + 31) / 32));  // vlist_cap words
-    __shared__ uint32_t s_nv, s_rb[9], s_re[9], s_rp[10], s_next;
+    __shared__ IsoBwdSlice<TC01> slices[kFWarps];
+    const int lane = threadIdx.x & 31;
+    IsoBwdSlice<TC01>& w = slices[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap_band);
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t ngroups = (a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
+    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mark_keys)
+    const uint32_t nslab = field_slabs(nlist);
     const float h2 = a.h * a.h, inv_h2 = 1.0f / h2;
     const float cr = cull_radius(a.h, a.sp.cs), cr2 = cr * cr;
-    __shared__ uint32_t s_g;
-    const uint32_t nlist = a.glist[0];
+    const float2 inv2 = make_float2(inv_h2, inv_h2), ninv2 = make_float2(-inv_h2, -inv_h2);
+    const float2 one2 = make_float2(1.0f, 1.0f), mone2 = make_float2(-1.0f, -1.0f);
 
-    // the groups holding gradient vertices, handed out one per block from
-    // the list k_mark_keys built
     for (;;) {
-        if (tid == 0) s_g = atomicAdd(&a.glist[2], 1u);
-        __syncthreads();
-        const uint32_t k = s_g;
-        __syncthreads();
-        if (k >= nlist) break;
-        const uint32_t g = a.glist[4 + k];
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(&a.glist[2], 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= nlist * nslab) break;
         int c[3], lo[3], hi[3];
-        if (!group_box(g, a.sp, a.sc, a.ratio, c, lo, hi)) continue;
-        if (tid == 0) s_next = 0;
-        list_grad_vertices(a.band, a.gphi, nb, a.sc, lo, hi, hist, vlist_cap, &s_nv,
-                           [&](uint32_t slot, int lx, int ly, int lz, uint32_t rank, float gv) {
-            av[slot] = make_float4(vpos1(lo[0] + lx, a.sc.min[0], a.sc.cs), vpos1(lo[1] + ly, a.sc.min[1], a.sc.cs),
-                                   vpos1(lo[2] + lz, a.sc.min[2], a.sc.cs), gv);
-            if (!TC01) {
-                const float4 m = __ldg(a.mv + rank);  // mean - v, weight sum
-                const float ml = sqrtf(fmaf(m.x, m.x, fmaf(m.y, m.y, m.z * m.z)));
+        if (!group_box(a.glist[4 + k / nslab], a.sp, a.sc, a.ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi))
+            continue;
+        const uint32_t total = window_rows(a.sp, a.ranges, c, w.rb, w.rp, lane);
+
+        auto pass = [&](uint32_t nv) {
+            float4 pl, ph;
+            pass_layout<true, kBwdVerts>(w.vloc, w.vrank, lo, a.sc, nullptr, w.hist, w.box, nv, lane, pl, ph);
+            const uint32_t ntiles = (nv + 31) / 32;
+            // the vertices' positions and factors; the places up to the last
+            // tile's end lie beyond h of everything
+            for (uint32_t q = lane; q < 32u * ntiles; q += 32) {
+                float4 vp = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f);
                 float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (m.w > 0.f && ml > 0.f) {
-                    const float f = gv / ml / m.w;
-                    e = make_float4(m.x * f, m.y * f, m.z * f, 0.f);
-                    e.w = fmaf(e.x, m.x, fmaf(e.y, m.y, e.z * m.z));
-                }
-                am[slot] = e;
-            }
-        });
-        // the +-1 window's rows (x-adjacent cells are contiguous in the sorted order)
-        if (tid < 9) {
-            const int x0 = clampi(c[0] - 1, 0, (int)a.sp.res[0] - 1), x1 = clampi(c[0] + 1, 0, (int)a.sp.res[0] - 1);
-            const int y0 = clampi(c[1] - 1, 0, (int)a.sp.res[1] - 1), y1 = clampi(c[1] + 1, 0, (int)a.sp.res[1] - 1);
-            const int z0 = clampi(c[2] - 1, 0, (int)a.sp.res[2] - 1), z1 = clampi(c[2] + 1, 0, (int)a.sp.res[2] - 1);
-            const int yy = y0 + tid % 3, zz = z0 + tid / 3;
-            uint32_t beg = kEmpty, end = 0;
-            if (yy <= y1 && zz <= z1) {
-                const uint32_t c0 = lin3(x0, yy, zz, a.sp);
-                for (int xx = 0; xx <= x1 - x0; ++xx) {
-                    const uint2 r = __ldg(&a.ranges[c0 + xx]);
-                    if (r.x != kEmpty) {
-                        beg = min(beg, r.x);
-                        end = max(end, r.y);
+                float gv = 0.f;
+                if (q < nv) {
+                    vp = vert_pos(w.vloc[q], lo, a.sc);
+                    const uint32_t rank = w.vrank[q];
+                    gv = __ldg(a.gphi + rank);
+                    if (!TC01) {
+                        const float4 m = __ldg(a.mv + rank);  // mean - v, weight sum
+                        const float ml = sqrtf(fmaf(m.x, m.x, fmaf(m.y, m.y, m.z * m.z)));
+                        if (m.w > 0.f && ml > 0.f) {
+                            const float f = gv / ml / m.w;
+                            e = make_float4(m.x * f, m.y * f, m.z * f, 0.f);
+                            e.w = fmaf(e.x, m.x, fmaf(e.y, m.y, e.z * m.z));
+                        }
                     }
                 }
-            }
-            s_rb[tid] = beg;
-            s_re[tid] = end > beg ? end : beg;
-        }
-        __syncthreads();
-        const uint32_t nv = min(s_nv, vlist_cap);
-        if (tid == 0) {
-            uint32_t acc = 0;
-            for (int r = 0; r < 9; ++r) {
-                s_rp[r] = acc;
-                acc += (s_rb[r] == kEmpty) ? 0u : s_re[r] - s_rb[r];
-            }
-            s_rp[9] = acc;
-        }
-        const uint32_t nch = (nv + 31) / 32;
-        for (uint32_t k = tid; k < nch; k += kBT) {
-            float4 l = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f), h = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.f);
-            for (uint32_t q = 32 * k; q < min(nv, 32 * k + 32); ++q) {
-                const float4 v = av[q];
-                l.x = fminf(l.x, v.x); l.y = fminf(l.y, v.y); l.z = fminf(l.z, v.z);
-                h.x = fmaxf(h.x, v.x); h.y = fmaxf(h.y, v.y); h.z = fmaxf(h.z, v.z);
-            }
-            cbox[2 * k] = l;
-            cbox[2 * k + 1] = h;
-        }
-        __syncthreads();
-        const uint32_t total = nv ? s_rp[9] : 0u;
-        // one candidate per thread; warps take the next 32 as they finish
-        for (;;) {
-            uint32_t cb = 0;
-            if (lane == 0) cb = atomicAdd(&s_next, 32u);
-            cb = __shfl_sync(0xffffffffu, cb, 0);
-            if (cb >= total) break;
-            const uint32_t jj = cb + lane;
-            if (jj >= total) continue;
-            int r = 0;
-            while (r < 8 && s_rp[r + 1] <= jj) ++r;
-            const uint32_t j = s_rb[r] + (jj - s_rp[r]);
-            const float4 q = __ldg(&a.sorted[j]);
-            float gx = 0.f, gy = 0.f, gz = 0.f;
-            for (uint32_t k = 0; k < nch; ++k) {
-                if (!(box_dist2(q.x, q.y, q.z, cbox[2 * k], cbox[2 * k + 1]) < cr2)) continue;
-                const uint32_t qe = min(nv, 32 * k + 32);
-                for (uint32_t t = 32 * k; t < qe; ++t) {
-                    const float4 v = av[t];
-                    const float dx = q.x - v.x, dy = q.y - v.y, dz = q.z - v.z;
-                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    if (TC01) {
-                        if (d2 > h2) continue;
-                        const float tt = d2 * inv_h2 * 0.5f;
-                        const float sg = v.w * (2.f * tt - 1.f) * inv_h2;
-                        gx = fmaf(sg, dx, gx);
-                        gy = fmaf(sg, dy, gy);
-                        gz = fmaf(sg, dz, gz);
-                    } else {
-                        if (d2 >= h2) continue;
-                        const float4 e = am[t];
-                        const float u = 1.0f - d2 * inv_h2;
-                        const float wt = u * u * u;
-                        // d phi / d xbar = (xbar - v) / |xbar - v|; d xbar / d x_j = (w I + (x_j - xbar)
-                        // (dw/dx_j)^T) / W with dw/dx_j = -6 u^2 (x_j - v) / h^2; with e as above
-                        // (x_j - xbar = d - (mean - v)):
-                        //   dL/dx_j += wt e + (e.d - e.(mean - v)) (-6 u^2 / h^2) d
-                        const float k2 = (fmaf(e.x, dx, fmaf(e.y, dy, e.z * dz)) - e.w) * (-6.0f * u * u * inv_h2);
-                        gx = fmaf(wt, e.x, fmaf(k2, dx, gx));
-                        gy = fmaf(wt, e.y, fmaf(k2, dy, gy));
-                        gz = fmaf(wt, e.z, fmaf(k2, dz, gz));
-                    }
+                const uint32_t p = q >> 1, s = q & 1u;
+                float* d = reinterpret_cast<float*>(w.vxy + p) + s;
+                d[0] = vp.x;
+                d[2] = vp.y;
+                reinterpret_cast<float*>(w.vz)[q] = vp.z;
+                if (TC01) {
+                    reinterpret_cast<float*>(w.g)[q] = gv;
+                } else {
+                    d = reinterpret_cast<float*>(w.exy + p) + s;
+                    d[0] = e.x;
+                    d[2] = e.y;
+                    d = reinterpret_cast<float*>(w.ezw + p) + s;
+                    d[0] = e.z;
+                    d[2] = e.w;
                 }
             }
-            if (gx != 0.f || gy != 0.f || gz != 0.f) atomicAdd(a.gx + j, make_float4(gx, gy, gz, 0.f));
-        }
-        __syncthreads();
+            __syncwarp();
+            uint32_t fill = 0;
+            auto tiles = [&]() {
+                for (uint32_t i = lane; i < fill; i += 32) w.gx[i] = w.gy[i] = w.gz[i] = 0.f;
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t t = 0; t < ntiles; ++t) {
+                    const float4 tl = w.box[2 * t], th = w.box[2 * t + 1];
+                    uint32_t cnt = 0;
+                    for (uint32_t b = 0; b < fill; b += 32) {
+                        const uint32_t i = b + (uint32_t)lane;
+                        bool in = false;
+                        if (i < fill) in = within(make_float4(w.cx[i], w.cy[i], w.cz[i], 0.f), tl, th, cr2);
+                        const uint32_t m = __ballot_sync(0xffffffffu, in);
+                        if (in) w.list[cnt + __popc(m & ((1u << lane) - 1u))] = i;
+                        cnt += __popc(m);
+                    }
+                    __syncwarp();
+                    const uint32_t pairs = (min(32u, nv - 32u * t) + 1u) >> 1;
+                    for (uint32_t b = lane; b < cnt; b += 32) {
+                        const uint32_t i = w.list[b];
+                        const float2 qx = make_float2(w.cx[i], w.cx[i]), qy = make_float2(w.cy[i], w.cy[i]),
+                                     qz = make_float2(w.cz[i], w.cz[i]);
+                        // (ZB05) sum w e; sum k d with the factors common to all pairs left out
+                        float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx, tx = sx, ty = sx, tz = sx;
+#pragma unroll 2
+                        for (uint32_t j = 0; j < pairs; ++j) {
+                            const float4 A = w.vxy[16u * t + j];
+                            const float2 dx = __ffma2_rn(make_float2(A.x, A.y), mone2, qx);
+                            const float2 dy = __ffma2_rn(make_float2(A.z, A.w), mone2, qy);
+                            const float2 dz = __ffma2_rn(w.vz[16u * t + j], mone2, qz);
+                            const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                            float2 kk;
+                            if (TC01) {
+                                kk = __ffma2_rn(d2, inv2, mone2);
+                                kk.x = fminf(kk.x, 0.f);
+                                kk.y = fminf(kk.y, 0.f);
+                                kk = __fmul2_rn(kk, w.g[16u * t + j]);
+                            } else {
+                                float2 u = __ffma2_rn(d2, ninv2, one2);
+                                u.x = fmaxf(u.x, 0.f);
+                                u.y = fmaxf(u.y, 0.f);
+                                const float2 u2 = __fmul2_rn(u, u), wt = __fmul2_rn(u2, u);
+                                const float4 E = w.exy[16u * t + j], Z = w.ezw[16u * t + j];
+                                const float2 ex = make_float2(E.x, E.y), ey = make_float2(E.z, E.w),
+                                             ez = make_float2(Z.x, Z.y), ew = make_float2(Z.z, Z.w);
+                                kk = __ffma2_rn(ex, dx, __ffma2_rn(ey, dy, __ffma2_rn(ez, dz, __fmul2_rn(ew, mone2))));
+                                kk = __fmul2_rn(kk, u2);
+                                sx = __ffma2_rn(wt, ex, sx);
+                                sy = __ffma2_rn(wt, ey, sy);
+                                sz = __ffma2_rn(wt, ez, sz);
+                            }
+                            tx = __ffma2_rn(kk, dx, tx);
+                            ty = __ffma2_rn(kk, dy, ty);
+                            tz = __ffma2_rn(kk, dz, tz);
+                        }
+                        const float f = TC01 ? inv_h2 : -6.0f * inv_h2;
+                        w.gx[i] += fmaf(f, tx.x + tx.y, sx.x + sx.y);
+                        w.gy[i] += fmaf(f, ty.x + ty.y, sy.x + sy.y);
+                        w.gz[i] += fmaf(f, tz.x + tz.y, sz.x + sz.y);
+                    }
+                    __syncwarp();
+                }
+                for (uint32_t i = lane; i < fill; i += 32) {
+                    const float4 g = make_float4(w.gx[i], w.gy[i], w.gz[i], 0.f);
+                    if (g.x != 0.f || g.y != 0.f || g.z != 0.f) atomicAdd(a.gx + w.cj[i], g);
+                }
+                __syncwarp();
+                fill = 0;
+            };
+            int row = 0;
+            for (uint32_t cb = 0; cb < total; cb += 32) {
+                const uint32_t j = cb + lane;
+                bool keep = false;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                uint32_t idx = 0;
+                if (j < total) {
+                    while (row < 8 && w.rp[row + 1] <= j) ++row;
+                    idx = w.rb[row] + (j - w.rp[row]);
+                    q = __ldg(&a.sorted[idx]);
+                    keep = within(q, pl, ph, cr2);
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const uint32_t pos = fill + __popc(m & ((1u << lane) - 1u));
+                    w.cx[pos] = q.x;
+                    w.cy[pos] = q.y;
+                    w.cz[pos] = q.z;
+                    w.cj[pos] = idx;
+                }
+                fill += __popc(m);
+                if (fill > kBwdSeg - 32) tiles();
+            }
+            if (fill) tiles();
+        };
+        // the vertices of a row segment with dL/dphi != 0
+        auto with_gradient = [&](uint32_t bits, uint32_t r0) {
+            uint32_t kept = 0;
+            for (uint32_t m = bits, r = r0; m; m &= m - 1u, ++r)
+                if (r < nb && __ldg(a.gphi + r) != 0.f) kept |= m & (0u - m);
+            return kept;
+        };
+        list_band_vertices<kBwdVerts>(a.sc, a.band, lo, hi, w.vloc, w.vrank, lane, with_gradient, pass);
+        __syncwarp();
     }
 }
 
@@ -1677,26 +1681,14 @@ void launch_field_aniso_grouped(const KernelCtx& c, const AnisoFieldArgs& f, con
     ++g_launches;
 }
 
-bool launch_field_iso_backward_grouped(const KernelCtx& c, const BwdArgs& a, bool tc01, const Counters* ctr)
+void launch_field_iso_backward(const KernelCtx& c, const BwdArgs& a, bool tc01, const Counters* ctr)
 {
-    const uint32_t vcap = (a.ratio + 2) * (a.ratio + 2) * (a.ratio + 2);
-    const size_t smem = sizeof(float4) * vcap * (tc01 ? 1 : 2) + sizeof(float4) * 2 * ((vcap + 31) / 32) +
-                        sizeof(uint32_t) * vcap;
-    if (smem > 200 * 1024) return false;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_field_iso_backward_grouped<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        cudaFuncSetAttribute(k_field_iso_backward_grouped<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             200 * 1024);
-        configured = true;
-    }
     const uint64_t groups = (uint64_t)(a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
-        groups, std::max<uint64_t>(1, (uint64_t)c.num_sms * 8 / std::max(1, c.grid_div)));
-    if (tc01) k_field_iso_backward_grouped<true><<<grid, kBT, smem, c.stream>>>(a, vcap, ctr);
-    else k_field_iso_backward_grouped<false><<<grid, kBT, smem, c.stream>>>(a, vcap, ctr);
+        (groups * kSlabMax + kFWarps - 1) / kFWarps, std::max<uint64_t>(1, (uint64_t)c.num_sms * 12 / std::max(1, c.grid_div)));
+    if (tc01) k_field_iso_backward<true><<<grid, kFT, 0, c.stream>>>(a, ctr);
+    else k_field_iso_backward<false><<<grid, kFT, 0, c.stream>>>(a, ctr);
     ++g_launches;
-    return true;
 }
 
 void launch_field_iso_grouped(const KernelCtx& c, bool tc01, const IsoFieldArgs& f, const BandView& band, uint32_t ratio,

@@ -32,66 +32,105 @@ namespace {
 constexpr int kT = 256;
 
 // ---------------------------------------------------------------- MC
-__global__ void k_mc_backward(BwdArgs a, const Counters* ctr)
+// One cube per thread.  The mesh vertices' terms are summed per corner in
+// shared memory first, one atomic per touched corner, and the corners are looked
+// up as four rows of two x-neighbours (as in k_mc_classify).  The cube also
+// marks the window centres (keys) its corners fall in; the first mark of a key
+// appends it to the list the grouped adjoints take their groups from (a key
+// without a gradient vertex is found empty there).  Measured with the marking,
+// which was a pass over the band of its own: 500k-particle ZB05 frame (1.1M
+// cubes) 116 -> @MB@ us.
+// kRadius: dL/d(particle radius) of ZB05, minus the sum of dL/dphi over the
+// vertices with weight.  An edge's two terms nearly cancel, -(ga + gb) =
+// dL/df / (phi_b - phi_a), so that difference is summed, in FP64 (the sum of the
+// FP32 gradients was off by 1e-6 to 1e-5, differently in each run).
+template <bool kRadius>
+__global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* ctr, double* radius)
 {
+    __shared__ float s_val[8 * kT], s_g[8 * kT];  // [corner][thread]
+    float* val = s_val + threadIdx.x;
+    float* g = s_g + threadIdx.x;
     const uint32_t nq = min(ctr->n_valid, a.cap_valid);
     const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
+    const uint32_t kx = a.sp.res[0] + 1, ky = a.sp.res[1] + 1;
+    double rad = 0.0;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const uint32_t t = a.valid[q];
         const uint32_t info = a.mc[t];
         const uint32_t cs = info >> 8, nv = info & 0xFFu, base = a.vofs[t];
         const uint32_t v = a.sv[t];
-        uint32_t rk[8];
-        float val[8];
+        uint32_t r0[4];  // rank of each row's x corner; its x + 1 corner follows
+        uint32_t weighted = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const uint32_t id = v + (uint32_t)mc::cornerDx(i) + (uint32_t)mc::cornerDy(i) * rx +
-                                (uint32_t)mc::cornerDz(i) * rxy;
-            rk[i] = band_rank(a.band, id);
-            val[i] = __ldg(a.band.phi + rk[i]);
+        for (int r = 0; r < 4; ++r) {
+            const int dy = r & 1, dz = r >> 1;
+            const int i0 = dy ? (dz ? 2 : 3) : (dz ? 1 : 0);  // corner (0, dy, dz); (1, dy, dz) is i0 + 4
+            r0[r] = r == 0 ? t : band_rank(a.band, v + (uint32_t)dy * rx + (uint32_t)dz * rxy);
+            val[i0 * kT] = __ldg(a.band.phi + r0[r]);
+            val[(i0 + 4) * kT] = __ldg(a.band.phi + r0[r] + 1);
+            g[i0 * kT] = g[(i0 + 4) * kT] = 0.f;
+            if (kRadius) {
+                if (__ldg(&a.mv[r0[r]].w) > 0.f) weighted |= 1u << i0;
+                if (__ldg(&a.mv[r0[r] + 1].w) > 0.f) weighted |= 1u << (i0 + 4);
+            }
         }
         const uint64_t tri = a.tri[cs];
+        float cube = 0.f;
         for (uint32_t k = 0; k < nv; ++k) {
             const int e = (int)((tri >> (4u * k)) & 0xFu);
             const int ia = mc::edgeA(e), ib = mc::edgeB(e);
-            float fa = 0.f, fb = 0.f;
-            uint32_t ra = 0, rb = 0;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (i == ia) { fa = val[i]; ra = rk[i]; }
-                if (i == ib) { fb = val[i]; rb = rk[i]; }
-            }
+            const float fa = val[ia * kT], fb = val[ib * kT];
             const float d = fb - fa;
             if (d > -1.0e-7f && d < 1.0e-7f) continue;  // f = 0.5 is constant there
             // p_b - p_a is one grid spacing along the edge's axis
             const int ax = mc::cornerDx(ib) != mc::cornerDx(ia) ? 0 : (mc::cornerDy(ib) != mc::cornerDy(ia) ? 1 : 2);
             const int sgn = (ax == 0 ? mc::cornerDx(ib) - mc::cornerDx(ia)
                                      : ax == 1 ? mc::cornerDy(ib) - mc::cornerDy(ia) : mc::cornerDz(ib) - mc::cornerDz(ia));
-            const float gp = a.gmesh[3ull * (base + k) + ax];
+            const float gp = __ldg(a.gmesh + 3ull * (base + k) + ax);
             const float gf = gp * (float)sgn * a.sc.cs;
             const float inv = 1.0f / (d * d);
-            atomicAdd(a.gphi + ra, gf * (a.iso - fb) * inv);
-            atomicAdd(a.gphi + rb, -gf * (a.iso - fa) * inv);
+            const float ga = gf * (a.iso - fb) * inv, gb = -gf * (a.iso - fa) * inv;
+            g[ia * kT] += ga;
+            g[ib * kT] += gb;
+            if (kRadius) {
+                const bool wa = (weighted >> ia) & 1u, wb = (weighted >> ib) & 1u;
+                cube += wa && wb ? gf / d : (wa ? -ga : 0.f) + (wb ? -gb : 0.f);
+            }
         }
-    }
-}
-
-// keys (window centres) holding a band vertex with a non-zero field gradient;
-// the first vertex to mark a key appends it to the list the grouped
-// adjoints take their groups from
-__global__ void k_mark_keys(BwdArgs a, const Counters* ctr)
-{
-    const uint32_t nb = min(ctr->n_band, a.cap_band);
-    const uint32_t kx = a.sp.res[0] + 1, ky = a.sp.res[1] + 1;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x) {
-        if (a.gphi[t] == 0.f) continue;
+        if (kRadius) rad += (double)cube;
+        bool any = false;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int dy = r & 1, dz = r >> 1;
+            const int i0 = dy ? (dz ? 2 : 3) : (dz ? 1 : 0);
+            const float g0 = g[i0 * kT], g1 = g[(i0 + 4) * kT];
+            if (g0 != 0.f) atomicAdd(a.gphi + r0[r], g0);
+            if (g1 != 0.f) atomicAdd(a.gphi + r0[r] + 1, g1);
+            any = any || g0 != 0.f || g1 != 0.f;
+        }
+        if (!any) continue;
+        // the keys of the corners: the cell of each end per axis
         uint32_t x, y, z;
-        unlin3(a.sv[t], a.sc, x, y, z);
-        const int cx = cell1(vpos1(x, a.sc.min[0], a.sc.cs), a.sp.min[0], a.sp.cs);
-        const int cy = cell1(vpos1(y, a.sc.min[1], a.sc.cs), a.sp.min[1], a.sp.cs);
-        const int cz = cell1(vpos1(z, a.sc.min[2], a.sc.cs), a.sp.min[2], a.sp.cs);
-        const uint32_t key = ((uint32_t)cz * ky + cy) * kx + cx;
-        if (a.gkey[key] == 0u && atomicExch(&a.gkey[key], 1u) == 0u) a.glist[4 + atomicAdd(&a.glist[0], 1u)] = key;
+        unlin3(v, a.sc, x, y, z);
+        const uint32_t p[3] = {x, y, z};
+        uint32_t lo[3], hi[3];
+#pragma unroll
+        for (int ax = 0; ax < 3; ++ax) {
+            lo[ax] = (uint32_t)cell1(vpos1(p[ax], a.sc.min[ax], a.sc.cs), a.sp.min[ax], a.sp.cs);
+            hi[ax] = (uint32_t)cell1(vpos1(p[ax] + 1, a.sc.min[ax], a.sc.cs), a.sp.min[ax], a.sp.cs);
+        }
+        for (uint32_t cz = lo[2]; cz <= hi[2]; ++cz)
+            for (uint32_t cy = lo[1]; cy <= hi[1]; ++cy)
+                for (uint32_t cx = lo[0]; cx <= hi[0]; ++cx) {
+                    const uint32_t key = (cz * ky + cy) * kx + cx;
+                    if (a.gkey[key] == 0u && atomicExch(&a.gkey[key], 1u) == 0u)
+                        a.glist[4 + atomicAdd(&a.glist[0], 1u)] = key;
+                }
+    }
+    if (kRadius) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) rad += __shfl_xor_sync(0xffffffffu, rad, o);
+        if ((threadIdx.x & 31) == 0 && rad != 0.0) atomicAdd(radius, rad);
     }
 }
 
@@ -161,31 +200,6 @@ __device__ __forceinline__ void window_box(const BwdArgs& a, const int c[3], int
         const int s1 = __float2int_ru((p[k] + r - a.sc.min[k]) * inv);
         lo[k] = max(w0[k], s0);
         hi[k] = min(w1[k], s1);
-    }
-}
-
-// ---------------------------------------------------------------- ZB05 radius
-// dL/d(particle radius) of ZB05: -sum of dL/dphi over vertices with weight.
-// Summed in FP64: millions of terms of both signs, and FP32 partial sums added
-// in the order of the atomics were off by up to 2e-6 of the result, differently
-// in each run.  Bound by the read of dL/dphi; the weight sums are read only
-// where it is not zero (500k-particle frame: 50 -> 35 us).
-__global__ void k_radius_grad(BwdArgs a, const Counters* ctr, double* out)
-{
-    const uint32_t nb = min(ctr->n_band, a.cap_band);
-    double s = 0.0;
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x) {
-        const float g = a.gphi[t];
-        if (g != 0.f && a.mv[t].w > 0.f) s -= (double)g;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ double warps[kT / 32];
-    if ((threadIdx.x & 31) == 0) warps[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        for (int w = 1; w < kT / 32; ++w) s += warps[w];
-        if (s != 0.0) atomicAdd(out, s);
     }
 }
 
@@ -611,11 +625,9 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
 {
     const unsigned pb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_valid + kT - 1) / kT,
                                                                           (uint64_t)c.num_sms * 16));
-    k_mc_backward<<<pb, kT, 0, c.stream>>>(a, ctr);
-    const unsigned bb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_band + kT - 1) / kT,
-                                                                          (uint64_t)c.num_sms * 16));
-    k_mark_keys<<<bb, kT, 0, c.stream>>>(a, ctr);
-    g_launches += 2;
+    if (radius_grad_dev) k_mc_backward<true><<<pb, kT, 0, c.stream>>>(a, ctr, radius_grad_dev);
+    else k_mc_backward<false><<<pb, kT, 0, c.stream>>>(a, ctr, nullptr);
+    ++g_launches;
     if (method == FSR_METHOD_YU13) {
         AnisoBwdArgs fb{};
         fb.sp = a.sp;
@@ -646,10 +658,6 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
         g_launches += 3;
     } else {
         launch_field_iso_backward(c, a, method == FSR_METHOD_TC01, ctr);
-        if (radius_grad_dev) {
-            k_radius_grad<<<bb, kT, 0, c.stream>>>(a, ctr, radius_grad_dev);
-            ++g_launches;
-        }
     }
     k_unsort<<<nblk(a.n), kT, 0, c.stream>>>(a.gx, a.perm, a.n, out_grad_xyz);
     ++g_launches;

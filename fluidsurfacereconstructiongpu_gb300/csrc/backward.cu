@@ -39,7 +39,7 @@ constexpr int kT = 256;
 // appends it to the list the grouped adjoints take their groups from (a key
 // without a gradient vertex is found empty there).  Measured with the marking,
 // which was a pass over the band of its own: 500k-particle ZB05 frame (1.1M
-// cubes) 116 -> @MB@ us.
+// cubes, with the radius) 151 -> 116 us.
 // kRadius: dL/d(particle radius) of ZB05, minus the sum of dL/dphi over the
 // vertices with weight.  An edge's two terms nearly cancel, -(ga + gb) =
 // dL/df / (phi_b - phi_a), so that difference is summed, in FP64 (the sum of the

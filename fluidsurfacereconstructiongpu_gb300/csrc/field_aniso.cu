@@ -94,6 +94,16 @@ __device__ __forceinline__ uint32_t field_slabs(uint32_t ngroups)
 {
     return ngroups >= kSlabTarget ? 1u : min(kSlabMax, (kSlabTarget + ngroups - 1) / max(ngroups, 1u));
 }
+// The anisotropic field's items run 0.1 to 0.3 ms each, two to twelve per
+// resident warp, so their order and size decide how long the last ones keep a
+// few SMs busy (ncu, 150k particles: the busiest scheduler issued 1.6 times the
+// average).  The dense groups come first (GroupList); the last kSplitItems of
+// them, about one per resident warp, are split in two, each half taking every
+// second tile of the passes; the sparse groups fill the end.  A vertex's sum does
+// not depend on the split.  Measured (ms, all / last 7296 / last 3648 split, none
+// before): 256k particles 1.00 / 0.98 / 0.99, 1.38 before; 1M 2.34 / 2.27 / 2.19,
+// 2.53; 8M 9.73 / 9.37 / 9.33, 9.67; in four parts 1M 2.29.
+constexpr uint32_t kSplitItems = 4096;
 // Restricts the box [lo, hi) to slab `part` of S along z; false when empty.
 __device__ __forceinline__ bool slab_box(uint32_t part, uint32_t S, int lo[3], int hi[3])
 {
@@ -715,21 +725,35 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
     const int lane = threadIdx.x & 31;
     WarpSlice& w = slices[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap);
-    const uint32_t ngroups = ctr->n_groups;  // groups holding band vertices
+    const GroupList groups(a.glist, a.sp, ctr);
+    const uint32_t ngroups = groups.size();
     const uint32_t nslab = field_slabs(ngroups);
+    const uint32_t dense = groups.dense * nslab, sparse = groups.sparse * nslab;
+    const uint32_t split = min(dense, kSplitItems), whole = dense - split;
 
     for (;;) {
         uint32_t k = 0;
         if (lane == 0) k = atomicAdd(&ctr->work_field, 1u);
         k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= ngroups * nslab) break;
-        const uint32_t g = a.glist[k / nslab];
+        if (k >= whole + 2u * split + sparse) break;
+        // a work item takes every nsub-th tile of its slab's passes
+        uint32_t nsub = 1u, sub = 0u, slab = k;
+        if (k >= whole + 2u * split) {
+            slab = k - split;
+        } else if (k >= whole) {
+            nsub = 2u;
+            sub = (k - whole) & 1u;
+            slab = whole + ((k - whole) >> 1);
+        }
+        const uint32_t g = groups[slab / nslab];
         int c[3], lo[3], hi[3];
-        if (!group_box(g, a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi)) continue;
+        if (!group_box(g, a.sp, a.sc, ratio, c, lo, hi) || !slab_box(slab % nslab, nslab, lo, hi)) continue;
         bool tables = false;
         uint32_t total = 0;
 
         auto pass = [&](uint32_t nv) {
+            const uint32_t ntiles = (nv + 31) / 32;
+            if (sub >= ntiles) return;
             if (!tables) {
                 const float b0[3] = {vpos1(lo[0], a.sc.min[0], a.sc.cs), vpos1(lo[1], a.sc.min[1], a.sc.cs),
                                      vpos1(lo[2], a.sc.min[2], a.sc.cs)};
@@ -765,7 +789,6 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 if (lane == 0) w.use_mom = (sqrtf(y2max) + zmax) * 1.001f < 0.5f ? 1u : 0u;
                 __syncwarp();
             }
-            const uint32_t ntiles = (nv + 31) / 32;
             // the pass's box, brick order and tile boxes
             float4 pl, ph;
             pass_layout<false>(w.vloc, w.vrank, lo, a.sc, w.order, reinterpret_cast<uint32_t*>(&w.psum[0][0]), w.box, nv, lane, pl, ph);  // psum is zeroed below
@@ -777,7 +800,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
             // the sums live in the warp's shared slice, so that the tile loops
             // need not be unrolled (the kernel's code stays small enough for
             // the instruction cache)
-            for (uint32_t t = 0; t < ntiles; ++t) w.psum[t][lane] = w.usum[t][lane] = 0.f;
+            for (uint32_t t = sub; t < ntiles; t += nsub) w.psum[t][lane] = w.usum[t][lane] = 0.f;
             const uint32_t total_inv = w.total_inv;
             // involved candidates: staged with their G, culled per tile by
             // their support sphere, evaluated two at a time
@@ -800,51 +823,49 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 __syncwarp();
                 if (any) {
 #pragma unroll 1
-                    for (int t = 0; t < kPassTiles; ++t) {
-                        if ((uint32_t)t < ntiles) {
-                            const uint32_t m = __ballot_sync(0xffffffffu, keep && reaches(r0, w.box[2 * t], w.box[2 * t + 1]));
-                            if (m) {
-                                // the candidates that reach the tile, listed in
-                                // lane order two to a pair block
-                                if ((m >> lane) & 1u)
-                                    list_pair_record(reinterpret_cast<const float2*>(w.rec), lane,
-                                                     reinterpret_cast<float*>(w.lst), __popc(m & ((1u << lane) - 1u)));
-                                __syncwarp();
-                                const uint32_t v = 32 * t + lane;
-                                if (v < nv) {
-                                    const float4 vp = vert_pos(w.vloc[w.order[v]], lo, a.sc);
-                                    // the chunk's terms are summed on their own and
-                                    // then added to the vertex's sum with the
-                                    // rounding error of that addition (two-sum)
-                                    // kept in the second sum: with tens of
-                                    // thousands of neighbours one running FP32 sum
-                                    // drifts by more than 1e-5 of the field
-                                    float s = 0.f;
-                                    // one pair block per step, both candidates
-                                    // evaluated at once by packed operations; the
-                                    // terms of vertices inside the support enter
-                                    // the sum in list (lane) order
-                                    const float2 nvx = make_float2(-vp.x, -vp.x), nvy = make_float2(-vp.y, -vp.y),
-                                                 nvz = make_float2(-vp.z, -vp.z);
-                                    const uint32_t cnt = __popc(m);
-                                    // not unrolled: copies of the body crowd the
-                                    // instruction cache (measured: fetch stalls
-                                    // doubled and the 2^18-particle frame slowed)
+                    for (uint32_t t = sub; t < ntiles; t += nsub) {
+                        const uint32_t m = __ballot_sync(0xffffffffu, keep && reaches(r0, w.box[2 * t], w.box[2 * t + 1]));
+                        if (m) {
+                            // the candidates that reach the tile, listed in
+                            // lane order two to a pair block
+                            if ((m >> lane) & 1u)
+                                list_pair_record(reinterpret_cast<const float2*>(w.rec), lane,
+                                                 reinterpret_cast<float*>(w.lst), __popc(m & ((1u << lane) - 1u)));
+                            __syncwarp();
+                            const uint32_t v = 32 * t + lane;
+                            if (v < nv) {
+                                const float4 vp = vert_pos(w.vloc[w.order[v]], lo, a.sc);
+                                // the chunk's terms are summed on their own and
+                                // then added to the vertex's sum with the
+                                // rounding error of that addition (two-sum)
+                                // kept in the second sum: with tens of
+                                // thousands of neighbours one running FP32 sum
+                                // drifts by more than 1e-5 of the field
+                                float s = 0.f;
+                                // one pair block per step, both candidates
+                                // evaluated at once by packed operations; the
+                                // terms of vertices inside the support enter
+                                // the sum in list (lane) order
+                                const float2 nvx = make_float2(-vp.x, -vp.x), nvy = make_float2(-vp.y, -vp.y),
+                                             nvz = make_float2(-vp.z, -vp.z);
+                                const uint32_t cnt = __popc(m);
+                                // not unrolled: copies of the body crowd the
+                                // instruction cache (measured: fetch stalls
+                                // doubled and the 2^18-particle frame slowed)
 #pragma unroll 1
-                                    for (uint32_t j = 0; j < cnt; j += 2) {
-                                        float2 q2, u3, c;
-                                        pair_terms(w.lst + (j >> 1) * kPairF4, nvx, nvy, nvz, q2, u3, c);
-                                        if (q2.x < 1.0f) s = fmaf(c.x, u3.x, s);
-                                        if (j + 1 < cnt && q2.y < 1.0f) s = fmaf(c.y, u3.y, s);
-                                    }
-                                    const float a0 = w.psum[t][lane];
-                                    const float t0 = a0 + s;
-                                    const float bp = t0 - a0;
-                                    w.psum[t][lane] = t0;
-                                    w.usum[t][lane] += (a0 - (t0 - bp)) + (s - bp);
+                                for (uint32_t j = 0; j < cnt; j += 2) {
+                                    float2 q2, u3, c;
+                                    pair_terms(w.lst + (j >> 1) * kPairF4, nvx, nvy, nvz, q2, u3, c);
+                                    if (q2.x < 1.0f) s = fmaf(c.x, u3.x, s);
+                                    if (j + 1 < cnt && q2.y < 1.0f) s = fmaf(c.y, u3.y, s);
                                 }
-                                __syncwarp();
+                                const float a0 = w.psum[t][lane];
+                                const float t0 = a0 + s;
+                                const float bp = t0 - a0;
+                                w.psum[t][lane] = t0;
+                                w.usum[t][lane] += (a0 - (t0 - bp)) + (s - bp);
                             }
+                            __syncwarp();
                         }
                     }
                 }
@@ -861,9 +882,9 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 const float oy = 0.5f * (vpos1(lo[1], a.sc.min[1], a.sc.cs) + vpos1(hi[1] - 1, a.sc.min[1], a.sc.cs));
                 const float oz = 0.5f * (vpos1(lo[2], a.sc.min[2], a.sc.cs) + vpos1(hi[2] - 1, a.sc.min[2], a.sc.cs));
 #pragma unroll 1
-                for (int t = 0; t < kPassTiles; ++t) {
+                for (uint32_t t = sub; t < ntiles; t += nsub) {
                     const uint32_t v = 32 * t + lane;
-                    if ((uint32_t)t < ntiles && v < nv) {
+                    if (v < nv) {
                         const float4 vp = vert_pos(w.vloc[w.order[v]], lo, a.sc);
                         w.usum[t][lane] += unscaled_sum(w.mom, vp.x - ox, vp.y - oy, vp.z - oz);
                     }
@@ -881,9 +902,9 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 const uint32_t cnt = min(32u, total - cb);
                 __syncwarp();
 #pragma unroll 1
-                for (int t = 0; t < kPassTiles; ++t) {
+                for (uint32_t t = sub; t < ntiles; t += nsub) {
                     const uint32_t v = 32 * t + lane;
-                    if ((uint32_t)t < ntiles && v < nv) {
+                    if (v < nv) {
                         const float4 vp = vert_pos(w.vloc[w.order[v]], lo, a.sc);
                         float su = 0.f;  // the chunk's terms, as for the involved candidates
                         uint32_t k = 0;
@@ -909,8 +930,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 }
                 __syncwarp();
             }
-#pragma unroll
-            for (int t = 0; t < kPassTiles; ++t) {
+            for (uint32_t t = sub; t < ntiles; t += nsub) {
                 const uint32_t v = 32 * t + lane;
                 if (v < nv) {
                     const uint32_t rank = w.vrank[w.order[v]];
@@ -1008,7 +1028,8 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, Ba
     const int lane = threadIdx.x & 31;
     IsoSlice& w = slices[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap);
-    const uint32_t ngroups = ctr->n_groups;  // groups holding band vertices
+    const GroupList groups(a.glist, a.sp, ctr);
+    const uint32_t ngroups = groups.size();
     const uint32_t nslab = field_slabs(ngroups);
     const float cr = cull_radius(a.h, a.sp.cs), cr2 = cr * cr;
     constexpr int kSums = TC01 ? 1 : 4;
@@ -1018,7 +1039,7 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, Ba
         if (lane == 0) k = atomicAdd(&ctr->work_field, 1u);
         k = __shfl_sync(0xffffffffu, k, 0);
         if (k >= ngroups * nslab) break;
-        const uint32_t g = a.glist[k / nslab];
+        const uint32_t g = groups[k / nslab];
         int c[3], lo[3], hi[3];
         if (!group_box(g, a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi)) continue;
         const uint32_t total = window_rows(a.sp, a.ranges, c, w.rb, w.rp, lane);

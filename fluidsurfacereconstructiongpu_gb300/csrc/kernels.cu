@@ -379,6 +379,25 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
     }
 }
 
+// Whether a group's cell and its six neighbours hold enough particles for its
+// field to be a long work item (an isolated particle's groups: one or two).
+constexpr uint32_t kDenseGroup = 16;
+__device__ __forceinline__ bool dense_group(const GroupMark& gm, int cx, int cy, int cz)
+{
+    const int x1 = (int)gm.sp.res[0] - 1, y1 = (int)gm.sp.res[1] - 1, z1 = (int)gm.sp.res[2] - 1;
+    const int x = min(cx, x1), y = min(cy, y1), z = min(cz, z1);
+    const int p[7][3] = {{x, y, z}, {max(x - 1, 0), y, z}, {min(x + 1, x1), y, z}, {x, max(y - 1, 0), z},
+                         {x, min(y + 1, y1), z}, {x, y, max(z - 1, 0)}, {x, y, min(z + 1, z1)}};
+    uint2 r[7];
+#pragma unroll
+    for (int k = 0; k < 7; ++k) r[k] = __ldg(gm.ranges + lin3(p[k][0], p[k][1], p[k][2], gm.sp));
+    uint32_t sum = 0;
+#pragma unroll
+    for (int k = 0; k < 7; ++k)
+        if (r[k].x != kEmpty) sum += r[k].y - r[k].x;
+    return sum >= kDenseGroup;
+}
+
 // compactSurfaceVertex (cu:293-304) over the bitset: every set bit writes
 // its vertex id at its rank.  The band vertices also mark their window
 // groups (the spatial cell a vertex's FP32 position falls in, as the grouped
@@ -389,7 +408,7 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
 __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix,
                             uint32_t nwords, uint32_t* __restrict__ sv, uint32_t cap, GroupMark gm, Counters* ctr)
 {
-    const uint32_t kx = gm.sp.res[0] + 1, ky = gm.sp.res[1] + 1;
+    const uint32_t kx = gm.sp.res[0] + 1, ky = gm.sp.res[1] + 1, gend = kx * ky * (gm.sp.res[2] + 1);
     const uint32_t rx = gm.sc.res[0], rxy = gm.sc.res[0] * gm.sc.res[1];
     const uint32_t nb = ctr->n_band;
     if (blockIdx.x == 0 && threadIdx.x == 0 && nb > cap) {
@@ -425,7 +444,10 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
                     const uint32_t g = (uint32_t)cx + kx * ((uint32_t)cy + ky * (uint32_t)cz);
                     if (g != last) {
                         last = g;
-                        if (atomicExch(gm.gflag + g, 1u) == 0u) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
+                        if (atomicExch(gm.gflag + g, 1u) == 0u) {
+                            if (dense_group(gm, cx, cy, cz)) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
+                            else gm.glist[gend - 1u - atomicAdd(&ctr->n_sparse, 1u)] = g;
+                        }
                     }
                 }
             }

@@ -50,10 +50,11 @@ void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t*
 
 // The band list, and the list of the window groups (spatial cells of the
 // (res + 1)^3 grid the grouped field kernels walk) that hold band vertices:
-// glist[0 .. ctr->n_groups), in no particular order; gflag (one word per
-// group) must start at zero.
+// the ones among many particles from the list's front, the others from its end
+// (GroupList); gflag (one word per group) must start at zero.
 struct GroupMark {
     Grid sp, sc;
+    const uint2* ranges;
     uint32_t* gflag;
     uint32_t* glist;
 };
@@ -68,7 +69,7 @@ struct IsoFieldArgs {
     const uint32_t* sv;
     float* phi;
     float4* mv;  // optional (ZB05): per band vertex (mean - v, weight sum), kept for the backward pass
-    const uint32_t* glist;  // groups holding band vertices (ctr->n_groups of them)
+    const uint32_t* glist;  // groups holding band vertices (GroupList)
     float h, h2, inv_h2, rp;
     uint32_t cap;
 };
@@ -121,7 +122,7 @@ struct AnisoFieldArgs {
     const float* cell_rmax;
     const uint32_t* sv;
     float* phi;
-    const uint32_t* glist;  // groups holding band vertices (ctr->n_groups of them)
+    const uint32_t* glist;  // groups holding band vertices (GroupList)
     float sigma;
     uint32_t cap;
 };

@@ -364,7 +364,7 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     const uint64_t G = (uint64_t)(sp.res[0] + 1) * (sp.res[1] + 1) * (sp.res[2] + 1);
     CK(cudaMemsetAsync(h->gflag.ptr, 0, 4ull * G, st));
     launch_band_list(kc, bits, prefix, nwords, sv, h->cap_band,
-                     GroupMark{sp, sc, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
+                     GroupMark{sp, sc, ranges, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
     mark(4);
 
     // ---- field

@@ -191,19 +191,66 @@ __global__ void k_involved_cells(Grid sp, const uint8_t* __restrict__ occ, const
     invol[t] = v;
 }
 
+// Lanes whose windows span few cells together walk their union together
+// (below); a warp whose windows lie further apart (its particles run over the
+// end of a row of cells) is cut into such sets of lanes, each walked on its own.
+// The lanes of `left` that form a set with its first lane: together with that
+// lane's window theirs spans at most span + 1 cells per axis.
+constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
+__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
+{
+    const int lead = __ffs((int)left) - 1;
+    bool ok = (left >> lane) & 1u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
+        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
+    }
+    return __ballot_sync(0xffffffffu, ok || lane == lead);
+}
+
+// The gradient's factor of a neighbour at squared distance d2 (0 < d2 < h^2),
+// float(k x x) with x = 1 - d / h, and 1 / d, in the reference's roundings.
+template <bool kFast>
+__device__ __forceinline__ void colour_gradient(float d2, float h, float h_rcp, float tiny, double k_spiky, float khi,
+                                                float klo, float& grad, float& inv)
+{
+    float ratio;
+    if (kFast && d2 >= tiny) {
+        const float d = root_exact(d2);
+        inv = rcp_exact(d);
+        const float q = __fmul_rn(d, h_rcp);
+        ratio = fmaf(fmaf(-q, h, d), h_rcp, q);
+    } else {
+        const float d = __fsqrt_rn(d2);
+        inv = __fdiv_rn(1.0f, d);
+        ratio = div_exact(d, h, h_rcp);
+    }
+    // x = float(1.0 - (double)(d / h)): the double difference of 1 and a
+    // float is exact, so rounding it to float is the correctly rounded
+    // FP32 difference (no FP64 work needed)
+    const float x = __fsub_rn(1.0f, ratio);
+    // float(k x x) in double (cu:957); in FP32 when |k| is in range (khi > 0)
+    grad = khi > 0.f ? spiky_grad(x, khi, klo, k_spiky) : spiky_grad_double(x, k_spiky);
+}
+
 // extractionOfSurfaceParticlesUsingColorField (cu:909-971, wSpikyGrad
 // cuh:324-334).  The decision |grad c| > 3 depends on a sum, so the sum is
 // taken in the reference's order with the reference's roundings (FP64 where
-// the source promotes).
+// the source promotes).  Issue-bound on the pairs (16.5 of 32 threads per
+// instruction: each lane has its own neighbours); with the root, the division
+// and the reciprocal by FMA corrections, the gradient's rounding test halved and
+// the window test on sorted indices: 1M particles 1.68 -> 1.29 ms, 262k 0.49 ->
+// 0.40.
+template <bool kFast>
 __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restrict__ sorted, uint32_t n,
-                                                         const uint2* __restrict__ ranges,
-                                                         const uint32_t* __restrict__ skeys, Grid sp, float h,
-                                                         float h_rcp, float h_lt2, double k_spiky, float khi,
+                                                         const uint2* __restrict__ ranges, Grid sp, float h,
+                                                         float h_rcp, float h_lt2, float tiny, double k_spiky, float khi,
                                                          float klo, float mass, uint8_t* __restrict__ psurf)
 {
     __shared__ float4 s_q[kThreads];    // staged candidates, per warp
     __shared__ float s_mr[kThreads];    // their m / rho
-    __shared__ uint32_t s_cx[kThreads]; // their cells' x index
+    __shared__ uint32_t s_idx[kThreads]; // their sorted index
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = t < n;
     if (__all_sync(0xffffffffu, !active)) return;
@@ -217,14 +264,8 @@ __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restric
     // and +0 / -0 terms leave the sums, never -0, unchanged)
     auto add = [&](float4 q, float d2, float m_rho) {
         float rx = __fsub_rn(p.x, q.x), ry = __fsub_rn(p.y, q.y), rz = __fsub_rn(p.z, q.z);
-        const float d = __fsqrt_rn(d2);
-        // x = float(1.0 - (double)(d / h)): the double difference of 1 and a
-        // float is exact, so rounding it to float is the correctly rounded
-        // FP32 difference (no FP64 work needed)
-        const float x = __fsub_rn(1.0f, div_exact(d, h, h_rcp));
-        // float(k x x) in double (cu:957); in FP32 when |k| is in range (khi > 0)
-        const float grad = khi > 0.f ? spiky_grad(x, khi, klo, k_spiky) : spiky_grad_double(x, k_spiky);
-        const float inv = __fdiv_rn(1.0f, d);
+        float grad, inv;
+        colour_gradient<kFast>(d2, h, h_rcp, tiny, k_spiky, khi, klo, grad, inv);
         rx = __fmul_rn(rx, inv);
         ry = __fmul_rn(ry, inv);
         rz = __fmul_rn(rz, inv);
@@ -270,19 +311,16 @@ __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restric
         // each lane takes the staged particles of its own window in window
         // order (rows from the loop, x from the cell index)
         uint32_t in_window = 0, zeros = 0;
-        if (active)
-            for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
-                for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
-                    uint32_t b, e, c;
-                    row_range(w.lo[0], w.hi[0], yy, zz, b, e, c);
-                    in_window += c;
-                }
         const WarpBox box = warp_box(active, p.x, p.y, p.z, cull_radius(h, sp.cs));
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 const bool row_in = active && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1];
                 if (!__any_sync(0xffffffffu, row_in)) continue;
-                uint32_t beg, end, c;
+                // the run of sorted particles that the row has in this lane's window
+                uint32_t beg, end, own = 0, own_end = 0, len = 0;
+                if (row_in) row_range(w.lo[0], w.hi[0], yy, zz, own, own_end, len);
+                in_window += len;
+                uint32_t c;
                 row_range(ulo[0], uhi[0], yy, zz, beg, end, c);
                 for (uint32_t b = beg; b < end; b += 32) {
                     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -296,14 +334,13 @@ __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restric
                         const uint32_t slot = wb + __popc(mk & ((1u << lane) - 1u));
                         s_q[slot] = q;
                         s_mr[slot] = __fdiv_rn(mass, q.w);
-                        s_cx[slot] = __ldg(&skeys[b + lane]) % sp.res[0];
+                        s_idx[slot] = b + lane;
                     }
                     __syncwarp();
                     const uint32_t cnt = __popc(mk);
                     if (row_in)
                         for (uint32_t k = 0; k < cnt; ++k) {
-                            const int cx = (int)s_cx[wb + k];
-                            if (cx < w.lo[0] || cx > w.hi[0]) continue;
+                            if (s_idx[wb + k] - own >= len) continue;
                             const float4 q2 = s_q[wb + k];
                             const float d2 = dist2(q2);
                             if (!(d2 > 0.0f)) {
@@ -331,6 +368,170 @@ __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restric
             }
     }
     if (!active) return;
+    const bool s = nn < 25u || __fsqrt_rn(dot3_rn(sx, sy, sz)) > 3.0f;
+    psurf[t] = s ? 1 : 0;
+}
+
+// Small frames: four lanes per particle, eight particles per warp.  The
+// particles walk the union of their windows row by row; candidates within h of
+// their box are staged, each particle's lanes test 32 of them at a time (a bit
+// per hit), share its hits out evenly, write the three components of each hit's
+// term, and then add one component each in the candidates' order.
+constexpr int kColorThreads = 128;
+constexpr uint32_t kColorCap = 96;  // staged candidates of a warp
+constexpr uint32_t kHitRow = 36;    // pitch of a particle's 32 hits
+
+struct ColorSlice {
+    float x[kColorCap], y[kColorCap], z[kColorCap], mr[kColorCap];  // staged candidates, m / rho
+    uint32_t idx[kColorCap];                                      // their sorted index
+    uint32_t hit[8][kHitRow];                                     // per particle: its hits among 32 candidates
+    float term[8][3][kHitRow];                                    // and their terms
+};
+
+template <bool kFast>
+__global__ void __launch_bounds__(kColorThreads, 8) k_colorfield_quads(const float4* __restrict__ sorted, uint32_t n,
+                                                         const uint2* __restrict__ ranges, Grid sp, float h,
+                                                         float h_rcp, float h_lt2, float tiny, double k_spiky, float khi,
+                                                         float klo, float mass, uint8_t* __restrict__ psurf)
+{
+    __shared__ __align__(16) ColorSlice slices[kColorThreads / 32];
+    ColorSlice& S = slices[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31, part = lane >> 2;
+    const uint32_t sub = lane & 3u;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
+    const bool active = t < n;
+    if (__all_sync(0xffffffffu, !active)) return;
+    const float4 p = active ? sorted[t] : make_float4(0.f, 0.f, 0.f, 1.f);
+    const Window w = window(cell1(p.x, sp.min[0], sp.cs), cell1(p.y, sp.min[1], sp.cs),
+                            cell1(p.z, sp.min[2], sp.cs), 1, sp);
+    auto row_range = [&](int x0, int x1, int yy, int zz, uint32_t& beg, uint32_t& end) {
+        // the particles of a row of x-adjacent cells are contiguous in sorted order
+        const uint32_t c0 = lin3(x0, yy, zz, sp);
+        beg = kEmpty;
+        end = 0;
+        for (int xx = 0; xx <= x1 - x0; ++xx) {
+            const uint2 r = __ldg(&ranges[c0 + xx]);
+            if (r.x != kEmpty) {
+                beg = min(beg, r.x);
+                end = max(end, r.y);
+            }
+        }
+    };
+    auto dist2 = [&](uint32_t k) {
+        return dot3_rn(__fsub_rn(p.x, S.x[k]), __fsub_rn(p.y, S.y[k]), __fsub_rn(p.z, S.z[k]));
+    };
+    float sum = 0.f;         // component `sub` of the gradient (three lanes)
+    uint32_t zeros = 0;      // this lane's tested candidates at distance 0
+    uint32_t in_window = 0;  // particles of the window
+    // the staged candidates [0, fill); own, len: the run of sorted particles
+    // that the row has in this particle's window
+    auto take = [&](uint32_t fill, uint32_t own, uint32_t len) {
+        __syncwarp();
+        for (uint32_t b = 0; b < fill; b += 32) {
+            const uint32_t lim = min(32u, fill - b);
+            uint32_t m = 0;
+            for (uint32_t k = sub; k < lim; k += 4)
+                if (S.idx[b + k] - own < len) {
+                    const float d2 = dist2(b + k);
+                    if (!(d2 > 0.0f)) ++zeros;
+                    // (the gradient is 0 at d >= h, and +0 / -0 terms leave the
+                    // sums, never -0, unchanged)
+                    else if (d2 < h_lt2) m |= 1u << k;
+                }
+            const uint32_t mine = m;
+            m |= __shfl_xor_sync(0xffffffffu, m, 1);
+            m |= __shfl_xor_sync(0xffffffffu, m, 2);
+            const uint32_t cnt = __popc(m);
+            for (uint32_t r = mine; r; r &= r - 1u) {
+                const uint32_t k = __ffs(r) - 1;
+                S.hit[part][__popc(m & ((1u << k) - 1u))] = b + k;
+            }
+            __syncwarp();
+            for (uint32_t r = sub; r < cnt; r += 4) {
+                const uint32_t k = S.hit[part][r];
+                float rx = __fsub_rn(p.x, S.x[k]), ry = __fsub_rn(p.y, S.y[k]), rz = __fsub_rn(p.z, S.z[k]);
+                const float d2 = dot3_rn(rx, ry, rz);
+                float grad, inv;
+                colour_gradient<kFast>(d2, h, h_rcp, tiny, k_spiky, khi, klo, grad, inv);
+                const float coef = __fmul_rn(S.mr[k], grad);
+                S.term[part][0][r] = __fmul_rn(coef, __fmul_rn(rx, inv));
+                S.term[part][1][r] = __fmul_rn(coef, __fmul_rn(ry, inv));
+                S.term[part][2][r] = __fmul_rn(coef, __fmul_rn(rz, inv));
+            }
+            const uint32_t end = (cnt + 3u) & ~3u;
+            if (cnt + sub < end)
+                S.term[part][0][cnt + sub] = S.term[part][1][cnt + sub] = S.term[part][2][cnt + sub] = 0.f;
+            __syncwarp();
+            if (sub < 3u)
+                for (uint32_t r = 0; r < end; r += 4) {
+                    const float4 v = *reinterpret_cast<const float4*>(&S.term[part][sub][r]);
+                    sum = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sum, v.x), v.y), v.z), v.w);
+                }
+            __syncwarp();
+        }
+    };
+    // particles whose windows lie apart are walked in sets (window_mates)
+    const float reach = cull_radius(h, sp.cs);
+    uint32_t left = __ballot_sync(0xffffffffu, active);
+    while (left != 0u) {
+        const uint32_t set = window_mates(left, w, 4, lane);
+        left &= ~set;
+        const bool in_set = (set >> lane) & 1u;
+        int ulo[3], uhi[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            ulo[a] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)w.lo[a] : 0x7fffffffu);
+            uhi[a] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
+        }
+        // staging drops what lies beyond h of every particle of the set (zero
+        // gradient, and such a particle is at a distance > 0, counted through
+        // the cell counts)
+        const WarpBox box = warp_box(in_set, p.x, p.y, p.z, reach);
+        for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
+            for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
+                uint32_t beg, end, own = 0, len = 0, fill = 0;
+                if (in_set && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
+                    row_range(w.lo[0], w.hi[0], yy, zz, own, len);
+                    len = len > own ? len - own : 0u;
+                    in_window += len;
+                }
+                if (!__any_sync(0xffffffffu, len != 0u)) continue;
+                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                for (uint32_t base = beg; base < end; base += 32) {
+                    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                    bool keep = false;
+                    if (base + lane < end) {
+                        q = __ldg(&sorted[base + lane]);
+                        keep = box.keeps(q);
+                    }
+                    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        const uint32_t k = fill + __popc(m & ((1u << lane) - 1u));
+                        S.x[k] = q.x;
+                        S.y[k] = q.y;
+                        S.z[k] = q.z;
+                        S.mr[k] = __fdiv_rn(mass, q.w);
+                        S.idx[k] = base + lane;
+                    }
+                    fill += __popc(m);
+                    if (fill + 32u > kColorCap) {
+                        take(fill, own, len);
+                        fill = 0;
+                    }
+                }
+                if (fill) take(fill, own, len);
+            }
+    }
+    zeros += __shfl_xor_sync(0xffffffffu, zeros, 1);
+    zeros += __shfl_xor_sync(0xffffffffu, zeros, 2);
+    const int lead = lane & 28;
+    const float sx = __shfl_sync(0xffffffffu, sum, lead), sy = __shfl_sync(0xffffffffu, sum, lead + 1),
+                sz = __shfl_sync(0xffffffffu, sum, lead + 2);
+    if (!active || sub != 0u) return;
+    // nn: the particles of the window at a distance > 0 (the reference counts
+    // every particle of the 27 cells, cu:930-950) = the window's particles
+    // minus those at distance 0 (the particle itself and exact duplicates)
+    const uint32_t nn = in_window - zeros;
     const bool s = nn < 25u || __fsqrt_rn(dot3_rn(sx, sy, sz)) > 3.0f;
     psurf[t] = s ? 1 : 0;
 }
@@ -484,24 +685,6 @@ __device__ __forceinline__ uint32_t stage_in_box(const float4* __restrict__ src,
     const uint32_t m = __ballot_sync(0xffffffffu, keep);
     if (keep) sq[__popc(m & ((1u << lane) - 1u))] = q;
     return __popc(m);
-}
-
-// Lanes whose windows span few cells together walk their union together
-// (below); a warp whose windows lie further apart (its particles run over the
-// end of a row of cells) is cut into such sets of lanes, each walked on its own.
-// The lanes of `left` that form a set with its first lane: together with that
-// lane's window theirs spans at most span + 1 cells per axis.
-constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
-__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
-{
-    const int lead = __ffs((int)left) - 1;
-    bool ok = (left >> lane) & 1u;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
-        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
-    }
-    return __ballot_sync(0xffffffffu, ok || lane == lead);
 }
 
 // ------------------------------------------------------------ anisotropic path
@@ -1584,8 +1767,19 @@ void launch_colorfield(const KernelCtx& c, const float4* sorted, uint32_t n, con
         khi = (float)K;
         klo = (float)(K - (double)khi);
     }
-    k_colorfield<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, skeys, sp, h, 1.0f / h,
-                                                           sqrt_threshold(h, false), k, khi, klo, mass, psurf);
+    const bool fast = fast_radius(h);
+    // one lane per particle / four (ms): 4k particles 0.17 / 0.06, 20k 0.28 /
+    // 0.11, 60k 0.29 / 0.18, 100k 0.20-0.33 / 0.20-0.34, 262k 0.40 / 0.46, 1M
+    // 1.29 / 1.75
+    if (n < 98304u) {
+        const auto kernel = fast ? k_colorfield_quads<true> : k_colorfield_quads<false>;
+        kernel<<<blocks_for(4ull * n, kColorThreads), kColorThreads, 0, c.stream>>>(
+            sorted, n, ranges, sp, h, 1.0f / h, sqrt_threshold(h, false), tiny_d2(h), k, khi, klo, mass, psurf);
+    } else {
+        const auto kernel = fast ? k_colorfield<true> : k_colorfield<false>;
+        kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, h, 1.0f / h, sqrt_threshold(h, false),
+                                                             tiny_d2(h), k, khi, klo, mass, psurf);
+    }
     ++g_launches;
 }
 

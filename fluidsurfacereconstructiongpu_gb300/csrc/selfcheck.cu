@@ -29,7 +29,8 @@ __global__ void k_check_division(uint32_t hi_bits, float b, float rb, unsigned l
     if (local) atomicAdd(bad, local);
 }
 
-// Every float x in [2^-100, 2^100]: root_exact must equal __fsqrt_rn.  And
+// Every float x in [2^-100, 2^100]: root_exact must equal __fsqrt_rn and
+// rcp_exact __fdiv_rn(1, x).  And
 // every float d2 in [0, R^2]: the weight 1 - (d/R)^3 formed through
 // dist_over<true> must equal the one through __fsqrt_rn and __fdiv_rn.
 __global__ void k_check_root(uint32_t lo_bits, uint32_t hi_bits, float R, float rR, float tiny, uint32_t r2_bits,
@@ -40,7 +41,8 @@ __global__ void k_check_root(uint32_t lo_bits, uint32_t hi_bits, float R, float 
     unsigned long long local = 0;
     for (uint64_t i = lo_bits + start; i <= hi_bits; i += stride) {
         const float x = __uint_as_float((uint32_t)i);
-        if (__float_as_uint(fsr::root_exact(x)) != __float_as_uint(__fsqrt_rn(x))) {
+        if (__float_as_uint(fsr::root_exact(x)) != __float_as_uint(__fsqrt_rn(x)) ||
+            __float_as_uint(fsr::rcp_exact(x)) != __float_as_uint(__fdiv_rn(1.0f, x))) {
             ++local;
             atomicMin(first_bad, (unsigned long long)i);
         }

@@ -385,8 +385,9 @@ fsr_status fsr_check_division(float R, uint64_t* n_checked, uint64_t* n_mismatch
 /* Self-check of the square root the same kernels use (an FMA correction of an
  * approximate root, Markstein) for R in [2^-20, 2^40]: the root of every
  * float in [2^-100, 2^100] against the correctly rounded one, and the weight
- * 1 - (d/R)^3 of every squared distance in [0, R^2]; counts the results that
- * differ (0 expected). */
+ * 1 - (d/R)^3 of every squared distance in [0, R^2]; the colour field's
+ * reciprocal of every float in [2^-100, 2^100]; counts the results that differ
+ * (0 expected). */
 fsr_status fsr_check_root(float R, uint64_t* n_checked, uint64_t* n_mismatch);
 
 /* Self-check of the FP32 form of the colour field's gradient float(k x x)

@@ -58,3 +58,37 @@ def test_both_sides_of_the_lanes_per_particle_rule(n_side, settings):
     from fluidsurfacereconstructiongpu_gb300 import synthetic
     fr = synthetic.lattice_cube(n_side, 0.008, seed=n_side, jitter_frac=0.3, origin=(0.2, 0.2, 0.2))
     _run("yu13", fr, **SETTINGS[settings])
+
+
+@pytest.mark.parametrize("scale", [1.0, 1.4])
+@pytest.mark.parametrize("case", ["few1", "few40", "scattered", "slab", "duplicates", "below", "above"])
+def test_colour_field_walks(case, scale):
+    """The Akinci12 colour field by four lanes per particle and by one (97,336 /
+    103,823 particles); windows in one set, in several, scattered; particles on
+    top of one another (at distance 0, not counted).  The flags are exact (the
+    field is not looked at: isolated vertices' weights are ill-conditioned)."""
+    from fluidsurfacereconstructiongpu_gb300 import synthetic
+    if case.startswith("few"):
+        fr = _frame(int(case[3:]), 0.08, 0.3, 3)
+    elif case == "scattered":
+        fr = _frame(3000, 0.05, 0.95, 5)
+    elif case == "slab":
+        fr = _frame(4000, 0.04, 0.9, 6)
+        fr.pos[:, 0] = 0.5 + (fr.pos[:, 0] - 0.5) * 0.1
+    elif case == "duplicates":
+        fr = _frame(1500, 0.06, 0.3, 7)
+        fr.pos[1::3] = fr.pos[::3]
+    else:
+        fr = synthetic.lattice_cube(46 if case == "below" else 47, 0.008, seed=9, jitter_frac=0.3,
+                                    origin=(0.2, 0.2, 0.2))
+    import torch
+    from fluidsurfacereconstructiongpu_gb300 import api
+    from oracle import pipeline as P
+    rec = api.Reconstructor("akinci", 0, keep_intermediates=True, cell_size_scale=scale, grid_ratio=2)
+    rec.reconstruct(torch.from_numpy(fr.pos).cuda(), torch.from_numpy(fr.density).cuda(), api.header_of(fr))
+    params = P.FrameParams(method="akinci", h=fr.h, particle_radius=fr.particle_radius, mass=fr.mass,
+                           cell_scale=scale, ratio=2)
+    o32 = P.run_frame("oracle32", fr.pos, fr.density, fr.bbox_min, fr.bbox_max, params)
+    assert np.array_equal(rec.debug("surface_flags"), o32.sflag)
+    assert np.array_equal(rec.debug("band"), o32.sv)
+    rec.close()

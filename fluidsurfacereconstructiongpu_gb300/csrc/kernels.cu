@@ -98,6 +98,24 @@ __global__ void k_ranges_gather(const uint32_t* __restrict__ skeys, const uint32
     sorted[k] = make_float4(xyz[3ull * s], xyz[3ull * s + 1], xyz[3ull * s + 2], dens ? dens[s] : 0.0f);
 }
 
+// Lanes whose windows span few cells together walk their union together
+// (below); a warp whose windows lie further apart (its particles run over the
+// end of a row of cells) is cut into such sets of lanes, each walked on its own.
+// The lanes of `left` that form a set with its first lane: together with that
+// lane's window theirs spans at most span + 1 cells per axis.
+constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
+__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
+{
+    const int lead = __ffs((int)left) - 1;
+    bool ok = (left >> lane) & 1u;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
+        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
+    }
+    return __ballot_sync(0xffffffffu, ok || lane == lead);
+}
+
 // SPH density of each sorted particle, for frames without a density column
 // (the reference's .xyz files carry the simulator's densities and the
 // reference computes none): rho_i = m sigma / h^3 sum_j (1 - |x_i - x_j|^2 /
@@ -105,40 +123,119 @@ __global__ void k_ranges_gather(const uint32_t* __restrict__ skeys, const uint32
 // (64 pi) - the poly6 kernel with the normalisation of the reference's own
 // field kernel (anisotropicW, cuh:294-310, at G = I / h).  Each particle's
 // sum runs over its window's cells in order, so results are deterministic.
-__global__ void __launch_bounds__(kThreads) k_density(const float4* __restrict__ sorted, uint32_t n,
+//
+// A warp's lanes walk the union of their windows together (sets of lanes as in
+// window_mates), the candidates within h of their box staged in shared memory
+// and evaluated two at a time with packed FP32x2 operations; a candidate
+// outside a lane's window lies beyond h of it.  (Each lane on a window of its
+// own: 120k particles 0.25 -> 0.11 ms, 1M 0.92 -> 0.33.)
+constexpr int kDensityThreads = 128;
+constexpr uint32_t kDensityCap = 64;
+struct DensitySlice {
+    float x[kDensityCap], y[kDensityCap], z[kDensityCap];
+};
+__global__ void __launch_bounds__(kDensityThreads) k_density(const float4* __restrict__ sorted, uint32_t n,
                                                       const uint2* __restrict__ ranges, Grid sp, int ext, float h,
                                                       float h2, float inv_h2, float scale, float* __restrict__ rho)
 {
+    __shared__ __align__(16) DensitySlice slices[kDensityThreads / 32];
+    DensitySlice& S = slices[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n) return;
-    const float4 p = sorted[t];
+    const bool active = t < n;
+    if (__all_sync(0xffffffffu, !active)) return;
+    const float4 p = active ? sorted[t] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float reach = cull_radius(h, sp.cs);
     const Window w = narrow(window(cell1(p.x, sp.min[0], sp.cs), cell1(p.y, sp.min[1], sp.cs),
                                    cell1(p.z, sp.min[2], sp.cs), ext, sp),
-                            p.x, p.y, p.z, cull_radius(h, sp.cs), sp);
-    float sum = 0.f;
-    for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
-        for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
-            // the row's cells are contiguous in the sorted array
-            const uint32_t c0 = lin3(w.lo[0], yy, zz, sp);
-            uint32_t beg = kEmpty, end = 0;
-            for (int xx = 0; xx <= w.hi[0] - w.lo[0]; ++xx) {
-                const uint2 r = __ldg(&ranges[c0 + xx]);
-                if (r.x != kEmpty) {
-                    beg = min(beg, r.x);
-                    end = max(end, r.y);
-                }
-            }
-            for (uint32_t i = beg; i < end; ++i) {
-                const float4 q = __ldg(&sorted[i]);
-                const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
-                const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                if (d2 < h2) {
-                    const float u = 1.0f - d2 * inv_h2;
-                    sum = fmaf(u * u, u, sum);
-                }
+                            p.x, p.y, p.z, reach, sp);
+    auto row_range = [&](int x0, int x1, int yy, int zz, uint32_t& beg, uint32_t& end) {
+        // the row's cells are contiguous in the sorted array
+        const uint32_t c0 = lin3(x0, yy, zz, sp);
+        beg = kEmpty;
+        end = 0;
+        for (int xx = 0; xx <= x1 - x0; ++xx) {
+            const uint2 r = __ldg(&ranges[c0 + xx]);
+            if (r.x != kEmpty) {
+                beg = min(beg, r.x);
+                end = max(end, r.y);
             }
         }
-    rho[t] = scale * sum;
+    };
+    float sum = 0.f;
+    const float2 nx = make_float2(-p.x, -p.x), ny = make_float2(-p.y, -p.y), nz = make_float2(-p.z, -p.z);
+    const float2 ninv = make_float2(-inv_h2, -inv_h2), one = make_float2(1.0f, 1.0f);
+    auto take = [&](uint32_t fill, bool in_set) {
+        if ((fill & 1u) && lane == 0) S.x[fill] = S.y[fill] = S.z[fill] = 1.0e18f;  // beyond h of everything
+        __syncwarp();
+        if (in_set)
+#pragma unroll 4
+            for (uint32_t k = 0; k < fill; k += 2) {
+                const float2 dx = __fadd2_rn(*reinterpret_cast<const float2*>(S.x + k), nx);
+                const float2 dy = __fadd2_rn(*reinterpret_cast<const float2*>(S.y + k), ny);
+                const float2 dz = __fadd2_rn(*reinterpret_cast<const float2*>(S.z + k), nz);
+                const float2 d2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                const float2 u = __ffma2_rn(d2, ninv, one);
+                const float2 uu = __fmul2_rn(u, u);
+                if (d2.x < h2) sum = fmaf(uu.x, u.x, sum);
+                if (d2.y < h2) sum = fmaf(uu.y, u.y, sum);
+            }
+        __syncwarp();
+    };
+    uint32_t left = __ballot_sync(0xffffffffu, active);
+    for (int sets = 0; left != 0u && sets < kMaxSets; ++sets) {
+        const uint32_t set = window_mates(left, w, 2 * ext + 1, lane);
+        left &= ~set;
+        const bool in_set = (set >> lane) & 1u;
+        int ulo[3], uhi[3];
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+            ulo[a] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)w.lo[a] : 0x7fffffffu);
+            uhi[a] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
+        }
+        const WarpBox box = warp_box(in_set, p.x, p.y, p.z, reach);
+        uint32_t fill = 0;
+        for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
+            for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
+                uint32_t beg, end;
+                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                for (uint32_t base = beg; base < end; base += 32) {
+                    float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                    bool keep = false;
+                    if (base + lane < end) {
+                        q = __ldg(&sorted[base + lane]);
+                        keep = box.keeps(q);
+                    }
+                    const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                    if (keep) {
+                        const uint32_t k = fill + __popc(m & ((1u << lane) - 1u));
+                        S.x[k] = q.x;
+                        S.y[k] = q.y;
+                        S.z[k] = q.z;
+                    }
+                    fill += __popc(m);
+                    if (fill + 32u > kDensityCap) {
+                        take(fill, in_set);
+                        fill = 0;
+                    }
+                }
+            }
+        if (fill) take(fill, in_set);
+    }
+    if ((left >> lane) & 1u)
+        for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
+            for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
+                uint32_t beg, end;
+                row_range(w.lo[0], w.hi[0], yy, zz, beg, end);
+                for (uint32_t i = beg; i < end; ++i) {
+                    const float4 q = __ldg(&sorted[i]);
+                    const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+                    const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                    const float u = fmaf(-d2, inv_h2, 1.0f);
+                    if (d2 < h2) sum = fmaf(u * u, u, sum);
+                }
+            }
+    if (active) rho[t] = scale * sum;
 }
 
 __global__ void k_set_density(float4* __restrict__ sorted, const float* __restrict__ rho, uint32_t n)
@@ -189,24 +286,6 @@ __global__ void k_involved_cells(Grid sp, const uint8_t* __restrict__ occ, const
                     if (surf[lin3(xx, yy, zz, sp)]) { v = 1; break; }
     }
     invol[t] = v;
-}
-
-// Lanes whose windows span few cells together walk their union together
-// (below); a warp whose windows lie further apart (its particles run over the
-// end of a row of cells) is cut into such sets of lanes, each walked on its own.
-// The lanes of `left` that form a set with its first lane: together with that
-// lane's window theirs spans at most span + 1 cells per axis.
-constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
-__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
-{
-    const int lead = __ffs((int)left) - 1;
-    bool ok = (left >> lane) & 1u;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
-        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
-    }
-    return __ballot_sync(0xffffffffu, ok || lane == lead);
 }
 
 // The gradient's factor of a neighbour at squared distance d2 (0 < d2 < h^2),
@@ -1733,7 +1812,7 @@ void launch_density(const KernelCtx& c, float4* sorted, uint32_t n, const uint2*
     const float h2 = h * h;
     const float sigma = 315.0f / (64.0f * 3.1415926535898f);
     const float scale = mass * sigma / (h * h * h);
-    k_density<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, ext, h, h2, 1.0f / h2, scale, rho);
+    k_density<<<blocks_for(n, kDensityThreads), kDensityThreads, 0, c.stream>>>(sorted, n, ranges, sp, ext, h, h2, 1.0f / h2, scale, rho);
     k_set_density<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, rho, n);
     g_launches += 2;
 }

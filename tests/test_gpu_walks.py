@@ -92,3 +92,27 @@ def test_colour_field_walks(case, scale):
     assert np.array_equal(rec.debug("surface_flags"), o32.sflag)
     assert np.array_equal(rec.debug("band"), o32.sv)
     rec.close()
+
+
+@pytest.mark.parametrize("scale", [0.7, 1.0, 1.4])
+@pytest.mark.parametrize("case", ["few1", "few40", "scattered", "slab", "dense"])
+def test_density_walks(case, scale):
+    """Windows of one, several and many sets of lanes, cells smaller than h."""
+    import torch
+    from fluidsurfacereconstructiongpu_gb300 import api
+    from oracle.pipeline import sph_density
+    if case.startswith("few"):
+        fr = _frame(int(case[3:]), 0.08, 0.3, 3)
+    elif case == "dense":
+        fr = _frame(3001, 0.08, 0.3, 4)
+    else:
+        fr = _frame(3000, 0.05, 0.95, 5)
+        if case == "slab":
+            fr.pos[:, 0] = 0.5 + (fr.pos[:, 0] - 0.5) * 0.1
+    rec = api.Reconstructor("zb05", 0, compute_density=True, cell_size_scale=scale)
+    rec.reconstruct(torch.from_numpy(fr.pos).cuda(), None, api.header_of(fr))
+    got = rec.debug("density").astype(np.float64)
+    perm = rec.debug("perm")
+    rec.close()
+    want = sph_density(fr.pos, fr.h, fr.mass)[perm]
+    assert np.all(np.abs(got - want) <= 1e-5 * want)

@@ -69,6 +69,7 @@ struct fsr_handle {
     fsr::DevBuf rho;                     // computed densities, sorted order (FSR_FLAG_COMPUTE_DENSITY)
     // cell-sized
     fsr::DevBuf ranges, occ, surf, invol, cell_rmax;
+    fsr::DevBuf cell_first;              // counting sort: first place of each cell (cell_sort.cu)
     // vertex-sized
     fsr::DevBuf bits, prefix, scan_tmp;
     fsr::DevBuf gflag, glist;            // window groups holding band vertices: flags, list

@@ -62,15 +62,8 @@ __global__ void k_hash(const float* __restrict__ xyz, uint32_t n, Grid sp, uint3
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float p[3] = {xyz[3ull * i], xyz[3ull * i + 1], xyz[3ull * i + 2]};
-    int c[3];
-    bool ok = true;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const float q = __fdiv_rn(__fsub_rn(p[a], sp.min[a]), sp.cs);
-        ok = ok && (q > -1.0f) && (q < (float)sp.res[a]);  // NaN fails too
-        c[a] = ok ? __float2int_rz(q) : 0;
-    }
-    keys[i] = ok ? lin3((uint32_t)c[0], (uint32_t)c[1], (uint32_t)c[2], sp) : 0u;
+    bool ok;
+    keys[i] = cell_key(p, sp, ok);
     vals[i] = i;
     if (!ok) atomicAdd(&ctr->out_of_grid, 1u);
 }

@@ -153,6 +153,29 @@ struct AnisoBwdArgs {
 bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs& a, uint32_t ratio,
                                          const Counters* ctr);
 
+// Spatial hashing as a counting sort by cell (cell_sort.cu): sorted particles,
+// their keys and input numbers, cell ranges and occupancy (ranges must start
+// empty and occ at zero).
+struct CellSort {
+    const float* xyz;
+    const float* dens;   // may be null (densities computed later)
+    uint32_t n;
+    Grid sp;
+    uint32_t* keys;      // n words each: scratch
+    uint32_t* arrival;
+    uint32_t* grouped;
+    uint32_t* first;     // cells + 1 words
+    uint32_t* scan_tmp;  // scan_scratch_words(cells + 1)
+    uint32_t* big;       // n / 1024 words
+    float4* sorted;
+    uint32_t* skeys;     // may be `arrival`
+    uint32_t* perm;
+    uint2* ranges;
+    uint8_t* occ;
+};
+bool cell_sort_wanted(uint64_t cells, uint32_t n);
+cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ctr);
+
 struct McArgs {
     Grid sc;
     BandView band;

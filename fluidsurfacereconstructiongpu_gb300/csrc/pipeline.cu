@@ -187,7 +187,7 @@ fsr_handle::~fsr_handle()
 
 std::vector<DevBuf*> fsr_handle::all_buffers()
 {
-    return {&in_xyz, &in_den,  &keys0,  &vals0,  &keys1, &vals1,  &radix_tmp, &sorted, &ranges,  &occ,
+    return {&in_xyz, &in_den,  &keys0,  &vals0,  &keys1, &vals1,  &radix_tmp, &sorted, &ranges,  &cell_first, &occ,
             &surf,   &invol, &cell_rmax,   &psurf,  &bits,   &prefix, &gflag, &glist, &scan_tmp, &sv,       &phi,    &mc,      &vofs,
             &valid,   &mean,   &mean32, &smoothed, &grec, &qrec, &covrec, &mesh_pos, &mesh_nrm, &wkey, &wslot, &wrank, &widx, &wpos, &wnrm, &wtable_keys, &wtable_first, &rho, &pflags, &ctr, &mv, &gphi, &gkey, &gklist, &gsmooth, &gG, &gmean, &gx, &gscalar, &tri, &in_xyz_b, &in_den_b, &mesh_pos_b, &mesh_nrm_b};
 }
@@ -238,6 +238,8 @@ fsr_status frame_buffers(fsr_handle* h, const FramePlan& fp)
     CK(h->radix_tmp.ensure(4ull * radix_scratch_words((uint32_t)nn)));
     CK(h->sorted.ensure(16ull * nn));
     CK(h->ranges.ensure(8ull * C));
+    const bool by_cell = cell_sort_wanted(C, fp.n);
+    if (by_cell) CK(h->cell_first.ensure(4ull * (C + 1)));
     CK(h->occ.ensure(C));
     CK(h->surf.ensure(C));
     CK(h->bits.ensure(4ull * nwords + 4));
@@ -266,6 +268,7 @@ fsr_status frame_buffers(fsr_handle* h, const FramePlan& fp)
     }
     const bool weld = (p.flags & FSR_FLAG_WELD) != 0;
     uint64_t scan_words = std::max<uint64_t>(scan_scratch_words(nwords), mc_offsets_scratch_words(h->cap_band));
+    if (by_cell) scan_words = std::max<uint64_t>(scan_words, scan_scratch_words(C + 1));
     if (weld) {
         scan_words = std::max<uint64_t>(scan_words, scan_scratch_words(h->cap_mesh));
         const uint64_t cm = h->cap_mesh, ts = weld_table_size(h->cap_mesh);
@@ -323,20 +326,45 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     uint32_t* v0 = (uint32_t*)h->vals0.ptr;
     uint32_t* k1 = (uint32_t*)h->keys1.ptr;
     uint32_t* v1 = (uint32_t*)h->vals1.ptr;
-    launch_hash(kc, d_xyz, n, sp, k0, v0, ctr);
-    cudaError_t se = cudaSuccess;
-    const int which = radix_sort_pairs(k0, v0, k1, v1, n, bits_for(C), (uint32_t*)h->radix_tmp.ptr, st, &se);
-    if (se != cudaSuccess) return cuda_fail(h, se, "radix sort");
-    const uint32_t* skeys = which ? k1 : k0;
-    const uint32_t* perm = which ? v1 : v0;
-    h->perm_ptr = perm;
-    h->skeys_ptr = skeys;
-    mark(0);
     float4* sorted = (float4*)h->sorted.ptr;
     uint2* ranges = (uint2*)h->ranges.ptr;
     uint8_t* occ = (uint8_t*)h->occ.ptr;
     const bool own_density = (p.flags & FSR_FLAG_COMPUTE_DENSITY) != 0;
-    launch_ranges_gather(kc, skeys, perm, n, d_xyz, own_density ? nullptr : d_den, sorted, ranges, occ);
+    const float* density = own_density ? nullptr : d_den;
+    const uint32_t *skeys, *perm;
+    if (cell_sort_wanted(C, n)) {
+        CellSort cs{};
+        cs.xyz = d_xyz;
+        cs.dens = density;
+        cs.n = n;
+        cs.sp = sp;
+        cs.keys = k0;
+        cs.arrival = v0;
+        cs.grouped = k1;
+        cs.first = (uint32_t*)h->cell_first.ptr;
+        cs.scan_tmp = (uint32_t*)h->scan_tmp.ptr;
+        cs.big = (uint32_t*)h->radix_tmp.ptr;
+        cs.sorted = sorted;
+        cs.skeys = v0;
+        cs.perm = v1;
+        cs.ranges = ranges;
+        cs.occ = occ;
+        CK(launch_cell_sort(kc, cs, ctr));
+        skeys = v0;
+        perm = v1;
+        mark(0);
+    } else {
+        launch_hash(kc, d_xyz, n, sp, k0, v0, ctr);
+        cudaError_t se = cudaSuccess;
+        const int which = radix_sort_pairs(k0, v0, k1, v1, n, bits_for(C), (uint32_t*)h->radix_tmp.ptr, st, &se);
+        if (se != cudaSuccess) return cuda_fail(h, se, "radix sort");
+        skeys = which ? k1 : k0;
+        perm = which ? v1 : v0;
+        mark(0);
+        launch_ranges_gather(kc, skeys, perm, n, d_xyz, density, sorted, ranges, occ);
+    }
+    h->perm_ptr = perm;
+    h->skeys_ptr = skeys;
     if (own_density)
         launch_density(kc, sorted, n, ranges, sp, hdr.kernel_radius, hdr.particle_mass, (float*)h->rho.ptr);
     mark(1);

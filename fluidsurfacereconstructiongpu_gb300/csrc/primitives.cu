@@ -285,6 +285,15 @@ cudaError_t scan_u32(const uint32_t* in, uint32_t* out, uint32_t n_host, const u
     return cudaGetLastError();
 }
 
+cudaError_t scan_counts(uint32_t* counts, uint32_t n, uint32_t* scratch, cudaStream_t stream)
+{
+    if (n > kSingleMax)
+        return scan_u32(counts, counts, n, nullptr, n, nullptr, ScanInput::kValue, scratch, stream);
+    k_scan_single<<<1, kSingleThreads, 0, stream>>>(counts, counts, n);
+    ++g_launches;
+    return cudaGetLastError();
+}
+
 size_t radix_scratch_words(uint32_t n)
 {
     const uint64_t ntiles = ((uint64_t)n + kRadixTile - 1) / kRadixTile;
@@ -308,13 +317,8 @@ int radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uin
         uint32_t* kout = cur ? k0 : k1;
         uint32_t* vout = cur ? v0 : v1;
         k_radix_hist<<<ntiles, kRadixThreads, 0, stream>>>(kin, n, shift, ntiles, hist);
-        if (nhist <= kSingleMax) {
-            k_scan_single<<<1, kSingleThreads, 0, stream>>>(hist, hist, nhist);
-            ++g_launches;
-        } else {
-            cudaError_t e = scan_u32(hist, hist, nhist, nullptr, nhist, nullptr, ScanInput::kValue, scan_tmp, stream);
-            if (e != cudaSuccess) { *err = e; return cur; }
-        }
+        const cudaError_t e = scan_counts(hist, nhist, scan_tmp, stream);
+        if (e != cudaSuccess) { *err = e; return cur; }
         k_radix_scatter<<<ntiles, kRadixThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, ntiles, hist);
         g_launches += 2;
         cur ^= 1;

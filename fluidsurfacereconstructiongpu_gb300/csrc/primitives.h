@@ -58,6 +58,10 @@ cudaError_t scan_u32(const uint32_t* in, uint32_t* out, uint32_t n_host, const u
                      uint32_t n_max, uint32_t* total, ScanInput mode, uint32_t* scratch,
                      cudaStream_t stream);
 
+// Exclusive scan of n counts in place: one block for short arrays.  scratch:
+// scan_scratch_words(n).
+cudaError_t scan_counts(uint32_t* counts, uint32_t n, uint32_t* scratch, cudaStream_t stream);
+
 // Stable sort of (key, value) pairs by the low `key_bits` bits of key.  The
 // sorted pairs end in (k0, v0) when the function returns 0 and in (k1, v1)
 // when it returns 1 (ping-pong buffers).  scratch: radix_scratch_words(n).

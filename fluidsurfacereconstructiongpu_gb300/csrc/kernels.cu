@@ -1544,7 +1544,7 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
                                                                const uint32_t* tile_prefix, uint32_t ntiles_max)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
-    __shared__ uint32_t tile_vals[kScanTile];
+    __shared__ uint32_t tile_vals[kScanTilePadded];
     const uint32_t n = min(ctr->n_band, a.cap_band);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -1553,7 +1553,7 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint32_t j = k * kScanThreads + threadIdx.x;
             const uint64_t i = base + j;
-            tile_vals[j] = i < n ? mc_pair(__ldg(a.mc + i)) : 0u;
+            tile_vals[scan_slot(j)] = i < n ? mc_pair(__ldg(a.mc + i)) : 0u;
         }
         __syncthreads();
         // each thread owns kScanItems consecutive positions
@@ -1561,7 +1561,7 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
         uint32_t s = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kScanItems; ++k) {
-            local[k] = tile_vals[threadIdx.x * kScanItems + k];
+            local[k] = tile_vals[scan_slot(threadIdx.x * kScanItems + k)];
             s += local[k];
         }
         const uint32_t incl = block_inclusive_scan(s, warp_sums);
@@ -1574,7 +1574,7 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
                 const uint32_t q = pq + (run >> 16);
                 if (q < a.cap_valid) a.valid[q] = (uint32_t)t;
             }
-            tile_vals[threadIdx.x * kScanItems + k] = pv + (run & 0xFFFFu);
+            tile_vals[scan_slot(threadIdx.x * kScanItems + k)] = pv + (run & 0xFFFFu);
             run += local[k];
         }
         __syncthreads();
@@ -1582,7 +1582,7 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint32_t j = k * kScanThreads + threadIdx.x;
             const uint64_t i = base + j;
-            if (i < n) a.vofs[i] = tile_vals[j];
+            if (i < n) a.vofs[i] = tile_vals[scan_slot(j)];
         }
         __syncthreads();
     }

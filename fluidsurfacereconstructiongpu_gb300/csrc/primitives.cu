@@ -74,7 +74,7 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
                                                             uint32_t n_max, const uint32_t* tile_prefix)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
-    __shared__ uint32_t tile_vals[kScanTile];
+    __shared__ uint32_t tile_vals[kScanTilePadded];
     const uint32_t n = count_of(n_host, n_dev, n_max);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint32_t j = k * kScanThreads + threadIdx.x;
             const uint64_t i = base + j;
-            tile_vals[j] = i < n ? scan_load<M>(in, (uint32_t)i) : 0u;
+            tile_vals[scan_slot(j)] = i < n ? scan_load<M>(in, (uint32_t)i) : 0u;
         }
         __syncthreads();
         // each thread owns kScanItems consecutive elements
@@ -92,14 +92,14 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
         uint32_t s = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kScanItems; ++k) {
-            local[k] = tile_vals[threadIdx.x * kScanItems + k];
+            local[k] = tile_vals[scan_slot(threadIdx.x * kScanItems + k)];
             s += local[k];
         }
         const uint32_t incl = block_inclusive_scan(s, warp_sums);
         uint32_t run = tile_prefix[tile] + incl - s;
 #pragma unroll
         for (uint32_t k = 0; k < kScanItems; ++k) {
-            tile_vals[threadIdx.x * kScanItems + k] = run;
+            tile_vals[scan_slot(threadIdx.x * kScanItems + k)] = run;
             run += local[k];
         }
         __syncthreads();
@@ -107,7 +107,7 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint32_t j = k * kScanThreads + threadIdx.x;
             const uint64_t i = base + j;
-            if (i < n) out[i] = tile_vals[j];
+            if (i < n) out[i] = tile_vals[scan_slot(j)];
         }
         __syncthreads();
     }

@@ -7,8 +7,7 @@
 //   3. particle numbers to first place + arrival number: grouped by cell, in
 //      no particular order inside one;
 //   4. each particle's place inside its cell is the number of smaller particle
-//      numbers there (the sort is stable), which also gathers the particles and
-//      writes the cell ranges.
+//      numbers there (the sort is stable), which also gathers the particles.
 // Five launches with a scan in one block (seven with a tiled scan) instead of
 // the radix sort's two or three passes of three to five; the radix sort stays
 // for sparse grids, whose scan would cost more than its passes.  Cells of more
@@ -49,11 +48,25 @@ __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp,
     if (there) arrival[i] = base + (uint32_t)__popc(peers & ((1u << lane) - 1u));
 }
 
+// Step 3, and per cell what the frame starts from: its range and occupancy, and
+// zeros in the cell-sized arrays of later stages (a memset each before).
 __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ arrival,
-                        const uint32_t* __restrict__ first, uint32_t n, uint32_t* __restrict__ grouped)
+                        const uint32_t* __restrict__ first, uint32_t n, uint32_t cells, uint32_t groups,
+                        uint32_t* __restrict__ grouped, uint2* __restrict__ ranges, uint8_t* __restrict__ occ,
+                        float* __restrict__ cell_rmax, uint32_t* __restrict__ gflag, uint32_t* __restrict__ big,
+                        Counters* ctr)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
+    const uint32_t stride = gridDim.x * blockDim.x, start = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t i = start; i < n; i += stride) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
+    for (uint32_t c = start; c < groups; c += stride) {
+        gflag[c] = 0u;
+        if (c >= cells) continue;
+        const uint32_t s = __ldg(first + c), e = __ldg(first + c + 1);
+        ranges[c] = e > s ? make_uint2(s, e) : make_uint2(kEmpty, kEmpty);
+        occ[c] = e > s ? 1 : 0;
+        if (cell_rmax) cell_rmax[c] = 0.f;
+        if (e - s > kBigCell) big[atomicAdd(&ctr->n_big_cells, 1u)] = c;
+    }
 }
 
 struct CellSortOut {
@@ -72,21 +85,14 @@ struct CellSortOut {
 };
 
 __global__ void k_cell_rank(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ first,
-                            const uint32_t* __restrict__ grouped, uint32_t n, CellSortOut out,
-                            uint2* __restrict__ ranges, uint8_t* __restrict__ occ, uint32_t* __restrict__ big,
-                            Counters* ctr)
+                            const uint32_t* __restrict__ grouped, uint32_t n, CellSortOut out)
 {
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t i = grouped[k];
     const uint32_t key = __ldg(keys + i);
     const uint32_t s = __ldg(first + key), e = __ldg(first + key + 1);
-    if (k == s) {
-        ranges[key] = make_uint2(s, e);
-        occ[key] = 1;
-        if (e - s > kBigCell) big[atomicAdd(&ctr->n_big_cells, 1u)] = key;
-    }
-    if (e - s > kBigCell) return;
+    if (e - s > kBigCell) return;  // k_big_cells
     uint32_t r = 0;
     uint32_t j = s;
     for (; j + 4 <= e; j += 4) {
@@ -180,15 +186,18 @@ cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ct
     const int threads = 256;
     const unsigned blocks = (unsigned)((a.n + threads - 1) / threads);
     const uint32_t cells = a.sp.res[0] * a.sp.res[1] * a.sp.res[2];
-    cudaError_t e = cudaMemsetAsync(a.first, 0, 4ull * (cells + 1ull), c.stream);
-    if (e != cudaSuccess) return e;
+    const uint32_t groups = (a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
+    cudaError_t e = cudaSuccess;
     k_hash_count<<<blocks, threads, 0, c.stream>>>(a.xyz, a.n, a.sp, a.keys, a.arrival, a.first, ctr);
     ++g_launches;
     // in place: first[cells] becomes the number of particles
     if ((e = scan_counts(a.first, cells + 1u, a.scan_tmp, c.stream)) != cudaSuccess) return e;
-    k_group<<<blocks, threads, 0, c.stream>>>(a.keys, a.arrival, a.first, a.n, a.grouped);
+    const unsigned gblocks = (unsigned)std::min<uint64_t>(((uint64_t)std::max(a.n, groups) + threads - 1) / threads,
+                                                          (uint64_t)std::max(1, c.num_sms) * 32);
+    k_group<<<gblocks, threads, 0, c.stream>>>(a.keys, a.arrival, a.first, a.n, cells, groups, a.grouped, a.ranges, a.occ,
+                                               a.cell_rmax, a.gflag, a.big, ctr);
     const CellSortOut out{a.xyz, a.dens, a.sorted, a.skeys, a.perm};
-    k_cell_rank<<<blocks, threads, 0, c.stream>>>(a.keys, a.first, a.grouped, a.n, out, a.ranges, a.occ, a.big, ctr);
+    k_cell_rank<<<blocks, threads, 0, c.stream>>>(a.keys, a.first, a.grouped, a.n, out);
     g_launches += 2;
     if (a.n > kBigCell) {
         const uint32_t most = a.n / kBigCell;

@@ -69,7 +69,6 @@ struct fsr_handle {
     fsr::DevBuf rho;                     // computed densities, sorted order (FSR_FLAG_COMPUTE_DENSITY)
     // cell-sized
     fsr::DevBuf ranges, occ, surf, invol, cell_rmax;
-    fsr::DevBuf cell_first;              // counting sort: first place of each cell (cell_sort.cu)
     // vertex-sized
     fsr::DevBuf bits, prefix, scan_tmp;
     fsr::DevBuf gflag, glist;            // window groups holding band vertices: flags, list
@@ -79,7 +78,7 @@ struct fsr_handle {
     fsr::DevBuf mesh_pos, mesh_nrm;
     // vertex welding (FSR_FLAG_WELD)
     fsr::DevBuf wkey, wslot, wrank, widx, wpos, wnrm, wtable_keys, wtable_first;
-    fsr::DevBuf ctr;
+    fsr::DevBuf ctr;                     // Counters, then the counting sort's cell counts (cell_sort.cu)
     // backward pass
     fsr::DevBuf mv;                      // ZB05/Akinci12: per band vertex (mean - v, weight sum)
     fsr::DevBuf gphi, gkey, gklist, gsmooth, gG, gmean, gx, gscalar, tri;  // gklist: keys with gradient vertices

@@ -154,8 +154,8 @@ bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs&
                                          const Counters* ctr);
 
 // Spatial hashing as a counting sort by cell (cell_sort.cu): sorted particles,
-// their keys and input numbers, cell ranges and occupancy (ranges must start
-// empty and occ at zero).
+// their keys and input numbers, cell ranges and occupancy; zeroes cell_rmax (may
+// be null) and gflag ((res + 1)^3 words).  first must start at zero.
 struct CellSort {
     const float* xyz;
     const float* dens;   // may be null (densities computed later)
@@ -172,6 +172,8 @@ struct CellSort {
     uint32_t* perm;
     uint2* ranges;
     uint8_t* occ;
+    float* cell_rmax;
+    uint32_t* gflag;
 };
 bool cell_sort_wanted(uint64_t cells, uint32_t n);
 cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ctr);

@@ -187,7 +187,7 @@ fsr_handle::~fsr_handle()
 
 std::vector<DevBuf*> fsr_handle::all_buffers()
 {
-    return {&in_xyz, &in_den,  &keys0,  &vals0,  &keys1, &vals1,  &radix_tmp, &sorted, &ranges,  &cell_first, &occ,
+    return {&in_xyz, &in_den,  &keys0,  &vals0,  &keys1, &vals1,  &radix_tmp, &sorted, &ranges,  &occ,
             &surf,   &invol, &cell_rmax,   &psurf,  &bits,   &prefix, &gflag, &glist, &scan_tmp, &sv,       &phi,    &mc,      &vofs,
             &valid,   &mean,   &mean32, &smoothed, &grec, &qrec, &covrec, &mesh_pos, &mesh_nrm, &wkey, &wslot, &wrank, &widx, &wpos, &wnrm, &wtable_keys, &wtable_first, &rho, &pflags, &ctr, &mv, &gphi, &gkey, &gklist, &gsmooth, &gG, &gmean, &gx, &gscalar, &tri, &in_xyz_b, &in_den_b, &mesh_pos_b, &mesh_nrm_b};
 }
@@ -239,7 +239,6 @@ fsr_status frame_buffers(fsr_handle* h, const FramePlan& fp)
     CK(h->sorted.ensure(16ull * nn));
     CK(h->ranges.ensure(8ull * C));
     const bool by_cell = cell_sort_wanted(C, fp.n);
-    if (by_cell) CK(h->cell_first.ensure(4ull * (C + 1)));
     CK(h->occ.ensure(C));
     CK(h->surf.ensure(C));
     CK(h->bits.ensure(4ull * nwords + 4));
@@ -247,7 +246,8 @@ fsr_status frame_buffers(fsr_handle* h, const FramePlan& fp)
     const uint64_t G = (uint64_t)(fp.sp.res[0] + 1) * (fp.sp.res[1] + 1) * (fp.sp.res[2] + 1);
     CK(h->gflag.ensure(4ull * G));
     CK(h->glist.ensure(4ull * G));
-    CK(h->ctr.ensure(sizeof(Counters)));
+    // the counting sort's cell counts follow the counters: one memset for both
+    CK(h->ctr.ensure(sizeof(Counters) + (by_cell ? 4ull * (C + 1) : 0)));
     if (yu13) {
         CK(h->invol.ensure(C));
         CK(h->cell_rmax.ensure(4ull * C));
@@ -315,11 +315,16 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     if (timing) cudaEventRecord(h->ev_start, st);
 
     h->launches_mark = g_launches;
-    CK(cudaMemsetAsync(ctr, 0, sizeof(Counters), st));
-    CK(cudaMemsetAsync(h->ranges.ptr, 0xFF, 8ull * C, st));
-    CK(cudaMemsetAsync(h->occ.ptr, 0, C, st));
+    const bool by_cell = cell_sort_wanted(C, n);
+    const uint64_t G = (uint64_t)(sp.res[0] + 1) * (sp.res[1] + 1) * (sp.res[2] + 1);
+    CK(cudaMemsetAsync(ctr, 0, sizeof(Counters) + (by_cell ? 4ull * (C + 1) : 0), st));
     CK(cudaMemsetAsync(h->bits.ptr, 0, 4ull * nwords + 4, st));
-    if (yu13) CK(cudaMemsetAsync(h->cell_rmax.ptr, 0, 4ull * C, st));
+    if (!by_cell) {
+        CK(cudaMemsetAsync(h->ranges.ptr, 0xFF, 8ull * C, st));
+        CK(cudaMemsetAsync(h->occ.ptr, 0, C, st));
+        CK(cudaMemsetAsync(h->gflag.ptr, 0, 4ull * G, st));
+        if (yu13) CK(cudaMemsetAsync(h->cell_rmax.ptr, 0, 4ull * C, st));
+    }
 
     // ---- spatial hashing (ReconstructorGPU.cpp:292-313)
     uint32_t* k0 = (uint32_t*)h->keys0.ptr;
@@ -332,7 +337,7 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     const bool own_density = (p.flags & FSR_FLAG_COMPUTE_DENSITY) != 0;
     const float* density = own_density ? nullptr : d_den;
     const uint32_t *skeys, *perm;
-    if (cell_sort_wanted(C, n)) {
+    if (by_cell) {
         CellSort cs{};
         cs.xyz = d_xyz;
         cs.dens = density;
@@ -341,7 +346,7 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
         cs.keys = k0;
         cs.arrival = v0;
         cs.grouped = k1;
-        cs.first = (uint32_t*)h->cell_first.ptr;
+        cs.first = (uint32_t*)(ctr + 1);
         cs.scan_tmp = (uint32_t*)h->scan_tmp.ptr;
         cs.big = (uint32_t*)h->radix_tmp.ptr;
         cs.sorted = sorted;
@@ -349,6 +354,8 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
         cs.perm = v1;
         cs.ranges = ranges;
         cs.occ = occ;
+        cs.cell_rmax = yu13 ? (float*)h->cell_rmax.ptr : nullptr;
+        cs.gflag = (uint32_t*)h->gflag.ptr;
         CK(launch_cell_sort(kc, cs, ctr));
         skeys = v0;
         perm = v1;
@@ -389,8 +396,6 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     CK(scan_u32(bits, prefix, nwords, nullptr, nwords, &ctr->n_band, ScanInput::kPopcount,
                 (uint32_t*)h->scan_tmp.ptr, st));
     uint32_t* sv = (uint32_t*)h->sv.ptr;
-    const uint64_t G = (uint64_t)(sp.res[0] + 1) * (sp.res[1] + 1) * (sp.res[2] + 1);
-    CK(cudaMemsetAsync(h->gflag.ptr, 0, 4ull * G, st));
     launch_band_list(kc, bits, prefix, nwords, sv, h->cap_band,
                      GroupMark{sp, sc, ranges, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
     mark(4);

@@ -1404,15 +1404,33 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
 }
 
 // ------------------------------------------------------------ marching cubes
-__device__ __forceinline__ float field_at(const McArgs& a, int x, int y, int z)
+// The field at the grid positions (x0 + k, y, z), k = 0 .. N - 1 (N <= 4): 0
+// outside the grid (getValue, cuh:410-416), the fill value off the band.  x0 >= -1
+// and x0 + 1 inside.  One or two bitset words and one prefix give the four
+// memberships and ranks; the values of neighbouring band vertices follow one
+// another.
+template <int N>
+__device__ __forceinline__ void field_row(const McArgs& a, int x0, int y, int z, float out[N])
 {
-    if (x < 0 || y < 0 || z < 0 || (uint32_t)x >= a.sc.res[0] || (uint32_t)y >= a.sc.res[1] ||
-        (uint32_t)z >= a.sc.res[2])
-        return 0.f;  // getValue outside the grid (cuh:410-416)
-    const uint32_t v = lin3(x, y, z, a.sc);
-    if (!band_has(a.band, v)) return a.fill;
-    const uint32_t r = band_rank(a.band, v);
-    return r < a.cap_band ? __ldg(a.band.phi + r) : a.fill;  // r >= cap only in a frame that is re-run
+#pragma unroll
+    for (int k = 0; k < N; ++k) out[k] = 0.f;
+    if ((uint32_t)y >= a.sc.res[1] || (uint32_t)z >= a.sc.res[2]) return;
+    // the first position inside the grid, and the number of those before it
+    const int skip = x0 < 0 ? 1 : 0;
+    const uint32_t v = lin3((uint32_t)(x0 + skip), (uint32_t)y, (uint32_t)z, a.sc);
+    const uint32_t w = v >> 5, sh = v & 31u;
+    const uint32_t lo = __ldg(a.band.bits + w), hi = sh + N > 32u ? __ldg(a.band.bits + w + 1) : 0u;
+    const uint32_t f = (uint32_t)((((uint64_t)hi << 32) | lo) >> sh) << skip;
+    uint32_t r = __ldg(a.band.prefix + w) + __popc(lo & ((1u << sh) - 1u));
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        if (x0 + k < 0 || x0 + k >= (int)a.sc.res[0]) continue;
+        out[k] = a.fill;
+        if ((f >> k) & 1u) {
+            if (r < a.cap_band) out[k] = __ldg(a.band.phi + r);  // r >= cap only in a frame that is re-run
+            ++r;
+        }
+    }
 }
 
 // detectValidSurfaceCubes (cu:328-364): a band vertex as cube origin is
@@ -1653,18 +1671,31 @@ __global__ void __launch_bounds__(kThreads) k_mc_generate(McArgs a, const Counte
             X = (int)x;
             Y = (int)y;
             Z = (int)z;
-            // the 32 positions, each looked up once (the corner-by-corner form
-            // reads 56)
+            // the 32 positions as 12 rows of x-neighbours (one by one, each
+            // with its bitset word, prefix and value in turn, the lookups took
+            // longest: 188 -> 119 us for 2.5M triangles, 97 -> 54 us for 0.93M)
+#pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const int cy = r & 1, cz = r >> 1;
-                for (int xi = 0; xi < 4; ++xi) S(r * 4 + xi) = field_at(a, X + xi - 1, Y + cy, Z + cz);
-            }
-            for (int k = 0; k < 4; ++k) {
-                const int c0 = k & 1, c1 = k >> 1;
-                S(16 + k * 2) = field_at(a, X + c0, Y - 1, Z + c1);      // (cx, cz) = (c0, c1)
-                S(16 + k * 2 + 1) = field_at(a, X + c0, Y + 2, Z + c1);
-                S(24 + k * 2) = field_at(a, X + c0, Y + c1, Z - 1);      // (cx, cy) = (c0, c1)
-                S(24 + k * 2 + 1) = field_at(a, X + c0, Y + c1, Z + 2);
+                float row[4], below[2], above[2];
+                field_row<4>(a, X - 1, Y + cy, Z + cz, row);
+                // (cy as the row's x-independent place: rows at y = -1, 2 for z = cz,
+                // rows at z = -1, 2 for y = cz)
+                if (cy == 0) {
+                    field_row<2>(a, X, Y - 1, Z + cz, below);
+                    field_row<2>(a, X, Y + 2, Z + cz, above);
+                } else {
+                    field_row<2>(a, X, Y + cz, Z - 1, below);
+                    field_row<2>(a, X, Y + cz, Z + 2, above);
+                }
+#pragma unroll
+                for (int xi = 0; xi < 4; ++xi) S(r * 4 + xi) = row[xi];
+                const int base = cy == 0 ? 16 : 24;
+#pragma unroll
+                for (int cx = 0; cx < 2; ++cx) {  // slots of (cx, cz) or (cx, cy = cz)
+                    S(base + (cz * 2 + cx) * 2) = below[cx];
+                    S(base + (cz * 2 + cx) * 2 + 1) = above[cx];
+                }
             }
             // corner normals, f(p - e) - f(p + e) per axis, over their slots
             for (int i = 0; i < 8; ++i) {

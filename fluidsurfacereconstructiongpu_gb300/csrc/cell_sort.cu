@@ -25,6 +25,7 @@ namespace fsr {
 namespace {
 
 constexpr uint32_t kBigCell = 1024;
+constexpr uint32_t kDenseParticles = 16;
 
 __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp, uint32_t* __restrict__ keys,
                              uint32_t* __restrict__ arrival, uint32_t* __restrict__ count, Counters* ctr)
@@ -50,16 +51,29 @@ __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp,
 
 // Step 3, and per cell what the frame starts from: its range and occupancy, and
 // zeros in the cell-sized arrays of later stages (a memset each before).
+// gflag: kDenseGroup for the window groups whose cell and its six neighbours hold
+// enough particles for their field to be a long work item (an isolated
+// particle's groups: one or two), which k_band_list lists first.
 __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ arrival,
-                        const uint32_t* __restrict__ first, uint32_t n, uint32_t cells, uint32_t groups,
+                        const uint32_t* __restrict__ first, uint32_t n, Grid sp, uint32_t cells, uint32_t groups,
                         uint32_t* __restrict__ grouped, uint2* __restrict__ ranges, uint8_t* __restrict__ occ,
                         float* __restrict__ cell_rmax, uint32_t* __restrict__ gflag, uint32_t* __restrict__ big,
                         Counters* ctr)
 {
     const uint32_t stride = gridDim.x * blockDim.x, start = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t i = start; i < n; i += stride) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
+    const uint32_t kx = sp.res[0] + 1, ky = sp.res[1] + 1;
     for (uint32_t c = start; c < groups; c += stride) {
-        gflag[c] = 0u;
+        // (groups beyond the last cell of an axis count as that cell)
+        const uint32_t gz = c / (kx * ky), gy = (c - gz * kx * ky) / kx, gx = c - (gz * ky + gy) * kx;
+        const uint32_t x1 = sp.res[0] - 1, y1 = sp.res[1] - 1, z1 = sp.res[2] - 1;
+        const uint32_t x = min(gx, x1), y = min(gy, y1), z = min(gz, z1);
+        const uint32_t row = lin3(0, y, z, sp);
+        auto held = [&](uint32_t a, uint32_t b) { return __ldg(first + b + 1) - __ldg(first + a); };
+        uint32_t sum = held(row + (x ? x - 1 : 0u), row + min(x + 1, x1));  // x-neighbours are one run
+        auto one = [&](uint32_t yy, uint32_t zz) { const uint32_t k = lin3(x, yy, zz, sp); return held(k, k); };
+        sum += one(y ? y - 1 : 0u, z) + one(min(y + 1, y1), z) + one(y, z ? z - 1 : 0u) + one(y, min(z + 1, z1));
+        gflag[c] = sum >= kDenseParticles ? kDenseGroup : 0u;
         if (c >= cells) continue;
         const uint32_t s = __ldg(first + c), e = __ldg(first + c + 1);
         ranges[c] = e > s ? make_uint2(s, e) : make_uint2(kEmpty, kEmpty);
@@ -194,7 +208,7 @@ cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ct
     if ((e = scan_counts(a.first, cells + 1u, a.scan_tmp, c.stream)) != cudaSuccess) return e;
     const unsigned gblocks = (unsigned)std::min<uint64_t>(((uint64_t)std::max(a.n, groups) + threads - 1) / threads,
                                                           (uint64_t)std::max(1, c.num_sms) * 32);
-    k_group<<<gblocks, threads, 0, c.stream>>>(a.keys, a.arrival, a.first, a.n, cells, groups, a.grouped, a.ranges, a.occ,
+    k_group<<<gblocks, threads, 0, c.stream>>>(a.keys, a.arrival, a.first, a.n, a.sp, cells, groups, a.grouped, a.ranges, a.occ,
                                                a.cell_rmax, a.gflag, a.big, ctr);
     const CellSortOut out{a.xyz, a.dens, a.sorted, a.skeys, a.perm};
     k_cell_rank<<<blocks, threads, 0, c.stream>>>(a.keys, a.first, a.grouped, a.n, out);

@@ -616,59 +616,48 @@ __global__ void __launch_bounds__(kColorThreads, 8) k_colorfield_quads(const flo
 // kernel tests the squared distance against thr2 = sqrt_threshold(thr,
 // true), the same decision without the square root.
 // Each (y,z) row of at most 6 vertices is OR-ed into the bitset with at most
-// two atomics.
+// two atomics.  kLanes lanes share a particle's z planes: one lane walks 49 rows,
+// which is most of a tiny frame's kernel; more lanes only cost flag reads in a
+// large one.  kCheck: the words are read first (a stale value only costs an
+// atomic), since on a surface a vertex is stamped by seven particles or, on
+// coarse grids, by fifty; Akinci12's flags on a fine grid keep every other warp
+// full of surface particles, and there the reads cost more than the atomics.
+// Measured (us; one lane without the check / 8 or 2 lanes with it): 1.5k particles
+// on the coarse grid 25 / 10, 32k 27 / 17, 300k on the coarse grid 87 / 49, 1M 102
+// / 93, 8M 453 / 336; Akinci12 262k on the fine grid, 2 lanes: 74 without, 88 with.
+template <int kLanes, bool kCheck>
 __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* __restrict__ skeys,
                              const uint8_t* __restrict__ surf, const uint8_t* __restrict__ psurf, uint32_t n,
                              Grid sc, float thr2, uint32_t* __restrict__ bits, Counters* ctr)
 {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = i / kLanes, plane = i % kLanes;
     bool is_s = false;
     if (t < n) is_s = psurf ? psurf[t] != 0 : surf[skeys[t]] != 0;
-    warp_count(&ctr->n_surface, is_s);
+    warp_count(&ctr->n_surface, is_s && plane == 0);
     if (!is_s) return;
     const float4 p = sorted[t];
     const Window w = window(cell1(p.x, sc.min[0], sc.cs), cell1(p.y, sc.min[1], sc.cs),
                             cell1(p.z, sc.min[2], sc.cs), 3, sc);
     if (w.hi[0] <= w.lo[0]) return;
-    for (int z = w.lo[2]; z <= w.hi[2]; ++z) {
+    for (int z = w.lo[2] + (int)plane; z <= w.hi[2]; z += kLanes) {
         const float dz = __fsub_rn(vpos1(z, sc.min[2], sc.cs), p.z);
         for (int y = w.lo[1]; y <= w.hi[1]; ++y) {
             const float dy = __fsub_rn(vpos1(y, sc.min[1], sc.cs), p.y);
             const uint32_t v0 = lin3(w.lo[0], y, z, sc);
             const uint32_t word0 = v0 >> 5;
-            uint32_t m0 = 0, m1 = 0;
+            uint64_t m = 0;
             for (int x = w.lo[0]; x < w.hi[0]; ++x) {
                 const float dx = __fsub_rn(vpos1(x, sc.min[0], sc.cs), p.x);
                 // sqrt_rn(d2) <= thr  <=>  d2 < thr2 (the smallest float whose root exceeds thr)
-                if (dot3_rn(dx, dy, dz) < thr2) {
-                    const uint32_t v = v0 + (uint32_t)(x - w.lo[0]);
-                    if ((v >> 5) == word0) m0 |= 1u << (v & 31u);
-                    else m1 |= 1u << (v & 31u);
-                }
+                if (dot3_rn(dx, dy, dz) < thr2) m |= 1ull << (x - w.lo[0]);
             }
-            if (m0) atomicOr(bits + word0, m0);
-            if (m1) atomicOr(bits + word0 + 1, m1);
+            m <<= v0 & 31u;
+            const uint32_t m0 = (uint32_t)m, m1 = (uint32_t)(m >> 32);
+            if (m0 && (!kCheck || (m0 & ~bits[word0]))) atomicOr(bits + word0, m0);
+            if (m1 && (!kCheck || (m1 & ~bits[word0 + 1]))) atomicOr(bits + word0 + 1, m1);
         }
     }
-}
-
-// Whether a group's cell and its six neighbours hold enough particles for its
-// field to be a long work item (an isolated particle's groups: one or two).
-constexpr uint32_t kDenseGroup = 16;
-__device__ __forceinline__ bool dense_group(const GroupMark& gm, int cx, int cy, int cz)
-{
-    const int x1 = (int)gm.sp.res[0] - 1, y1 = (int)gm.sp.res[1] - 1, z1 = (int)gm.sp.res[2] - 1;
-    const int x = min(cx, x1), y = min(cy, y1), z = min(cz, z1);
-    const int p[7][3] = {{x, y, z}, {max(x - 1, 0), y, z}, {min(x + 1, x1), y, z}, {x, max(y - 1, 0), z},
-                         {x, min(y + 1, y1), z}, {x, y, max(z - 1, 0)}, {x, y, min(z + 1, z1)}};
-    uint2 r[7];
-#pragma unroll
-    for (int k = 0; k < 7; ++k) r[k] = __ldg(gm.ranges + lin3(p[k][0], p[k][1], p[k][2], gm.sp));
-    uint32_t sum = 0;
-#pragma unroll
-    for (int k = 0; k < 7; ++k)
-        if (r[k].x != kEmpty) sum += r[k].y - r[k].x;
-    return sum >= kDenseGroup;
 }
 
 // compactSurfaceVertex (cu:293-304) over the bitset: every set bit writes
@@ -688,17 +677,22 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
         atomicOr(&ctr->overflow, 1u);
         atomicMax(&ctr->need_band, nb);
     }
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += gridDim.x * blockDim.x) {
-        const uint32_t w0 = bits[i];
-        if (w0 == 0u) continue;
-        uint32_t w = w0;
-        uint32_t r = prefix[i];
-        while (w) {
-            const uint32_t b = __ffs(w) - 1;
-            w &= w - 1;
-            if (r < cap) sv[r] = (i << 5) | b;
-            ++r;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < nwords; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + lane;
+        const uint32_t w0 = i < nwords ? bits[i] : 0u;
+        const uint32_t r0 = w0 ? prefix[i] : 0u;
+        // the warp writes its words' vertices one word at a time, a lane per bit:
+        // consecutive lanes on consecutive entries (each lane writing its own
+        // word's, 4 bytes at a time, and each new group's cells read here: 1M ZB05
+        // frame, scan and list, 119 -> 90 us, 8M 382 -> 257)
+        for (uint32_t m = __ballot_sync(0xffffffffu, w0 != 0u); m; m &= m - 1u) {
+            const int src = __ffs((int)m) - 1;
+            const uint32_t w = __shfl_sync(0xffffffffu, w0, src), r = __shfl_sync(0xffffffffu, r0, src);
+            const uint32_t at = r + (uint32_t)__popc(w & ((1u << lane) - 1u));
+            if (((w >> lane) & 1u) && at < cap) sv[at] = ((i0 + (uint32_t)src) << 5) | lane;
         }
+        if (w0 == 0u) continue;
         // the word's rows: bits [s, e) lie in row (y, z) from column x on
         const uint32_t v0 = i << 5;
         uint32_t z = v0 / rxy, y = (v0 - z * rxy) / rx, x = v0 - z * rxy - y * rx;
@@ -717,10 +711,11 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
                     const uint32_t g = (uint32_t)cx + kx * ((uint32_t)cy + ky * (uint32_t)cz);
                     if (g != last) {
                         last = g;
-                        if (atomicExch(gm.gflag + g, 1u) == 0u) {
-                            if (dense_group(gm, cx, cy, cz)) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
-                            else gm.glist[gend - 1u - atomicAdd(&ctr->n_sparse, 1u)] = g;
-                        }
+                        if (gm.gflag[g] & kMarkedGroup) continue;  // (a stale value only costs the atomic)
+                        const uint32_t flag = atomicOr(gm.gflag + g, kMarkedGroup);
+                        if (flag & kMarkedGroup) continue;
+                        if (flag & kDenseGroup) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
+                        else gm.glist[gend - 1u - atomicAdd(&ctr->n_sparse, 1u)] = g;
                     }
                 }
             }
@@ -1887,12 +1882,18 @@ void launch_colorfield(const KernelCtx& c, const float4* sorted, uint32_t n, con
 }
 
 void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t* skeys, const uint8_t* surf,
-                       const uint8_t* psurf, uint32_t n, const Grid& sc, float thr, uint32_t* bits,
+                       const uint8_t* psurf, uint32_t n, const Grid& sp, const Grid& sc, float thr, uint32_t* bits,
                        Counters* ctr)
 {
     if (!n) return;
-    k_band_stamp<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, skeys, surf, psurf, n, sc,
-                                                           sqrt_threshold(thr, true), bits, ctr);
+    const float thr2 = sqrt_threshold(thr, true);
+    auto launch = [&](auto kernel, uint32_t lanes) {
+        kernel<<<blocks_for((uint64_t)n * lanes, bs(c)), bs(c), 0, c.stream>>>(sorted, skeys, surf, psurf, n, sc, thr2, bits,
+                                                                            ctr);
+    };
+    const bool check = !psurf || sc.cs * 4.0f >= sp.cs;  // (at most 4 grid vertices per cell)
+    if (n < 65536u) launch(check ? k_band_stamp<8, true> : k_band_stamp<8, false>, 8);
+    else launch(check ? k_band_stamp<2, true> : k_band_stamp<2, false>, 2);
     ++g_launches;
 }
 

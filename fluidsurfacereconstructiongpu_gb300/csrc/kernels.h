@@ -45,16 +45,16 @@ void launch_colorfield(const KernelCtx& c, const float4* sorted, uint32_t n, con
 // Band stamp around surface particles.  Surface particles are those with
 // psurf[i] != 0 when psurf is given, else those whose cell has surf != 0.
 void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t* skeys,
-                       const uint8_t* surf, const uint8_t* psurf, uint32_t n, const Grid& sc,
+                       const uint8_t* surf, const uint8_t* psurf, uint32_t n, const Grid& sp, const Grid& sc,
                        float thr, uint32_t* bits, Counters* ctr);
 
 // The band list, and the list of the window groups (spatial cells of the
 // (res + 1)^3 grid the grouped field kernels walk) that hold band vertices:
 // the ones among many particles from the list's front, the others from its end
-// (GroupList); gflag (one word per group) must start at zero.
+// (GroupList).  gflag: one word per group, starting at 0 or kDenseGroup (cell_sort.cu).
+constexpr uint32_t kMarkedGroup = 1u, kDenseGroup = 2u;
 struct GroupMark {
     Grid sp, sc;
-    const uint2* ranges;
     uint32_t* gflag;
     uint32_t* glist;
 };

@@ -391,13 +391,13 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     // ---- narrow band
     uint32_t* bits = (uint32_t*)h->bits.ptr;
     uint32_t* prefix = (uint32_t*)h->prefix.ptr;
-    launch_band_stamp(kc, sorted, skeys, surf, psurf, n, sc, band_threshold(h_r), bits, ctr);
+    launch_band_stamp(kc, sorted, skeys, surf, psurf, n, sp, sc, band_threshold(h_r), bits, ctr);
     mark(3);
     CK(scan_u32(bits, prefix, nwords, nullptr, nwords, &ctr->n_band, ScanInput::kPopcount,
                 (uint32_t*)h->scan_tmp.ptr, st));
     uint32_t* sv = (uint32_t*)h->sv.ptr;
     launch_band_list(kc, bits, prefix, nwords, sv, h->cap_band,
-                     GroupMark{sp, sc, ranges, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
+                     GroupMark{sp, sc, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
     mark(4);
 
     // ---- field

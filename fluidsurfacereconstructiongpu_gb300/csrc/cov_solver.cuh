@@ -129,9 +129,8 @@ struct CovAccum {
 struct CovChunkAccum {
     CovAccum tot;
     float w = 0.f, c11 = 0.f, c22 = 0.f, c33 = 0.f, c12 = 0.f, c13 = 0.f, c23 = 0.f;
-    __device__ __forceinline__ void add(float vx, float vy, float vz, float s)
+    __device__ __forceinline__ void add(float vx, float vy, float vz, float wt)
     {
-        const float wt = 1.0f - s * s * s;
         w += wt;
         const float wx = wt * vx, wy = wt * vy;
         c11 = fmaf(wx, vx, c11);

@@ -1197,8 +1197,6 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
         dm = sqrtf(fmaf(m.x - m32.x, m.x - m32.x, fmaf(m.y - m32.y, m.y - m32.y, (m.z - m32.z) * (m.z - m32.z))));
     }
     const float cr = cull_radius(a.R, a.sp.cs) + 2.0f * dm;
-    // a candidate within R of either mean lies within R + dm of m
-    const float pre2 = (a.R * 1.0001f + 2.0f * dm) * (a.R * 1.0001f + 2.0f * dm);
     // |q - m|^2 below in2 (above out2) puts q within (beyond) R of m32 with a
     // margin far above the roundings of both squared distances: only
     // candidates in the shell between them take the reference's test
@@ -1217,20 +1215,21 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
         since = 0;
     };
     uint32_t nn = 0;
-    // d > R: neither counted nor weighed
+    // d > R: neither counted nor weighed (out2 > R^2; a weight of 0 adds nothing)
     auto take = [&](const float4& q) {
         const float vx = __fsub_rn(q.x, m.x), vy = __fsub_rn(q.y, m.y), vz = __fsub_rn(q.z, m.z);
         const float d2 = dot3_rn(vx, vy, vz);
-        if (d2 < in2) {
-            ++nn;
-        } else if (d2 < out2) {  // rare: m32 is loaded again (L1) rather than kept in registers
+        if (d2 < in2) ++nn;
+        else if (d2 < out2) {  // rare: m32 is loaded again (L1) rather than kept in registers
             const float4 m32 = a.mean32[t];
             if (dot3_rn(__fsub_rn(q.x, m32.x), __fsub_rn(q.y, m32.y), __fsub_rn(q.z, m32.z)) < a.R_le2) ++nn;
         }
-        if (d2 < a.R_lt2) acc.add(vx, vy, vz, dist_over<kFast>(d2, a.R, a.R_rcp, a.tiny));
+        const float s = dist_over<kFast>(d2, a.R, a.R_rcp, a.tiny);
+        const float wt = 1.0f - s * s * s;
+        acc.add(vx, vy, vz, d2 < a.R_lt2 ? wt : 0.f);
     };
     auto near = [&](const float4& q) {
-        return dot3_rn(__fsub_rn(q.x, m.x), __fsub_rn(q.y, m.y), __fsub_rn(q.z, m.z)) < pre2;
+        return dot3_rn(__fsub_rn(q.x, m.x), __fsub_rn(q.y, m.y), __fsub_rn(q.z, m.z)) < out2;
     };
     auto row_range = [&](int x0, int x1, int yy, int zz, uint32_t& beg, uint32_t& end) {
         const uint32_t c0 = lin3(x0, yy, zz, a.sp);
@@ -1290,7 +1289,7 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
                         }
                         for (; k < cnt; k += P) {
                             const float4 q = sq[k];
-                            if (mine(q)) take(q);
+                            if (near(q) && mine(q)) take(q);
                         }
                         since += kSets ? (nbox + P - 1) / P : nbox / P;
                         if (since >= 32) fold();
@@ -1340,7 +1339,10 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
                     since += 4;
                     if (since >= 32) fold();
                 }
-                for (; i < end; ++i) take(__ldg(&a.sorted[i]));
+                for (; i < end; ++i) {
+                    const float4 q = __ldg(&a.sorted[i]);
+                    if (near(q)) take(q);
+                }
             }
     }
     fold();

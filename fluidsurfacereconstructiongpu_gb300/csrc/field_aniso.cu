@@ -688,6 +688,30 @@ struct MomAcc {
         m[33] = fmaf(czz, yy, m[33]);  // yzz
         m[34] = fmaf(cx * yy, yz, m[34]);  // xyz
     }
+    // The warp's sums to out.  32 of the moments are halved from lane to lane: a
+    // lane hands over half of what it holds and keeps the sums of the other
+    // half, so that 31 shuffles leave one moment per lane (in the order of the
+    // pairwise sums of an all-lanes reduction, which takes 160).
+    __device__ __forceinline__ void store(float* out, int lane)
+    {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const bool up = (lane & o) != 0;
+#pragma unroll
+            for (int k = 0; k < o; ++k) {
+                const float give = up ? m[k] : m[k + o], keep = up ? m[k + o] : m[k];
+                m[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+            }
+        }
+        out[lane] = m[0];
+#pragma unroll
+        for (int k = 32; k < kMoments; ++k) {
+            float v = m[k];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == 0) out[k] = v;
+        }
+    }
 };
 
 // The polynomial at z = v - o.
@@ -764,29 +788,26 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                 // moments of the non-involved candidates about the box centre
                 const float ox = 0.5f * (b0[0] + b1[0]), oy = 0.5f * (b0[1] + b1[1]), oz = 0.5f * (b0[2] + b1[2]);
                 const float hx = 0.5f * (b1[0] - b0[0]), hy = 0.5f * (b1[1] - b0[1]), hz = 0.5f * (b1[2] - b0[2]);
-                MomAcc acc;
-                acc.zero();
-                float y2max = 0.f;
-                const CandTables tabs{w.cstart, w.cpre, w.cinv};
-                for (uint32_t j = w.total_inv + lane; j < total; j += 32) {
-                    int cell;
-                    const uint32_t i = candidate(j, tabs, &cell, (int)w.ncells);
-                    const float4 sm = __ldg(&a.smoothed[i]);
-                    const float yx = sm.x - ox, yy = sm.y - oy, yz = sm.z - oz;
-                    y2max = fmaxf(y2max, fmaf(yx, yx, fmaf(yy, yy, yz * yz)));
-                    acc.add(a.sigma * sm.w, yx, yy, yz);
+                // (a group without such candidates has no unscaled part)
+                if (total > w.total_inv) {
+                    MomAcc acc;
+                    acc.zero();
+                    float y2max = 0.f;
+                    const CandTables tabs{w.cstart, w.cpre, w.cinv};
+                    for (uint32_t j = w.total_inv + lane; j < total; j += 32) {
+                        int cell;
+                        const uint32_t i = candidate(j, tabs, &cell, (int)w.ncells);
+                        const float4 sm = __ldg(&a.smoothed[i]);
+                        const float yx = sm.x - ox, yy = sm.y - oy, yz = sm.z - oz;
+                        y2max = fmaxf(y2max, fmaf(yx, yx, fmaf(yy, yy, yz * yz)));
+                        acc.add(a.sigma * sm.w, yx, yy, yz);
+                    }
+                    acc.store(w.mom, lane);
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) y2max = fmaxf(y2max, __shfl_xor_sync(0xffffffffu, y2max, o));
+                    const float zmax = sqrtf(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
+                    if (lane == 0) w.use_mom = (sqrtf(y2max) + zmax) * 1.001f < 0.5f ? 1u : 0u;
                 }
-#pragma unroll
-                for (int k = 0; k < kMoments; ++k) {
-                    float v = acc.m[k];
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                    if (lane == 0) w.mom[k] = v;
-                }
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) y2max = fmaxf(y2max, __shfl_xor_sync(0xffffffffu, y2max, o));
-                const float zmax = sqrtf(fmaf(hx, hx, fmaf(hy, hy, hz * hz)));
-                if (lane == 0) w.use_mom = (sqrtf(y2max) + zmax) * 1.001f < 0.5f ? 1u : 0u;
                 __syncwarp();
             }
             // the pass's box, brick order and tile boxes
@@ -876,7 +897,7 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
             // moment polynomial when it applies; else they are streamed: only
             // the position and the coefficient sigma m / rho are staged, and
             // q2 is |x~ - v|^2
-            const bool use_mom = w.use_mom != 0u;
+            const bool use_mom = total > total_inv && w.use_mom != 0u;
             if (use_mom) {
                 const float ox = 0.5f * (vpos1(lo[0], a.sc.min[0], a.sc.cs) + vpos1(hi[0] - 1, a.sc.min[0], a.sc.cs));
                 const float oy = 0.5f * (vpos1(lo[1], a.sc.min[1], a.sc.cs) + vpos1(hi[1] - 1, a.sc.min[1], a.sc.cs));

@@ -852,6 +852,9 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                             if ((m >> lane) & 1u)
                                 list_pair_record(reinterpret_cast<const float2*>(w.rec), lane,
                                                  reinterpret_cast<float*>(w.lst), __popc(m & ((1u << lane) - 1u)));
+                            // the other half of a last single: zeros, which add 0
+                            if ((__popc(m) & 1) && lane < 10)
+                                reinterpret_cast<float*>(w.lst)[(__popc(m) >> 1) * (4 * kPairF4) + 1 + 2 * lane] = 0.f;
                             __syncwarp();
                             const uint32_t v = 32 * t + lane;
                             if (v < nv) {
@@ -870,15 +873,14 @@ __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_group
                                 const float2 nvx = make_float2(-vp.x, -vp.x), nvy = make_float2(-vp.y, -vp.y),
                                              nvz = make_float2(-vp.z, -vp.z);
                                 const uint32_t cnt = __popc(m);
-                                // not unrolled: copies of the body crowd the
-                                // instruction cache (measured: fetch stalls
-                                // doubled and the 2^18-particle frame slowed)
-#pragma unroll 1
+                                // (two copies: 8M particles 9.36 -> 9.21 ms; three
+                                // crowd the instruction cache: 9.62)
+#pragma unroll 2
                                 for (uint32_t j = 0; j < cnt; j += 2) {
                                     float2 q2, u3, c;
                                     pair_terms(w.lst + (j >> 1) * kPairF4, nvx, nvy, nvz, q2, u3, c);
                                     if (q2.x < 1.0f) s = fmaf(c.x, u3.x, s);
-                                    if (j + 1 < cnt && q2.y < 1.0f) s = fmaf(c.y, u3.y, s);
+                                    if (q2.y < 1.0f) s = fmaf(c.y, u3.y, s);
                                 }
                                 const float a0 = w.psum[t][lane];
                                 const float t0 = a0 + s;

@@ -390,22 +390,26 @@ __device__ void g_to_c(const T V[3][3], const T l[3], float h_inv, const float g
         }
 }
 
-// Calls fn(i, q) for the sorted particles of each lane's cell window (rows of
-// x-adjacent cells merged).  Every lane of the warp calls it; lanes with
-// active = false take no particles.  A warp whose active windows span at
-// most 4 cells per axis walks their union together, 32 particles staged in
-// sq at a time (one load per particle for the whole warp); the caller sets
-// coop only when every particle the union adds fails each lane's own range
-// test, so each lane still sees exactly the particles that matter to it.
-// Staged particles beyond r of the box of the active lanes' centres (cx,
-// cy, cz) are dropped (they fail every lane's range test); the others keep
-// their order, their index rides in the staged w.
-template <class Fn>
+// Calls fn(i, q) for the sorted particles of each particle's cell window (rows
+// of x-adjacent cells merged), P lanes per particle taking every P-th of them.
+// Every lane of the warp calls it; lanes with active = false take none.
+// Lanes whose windows span few cells per axis walk their union together, 32
+// particles staged in sq at a time (one load per particle for the whole warp).
+// Staged particles beyond r of the box of the active lanes' centres (cx, cy, cz)
+// are dropped (they fail every lane's range test); their index rides in the
+// staged w.
+// kSets = false: the whole warp is one set, or each lane walks on its own; coop
+// says that every particle the union adds fails each lane's own range test.
+// kSets = true (wide windows, which may cut the range): sets of lanes
+// (window_mates), and a lane takes only its own window's particles, a run of the
+// sorted ones in each row.
+template <int P, bool kSets, class Fn>
 __device__ __forceinline__ void walk_windows(const Window& w, bool active, bool coop, const Grid& sp,
                                              const uint2* __restrict__ ranges, const float4* __restrict__ sorted,
                                              float4* sq, float cx, float cy, float cz, float r, Fn fn)
 {
     const int lane = threadIdx.x & 31;
+    const uint32_t sub = threadIdx.x % P;
     auto row_range = [&](int x0, int x1, int yy, int zz, uint32_t& beg, uint32_t& end) {
         const uint32_t c0 = lin3(x0, yy, zz, sp);
         beg = kEmpty;
@@ -418,20 +422,25 @@ __device__ __forceinline__ void walk_windows(const Window& w, bool active, bool 
             }
         }
     };
-    int ulo[3], uhi[3];
-    bool compact = coop;
+    auto walk = [&](bool in_set) {
+        int ulo[3], uhi[3];
+        bool compact = coop;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        ulo[a] = (int)__reduce_min_sync(0xffffffffu, active ? (unsigned)w.lo[a] : 0x7fffffffu);
-        uhi[a] = (int)__reduce_max_sync(0xffffffffu, active ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
-        compact = compact && uhi[a] - ulo[a] <= 3;
-    }
-    if (compact) {
-        const WarpBox box = warp_box(active, cx, cy, cz, r);
+        for (int a = 0; a < 3; ++a) {
+            ulo[a] = (int)__reduce_min_sync(0xffffffffu, in_set ? (unsigned)w.lo[a] : 0x7fffffffu);
+            uhi[a] = (int)__reduce_max_sync(0xffffffffu, in_set ? (unsigned)(w.hi[a] + 1) : 0u) - 1;
+            compact = compact && uhi[a] - ulo[a] <= 3;
+        }
+        if (!kSets && !compact) return false;
+        const WarpBox box = warp_box(in_set, cx, cy, cz, r);
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
-                uint32_t beg, end;
+                uint32_t beg, end, own = 0, len = 0;
                 row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                if (kSets && in_set && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
+                    row_range(w.lo[0], w.hi[0], yy, zz, own, len);
+                    len = len > own ? len - own : 0u;
+                }
                 for (uint32_t b = beg; b < end; b += 32) {
                     float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
                     bool keep = false;
@@ -443,22 +452,45 @@ __device__ __forceinline__ void walk_windows(const Window& w, bool active, bool 
                     if (keep) sq[__popc(m & ((1u << lane) - 1u))] = make_float4(q.x, q.y, q.z, __uint_as_float(b + lane));
                     __syncwarp();
                     const uint32_t cnt = __popc(m);
-                    if (active)
-                        for (uint32_t k = 0; k < cnt; ++k) {
+                    if (in_set)
+                        for (uint32_t k = sub; k < cnt; k += P) {
                             const float4 e = sq[k];
-                            fn(__float_as_uint(e.w), e);
+                            const uint32_t i = __float_as_uint(e.w);
+                            if (!kSets || i - own < len) fn(i, e);
                         }
                     __syncwarp();
                 }
             }
-    } else if (active) {
+        return true;
+    };
+    uint32_t left = __ballot_sync(0xffffffffu, active);
+    if (kSets) {
+        for (int sets = 0; left != 0u && sets < kMaxSets; ++sets) {
+            const uint32_t set = window_mates(left, w, 5, lane);
+            left &= ~set;
+            walk((set >> lane) & 1u);
+        }
+    } else if (walk(active)) {
+        left = 0u;
+    }
+    if ((left >> lane) & 1u) {
         for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
             for (int yy = w.lo[1]; yy <= w.hi[1]; ++yy) {
                 uint32_t beg, end;
                 row_range(w.lo[0], w.hi[0], yy, zz, beg, end);
-                for (uint32_t i = beg; i < end; ++i) fn(i, __ldg(&sorted[i]));
+                for (uint32_t i = beg + sub; i < end; i += P) fn(i, __ldg(&sorted[i]));
             }
     }
+    __syncwarp();
+}
+
+// The sum of v over a particle's P lanes.
+template <int P>
+__device__ __forceinline__ float lanes_sum(float v)
+{
+#pragma unroll
+    for (int o = 1; o < P; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
 }
 
 // Blocks of two warps (at the registers of 3 blocks of 256 threads per SM):
@@ -466,10 +498,17 @@ __device__ __forceinline__ void walk_windows(const Window& w, bool active, bool 
 // back as soon as its two warps are done.
 constexpr int kCovBT = 64;
 
+// P lanes per particle (neither kernel has an order to keep), kSets for radii of
+// a cell and more, as in the forward walks.  The whole backward pass, P = 1 / 4 /
+// 8 (ms): R = 0.8 cells: 3k particles 0.40 / 0.26 / 0.23, 60k 0.49 / 0.34 / 0.35,
+// 150k 0.61 / 0.50 / 0.54, 4M 3.60 / 3.86 / 4.68; R = 1.54 cells, P = 1 / 4 / 8 with
+// sets and P = 1 without: 20k 1.85 / 0.68 / 0.59, 2.11; 60k 2.29 / 1.18 / 1.07, 2.82.
+template <int P, bool kSets>
 __global__ void __launch_bounds__(kCovBT, 12) k_cov_backward(BwdArgs a, CovArgs f)
 {
     __shared__ float4 s_q[kCovBT];  // 32 staged particles per warp
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / P;
+    const bool first = threadIdx.x % P == 0;
     const bool valid = t < f.n;
     float4 gmo = make_float4(0.f, 0.f, 0.f, 0.f);
     float gG[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -493,7 +532,7 @@ __global__ void __launch_bounds__(kCovBT, 12) k_cov_backward(BwdArgs a, CovArgs 
         }
     }
     if (__all_sync(0xffffffffu, !act)) {
-        if (valid) a.gmean[t] = gmo;
+        if (valid && first) a.gmean[t] = gmo;
         return;
     }
     const float4 p = act ? f.sorted[t] : make_float4(0.f, 0.f, 0.f, 1.f);
@@ -533,8 +572,8 @@ __global__ void __launch_bounds__(kCovBT, 12) k_cov_backward(BwdArgs a, CovArgs 
     }
     const float R = f.R, invR = 1.0f / R, invR3 = invR * invR * invR;
     float gmx = 0.f, gmy = 0.f, gmz = 0.f;
-    walk_windows(w, act, f.coop_ok != 0, f.sp, f.ranges, f.sorted, s_q + (threadIdx.x & ~31u), m.x, m.y, m.z,
-                 cull_radius(R, f.sp.cs), [&](uint32_t i, const float4& q) {
+    walk_windows<P, kSets>(w, act, f.coop_ok != 0, f.sp, f.ranges, f.sorted, s_q + (threadIdx.x & ~31u), m.x, m.y, m.z,
+                           cull_radius(R, f.sp.cs), [&](uint32_t i, const float4& q) {
         const float vx = __fsub_rn(q.x, m.x), vy = __fsub_rn(q.y, m.y), vz = __fsub_rn(q.z, m.z);
         const float d2 = dot3_rn(vx, vy, vz);
         if (!(d2 < f.R_lt2)) return;  // the forward's weight test (d < R), exactly
@@ -553,16 +592,19 @@ __global__ void __launch_bounds__(kCovBT, 12) k_cov_backward(BwdArgs a, CovArgs 
         gmy -= gy;
         gmz -= gz;
     });
-    if (act) gmo = make_float4(gmx, gmy, gmz, 0.f);
-    if (valid) a.gmean[t] = gmo;
+    gmo = make_float4(lanes_sum<P>(gmx), lanes_sum<P>(gmy), lanes_sum<P>(gmz), 0.f);  // (0 when not active)
+    if (valid && first) a.gmean[t] = gmo;
 }
 
 // ---------------------------------------------------------------- smoothing
-__global__ void k_smooth_backward(BwdArgs a, const float4* sorted, const float4* mean, const uint2* ranges, Grid sp,
-                                  uint32_t n, float R, float R_lt2, int coop_ok, float lambda)
+template <int P, bool kSets>
+__global__ void __launch_bounds__(kT) k_smooth_backward(BwdArgs a, const float4* sorted, const float4* mean,
+                                                        const uint2* ranges, Grid sp, uint32_t n, float R, float R_lt2,
+                                                        int coop_ok, float lambda)
 {
     __shared__ float4 s_q[kT];  // 32 staged particles per warp
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / P;
+    const bool first = threadIdx.x % P == 0;
     const bool valid = t < n;
     float4 gs = make_float4(0.f, 0.f, 0.f, 0.f), gmc = gs;
     if (valid) {
@@ -570,7 +612,7 @@ __global__ void k_smooth_backward(BwdArgs a, const float4* sorted, const float4*
         gmc = a.gmean[t];
     }
     const float gmx = lambda * gs.x + gmc.x, gmy = lambda * gs.y + gmc.y, gmz = lambda * gs.z + gmc.z;
-    float gix = (1.0f - lambda) * gs.x, giy = (1.0f - lambda) * gs.y, giz = (1.0f - lambda) * gs.z;
+    float gix = 0.f, giy = 0.f, giz = 0.f;
     const bool act = valid && (gmx != 0.f || gmy != 0.f || gmz != 0.f);
     if (__any_sync(0xffffffffu, act)) {
         const float4 p = act ? sorted[t] : make_float4(0.f, 0.f, 0.f, 1.f);
@@ -581,9 +623,8 @@ __global__ void k_smooth_backward(BwdArgs a, const float4* sorted, const float4*
         const float iw = 1.0f / m.w;
         const float gnx = gmx * iw, gny = gmy * iw, gnz = gmz * iw;
         const float invR = 1.0f / R, invR3 = invR * invR * invR;
-        walk_windows(w, act, coop_ok != 0, sp, ranges, sorted, s_q + (threadIdx.x & ~31u), p.x, p.y, p.z,
-                     cull_radius(R, sp.cs),
-                     [&](uint32_t i, const float4& q) {
+        walk_windows<P, kSets>(w, act, coop_ok != 0, sp, ranges, sorted, s_q + (threadIdx.x & ~31u), p.x, p.y, p.z,
+                               cull_radius(R, sp.cs), [&](uint32_t i, const float4& q) {
             // the forward's neighbour decision, exactly
             const float d2 = dot3_rn(__fsub_rn(p.x, q.x), __fsub_rn(p.y, q.y), __fsub_rn(p.z, q.z));
             if (!(d2 < R_lt2)) return;
@@ -602,7 +643,10 @@ __global__ void k_smooth_backward(BwdArgs a, const float4* sorted, const float4*
             atomicAdd(a.gx + i, make_float4(wt * gnx - ex, wt * gny - ey, wt * gnz - ez, 0.f));
         });
     }
-    if (valid) atomicAdd(a.gx + t, make_float4(gix, giy, giz, 0.f));
+    gix = lanes_sum<P>(gix) + (1.0f - lambda) * gs.x;
+    giy = lanes_sum<P>(giy) + (1.0f - lambda) * gs.y;
+    giz = lanes_sum<P>(giz) + (1.0f - lambda) * gs.z;
+    if (valid && first) atomicAdd(a.gx + t, make_float4(gix, giy, giz, 0.f));
 }
 
 __global__ void k_unsort(const float4* gx, const uint32_t* perm, uint32_t n, float* out)
@@ -650,11 +694,24 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
         } else {
             k_field_backward_aniso<<<nblk(a.n), kT, 0, c.stream>>>(a);
         }
-        k_cov_backward<<<(unsigned)std::max<uint64_t>(1, (a.n + kCovBT - 1) / kCovBT), kCovBT, 0, c.stream>>>(a, *cov);
         // warps may walk the union of their windows when the cull radius stays below 2 cells
         const int smooth_coop = (R * 1.0001f + 1e-4f * cov->sp.cs) < 2.0f * cov->sp.cs * 0.9999f ? 1 : 0;
-        k_smooth_backward<<<nblk(a.n), kT, 0, c.stream>>>(a, cov->sorted, cov->mean, cov->ranges, cov->sp, a.n, R,
-                                                           cov->R_lt2, smooth_coop, lambda);
+        auto launch = [&](auto cov_kernel, auto smooth_kernel, uint64_t lanes) {
+            cov_kernel<<<(unsigned)((a.n * lanes + kCovBT - 1) / kCovBT), kCovBT, 0, c.stream>>>(a, *cov);
+            smooth_kernel<<<nblk(a.n * lanes), kT, 0, c.stream>>>(a, cov->sorted, cov->mean, cov->ranges, cov->sp, a.n, R,
+                                                                  cov->R_lt2, smooth_coop, lambda);
+        };
+        const bool sets = cov->coop_ok == 0;  // R near or above a cell
+        if (a.n < (sets ? 131072u : 40960u)) {
+            if (sets) launch(k_cov_backward<8, true>, k_smooth_backward<8, true>, 8);
+            else launch(k_cov_backward<8, false>, k_smooth_backward<8, false>, 8);
+        } else if (a.n < (1u << 21)) {
+            if (sets) launch(k_cov_backward<4, true>, k_smooth_backward<4, true>, 4);
+            else launch(k_cov_backward<4, false>, k_smooth_backward<4, false>, 4);
+        } else {
+            if (sets) launch(k_cov_backward<1, true>, k_smooth_backward<1, true>, 1);
+            else launch(k_cov_backward<1, false>, k_smooth_backward<1, false>, 1);
+        }
         g_launches += 3;
     } else {
         launch_field_iso_backward(c, a, method == FSR_METHOD_TC01, ctr);

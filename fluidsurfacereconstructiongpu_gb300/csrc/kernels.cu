@@ -91,24 +91,6 @@ __global__ void k_ranges_gather(const uint32_t* __restrict__ skeys, const uint32
     sorted[k] = make_float4(xyz[3ull * s], xyz[3ull * s + 1], xyz[3ull * s + 2], dens ? dens[s] : 0.0f);
 }
 
-// Lanes whose windows span few cells together walk their union together
-// (below); a warp whose windows lie further apart (its particles run over the
-// end of a row of cells) is cut into such sets of lanes, each walked on its own.
-// The lanes of `left` that form a set with its first lane: together with that
-// lane's window theirs spans at most span + 1 cells per axis.
-constexpr int kMaxSets = 4;  // lanes left over after these walk alone (scattered particles: small windows)
-__device__ __forceinline__ uint32_t window_mates(uint32_t left, const Window& w, int span, int lane)
-{
-    const int lead = __ffs((int)left) - 1;
-    bool ok = (left >> lane) & 1u;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-        const int lo = __shfl_sync(0xffffffffu, w.lo[a], lead), hi = __shfl_sync(0xffffffffu, w.hi[a], lead);
-        ok = ok && max(hi, w.hi[a]) - min(lo, w.lo[a]) <= span;
-    }
-    return __ballot_sync(0xffffffffu, ok || lane == lead);
-}
-
 // SPH density of each sorted particle, for frames without a density column
 // (the reference's .xyz files carry the simulator's densities and the
 // reference computes none): rho_i = m sigma / h^3 sum_j (1 - |x_i - x_j|^2 /

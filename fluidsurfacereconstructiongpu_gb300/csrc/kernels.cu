@@ -913,6 +913,7 @@ struct QuadSlice {
     float q[4][kQuadRow];  // 1, x, y, z of the staged candidates
     float w[8][kQuadRow];  // per particle: their weights (0 at and beyond R)
     uint32_t gend[kQuadGroups];  // ends of the closed chunk sums
+    uint32_t idx[kQuadRow];      // the staged candidates' sorted index (own_folds)
 };
 
 template <bool kFast>
@@ -1004,6 +1005,24 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
     };
     // Particles whose windows span few cells per axis walk their union
     // together (window_mates), as in k_smooth; the sets are the block's.
+    // The chunk sums end where k_smooth's do, so that both kernels' sums agree
+    // bit for bit for radii below a cell (max_span 3): where the whole block is
+    // one set, at 32 candidates of its box; else at every 32 of the particle's own
+    // window, row by row (own_folds).
+    bool one_set = max_span >= 0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const int lo = (int)__reduce_min_sync(0xffffffffu, there ? (unsigned)wl.lo[a] : 0x7fffffffu);
+        const int hi = (int)__reduce_max_sync(0xffffffffu, there ? (unsigned)(wl.hi[a] + 1) : 0u) - 1;
+        one_set = one_set && hi - lo <= max_span;
+    }
+    const bool own_folds = max_span == 3 && !one_set;
+    Window w;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        w.lo[a] = __shfl_sync(0xffffffffu, wl.lo[a], src);
+        w.hi[a] = __shfl_sync(0xffffffffu, wl.hi[a], src);
+    }
     for (uint32_t k = lane; k < kQuadRow; k += 32) S.q[0][k] = 1.0f;
     const float r = cull_radius(R, sp.cs);
     uint32_t left = __ballot_sync(0xffffffffu, there);
@@ -1026,6 +1045,7 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
         const WarpBox box = warp_box(in_set, pl.x, pl.y, pl.z, r);
         const WarpBox mine = warp_box(mine_in, p.x, p.y, p.z, r);
         uint32_t fill = 0, ngr = 0;
+        uint32_t own = 0, len = 0, chunk_at = 0;  // own_folds: the row's run of this particle's window, its chunk
         since = 0;
         // pads the staged candidates to a multiple of 4 with ones of weight 0
         auto pad = [&]() {
@@ -1034,8 +1054,23 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
             fill += m;
         };
         auto flush = [&]() {
+            const uint32_t staged = fill;
             pad();
             weights(fill, mine_in);
+            if (own_folds) {
+                for (uint32_t k = 0; k < staged; ++k) {
+                    const float wt = S.w[part][k];  // 0: beyond R, or of another window
+                    const uint32_t c = (S.idx[k] - own) >> 5;
+                    if (wt != 0.f && c != chunk_at) {
+                        fold();
+                        chunk_at = c;
+                    }
+                    sum(S.q[comp][k], wt);
+                }
+                fill = 0;
+                __syncwarp();
+                return;
+            }
             uint32_t s = 0;
             for (uint32_t g = 0; g < ngr; ++g) {
                 const uint32_t e = S.gend[g];
@@ -1051,6 +1086,13 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 uint32_t beg, end;
                 row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                if (own_folds) {
+                    own = len = chunk_at = 0;
+                    if (mine_in && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
+                        row_range(w.lo[0], w.hi[0], yy, zz, own, len);
+                        len = len > own ? len - own : 0u;
+                    }
+                }
                 float4 next = beg + lane < end ? __ldg(&sorted[beg + lane]) : make_float4(0.f, 0.f, 0.f, 0.f);
                 for (uint32_t base = beg; base < end; base += 32) {
                     const float4 q = next;
@@ -1065,10 +1107,11 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
                         S.q[1][k] = q.x;
                         S.q[2][k] = q.y;
                         S.q[3][k] = q.z;
+                        if (own_folds) S.idx[k] = base + lane;
                     }
                     fill += __popc(m);
-                    since += nbox;
-                    if (since >= 32) {
+                    since += own_folds ? 0u : nbox;
+                    if (since >= 32 && !own_folds) {
                         since = 0;
                         pad();
                         if (lane == 0) S.gend[ngr] = fill;
@@ -1076,17 +1119,24 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
                     }
                     if (fill + 35u > kQuadCap || ngr == kQuadGroups) flush();
                 }
+                if (own_folds) {
+                    flush();
+                    // the row's full chunks have ended, its rest waits for more
+                    if (len >= 32u) {
+                        if (chunk_at < (len >> 5)) fold();
+                        since = 0;
+                    }
+                    since += len & 31u;
+                    if (since >= 32u) {
+                        fold();
+                        since = 0;
+                    }
+                }
             }
         flush();
     }
     if (left != 0u) {
         // each particle walks its own window, 32 candidates at a time
-        Window w;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-            w.lo[a] = __shfl_sync(0xffffffffu, wl.lo[a], src);
-            w.hi[a] = __shfl_sync(0xffffffffu, wl.hi[a], src);
-        }
         since = 0;
         if ((left >> src) & 1u)
             for (int zz = w.lo[2]; zz <= w.hi[2]; ++zz)
@@ -1903,7 +1953,7 @@ void launch_smooth(const KernelCtx& c, const float4* sorted, uint32_t n, const u
     // Four lanes per particle while one would leave the SMs with two or three
     // warps per scheduler; more lanes cost more instructions per particle once
     // the GPU is full.  Measured, one lane / four (ms): R = 0.8 cells: 20k
-    // particles 0.19 / 0.07, 32k 0.12 / 0.09, 64k 0.11-0.23 / 0.14-0.18, 120k
+    // particles 0.16 / 0.08, 32k 0.12 / 0.09, 64k 0.11-0.23 / 0.14-0.18, 120k
     // 0.28 / 0.31; R = 1.54 cells: 20k 0.62 / 0.25, 40k 0.80 / 0.46, 100k 0.87 /
     // 1.03.
     const bool wide = max_span > 3, fast = fast_radius(R);

@@ -60,6 +60,32 @@ def test_both_sides_of_the_lanes_per_particle_rule(n_side, settings):
     _run("yu13", fr, **SETTINGS[settings])
 
 
+@pytest.mark.parametrize("case", ["lattice", "scattered", "slab"])
+def test_smoothing_of_the_same_particles_by_both_kernels(case):
+    """Below a cell's radius, four lanes per particle and one sum in the same
+    order and the same chunks: particles that sort first smooth to the same bits
+    whether 40,000 others further up bring the frame past the line or not."""
+    import torch
+    from fluidsurfacereconstructiongpu_gb300 import api, synthetic
+    fr = _frame(8000, 0.02, 0.5, 8)
+    if case == "lattice":
+        fr.pos = (0.3 + 0.2 * synthetic.lattice_cube(20, 0.025, seed=2, jitter_frac=0.3).pos).astype(np.float32)
+    elif case == "slab":
+        fr.pos[:, 0] = 0.5 + (fr.pos[:, 0] - 0.5) * 0.1
+    fr.pos[:, 2] = 0.1 + 0.5 * (fr.pos[:, 2] - fr.pos[:, 2].min())
+    n = len(fr.pos)
+    far = np.random.default_rng(9).random((49152 - n + 100, 3)) * [0.9, 0.9, 0.2] + [0.05, 0.05, 0.75]
+    got = []
+    for pos in (fr.pos, np.concatenate([fr.pos, far.astype(np.float32)])):
+        rec = api.Reconstructor("yu13", 0, keep_intermediates=True, **SETTINGS["fine"])
+        fr.density = np.full(len(pos), 1000.0, np.float32)
+        rec.reconstruct(torch.from_numpy(pos).cuda(), torch.from_numpy(fr.density).cuda(), api.header_of(fr))
+        got.append((np.array(rec.debug("perm"))[:n], np.array(rec.debug("smoothed"))[:n]))
+        rec.close()
+    assert np.array_equal(got[0][0], got[1][0])
+    assert np.array_equal(got[0][1], got[1][1])
+
+
 @pytest.mark.parametrize("scale", [1.0, 1.4])
 @pytest.mark.parametrize("case", ["few1", "few40", "scattered", "slab", "duplicates", "below", "above"])
 def test_colour_field_walks(case, scale):

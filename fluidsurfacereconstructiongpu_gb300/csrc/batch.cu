@@ -475,6 +475,8 @@ fsr_status fsr_batch_copy_mesh(const fsr_batch* b, uint32_t frame, float* pos, f
     if (nv == 0) return FSR_OK;
     if (!pos || !nrm) return FSR_ERR_INVALID_ARGUMENT;
     DeviceScope g(b->device);
+    populate_host(pos, 12ull * nv);
+    populate_host(nrm, 12ull * nv);
     if (cudaMemcpy(pos, h->mesh_pos.ptr, 12ull * nv, cudaMemcpyDefault) != cudaSuccess ||
         cudaMemcpy(nrm, h->mesh_nrm.ptr, 12ull * nv, cudaMemcpyDefault) != cudaSuccess) {
         cudaGetLastError();

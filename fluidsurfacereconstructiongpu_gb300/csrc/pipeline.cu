@@ -9,8 +9,13 @@
 // pooled buffer turned out too small the frame is re-queued with the grown
 // capacities (only the first frames of a new workload pay for that).
 #include <cuda_runtime.h>
+#ifdef __linux__
+#include <sys/mman.h>
+#include <unistd.h>
+#endif
 
 #include <algorithm>
+#include <cerrno>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -136,6 +141,26 @@ struct DeviceGuard {
 }  // namespace
 
 // ------------------------------------------------------------ DevBuf
+
+void fsr::populate_host(void* p, size_t bytes)
+{
+#ifdef __linux__
+    constexpr int kPopulateWrite = 23;  // MADV_POPULATE_WRITE (Linux 5.14; older kernels refuse it)
+    if (!p || !bytes) return;
+    const int saved = errno;
+    const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE), end = (uintptr_t)p + bytes;
+    unsigned char there[1024];
+    for (uintptr_t a = (uintptr_t)p & ~(page - 1); a < end; a += page * sizeof(there)) {
+        const uintptr_t len = std::min<uintptr_t>(end - a, page * sizeof(there)), pages = (len + page - 1) / page;
+        if (mincore((void*)a, len, there) != 0) break;  // not the host's memory
+        if (!std::all_of(there, there + pages, [](unsigned char c) { return c & 1; }))
+            (void)madvise((void*)a, len, kPopulateWrite);
+    }
+    errno = saved;
+#else
+    (void)p, (void)bytes;
+#endif
+}
 
 cudaError_t DevBuf::ensure(size_t want)
 {
@@ -584,6 +609,7 @@ fsr_status run_frame(fsr_handle* h, const fsr_frame_header& hdr, const float* d_
     for (int attempt = 0; attempt < 4; ++attempt) {
         if ((s = frame_buffers(h, fp)) != FSR_OK) return s;
         if ((s = frame_enqueue(h, fp, d_xyz, d_den, st, timing)) != FSR_OK) return s;
+        for (void* p : h->host_out) populate_host(p, h->host_out_bytes);
         CK(cudaStreamSynchronize(st));
         bool retry = false;
         if ((s = frame_finish(h, fp, timing, &retry)) != FSR_OK || !retry) return s;
@@ -705,7 +731,11 @@ fsr_status fsr_reconstruct_host(fsr_handle* h, const fsr_frame_header* hdr, cons
         if (!own_density) CK(cudaMemcpyAsync(h->in_den.ptr, density, 4ull * n, cudaMemcpyHostToDevice, st));
     }
     h->frame_ready = false;
+    h->host_out[0] = out_pos;
+    h->host_out[1] = out_nrm;
+    h->host_out_bytes = 12ull * std::min<uint64_t>(capacity, h->stats.n_mesh_vertices);
     fsr_status s = run_frame(h, *hdr, (const float*)h->in_xyz.ptr, (const float*)h->in_den.ptr, n, st);
+    h->host_out[0] = h->host_out[1] = nullptr;
     if (s != FSR_OK) return s;
     const uint64_t nv = h->stats.n_mesh_vertices;
     *n_vertices = nv;
@@ -713,6 +743,10 @@ fsr_status fsr_reconstruct_host(fsr_handle* h, const fsr_frame_header* hdr, cons
                                    (unsigned long long)nv, (unsigned long long)capacity);
     if (nv) {
         if (!out_pos || !out_nrm) return fail(h, FSR_ERR_INVALID_ARGUMENT, "null mesh output");
+        if (12ull * nv > h->host_out_bytes) {
+            populate_host(out_pos, 12ull * nv);
+            populate_host(out_nrm, 12ull * nv);
+        }
         CK(cudaMemcpyAsync(out_pos, h->mesh_pos.ptr, 12ull * nv, cudaMemcpyDeviceToHost, st));
         CK(cudaMemcpyAsync(out_nrm, h->mesh_nrm.ptr, 12ull * nv, cudaMemcpyDeviceToHost, st));
         CK(cudaStreamSynchronize(st));
@@ -740,6 +774,8 @@ fsr_status fsr_copy_mesh(fsr_handle* h, float* out_pos, float* out_nrm, uint64_t
     if (nv > capacity) return fail(h, FSR_ERR_CAPACITY, "mesh buffer too small");
     if (nv) {
         if (!out_pos || !out_nrm) return FSR_ERR_INVALID_ARGUMENT;
+        populate_host(out_pos, 12ull * nv);
+        populate_host(out_nrm, 12ull * nv);
         CK(cudaMemcpy(out_pos, h->mesh_pos.ptr, 12ull * nv, cudaMemcpyDeviceToHost));
         CK(cudaMemcpy(out_nrm, h->mesh_nrm.ptr, 12ull * nv, cudaMemcpyDeviceToHost));
     }
@@ -759,6 +795,9 @@ fsr_status fsr_copy_indexed_mesh(fsr_handle* h, float* pos, float* nrm, uint64_t
     if (nv > vertex_capacity || ni > index_capacity) return fail(h, FSR_ERR_CAPACITY, "indexed mesh buffers too small");
     if (nv) {
         if (!pos || !nrm || !indices) return FSR_ERR_INVALID_ARGUMENT;
+        populate_host(pos, 12ull * nv);
+        populate_host(nrm, 12ull * nv);
+        populate_host(indices, 4ull * ni);
         CK(cudaMemcpy(pos, h->wpos.ptr, 12ull * nv, cudaMemcpyDefault));
         CK(cudaMemcpy(nrm, h->wnrm.ptr, 12ull * nv, cudaMemcpyDefault));
         CK(cudaMemcpy(indices, h->widx.ptr, 4ull * ni, cudaMemcpyDefault));

@@ -642,6 +642,28 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
     }
 }
 
+__device__ __forceinline__ void mark_group(const GroupMark& gm, uint32_t g, Counters* ctr)
+{
+    const uint32_t flag = atomicOr(gm.gflag + g, kMarkedGroup);
+    if (flag & kMarkedGroup) return;
+    const uint32_t gend = (gm.sp.res[0] + 1) * (gm.sp.res[1] + 1) * (gm.sp.res[2] + 1);
+    if (flag & kDenseGroup) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
+    else gm.glist[gend - 1u - atomicAdd(&ctr->n_sparse, 1u)] = g;
+}
+
+// What both list kernels do besides: the overflow flag, and the zeros that the
+// classification adds the offsets' tile sums to.
+__device__ __forceinline__ void band_list_prologue(const GroupMark& gm, uint32_t cap, Counters* ctr)
+{
+    const uint32_t nb = ctr->n_band;
+    if (blockIdx.x == 0 && threadIdx.x == 0 && nb > cap) {
+        atomicOr(&ctr->overflow, 1u);
+        atomicMax(&ctr->need_band, nb);
+    }
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < gm.ntiles; i += gridDim.x * blockDim.x)
+        gm.tile_sums[i] = 0u;
+}
+
 // compactSurfaceVertex (cu:293-304) over the bitset: every set bit writes
 // its vertex id at its rank.  The band vertices also mark their window
 // groups (the spatial cell a vertex's FP32 position falls in, as the grouped
@@ -652,13 +674,9 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
 __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix,
                             uint32_t nwords, uint32_t* __restrict__ sv, uint32_t cap, GroupMark gm, Counters* ctr)
 {
-    const uint32_t kx = gm.sp.res[0] + 1, ky = gm.sp.res[1] + 1, gend = kx * ky * (gm.sp.res[2] + 1);
+    const uint32_t kx = gm.sp.res[0] + 1, ky = gm.sp.res[1] + 1;
     const uint32_t rx = gm.sc.res[0], rxy = gm.sc.res[0] * gm.sc.res[1];
-    const uint32_t nb = ctr->n_band;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && nb > cap) {
-        atomicOr(&ctr->overflow, 1u);
-        atomicMax(&ctr->need_band, nb);
-    }
+    band_list_prologue(gm, cap, ctr);
     const uint32_t lane = threadIdx.x & 31u;
     for (uint32_t i0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u); i0 < nwords; i0 += gridDim.x * blockDim.x) {
         const uint32_t i = i0 + lane;
@@ -694,10 +712,7 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
                     if (g != last) {
                         last = g;
                         if (gm.gflag[g] & kMarkedGroup) continue;  // (a stale value only costs the atomic)
-                        const uint32_t flag = atomicOr(gm.gflag + g, kMarkedGroup);
-                        if (flag & kMarkedGroup) continue;
-                        if (flag & kDenseGroup) gm.glist[atomicAdd(&ctr->n_groups, 1u)] = g;
-                        else gm.glist[gend - 1u - atomicAdd(&ctr->n_sparse, 1u)] = g;
+                        mark_group(gm, g, ctr);
                     }
                 }
             }
@@ -708,6 +723,38 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
                 ++z;
             }
         }
+    }
+}
+
+// The list for few words (small or coarse grids): a warp per word, a lane per
+// bit.  On coarse grids a word crosses ten groups or more, whose flags one lane
+// fetched one after the other.  A lane marks its vertex's group and, as the kernel
+// above, those between it and the vertex before it in its row (the same groups are
+// marked by both).
+__global__ void k_band_list_words(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix,
+                                  uint32_t nwords, uint32_t* __restrict__ sv, uint32_t cap, GroupMark gm, Counters* ctr)
+{
+    const int kx = (int)gm.sp.res[0] + 1, ky = (int)gm.sp.res[1] + 1;
+    band_list_prologue(gm, cap, ctr);
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; i < nwords; i += (gridDim.x * blockDim.x) >> 5) {
+        const uint32_t w = bits[i];
+        if (w == 0u) continue;
+        const uint32_t below = w & ((1u << lane) - 1u), v = (i << 5) | lane;
+        const uint32_t at = prefix[i] + (uint32_t)__popc(below);
+        const bool set = (w >> lane) & 1u;
+        uint32_t x, y, z;
+        unlin3(v, gm.sc, x, y, z);
+        const int cx = clampi(cell1(vpos1(x, gm.sc.min[0], gm.sc.cs), gm.sp.min[0], gm.sp.cs), 0, kx - 1);
+        const int cy = clampi(cell1(vpos1(y, gm.sc.min[1], gm.sc.cs), gm.sp.min[1], gm.sp.cs), 0, ky - 1);
+        const int cz = clampi(cell1(vpos1(z, gm.sc.min[2], gm.sc.cs), gm.sp.min[2], gm.sp.cs), 0, (int)gm.sp.res[2]);
+        const int before = below ? 31 - __clz((int)below) : (int)lane;
+        const int px = __shfl_sync(0xffffffffu, cx, before);
+        // a vertex before it in the word lies in its row when no more columns lie between them than its own
+        const bool row = below != 0u && lane - (uint32_t)before <= x;
+        if (!set) continue;
+        if (at < cap) sv[at] = v;
+        for (int c = row ? px + 1 : cx; c <= cx; ++c) mark_group(gm, (uint32_t)(c + kx * (cy + ky * cz)), ctr);
     }
 }
 
@@ -1462,95 +1509,104 @@ __device__ __forceinline__ void field_row(const McArgs& a, int x0, int y, int z,
     }
 }
 
-// detectValidSurfaceCubes (cu:328-364): a band vertex as cube origin is
-// valid when all 8 corners are band vertices and the case emits triangles.
-__global__ void k_mc_classify(McArgs a, const Counters* ctr)
-{
-    const uint32_t nb = min(ctr->n_band, a.cap_band);
-    const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
-    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x) {
-        const uint32_t v = a.sv[t];
-        uint32_t x, y, z;
-        unlin3(v, a.sc, x, y, z);
-        uint32_t info = 0;
-        // the cube's corners as 4 rows of two x-neighbours, (dy, dz) in
-        // {0,1}^2: one bitset word (two when the pair straddles a word) and
-        // one prefix per row give both memberships and both ranks (the x + 1
-        // corner of a row in the band follows its x corner: rank + 1)
-        if (x < a.sc.res[0] - 1 && y < a.sc.res[1] - 1 && z < a.sc.res[2] - 1) {
-            uint32_t vr[4], wd[4];
-            bool all = true;
-#pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                vr[r] = v + (uint32_t)(r & 1) * rx + (uint32_t)(r >> 1) * rxy;
-                const uint32_t w = vr[r] >> 5, b = vr[r] & 31u;
-                wd[r] = __ldg(a.band.bits + w);
-                const uint32_t next = b < 31u ? (wd[r] >> (b + 1)) : __ldg(a.band.bits + w + 1);
-                all = all && ((wd[r] >> b) & 1u) && (next & 1u);
-            }
-            if (all) {
-                uint32_t cs = 0;
-                bool in_cap = true;
-#pragma unroll
-                for (int r = 0; r < 4; ++r) {
-                    const uint32_t b = vr[r] & 31u;
-                    const uint32_t r0 = r == 0 ? t : __ldg(a.band.prefix + (vr[r] >> 5)) + __popc(wd[r] & ((1u << b) - 1u));
-                    // ranks beyond the capacity only occur in a frame that overflowed and is re-run
-                    if (r0 + 1 >= a.cap_band) {
-                        in_cap = false;
-                        break;
-                    }
-                    const int dy = r & 1, dz = r >> 1;
-                    const int i0 = dy ? (dz ? 2 : 3) : (dz ? 1 : 0);  // corner (0, dy, dz); (1, dy, dz) is i0 + 4
-                    if (__ldg(a.band.phi + r0) <= a.iso) cs |= 1u << i0;
-                    if (__ldg(a.band.phi + r0 + 1) <= a.iso) cs |= 1u << (i0 + 4);
-                }
-                if (in_cap) info = (uint32_t)c_mc.nverts[cs] | (cs << 8);
-            }
-        }
-        a.mc[t] = info;
-    }
-}
-
 // The marching-cubes offsets in one reduce-then-scan over the classify
 // words (generateTriangles' vertex offsets and compactValidSurfaceCubes:
 // cu:367-380 with the scans of cu:1154-1172).  Per band position t: vofs[t]
 // = the vertices of the cubes before t, and a cube with vertices is listed
 // at valid[its rank among such cubes] = t.  Within a 4096-position tile both
 // counts fit 16 bits (at most 15 x 4096 vertices), so each element is one
-// word, vertices low and cubes high, and the block scans add such words;
-// the tile totals are kept apart, as full words.
+// word, vertices low and cubes high, and the block scans add such words.  The
+// classification adds up the tiles' words; the scan's blocks add up those of the
+// tiles before their own, in full words, or for many tiles one block scans them.
 __device__ __forceinline__ uint32_t mc_pair(uint32_t info)
 {
     const uint32_t nv = info & 0xFFu;
     return nv | (nv != 0u ? 0x10000u : 0u);
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_mc_tile_reduce(McArgs a, const Counters* ctr, uint32_t* tile_sums,
-                                                                 uint32_t ntiles_max)
+// detectValidSurfaceCubes (cu:328-364): a band vertex as cube origin is
+// valid when all 8 corners are band vertices and the case emits triangles.
+__global__ void k_mc_classify(McArgs a, const Counters* ctr, uint32_t* tile_sums)
 {
-    __shared__ uint32_t warp_sums[kScanThreads / 32];
-    const uint32_t n = min(ctr->n_band, a.cap_band);
-    const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t base = (uint64_t)tile * kScanTile;
-        uint32_t s = 0;
+    const uint32_t nb = min(ctr->n_band, a.cap_band);
+    const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
+    // Runs of 128 once the runs of 32 would put too many atomics on a tile's word:
+    // 9M band vertices 92 us, 80 with runs of 128, 84 with 256; below a million the
+    // shorter runs keep more warps busy (a 32k frame 10 / 12).
+    const uint32_t span = nb < 1u << 20 ? 32u : 128u;
+    for (uint32_t t0 = span * warp; t0 < nb; t0 += span * nwarps) {
+        uint32_t sum = 0;
+#pragma unroll 1
+        for (uint32_t t = t0 + lane; t < t0 + span; t += 32u) {
+            const uint32_t v = t < nb ? a.sv[t] : 0xffffffffu;
+            uint32_t x, y, z;
+            unlin3(v, a.sc, x, y, z);
+            uint32_t info = 0;
+            // the cube's corners as 4 rows of two x-neighbours, (dy, dz) in
+            // {0,1}^2: one bitset word (two when the pair straddles a word) and
+            // one prefix per row give both memberships and both ranks (the x + 1
+            // corner of a row in the band follows its x corner: rank + 1)
+            if (t < nb && x < a.sc.res[0] - 1 && y < a.sc.res[1] - 1 && z < a.sc.res[2] - 1) {
+                uint32_t vr[4], wd[4];
+                bool all = true;
 #pragma unroll
-        for (uint32_t k = 0; k < kScanItems; ++k) {
-            const uint64_t i = base + k * kScanThreads + threadIdx.x;
-            if (i < n) s += mc_pair(__ldg(a.mc + i));
+                for (int r = 0; r < 4; ++r) {
+                    vr[r] = v + (uint32_t)(r & 1) * rx + (uint32_t)(r >> 1) * rxy;
+                    const uint32_t w = vr[r] >> 5, b = vr[r] & 31u;
+                    wd[r] = __ldg(a.band.bits + w);
+                    const uint32_t next = b < 31u ? (wd[r] >> (b + 1)) : __ldg(a.band.bits + w + 1);
+                    all = all && ((wd[r] >> b) & 1u) && (next & 1u);
+                }
+                if (all) {
+                    uint32_t cs = 0;
+                    bool in_cap = true;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const uint32_t b = vr[r] & 31u;
+                        const uint32_t r0 =
+                            r == 0 ? t : __ldg(a.band.prefix + (vr[r] >> 5)) + __popc(wd[r] & ((1u << b) - 1u));
+                        // ranks beyond the capacity only occur in a frame that overflowed and is re-run
+                        if (r0 + 1 >= a.cap_band) {
+                            in_cap = false;
+                            break;
+                        }
+                        const int dy = r & 1, dz = r >> 1;
+                        const int i0 = dy ? (dz ? 2 : 3) : (dz ? 1 : 0);  // corner (0, dy, dz); (1, dy, dz) is i0 + 4
+                        if (__ldg(a.band.phi + r0) <= a.iso) cs |= 1u << i0;
+                        if (__ldg(a.band.phi + r0 + 1) <= a.iso) cs |= 1u << (i0 + 4);
+                    }
+                    if (in_cap) info = (uint32_t)c_mc.nverts[cs] | (cs << 8);
+                }
+            }
+            if (t < nb) a.mc[t] = info;
+            sum += mc_pair(info);
         }
-        const uint32_t incl = block_inclusive_scan(s, warp_sums);
-        if (threadIdx.x == kScanThreads - 1) {
-            tile_sums[tile] = incl & 0xFFFFu;
-            tile_sums[ntiles_max + tile] = incl >> 16;
-        }
-        __syncthreads();
+        // the tile's sums for the offsets (a kernel of its own before: offsets of 9M
+        // vertices 45 us, 35 without it)
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        if (lane == 0 && sum != 0u) atomicAdd(tile_sums + t0 / kScanTile, sum);
     }
 }
 
-// One block: exclusive scans of both tile totals in place; the frame's
-// vertex and cube counts, and the pool overflow flags.
+// The frame's vertex and cube counts, and the pool overflow flags.
+__device__ __forceinline__ void mc_counts(const McArgs& a, Counters* ctr, uint32_t verts, uint32_t cubes)
+{
+    ctr->n_mesh_verts = verts;
+    ctr->n_valid = cubes;
+    if (cubes > a.cap_valid) {
+        atomicOr(&ctr->overflow, 2u);
+        atomicMax(&ctr->need_valid, cubes);
+    }
+    if (verts > a.cap_mesh) {
+        atomicOr(&ctr->overflow, 4u);
+        atomicMax(&ctr->need_mesh, verts);
+    }
+}
+
+// One block: exclusive scans of both tile totals, over the tiles' words and
+// behind them.
 __global__ void __launch_bounds__(kScanThreads) k_mc_scan_tile_sums(McArgs a, Counters* ctr, uint32_t* tile_sums,
                                                                     uint32_t ntiles_max)
 {
@@ -1561,34 +1617,24 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_scan_tile_sums(McArgs a, Co
     uint32_t carry[2] = {0u, 0u};
     for (uint32_t b = 0; b < ntiles; b += kScanThreads) {
         const uint32_t i = b + threadIdx.x;
+        const uint32_t both = i < ntiles ? tile_sums[i] : 0u;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            uint32_t* ts = tile_sums + h * ntiles_max;
-            const uint32_t x = i < ntiles ? ts[i] : 0u;
+            const uint32_t x = h ? both >> 16 : both & 0xFFFFu;
             const uint32_t incl = block_inclusive_scan(x, warp_sums);
-            if (i < ntiles) ts[i] = carry[h] + incl - x;
+            if (i < ntiles) tile_sums[h * ntiles_max + i] = carry[h] + incl - x;
             if (threadIdx.x == kScanThreads - 1) last[h] = incl;
             __syncthreads();
             carry[h] += last[h];
         }
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        ctr->n_mesh_verts = carry[0];
-        ctr->n_valid = carry[1];
-        if (carry[1] > a.cap_valid) {
-            atomicOr(&ctr->overflow, 2u);
-            atomicMax(&ctr->need_valid, carry[1]);
-        }
-        if (carry[0] > a.cap_mesh) {
-            atomicOr(&ctr->overflow, 4u);
-            atomicMax(&ctr->need_mesh, carry[0]);
-        }
-    }
+    if (threadIdx.x == 0) mc_counts(a, ctr, carry[0], carry[1]);
 }
 
-__global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const Counters* ctr,
-                                                               const uint32_t* tile_prefix, uint32_t ntiles_max)
+template <bool kSums>
+__global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, Counters* ctr, const uint32_t* tile_sums,
+                                                               uint32_t ntiles_max)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t tile_vals[kScanTilePadded];
@@ -1613,7 +1659,21 @@ __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, const C
         }
         const uint32_t incl = block_inclusive_scan(s, warp_sums);
         uint32_t run = incl - s;  // packed exclusive prefix within the tile
-        const uint32_t pv = tile_prefix[tile], pq = tile_prefix[ntiles_max + tile];
+        uint32_t pv = 0, pq = 0;
+        if (kSums) {
+            for (uint32_t i = threadIdx.x; i < tile; i += kScanThreads) {
+                const uint32_t both = __ldg(tile_sums + i);
+                pv += both & 0xFFFFu;
+                pq += both >> 16;
+            }
+            pv = block_sum(pv, warp_sums);
+            pq = block_sum(pq, warp_sums);
+            if (tile == ntiles - 1 && threadIdx.x == kScanThreads - 1)
+                mc_counts(a, ctr, pv + (incl & 0xFFFFu), pq + (incl >> 16));
+        } else {
+            pv = tile_sums[tile];
+            pq = tile_sums[ntiles_max + tile];
+        }
 #pragma unroll
         for (uint32_t k = 0; k < kScanItems; ++k) {
             const uint64_t t = base + threadIdx.x * kScanItems + k;
@@ -1934,7 +1994,15 @@ void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t*
 void launch_band_list(const KernelCtx& c, const uint32_t* bits, const uint32_t* prefix, uint32_t nwords,
                       uint32_t* sv, uint32_t cap, const GroupMark& gm, Counters* ctr)
 {
-    k_band_list<<<persistent_blocks(c, nwords, 16), bs(c), 0, c.stream>>>(bits, prefix, nwords, sv, cap, gm, ctr);
+    // A warp per word while the words make no more than a few rounds of warps;
+    // most words of a large grid are empty.  Measured with the scan, a lane per
+    // word / a warp per word (us): coarse grids of 68 words 25 / 12, 2.5k 22 / 12,
+    // 19k 51 / 31; fine grids of 24k and of 130k 20.5 / 20.5, 754k 33 / 80.
+    if (nwords <= 1u << 17)
+        k_band_list_words<<<persistent_blocks(c, 32ull * nwords, 8), bs(c), 0, c.stream>>>(bits, prefix, nwords, sv,
+                                                                                        cap, gm, ctr);
+    else
+        k_band_list<<<persistent_blocks(c, nwords, 16), bs(c), 0, c.stream>>>(bits, prefix, nwords, sv, cap, gm, ctr);
     ++g_launches;
 }
 
@@ -1998,25 +2066,28 @@ void launch_cov(const KernelCtx& c, const CovArgs& a0, Counters* ctr)
     ++g_launches;
 }
 
-void launch_mc_classify(const KernelCtx& c, const McArgs& a, Counters* ctr)
+void launch_mc_classify(const KernelCtx& c, const McArgs& a, Counters* ctr, uint32_t* scratch)
 {
-    k_mc_classify<<<persistent_blocks(c, a.cap_band, 16), bs(c), 0, c.stream>>>(a, ctr);
+    k_mc_classify<<<persistent_blocks(c, a.cap_band, 16), bs(c), 0, c.stream>>>(a, ctr, scratch);
     ++g_launches;
 }
 
-size_t mc_offsets_scratch_words(uint32_t cap_band)
-{
-    return 2 * (size_t)((cap_band + kScanTile - 1) / kScanTile) + 2;
-}
+uint32_t mc_tiles(uint32_t cap_band) { return (cap_band + kScanTile - 1) / kScanTile; }
+
+size_t mc_offsets_scratch_words(uint32_t cap_band) { return 2 * (size_t)mc_tiles(cap_band) + 2; }
 
 void launch_mc_offsets(const KernelCtx& c, const McArgs& a, Counters* ctr, uint32_t* scratch)
 {
-    const uint32_t ntiles_max = (a.cap_band + kScanTile - 1) / kScanTile;
+    const uint32_t ntiles_max = mc_tiles(a.cap_band);
     const uint32_t g = std::max<uint32_t>(1, std::min<uint32_t>(ntiles_max, 65535));
-    k_mc_tile_reduce<<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
+    if (ntiles_max <= kSumTiles) {
+        k_mc_tile_scan<true><<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
+        ++g_launches;
+        return;
+    }
     k_mc_scan_tile_sums<<<1, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
-    k_mc_tile_scan<<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
-    g_launches += 3;
+    k_mc_tile_scan<false><<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
+    g_launches += 2;
 }
 
 void launch_mc_generate(const KernelCtx& c, const McArgs& a, Counters* ctr)

@@ -57,6 +57,8 @@ struct GroupMark {
     Grid sp, sc;
     uint32_t* gflag;
     uint32_t* glist;
+    uint32_t* tile_sums;  // zeroed on the way: ntiles words for launch_mc_classify
+    uint32_t ntiles;
 };
 void launch_band_list(const KernelCtx& c, const uint32_t* bits, const uint32_t* prefix, uint32_t nwords,
                       uint32_t* sv, uint32_t cap, const GroupMark& gm, Counters* ctr);
@@ -192,10 +194,13 @@ struct McArgs {
     int host_mc;           // Akinci12: the host marching cubes' normal/lerp rules
     uint32_t cap_band, cap_valid, cap_mesh;
 };
-void launch_mc_classify(const KernelCtx& c, const McArgs& a, Counters* ctr);
-// vofs, the valid cube list and the vertex / cube counts from the classify
-// words (3 launches); scratch: mc_offsets_scratch_words(cap_band) words
+// scratch: mc_offsets_scratch_words(cap_band) words, the first mc_tiles(cap_band)
+// of them 0 (launch_band_list); the classification leaves the tiles' sums there
+uint32_t mc_tiles(uint32_t cap_band);
 size_t mc_offsets_scratch_words(uint32_t cap_band);
+void launch_mc_classify(const KernelCtx& c, const McArgs& a, Counters* ctr, uint32_t* scratch);
+// vofs, the valid cube list and the vertex / cube counts from the classify
+// words and the tiles' sums
 void launch_mc_offsets(const KernelCtx& c, const McArgs& a, Counters* ctr, uint32_t* scratch);
 void launch_mc_generate(const KernelCtx& c, const McArgs& a, Counters* ctr);
 

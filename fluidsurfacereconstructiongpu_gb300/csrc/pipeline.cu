@@ -422,7 +422,9 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
                 (uint32_t*)h->scan_tmp.ptr, st));
     uint32_t* sv = (uint32_t*)h->sv.ptr;
     launch_band_list(kc, bits, prefix, nwords, sv, h->cap_band,
-                     GroupMark{sp, sc, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr}, ctr);
+                     GroupMark{sp, sc, (uint32_t*)h->gflag.ptr, (uint32_t*)h->glist.ptr, (uint32_t*)h->scan_tmp.ptr,
+                               mc_tiles(h->cap_band)},
+                     ctr);
     mark(4);
 
     // ---- field
@@ -511,7 +513,7 @@ fsr_status frame_enqueue(fsr_handle* h, const FramePlan& fp, const float* d_xyz,
     ma.cap_mesh = h->cap_mesh;
     const bool weld = (p.flags & FSR_FLAG_WELD) != 0;
     ma.out_key = weld ? (uint64_t*)h->wkey.ptr : nullptr;
-    launch_mc_classify(kc, ma, ctr);
+    launch_mc_classify(kc, ma, ctr, (uint32_t*)h->scan_tmp.ptr);
     mark(8);
     launch_mc_offsets(kc, ma, ctr, (uint32_t*)h->scan_tmp.ptr);
     mark(9);

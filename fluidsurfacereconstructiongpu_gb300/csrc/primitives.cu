@@ -68,15 +68,19 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(uint32_t* tile_
     if (threadIdx.x == 0 && total) *total = carry;
 }
 
-template <ScanInput M>
+// kSums: the tiles' sums come unscanned and each block adds up those before its
+// own tile; the last tile's block writes the total.
+template <ScanInput M, bool kSums>
 __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, uint32_t* out,
                                                             uint32_t n_host, const uint32_t* n_dev,
-                                                            uint32_t n_max, const uint32_t* tile_prefix)
+                                                            uint32_t n_max, const uint32_t* tile_sums,
+                                                            uint32_t* total)
 {
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t tile_vals[kScanTilePadded];
     const uint32_t n = count_of(n_host, n_dev, n_max);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
+    if (kSums && ntiles == 0 && total && blockIdx.x == 0 && threadIdx.x == 0) *total = 0u;
     for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t base = (uint64_t)tile * kScanTile;
         // coalesced load into shared memory
@@ -96,7 +100,9 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
             s += local[k];
         }
         const uint32_t incl = block_inclusive_scan(s, warp_sums);
-        uint32_t run = tile_prefix[tile] + incl - s;
+        const uint32_t before = kSums ? sum_before(tile_sums, tile, warp_sums) : tile_sums[tile];
+        uint32_t run = before + incl - s;
+        if (kSums && total && tile == ntiles - 1 && threadIdx.x == kScanThreads - 1) *total = before + incl;
 #pragma unroll
         for (uint32_t k = 0; k < kScanItems; ++k) {
             tile_vals[scan_slot(threadIdx.x * kScanItems + k)] = run;
@@ -118,8 +124,13 @@ void launch_scan(uint32_t g, const uint32_t* in, uint32_t* out, uint32_t n_host,
                  uint32_t n_max, uint32_t* total, uint32_t* scratch, cudaStream_t stream)
 {
     k_tile_reduce<M><<<g, kScanThreads, 0, stream>>>(in, n_host, n_dev, n_max, scratch);
+    if (g <= kSumTiles) {
+        k_tile_scan<M, true><<<g, kScanThreads, 0, stream>>>(in, out, n_host, n_dev, n_max, scratch, total);
+        g_launches += 2;
+        return;
+    }
     k_scan_tile_sums<<<1, kScanThreads, 0, stream>>>(scratch, n_host, n_dev, n_max, total);
-    k_tile_scan<M><<<g, kScanThreads, 0, stream>>>(in, out, n_host, n_dev, n_max, scratch);
+    k_tile_scan<M, false><<<g, kScanThreads, 0, stream>>>(in, out, n_host, n_dev, n_max, scratch, nullptr);
     g_launches += 3;
 }
 
@@ -134,7 +145,9 @@ uint32_t grid_for_tiles(uint64_t n_max)
 // tile and a running carry.  One launch instead of three.
 constexpr uint32_t kSingleThreads = 1024;
 constexpr uint32_t kSingleMax = 1u << 14;  // longer arrays take the tiled three-kernel scan (one block is slower from ~64k on)
-__global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* in, uint32_t* out, uint32_t n)
+template <ScanInput M>
+__global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* in, uint32_t* out, uint32_t n,
+                                                                uint32_t* total)
 {
     __shared__ uint32_t warp_sums[kSingleThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -143,7 +156,7 @@ __global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* 
         const uint32_t i0 = base + 4 * threadIdx.x;
         uint32_t v[4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = i0 + k < n ? in[i0 + k] : 0u;
+        for (int k = 0; k < 4; ++k) v[k] = i0 + k < n ? scan_load<M>(in, i0 + k) : 0u;
         const uint32_t s = v[0] + v[1] + v[2] + v[3];
         uint32_t x = s;
 #pragma unroll
@@ -172,6 +185,7 @@ __global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* 
         carry += warp_sums[kSingleThreads / 32 - 1];
         __syncthreads();  // warp_sums is rewritten by the next tile
     }
+    if (total && threadIdx.x == 0) *total = carry;
 }
 
 // ---------------------------------------------------------------- radix
@@ -276,6 +290,11 @@ cudaError_t scan_u32(const uint32_t* in, uint32_t* out, uint32_t n_host, const u
         if (total) return cudaMemsetAsync(total, 0, sizeof(uint32_t), stream);
         return cudaSuccess;
     }
+    if (mode == ScanInput::kPopcount && !n_dev && n_host <= kSingleMax && n_host <= n_max) {
+        k_scan_single<ScanInput::kPopcount><<<1, kSingleThreads, 0, stream>>>(in, out, n_host, total);
+        ++g_launches;
+        return cudaGetLastError();
+    }
     const uint32_t g = grid_for_tiles(n_max);
     switch (mode) {
     case ScanInput::kValue: launch_scan<ScanInput::kValue>(g, in, out, n_host, n_dev, n_max, total, scratch, stream); break;
@@ -289,7 +308,7 @@ cudaError_t scan_counts(uint32_t* counts, uint32_t n, uint32_t* scratch, cudaStr
 {
     if (n > kSingleMax)
         return scan_u32(counts, counts, n, nullptr, n, nullptr, ScanInput::kValue, scratch, stream);
-    k_scan_single<<<1, kSingleThreads, 0, stream>>>(counts, counts, n);
+    k_scan_single<ScanInput::kValue><<<1, kSingleThreads, 0, stream>>>(counts, counts, n, nullptr);
     ++g_launches;
     return cudaGetLastError();
 }

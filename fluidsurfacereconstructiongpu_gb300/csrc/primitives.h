@@ -13,6 +13,13 @@ constexpr uint32_t kScanThreads = 256;
 constexpr uint32_t kScanItems = 16;
 constexpr uint32_t kScanTile = kScanThreads * kScanItems;  // 4096
 
+// Up to this many tiles the blocks of a scan's last kernel add up the sums of the
+// tiles before their own, beyond it a kernel of one block scans them first.  With
+// the line at 4096 / 16384 tiles (us): marking and listing a band of 7652 tiles of
+// words 257 / 238, offsets of 9M vertices 35 / 29 (43 with that kernel and a pass
+// for the tiles' sums).
+constexpr uint32_t kSumTiles = 16384;
+
 // What the scan reads: u32 elements, or the popcount of each u32 word.
 enum class ScanInput : int {
     kValue = 0,          // the element
@@ -54,6 +61,25 @@ __device__ __forceinline__ uint32_t block_inclusive_scan(uint32_t x, uint32_t* w
     __syncthreads();
     const uint32_t add = warp ? warp_sums[warp - 1] : 0u;
     return x + add;
+}
+
+// Sum of one value per thread over the block, to every thread.
+__device__ __forceinline__ uint32_t block_sum(uint32_t x, uint32_t* warp_sums)
+{
+    x = __reduce_add_sync(0xffffffffu, x);
+    __syncthreads();  // warp_sums' last readers
+    if ((threadIdx.x & 31u) == 0) warp_sums[threadIdx.x >> 5] = x;
+    __syncthreads();
+    const uint32_t lane = threadIdx.x & 31u;
+    return __reduce_add_sync(0xffffffffu, lane < kScanThreads / 32 ? warp_sums[lane] : 0u);
+}
+
+// sums[0] + ... + sums[tile - 1], by the block.
+__device__ __forceinline__ uint32_t sum_before(const uint32_t* sums, uint32_t tile, uint32_t* warp_sums)
+{
+    uint32_t x = 0;
+    for (uint32_t i = threadIdx.x; i < tile; i += kScanThreads) x += __ldg(sums + i);
+    return block_sum(x, warp_sums);
 }
 #endif
 

@@ -47,6 +47,7 @@ constexpr int kT = 256;
 template <bool kRadius>
 __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* ctr, double* radius)
 {
+    after_launch();
     __shared__ float s_val[8 * kT], s_g[8 * kT];  // [corner][thread]
     float* val = s_val + threadIdx.x;
     float* g = s_g + threadIdx.x;
@@ -206,6 +207,7 @@ __device__ __forceinline__ void window_box(const BwdArgs& a, const int c[3], int
 // ---------------------------------------------------------------- anisotropic field
 __global__ void k_field_backward_aniso(BwdArgs a)
 {
+    after_launch();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= a.n) return;
     const float4 q = a.sorted[j];
@@ -281,6 +283,7 @@ __global__ void k_field_backward_aniso(BwdArgs a)
 // the grouped adjoint has accumulated the sum in gsmooth.w.
 __global__ void k_det_term(BwdArgs a)
 {
+    after_launch();
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= a.n || !a.invol[a.skeys[j]]) return;
     const float sc = a.gsmooth[j].w;
@@ -506,6 +509,7 @@ constexpr int kCovBT = 64;
 template <int P, bool kSets>
 __global__ void __launch_bounds__(kCovBT, 12) k_cov_backward(BwdArgs a, CovArgs f)
 {
+    after_launch();
     __shared__ float4 s_q[kCovBT];  // 32 staged particles per warp
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / P;
     const bool first = threadIdx.x % P == 0;
@@ -602,6 +606,7 @@ __global__ void __launch_bounds__(kT) k_smooth_backward(BwdArgs a, const float4*
                                                         const uint2* ranges, Grid sp, uint32_t n, float R, float R_lt2,
                                                         int coop_ok, float lambda)
 {
+    after_launch();
     __shared__ float4 s_q[kT];  // 32 staged particles per warp
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / P;
     const bool first = threadIdx.x % P == 0;
@@ -651,6 +656,7 @@ __global__ void __launch_bounds__(kT) k_smooth_backward(BwdArgs a, const float4*
 
 __global__ void k_unsort(const float4* gx, const uint32_t* perm, uint32_t n, float* out)
 {
+    after_launch();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const float4 g = gx[k];
@@ -669,8 +675,8 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
 {
     const unsigned pb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_valid + kT - 1) / kT,
                                                                           (uint64_t)c.num_sms * 16));
-    if (radius_grad_dev) k_mc_backward<true><<<pb, kT, 0, c.stream>>>(a, ctr, radius_grad_dev);
-    else k_mc_backward<false><<<pb, kT, 0, c.stream>>>(a, ctr, nullptr);
+    if (radius_grad_dev) launch_after(k_mc_backward<true>, pb, kT, 0, c.stream, a, ctr, radius_grad_dev);
+    else launch_after(k_mc_backward<false>, pb, kT, 0, c.stream, a, ctr, nullptr);
     ++g_launches;
     if (method == FSR_METHOD_YU13) {
         AnisoBwdArgs fb{};
@@ -690,16 +696,16 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
         fb.sigma = a.sigma;
         fb.cap = a.cap_band;
         if (launch_field_aniso_backward_grouped(c, fb, a.ratio, ctr)) {
-            k_det_term<<<nblk(a.n), kT, 0, c.stream>>>(a);
+            launch_after(k_det_term, nblk(a.n), kT, 0, c.stream, a);
         } else {
-            k_field_backward_aniso<<<nblk(a.n), kT, 0, c.stream>>>(a);
+            launch_after(k_field_backward_aniso, nblk(a.n), kT, 0, c.stream, a);
         }
         // warps may walk the union of their windows when the cull radius stays below 2 cells
         const int smooth_coop = (R * 1.0001f + 1e-4f * cov->sp.cs) < 2.0f * cov->sp.cs * 0.9999f ? 1 : 0;
         auto launch = [&](auto cov_kernel, auto smooth_kernel, uint64_t lanes) {
-            cov_kernel<<<(unsigned)((a.n * lanes + kCovBT - 1) / kCovBT), kCovBT, 0, c.stream>>>(a, *cov);
-            smooth_kernel<<<nblk(a.n * lanes), kT, 0, c.stream>>>(a, cov->sorted, cov->mean, cov->ranges, cov->sp, a.n, R,
-                                                                  cov->R_lt2, smooth_coop, lambda);
+            launch_after(cov_kernel, (unsigned)((a.n * lanes + kCovBT - 1) / kCovBT), kCovBT, 0, c.stream, a, *cov);
+            launch_after(smooth_kernel, nblk(a.n * lanes), kT, 0, c.stream, a, cov->sorted, cov->mean, cov->ranges,
+                         cov->sp, a.n, R, cov->R_lt2, smooth_coop, lambda);
         };
         const bool sets = cov->coop_ok == 0;  // R near or above a cell
         if (a.n < (sets ? 131072u : 40960u)) {
@@ -716,7 +722,7 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
     } else {
         launch_field_iso_backward(c, a, method == FSR_METHOD_TC01, ctr);
     }
-    k_unsort<<<nblk(a.n), kT, 0, c.stream>>>(a.gx, a.perm, a.n, out_grad_xyz);
+    launch_after(k_unsort, nblk(a.n), kT, 0, c.stream, a.gx, a.perm, a.n, out_grad_xyz);
     ++g_launches;
 }
 

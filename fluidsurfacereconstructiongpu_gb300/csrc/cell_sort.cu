@@ -30,6 +30,7 @@ constexpr uint32_t kDenseParticles = 16;
 __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp, uint32_t* __restrict__ keys,
                              uint32_t* __restrict__ arrival, uint32_t* __restrict__ count, Counters* ctr)
 {
+    after_launch();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     const bool there = i < n;
@@ -60,6 +61,7 @@ __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __res
                         float* __restrict__ cell_rmax, uint32_t* __restrict__ gflag, uint32_t* __restrict__ big,
                         Counters* ctr)
 {
+    after_launch();
     const uint32_t stride = gridDim.x * blockDim.x, start = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t i = start; i < n; i += stride) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
     const uint32_t kx = sp.res[0] + 1, ky = sp.res[1] + 1;
@@ -101,6 +103,7 @@ struct CellSortOut {
 __global__ void k_cell_rank(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ first,
                             const uint32_t* __restrict__ grouped, uint32_t n, CellSortOut out)
 {
+    after_launch();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t i = grouped[k];
@@ -126,6 +129,7 @@ __global__ void __launch_bounds__(kBigThreads) k_big_cells(const uint32_t* __res
                                                            uint32_t digits, CellSortOut out,
                                                            const uint32_t* __restrict__ big, const Counters* ctr)
 {
+    after_launch();
     __shared__ uint32_t whist[kBigWarps][256];
     __shared__ uint32_t base[256];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
@@ -202,21 +206,21 @@ cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ct
     const uint32_t cells = a.sp.res[0] * a.sp.res[1] * a.sp.res[2];
     const uint32_t groups = (a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
     cudaError_t e = cudaSuccess;
-    k_hash_count<<<blocks, threads, 0, c.stream>>>(a.xyz, a.n, a.sp, a.keys, a.arrival, a.first, ctr);
+    launch_after(k_hash_count, blocks, threads, 0, c.stream, a.xyz, a.n, a.sp, a.keys, a.arrival, a.first, ctr);
     ++g_launches;
     // in place: first[cells] becomes the number of particles
     if ((e = scan_counts(a.first, cells + 1u, a.scan_tmp, c.stream)) != cudaSuccess) return e;
     const unsigned gblocks = (unsigned)std::min<uint64_t>(((uint64_t)std::max(a.n, groups) + threads - 1) / threads,
                                                           (uint64_t)std::max(1, c.num_sms) * 32);
-    k_group<<<gblocks, threads, 0, c.stream>>>(a.keys, a.arrival, a.first, a.n, a.sp, cells, groups, a.grouped, a.ranges, a.occ,
-                                               a.cell_rmax, a.gflag, a.big, ctr);
+    launch_after(k_group, gblocks, threads, 0, c.stream, a.keys, a.arrival, a.first, a.n, a.sp, cells, groups,
+                 a.grouped, a.ranges, a.occ, a.cell_rmax, a.gflag, a.big, ctr);
     const CellSortOut out{a.xyz, a.dens, a.sorted, a.skeys, a.perm};
-    k_cell_rank<<<blocks, threads, 0, c.stream>>>(a.keys, a.first, a.grouped, a.n, out);
+    launch_after(k_cell_rank, blocks, threads, 0, c.stream, a.keys, a.first, a.grouped, a.n, out);
     g_launches += 2;
     if (a.n > kBigCell) {
         const uint32_t most = a.n / kBigCell;
-        k_big_cells<<<std::min<uint32_t>(most, (uint32_t)std::max(1, c.num_sms)), kBigThreads, 0, c.stream>>>(
-            a.first, a.grouped, (bits_for(a.n) + 7u) / 8u, out, a.big, ctr);
+        launch_after(k_big_cells, std::min<uint32_t>(most, (uint32_t)std::max(1, c.num_sms)), kBigThreads, 0, c.stream,
+                     a.first, a.grouped, (bits_for(a.n) + 7u) / 8u, out, a.big, ctr);
         ++g_launches;
     }
     return cudaGetLastError();

@@ -745,6 +745,7 @@ __device__ __forceinline__ float unscaled_sum(const float* m, float zx, float zy
 // A vertex's sum takes the candidates in window order.
 __global__ void __launch_bounds__(kFT, FSR_FIELD_MIN_BLOCKS) k_field_aniso_grouped(GroupArgs a, uint32_t ratio, Counters* ctr)
 {
+    after_launch();
     __shared__ WarpSlice slices[kFWarps];
     const int lane = threadIdx.x & 31;
     WarpSlice& w = slices[threadIdx.x >> 5];
@@ -1047,6 +1048,7 @@ __device__ __forceinline__ bool within(float4 q, float4 lo, float4 hi, float r2)
 template <bool TC01>
 __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, BandView band, uint32_t ratio, Counters* ctr)
 {
+    after_launch();
     __shared__ IsoSlice slices[kFWarps];
     const int lane = threadIdx.x & 31;
     IsoSlice& w = slices[threadIdx.x >> 5];
@@ -1271,6 +1273,7 @@ __device__ __forceinline__ float box_dist2(float x, float y, float z, float4 lo,
 
 __global__ void k_field_aniso_backward_grouped(BwdGroupArgs a, uint32_t ratio, const Counters* ctr)
 {
+    after_launch();
     extern __shared__ __align__(16) unsigned char smem[];
     const uint32_t nch_cap = (a.vlist_cap + 31) / 32;
     float4* av = reinterpret_cast<float4*>(smem);            // active vertices: (v, dL/dphi)
@@ -1493,6 +1496,7 @@ struct IsoBwdSlice {
 template <bool TC01>
 __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const Counters* ctr)
 {
+    after_launch();
     __shared__ IsoBwdSlice<TC01> slices[kFWarps];
     const int lane = threadIdx.x & 31;
     IsoBwdSlice<TC01>& w = slices[threadIdx.x >> 5];
@@ -1695,7 +1699,7 @@ bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs&
     const uint64_t groups = (uint64_t)(f.sp.res[0] + 1) * (f.sp.res[1] + 1) * (f.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
         groups, std::max<uint64_t>(1, (uint64_t)c.num_sms * 8 / std::max(1, c.grid_div)));
-    k_field_aniso_backward_grouped<<<grid, kBT, smem, c.stream>>>(a, ratio, ctr);
+    launch_after(k_field_aniso_backward_grouped, grid, kBT, smem, c.stream, a, ratio, ctr);
     ++g_launches;
     return true;
 }
@@ -1721,7 +1725,7 @@ void launch_field_aniso_grouped(const KernelCtx& c, const AnisoFieldArgs& f, con
     const uint64_t groups = (uint64_t)(f.sp.res[0] + 1) * (f.sp.res[1] + 1) * (f.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
         (groups + kFWarps - 1) / kFWarps, std::max<uint64_t>(1, (uint64_t)c.num_sms * 16 / std::max(1, c.grid_div)));
-    k_field_aniso_grouped<<<grid, kFT, 0, c.stream>>>(a, ratio, ctr);
+    launch_after(k_field_aniso_grouped, grid, kFT, 0, c.stream, a, ratio, ctr);
     ++g_launches;
 }
 
@@ -1730,8 +1734,8 @@ void launch_field_iso_backward(const KernelCtx& c, const BwdArgs& a, bool tc01, 
     const uint64_t groups = (uint64_t)(a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
         (groups * kSlabMax + kFWarps - 1) / kFWarps, std::max<uint64_t>(1, (uint64_t)c.num_sms * 12 / std::max(1, c.grid_div)));
-    if (tc01) k_field_iso_backward<true><<<grid, kFT, 0, c.stream>>>(a, ctr);
-    else k_field_iso_backward<false><<<grid, kFT, 0, c.stream>>>(a, ctr);
+    if (tc01) launch_after(k_field_iso_backward<true>, grid, kFT, 0, c.stream, a, ctr);
+    else launch_after(k_field_iso_backward<false>, grid, kFT, 0, c.stream, a, ctr);
     ++g_launches;
 }
 
@@ -1741,8 +1745,8 @@ void launch_field_iso_grouped(const KernelCtx& c, bool tc01, const IsoFieldArgs&
     const uint64_t groups = (uint64_t)(f.sp.res[0] + 1) * (f.sp.res[1] + 1) * (f.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
         (groups + kFWarps - 1) / kFWarps, std::max<uint64_t>(1, (uint64_t)c.num_sms * 16 / std::max(1, c.grid_div)));
-    if (tc01) k_field_iso_grouped<true><<<grid, kFT, 0, c.stream>>>(f, band, ratio, ctr);
-    else k_field_iso_grouped<false><<<grid, kFT, 0, c.stream>>>(f, band, ratio, ctr);
+    if (tc01) launch_after(k_field_iso_grouped<true>, grid, kFT, 0, c.stream, f, band, ratio, ctr);
+    else launch_after(k_field_iso_grouped<false>, grid, kFT, 0, c.stream, f, band, ratio, ctr);
     ++g_launches;
 }
 

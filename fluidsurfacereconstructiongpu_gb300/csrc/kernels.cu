@@ -59,6 +59,7 @@ __device__ __forceinline__ void warp_count(uint32_t* counter, bool pred)
 __global__ void k_hash(const float* __restrict__ xyz, uint32_t n, Grid sp, uint32_t* __restrict__ keys,
                        uint32_t* __restrict__ vals, Counters* ctr)
 {
+    after_launch();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float p[3] = {xyz[3ull * i], xyz[3ull * i + 1], xyz[3ull * i + 2]};
@@ -76,6 +77,7 @@ __global__ void k_ranges_gather(const uint32_t* __restrict__ skeys, const uint32
                                 float4* __restrict__ sorted, uint2* __restrict__ ranges,
                                 uint8_t* __restrict__ occ)
 {
+    after_launch();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
     const uint32_t key = skeys[k];
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(kDensityThreads) k_density(const float4* __res
                                                       const uint2* __restrict__ ranges, Grid sp, int ext, float h,
                                                       float h2, float inv_h2, float scale, float* __restrict__ rho)
 {
+    after_launch();
     __shared__ __align__(16) DensitySlice slices[kDensityThreads / 32];
     DensitySlice& S = slices[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31;
@@ -215,6 +218,7 @@ __global__ void __launch_bounds__(kDensityThreads) k_density(const float4* __res
 
 __global__ void k_set_density(float4* __restrict__ sorted, const float* __restrict__ rho, uint32_t n)
 {
+    after_launch();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < n) sorted[t].w = rho[t];
 }
@@ -225,6 +229,7 @@ __global__ void k_set_density(float4* __restrict__ sorted, const float* __restri
 // layer of each axis is never tested (cu:81).
 __global__ void k_surface_cells(Grid sp, const uint8_t* __restrict__ occ, uint8_t* __restrict__ surf)
 {
+    after_launch();
     const uint64_t C = (uint64_t)sp.res[0] * sp.res[1] * sp.res[2];
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= C) return;
@@ -247,6 +252,7 @@ __global__ void k_surface_cells(Grid sp, const uint8_t* __restrict__ occ, uint8_
 __global__ void k_involved_cells(Grid sp, const uint8_t* __restrict__ occ, const uint8_t* __restrict__ surf,
                                  uint8_t* __restrict__ invol)
 {
+    after_launch();
     const uint64_t C = (uint64_t)sp.res[0] * sp.res[1] * sp.res[2];
     const uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= C) return;
@@ -302,6 +308,7 @@ __global__ void __launch_bounds__(kThreads) k_colorfield(const float4* __restric
                                                          float h_rcp, float h_lt2, float tiny, double k_spiky, float khi,
                                                          float klo, float mass, uint8_t* __restrict__ psurf)
 {
+    after_launch();
     __shared__ float4 s_q[kThreads];    // staged candidates, per warp
     __shared__ float s_mr[kThreads];    // their m / rho
     __shared__ uint32_t s_idx[kThreads]; // their sorted index
@@ -448,6 +455,7 @@ __global__ void __launch_bounds__(kColorThreads, 8) k_colorfield_quads(const flo
                                                          float h_rcp, float h_lt2, float tiny, double k_spiky, float khi,
                                                          float klo, float mass, uint8_t* __restrict__ psurf)
 {
+    after_launch();
     __shared__ __align__(16) ColorSlice slices[kColorThreads / 32];
     ColorSlice& S = slices[threadIdx.x >> 5];
     const int lane = threadIdx.x & 31, part = lane >> 2;
@@ -612,6 +620,7 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
                              const uint8_t* __restrict__ surf, const uint8_t* __restrict__ psurf, uint32_t n,
                              Grid sc, float thr2, uint32_t* __restrict__ bits, Counters* ctr)
 {
+    after_launch();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t t = i / kLanes, plane = i % kLanes;
     bool is_s = false;
@@ -674,6 +683,7 @@ __device__ __forceinline__ void band_list_prologue(const GroupMark& gm, uint32_t
 __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix,
                             uint32_t nwords, uint32_t* __restrict__ sv, uint32_t cap, GroupMark gm, Counters* ctr)
 {
+    after_launch();
     const uint32_t kx = gm.sp.res[0] + 1, ky = gm.sp.res[1] + 1;
     const uint32_t rx = gm.sc.res[0], rxy = gm.sc.res[0] * gm.sc.res[1];
     band_list_prologue(gm, cap, ctr);
@@ -734,6 +744,7 @@ __global__ void k_band_list(const uint32_t* __restrict__ bits, const uint32_t* _
 __global__ void k_band_list_words(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ prefix,
                                   uint32_t nwords, uint32_t* __restrict__ sv, uint32_t cap, GroupMark gm, Counters* ctr)
 {
+    after_launch();
     const int kx = (int)gm.sp.res[0] + 1, ky = (int)gm.sp.res[1] + 1;
     band_list_prologue(gm, cap, ctr);
     const uint32_t lane = threadIdx.x & 31u;
@@ -809,6 +820,7 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
                                                      float one_minus_lambda, float lambda, float mass, float4* __restrict__ mean,
                                                      float4* __restrict__ mean32, float4* __restrict__ smoothed)
 {
+    after_launch();
     __shared__ float4 s_q[kThreads];  // 32 staged candidates per warp
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = t < n;
@@ -970,6 +982,7 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
                                                      float one_minus_lambda, float lambda, float mass, float4* __restrict__ mean,
                                                      float4* __restrict__ mean32, float4* __restrict__ smoothed)
 {
+    after_launch();
     __shared__ __align__(16) QuadSlice slices[kQuadThreads / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     QuadSlice& S = slices[warp];
@@ -1257,6 +1270,7 @@ constexpr uint32_t kCovWideBelow = 12288;      // and P = 16 with kSets
 template <int P, bool kFast, bool kSets>
 __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs a, Counters* ctr)
 {
+    after_launch();
     __shared__ float4 s_q[kCovThreads];  // 32 staged candidates per warp
     const uint32_t t = (blockIdx.x * blockDim.x + threadIdx.x) / P;
     const uint32_t sub = threadIdx.x % P;
@@ -1528,6 +1542,7 @@ __device__ __forceinline__ uint32_t mc_pair(uint32_t info)
 // valid when all 8 corners are band vertices and the case emits triangles.
 __global__ void k_mc_classify(McArgs a, const Counters* ctr, uint32_t* tile_sums)
 {
+    after_launch();
     const uint32_t nb = min(ctr->n_band, a.cap_band);
     const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
     const uint32_t lane = threadIdx.x & 31u;
@@ -1610,6 +1625,7 @@ __device__ __forceinline__ void mc_counts(const McArgs& a, Counters* ctr, uint32
 __global__ void __launch_bounds__(kScanThreads) k_mc_scan_tile_sums(McArgs a, Counters* ctr, uint32_t* tile_sums,
                                                                     uint32_t ntiles_max)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t last[2];
     const uint32_t n = min(ctr->n_band, a.cap_band);
@@ -1636,6 +1652,7 @@ template <bool kSums>
 __global__ void __launch_bounds__(kScanThreads) k_mc_tile_scan(McArgs a, Counters* ctr, const uint32_t* tile_sums,
                                                                uint32_t ntiles_max)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t tile_vals[kScanTilePadded];
     const uint32_t n = min(ctr->n_band, a.cap_band);
@@ -1731,6 +1748,7 @@ __device__ __forceinline__ int mc_nz_slot(int cx, int cy, int cz) { return 24 + 
 
 __global__ void __launch_bounds__(kThreads) k_mc_generate(McArgs a, const Counters* ctr)
 {
+    after_launch();
     // per thread: the cube's 32 field values, then corner values and normals
     // ([slot][thread]), so that the cut edges can index them without
     // spilling registers
@@ -1875,6 +1893,7 @@ __global__ void __launch_bounds__(kThreads) k_mc_generate(McArgs a, const Counte
 __global__ void k_particle_flags(const uint32_t* __restrict__ skeys, const uint8_t* __restrict__ surf,
                                  const uint8_t* __restrict__ psurf, uint32_t n, uint32_t* __restrict__ out)
 {
+    after_launch();
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= n) return;
     out[t] = psurf ? psurf[t] : surf[skeys[t]];
@@ -1905,7 +1924,7 @@ void launch_hash(const KernelCtx& c, const float* xyz, uint32_t n, const Grid& s
                  uint32_t* vals, Counters* ctr)
 {
     if (!n) return;
-    k_hash<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(xyz, n, sp, keys, vals, ctr);
+    launch_after(k_hash, blocks_for(n, bs(c)), bs(c), 0, c.stream, xyz, n, sp, keys, vals, ctr);
     ++g_launches;
 }
 
@@ -1913,7 +1932,8 @@ void launch_ranges_gather(const KernelCtx& c, const uint32_t* skeys, const uint3
                           const float* xyz, const float* dens, float4* sorted, uint2* ranges, uint8_t* occ)
 {
     if (!n) return;
-    k_ranges_gather<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(skeys, perm, n, xyz, dens, sorted, ranges, occ);
+    launch_after(k_ranges_gather, blocks_for(n, bs(c)), bs(c), 0, c.stream, skeys, perm, n, xyz, dens, sorted, ranges,
+                 occ);
     ++g_launches;
 }
 
@@ -1925,15 +1945,16 @@ void launch_density(const KernelCtx& c, float4* sorted, uint32_t n, const uint2*
     const float h2 = h * h;
     const float sigma = 315.0f / (64.0f * 3.1415926535898f);
     const float scale = mass * sigma / (h * h * h);
-    k_density<<<blocks_for(n, kDensityThreads), kDensityThreads, 0, c.stream>>>(sorted, n, ranges, sp, ext, h, h2, 1.0f / h2, scale, rho);
-    k_set_density<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, rho, n);
+    launch_after(k_density, blocks_for(n, kDensityThreads), kDensityThreads, 0, c.stream, sorted, n, ranges, sp, ext, h,
+                 h2, 1.0f / h2, scale, rho);
+    launch_after(k_set_density, blocks_for(n, bs(c)), bs(c), 0, c.stream, sorted, rho, n);
     g_launches += 2;
 }
 
 void launch_surface_cells(const KernelCtx& c, const Grid& sp, const uint8_t* occ, uint8_t* surf)
 {
     const uint64_t C = (uint64_t)sp.res[0] * sp.res[1] * sp.res[2];
-    k_surface_cells<<<blocks_for(C, bs(c)), bs(c), 0, c.stream>>>(sp, occ, surf);
+    launch_after(k_surface_cells, blocks_for(C, bs(c)), bs(c), 0, c.stream, sp, occ, surf);
     ++g_launches;
 }
 
@@ -1941,7 +1962,7 @@ void launch_involved_cells(const KernelCtx& c, const Grid& sp, const uint8_t* oc
                            uint8_t* invol)
 {
     const uint64_t C = (uint64_t)sp.res[0] * sp.res[1] * sp.res[2];
-    k_involved_cells<<<blocks_for(C, bs(c)), bs(c), 0, c.stream>>>(sp, occ, surf, invol);
+    launch_after(k_involved_cells, blocks_for(C, bs(c)), bs(c), 0, c.stream, sp, occ, surf, invol);
     ++g_launches;
 }
 
@@ -1965,12 +1986,12 @@ void launch_colorfield(const KernelCtx& c, const float4* sorted, uint32_t n, con
     // 1.29 / 1.75
     if (n < 98304u) {
         const auto kernel = fast ? k_colorfield_quads<true> : k_colorfield_quads<false>;
-        kernel<<<blocks_for(4ull * n, kColorThreads), kColorThreads, 0, c.stream>>>(
-            sorted, n, ranges, sp, h, 1.0f / h, sqrt_threshold(h, false), tiny_d2(h), k, khi, klo, mass, psurf);
+        launch_after(kernel, blocks_for(4ull * n, kColorThreads), kColorThreads, 0, c.stream, sorted, n, ranges, sp, h,
+                     1.0f / h, sqrt_threshold(h, false), tiny_d2(h), k, khi, klo, mass, psurf);
     } else {
         const auto kernel = fast ? k_colorfield<true> : k_colorfield<false>;
-        kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, h, 1.0f / h, sqrt_threshold(h, false),
-                                                             tiny_d2(h), k, khi, klo, mass, psurf);
+        launch_after(kernel, blocks_for(n, bs(c)), bs(c), 0, c.stream, sorted, n, ranges, sp, h, 1.0f / h,
+                     sqrt_threshold(h, false), tiny_d2(h), k, khi, klo, mass, psurf);
     }
     ++g_launches;
 }
@@ -1982,8 +2003,8 @@ void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t*
     if (!n) return;
     const float thr2 = sqrt_threshold(thr, true);
     auto launch = [&](auto kernel, uint32_t lanes) {
-        kernel<<<blocks_for((uint64_t)n * lanes, bs(c)), bs(c), 0, c.stream>>>(sorted, skeys, surf, psurf, n, sc, thr2, bits,
-                                                                            ctr);
+        launch_after(kernel, blocks_for((uint64_t)n * lanes, bs(c)), bs(c), 0, c.stream, sorted, skeys, surf, psurf, n,
+                     sc, thr2, bits, ctr);
     };
     const bool check = !psurf || sc.cs * 4.0f >= sp.cs;  // (at most 4 grid vertices per cell)
     if (n < 65536u) launch(check ? k_band_stamp<8, true> : k_band_stamp<8, false>, 8);
@@ -1999,10 +2020,11 @@ void launch_band_list(const KernelCtx& c, const uint32_t* bits, const uint32_t* 
     // word / a warp per word (us): coarse grids of 68 words 25 / 12, 2.5k 22 / 12,
     // 19k 51 / 31; fine grids of 24k and of 130k 20.5 / 20.5, 754k 33 / 80.
     if (nwords <= 1u << 17)
-        k_band_list_words<<<persistent_blocks(c, 32ull * nwords, 8), bs(c), 0, c.stream>>>(bits, prefix, nwords, sv,
-                                                                                        cap, gm, ctr);
+        launch_after(k_band_list_words, persistent_blocks(c, 32ull * nwords, 8), bs(c), 0, c.stream, bits, prefix,
+                     nwords, sv, cap, gm, ctr);
     else
-        k_band_list<<<persistent_blocks(c, nwords, 16), bs(c), 0, c.stream>>>(bits, prefix, nwords, sv, cap, gm, ctr);
+        launch_after(k_band_list, persistent_blocks(c, nwords, 16), bs(c), 0, c.stream, bits, prefix, nwords, sv, cap,
+                     gm, ctr);
     ++g_launches;
 }
 
@@ -2027,15 +2049,13 @@ void launch_smooth(const KernelCtx& c, const float4* sorted, uint32_t n, const u
     const bool wide = max_span > 3, fast = fast_radius(R);
     if (n < (wide ? 81920u : 49152u)) {
         const auto kernel = fast ? k_smooth_quads<true> : k_smooth_quads<false>;
-        kernel<<<blocks_for(n, 32), kQuadThreads, 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R,
-                                                                sqrt_threshold(R, false), tiny_d2(R), max_span, oml,
-                                                                lambda, mass, mean, mean32, smoothed);
+        launch_after(kernel, blocks_for(n, 32), kQuadThreads, 0, c.stream, sorted, n, ranges, sp, R, 1.0f / R,
+                     sqrt_threshold(R, false), tiny_d2(R), max_span, oml, lambda, mass, mean, mean32, smoothed);
     } else {
         const auto kernel = wide ? (fast ? k_smooth<true, true> : k_smooth<false, true>)
                                  : (fast ? k_smooth<true, false> : k_smooth<false, false>);
-        kernel<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(sorted, n, ranges, sp, R, 1.0f / R,
-                                                             sqrt_threshold(R, false), tiny_d2(R), max_span, oml, lambda,
-                                                             mass, mean, mean32, smoothed);
+        launch_after(kernel, blocks_for(n, bs(c)), bs(c), 0, c.stream, sorted, n, ranges, sp, R, 1.0f / R,
+                     sqrt_threshold(R, false), tiny_d2(R), max_span, oml, lambda, mass, mean, mean32, smoothed);
     }
     ++g_launches;
 }
@@ -2052,7 +2072,7 @@ void launch_cov(const KernelCtx& c, const CovArgs& a0, Counters* ctr)
     const bool fast = fast_radius(a.R);
     const bool sets = a.coop_ok == 0;
     auto launch = [&](auto kernel, uint32_t lanes) {
-        kernel<<<blocks_for((uint64_t)a.n * lanes, kCovThreads), kCovThreads, 0, c.stream>>>(a, ctr);
+        launch_after(kernel, blocks_for((uint64_t)a.n * lanes, kCovThreads), kCovThreads, 0, c.stream, a, ctr);
     };
     if (sets && a.n < kCovWideBelow) {
         launch(fast ? k_cov<16, true, true> : k_cov<16, false, true>, 16);
@@ -2068,7 +2088,7 @@ void launch_cov(const KernelCtx& c, const CovArgs& a0, Counters* ctr)
 
 void launch_mc_classify(const KernelCtx& c, const McArgs& a, Counters* ctr, uint32_t* scratch)
 {
-    k_mc_classify<<<persistent_blocks(c, a.cap_band, 16), bs(c), 0, c.stream>>>(a, ctr, scratch);
+    launch_after(k_mc_classify, persistent_blocks(c, a.cap_band, 16), bs(c), 0, c.stream, a, ctr, scratch);
     ++g_launches;
 }
 
@@ -2081,18 +2101,18 @@ void launch_mc_offsets(const KernelCtx& c, const McArgs& a, Counters* ctr, uint3
     const uint32_t ntiles_max = mc_tiles(a.cap_band);
     const uint32_t g = std::max<uint32_t>(1, std::min<uint32_t>(ntiles_max, 65535));
     if (ntiles_max <= kSumTiles) {
-        k_mc_tile_scan<true><<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
+        launch_after(k_mc_tile_scan<true>, g, kScanThreads, 0, c.stream, a, ctr, scratch, ntiles_max);
         ++g_launches;
         return;
     }
-    k_mc_scan_tile_sums<<<1, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
-    k_mc_tile_scan<false><<<g, kScanThreads, 0, c.stream>>>(a, ctr, scratch, ntiles_max);
+    launch_after(k_mc_scan_tile_sums, 1, kScanThreads, 0, c.stream, a, ctr, scratch, ntiles_max);
+    launch_after(k_mc_tile_scan<false>, g, kScanThreads, 0, c.stream, a, ctr, scratch, ntiles_max);
     g_launches += 2;
 }
 
 void launch_mc_generate(const KernelCtx& c, const McArgs& a, Counters* ctr)
 {
-    k_mc_generate<<<persistent_blocks(c, a.cap_valid, 16), bs(c), 0, c.stream>>>(a, ctr);
+    launch_after(k_mc_generate, persistent_blocks(c, a.cap_valid, 16), bs(c), 0, c.stream, a, ctr);
     ++g_launches;
 }
 
@@ -2100,7 +2120,7 @@ void launch_particle_flags(const KernelCtx& c, const uint32_t* skeys, const uint
                            uint32_t n, uint32_t* out)
 {
     if (!n) return;
-    k_particle_flags<<<blocks_for(n, bs(c)), bs(c), 0, c.stream>>>(skeys, surf, psurf, n, out);
+    launch_after(k_particle_flags, blocks_for(n, bs(c)), bs(c), 0, c.stream, skeys, surf, psurf, n, out);
     ++g_launches;
 }
 

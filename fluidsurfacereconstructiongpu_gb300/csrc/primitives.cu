@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_reduce(const uint32_t* in
                                                               const uint32_t* n_dev, uint32_t n_max,
                                                               uint32_t* tile_sums)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     const uint32_t n = count_of(n_host, n_dev, n_max);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
@@ -50,6 +51,7 @@ __global__ void __launch_bounds__(kScanThreads) k_scan_tile_sums(uint32_t* tile_
                                                                  const uint32_t* n_dev, uint32_t n_max,
                                                                  uint32_t* total)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     const uint32_t n = count_of(n_host, n_dev, n_max);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
@@ -76,6 +78,7 @@ __global__ void __launch_bounds__(kScanThreads) k_tile_scan(const uint32_t* in, 
                                                             uint32_t n_max, const uint32_t* tile_sums,
                                                             uint32_t* total)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kScanThreads / 32];
     __shared__ uint32_t tile_vals[kScanTilePadded];
     const uint32_t n = count_of(n_host, n_dev, n_max);
@@ -123,14 +126,14 @@ template <ScanInput M>
 void launch_scan(uint32_t g, const uint32_t* in, uint32_t* out, uint32_t n_host, const uint32_t* n_dev,
                  uint32_t n_max, uint32_t* total, uint32_t* scratch, cudaStream_t stream)
 {
-    k_tile_reduce<M><<<g, kScanThreads, 0, stream>>>(in, n_host, n_dev, n_max, scratch);
+    launch_after(k_tile_reduce<M>, g, kScanThreads, 0, stream, in, n_host, n_dev, n_max, scratch);
     if (g <= kSumTiles) {
-        k_tile_scan<M, true><<<g, kScanThreads, 0, stream>>>(in, out, n_host, n_dev, n_max, scratch, total);
+        launch_after(k_tile_scan<M, true>, g, kScanThreads, 0, stream, in, out, n_host, n_dev, n_max, scratch, total);
         g_launches += 2;
         return;
     }
-    k_scan_tile_sums<<<1, kScanThreads, 0, stream>>>(scratch, n_host, n_dev, n_max, total);
-    k_tile_scan<M, false><<<g, kScanThreads, 0, stream>>>(in, out, n_host, n_dev, n_max, scratch, nullptr);
+    launch_after(k_scan_tile_sums, 1, kScanThreads, 0, stream, scratch, n_host, n_dev, n_max, total);
+    launch_after(k_tile_scan<M, false>, g, kScanThreads, 0, stream, in, out, n_host, n_dev, n_max, scratch, nullptr);
     g_launches += 3;
 }
 
@@ -149,6 +152,7 @@ template <ScanInput M>
 __global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* in, uint32_t* out, uint32_t n,
                                                                 uint32_t* total)
 {
+    after_launch();
     __shared__ uint32_t warp_sums[kSingleThreads / 32];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     uint32_t carry = 0;
@@ -201,6 +205,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_hist(const uint32_t* ke
                                                               uint32_t shift, uint32_t ntiles,
                                                               uint32_t* hist)
 {
+    after_launch();
     __shared__ uint32_t h[kRadixBins];
     h[threadIdx.x] = 0;
     __syncthreads();
@@ -224,6 +229,7 @@ __global__ void __launch_bounds__(kRadixThreads) k_radix_scatter(const uint32_t*
                                                                  uint32_t shift, uint32_t ntiles,
                                                                  const uint32_t* offsets)
 {
+    after_launch();
     __shared__ uint32_t whist[kRadixWarps][kRadixBins];
     __shared__ uint32_t base[kRadixBins];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
@@ -291,7 +297,7 @@ cudaError_t scan_u32(const uint32_t* in, uint32_t* out, uint32_t n_host, const u
         return cudaSuccess;
     }
     if (mode == ScanInput::kPopcount && !n_dev && n_host <= kSingleMax && n_host <= n_max) {
-        k_scan_single<ScanInput::kPopcount><<<1, kSingleThreads, 0, stream>>>(in, out, n_host, total);
+        launch_after(k_scan_single<ScanInput::kPopcount>, 1, kSingleThreads, 0, stream, in, out, n_host, total);
         ++g_launches;
         return cudaGetLastError();
     }
@@ -308,7 +314,7 @@ cudaError_t scan_counts(uint32_t* counts, uint32_t n, uint32_t* scratch, cudaStr
 {
     if (n > kSingleMax)
         return scan_u32(counts, counts, n, nullptr, n, nullptr, ScanInput::kValue, scratch, stream);
-    k_scan_single<ScanInput::kValue><<<1, kSingleThreads, 0, stream>>>(counts, counts, n, nullptr);
+    launch_after(k_scan_single<ScanInput::kValue>, 1, kSingleThreads, 0, stream, counts, counts, n, nullptr);
     ++g_launches;
     return cudaGetLastError();
 }
@@ -335,10 +341,10 @@ int radix_sort_pairs(uint32_t* k0, uint32_t* v0, uint32_t* k1, uint32_t* v1, uin
         const uint32_t* vin = cur ? v1 : v0;
         uint32_t* kout = cur ? k0 : k1;
         uint32_t* vout = cur ? v0 : v1;
-        k_radix_hist<<<ntiles, kRadixThreads, 0, stream>>>(kin, n, shift, ntiles, hist);
+        launch_after(k_radix_hist, ntiles, kRadixThreads, 0, stream, kin, n, shift, ntiles, hist);
         const cudaError_t e = scan_counts(hist, nhist, scan_tmp, stream);
         if (e != cudaSuccess) { *err = e; return cur; }
-        k_radix_scatter<<<ntiles, kRadixThreads, 0, stream>>>(kin, vin, kout, vout, n, shift, ntiles, hist);
+        launch_after(k_radix_scatter, ntiles, kRadixThreads, 0, stream, kin, vin, kout, vout, n, shift, ntiles, hist);
         g_launches += 2;
         cur ^= 1;
     }

@@ -38,6 +38,7 @@ __device__ __forceinline__ uint32_t soup_count(const Counters* ctr, uint32_t cap
 
 __global__ void k_weld_insert(WeldArgs a, const Counters* ctr)
 {
+    after_launch();
     const uint32_t n = soup_count(ctr, a.cap);
     const uint32_t mask = a.table_size - 1u;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -60,6 +61,7 @@ __global__ void k_weld_insert(WeldArgs a, const Counters* ctr)
 
 __global__ void k_weld_first(WeldArgs a, const Counters* ctr)
 {
+    after_launch();
     const uint32_t n = soup_count(ctr, a.cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         a.rank[i] = a.table_first[a.slot[i]] == i ? 1u : 0u;
@@ -67,6 +69,7 @@ __global__ void k_weld_first(WeldArgs a, const Counters* ctr)
 
 __global__ void k_weld_emit(WeldArgs a, const Counters* ctr)
 {
+    after_launch();
     const uint32_t n = soup_count(ctr, a.cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t first = a.table_first[a.slot[i]];
@@ -100,13 +103,13 @@ cudaError_t launch_weld(const KernelCtx& c, WeldArgs a, Counters* ctr, uint32_t*
     if (e == cudaSuccess) e = cudaMemsetAsync(a.table_first, 0xFF, 4ull * a.table_size, c.stream);
     if (e != cudaSuccess) return e;
     const unsigned grid = (unsigned)std::max(1, c.num_sms * 8);
-    k_weld_insert<<<grid, 256, 0, c.stream>>>(a, ctr);
-    k_weld_first<<<grid, 256, 0, c.stream>>>(a, ctr);
+    launch_after(k_weld_insert, grid, 256, 0, c.stream, a, ctr);
+    launch_after(k_weld_first, grid, 256, 0, c.stream, a, ctr);
     // numbers of the first occurrences (in place); the count lands in n_weld
     e = scan_u32(a.rank, a.rank, 0, &ctr->n_mesh_verts, a.cap, &ctr->n_weld, ScanInput::kValue, scan_scratch,
                  c.stream);
     if (e != cudaSuccess) return e;
-    k_weld_emit<<<grid, 256, 0, c.stream>>>(a, ctr);
+    launch_after(k_weld_emit, grid, 256, 0, c.stream, a, ctr);
     g_launches += 3;
     return cudaGetLastError();
 }

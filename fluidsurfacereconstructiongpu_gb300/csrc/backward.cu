@@ -10,7 +10,8 @@
 //   Yu13:  phi = sum c_j (1 - |G_j (x~_j - v)|^2)^3 - 1/2, c_j = sigma det(G_j) m/rho_j
 //          (unscaled kernel with G = I, c = sigma m/rho for non-involved particles)
 //     -> dL/dx (ZB05, TC01) or dL/dx~ and dL/dG (Yu13), gathered per particle
-//        over the band vertices of its support and window (k_field_backward_*)
+//        over the band vertices of its support and window (k_field_iso_backward,
+//        k_field_aniso_backward: by window group)
 //   G = (1/h) cbrt(s1 s2 s3) V diag(1/s) V^T, s = eigenvalues of C clamped
 //       from below at max/4, C = (h^2 I + sum w v v^T) / sum w, v = x_j - mean
 //     -> dL/dC by the derivative of a spectral function (Daleckii-Krein form
@@ -133,149 +134,6 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
         for (int o = 16; o > 0; o >>= 1) rad += __shfl_xor_sync(0xffffffffu, rad, o);
         if ((threadIdx.x & 31) == 0 && rad != 0.0) atomicAdd(radius, rad);
     }
-}
-
-// Does any key within +-ext of the particle's cell hold a gradient vertex?
-__device__ __forceinline__ bool near_gradient(const BwdArgs& a, int cx, int cy, int cz, int ext)
-{
-    const int kx = (int)a.sp.res[0] + 1, ky = (int)a.sp.res[1] + 1, kz = (int)a.sp.res[2] + 1;
-    for (int z = max(cz - ext, 0); z <= min(cz + ext, kz - 1); ++z)
-        for (int y = max(cy - ext, 0); y <= min(cy + ext, ky - 1); ++y)
-            for (int x = max(cx - ext, 0); x <= min(cx + ext, kx - 1); ++x)
-                if (a.gkey[((uint32_t)z * ky + y) * kx + x]) return true;
-    return false;
-}
-
-// Visits every band vertex with a non-zero field gradient inside the vertex
-// index box [lo, hi] (inclusive): fn(rank, gphi, vx, vy, vz).
-template <class Fn>
-__device__ __forceinline__ void for_band_vertices(const BwdArgs& a, const int lo[3], const int hi[3], Fn fn)
-{
-    const int n = hi[0] - lo[0] + 1;
-    if (n <= 0 || hi[1] < lo[1] || hi[2] < lo[2]) return;
-    for (int z = lo[2]; z <= hi[2]; ++z) {
-        const float vz = vpos1(z, a.sc.min[2], a.sc.cs);
-        for (int y = lo[1]; y <= hi[1]; ++y) {
-            const float vy = vpos1(y, a.sc.min[1], a.sc.cs);
-            const uint32_t v0 = lin3(lo[0], y, z, a.sc);
-            const uint32_t v1 = v0 + (uint32_t)n;  // exclusive
-            for (uint32_t w = v0 >> 5; w <= (v1 - 1) >> 5; ++w) {
-                uint32_t bits = __ldg(a.band.bits + w);
-                const uint32_t wbase = w << 5;
-                if (wbase < v0) bits &= ~0u << (v0 - wbase);
-                if (v1 - wbase < 32u) bits &= (1u << (v1 - wbase)) - 1u;
-                if (!bits) continue;
-                const uint32_t pre = __ldg(a.band.prefix + w);
-                const uint32_t word = __ldg(a.band.bits + w);
-                while (bits) {
-                    const uint32_t b = __ffs(bits) - 1;
-                    bits &= bits - 1;
-                    const uint32_t rank = pre + __popc(word & ((1u << b) - 1u));
-                    if (rank >= a.cap_band) continue;
-                    const float g = a.gphi[rank];
-                    if (g == 0.f) continue;
-                    const int x = lo[0] + (int)(wbase + b - v0);
-                    fn(rank, g, vpos1(x, a.sc.min[0], a.sc.cs), vy, vz);
-                }
-            }
-        }
-    }
-}
-
-// Vertex index box of the particle's reverse window (vertices whose window,
-// centred on their FP32 cell, contains cell c) intersected with the box of
-// grid vertices within r of point p.
-__device__ __forceinline__ void window_box(const BwdArgs& a, const int c[3], int ext, const float p[3], float r,
-                                           int lo[3], int hi[3])
-{
-    const int w0[3] = {first_vertex<0>(max(c[0] - ext, 0), a.sc, a.sp, a.ratio),
-                       first_vertex<1>(max(c[1] - ext, 0), a.sc, a.sp, a.ratio),
-                       first_vertex<2>(max(c[2] - ext, 0), a.sc, a.sp, a.ratio)};
-    const int w1[3] = {first_vertex<0>(c[0] + ext + 1, a.sc, a.sp, a.ratio) - 1,
-                       first_vertex<1>(c[1] + ext + 1, a.sc, a.sp, a.ratio) - 1,
-                       first_vertex<2>(c[2] + ext + 1, a.sc, a.sp, a.ratio) - 1};
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float inv = 1.0f / a.sc.cs;
-        const int s0 = __float2int_rd((p[k] - r - a.sc.min[k]) * inv);
-        const int s1 = __float2int_ru((p[k] + r - a.sc.min[k]) * inv);
-        lo[k] = max(w0[k], s0);
-        hi[k] = min(w1[k], s1);
-    }
-}
-
-// ---------------------------------------------------------------- anisotropic field
-__global__ void k_field_backward_aniso(BwdArgs a)
-{
-    after_launch();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= a.n) return;
-    const float4 q = a.sorted[j];
-    const int c[3] = {cell1(q.x, a.sp.min[0], a.sp.cs), cell1(q.y, a.sp.min[1], a.sp.cs),
-                      cell1(q.z, a.sp.min[2], a.sp.cs)};
-    const bool involved = a.invol[a.skeys[j]] != 0;
-    float gxs = 0.f, gys = 0.f, gzs = 0.f;                    // dL/dx~
-    float gg[9] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // dL/dG without the det term
-    float sc = 0.f;                                          // sum of dL/dphi (1 - q2)^3
-    if (near_gradient(a, c[0], c[1], c[2], 2)) {
-        float4 r0, g0, g1, g2;
-        if (involved) {
-            r0 = a.grec[4ull * j];
-            g0 = a.grec[4ull * j + 1];
-            g1 = a.grec[4ull * j + 2];
-            g2 = a.grec[4ull * j + 3];
-        } else {
-            const float4 s = a.smoothed[j];
-            r0 = make_float4(s.x, s.y, s.z, 1.0f);
-            g0 = make_float4(1.f, 0.f, 0.f, a.sigma * s.w);
-            g1 = make_float4(0.f, 1.f, 0.f, 0.f);
-            g2 = make_float4(0.f, 0.f, 1.f, 0.f);
-        }
-        const float coef = g0.w;
-        const float p[3] = {r0.x, r0.y, r0.z};
-        int lo[3], hi[3];
-        window_box(a, c, 2, p, sqrtf(r0.w), lo, hi);
-        for_band_vertices(a, lo, hi, [&](uint32_t rank, float g, float vx, float vy, float vz) {
-            const float rx = r0.x - vx, ry = r0.y - vy, rz = r0.z - vz;
-            const float tx = fmaf(g0.x, rx, fmaf(g0.y, ry, g0.z * rz));
-            const float ty = fmaf(g1.x, rx, fmaf(g1.y, ry, g1.z * rz));
-            const float tz = fmaf(g2.x, rx, fmaf(g2.y, ry, g2.z * rz));
-            const float q2 = fmaf(tx, tx, fmaf(ty, ty, tz * tz));
-            if (!(q2 < 1.0f)) return;
-            const float u = 1.0f - q2;
-            const float A = -6.0f * g * coef * u * u;
-            // d/dr of (1 - |G r|^2)^3 = -6 (1 - q2)^2 G^T G r
-            gxs += A * (g0.x * tx + g1.x * ty + g2.x * tz);
-            gys += A * (g0.y * tx + g1.y * ty + g2.y * tz);
-            gzs += A * (g0.z * tx + g1.z * ty + g2.z * tz);
-            gg[0] += A * tx * rx; gg[1] += A * tx * ry; gg[2] += A * tx * rz;
-            gg[3] += A * ty * rx; gg[4] += A * ty * ry; gg[5] += A * ty * rz;
-            gg[6] += A * tz * rx; gg[7] += A * tz * ry; gg[8] += A * tz * rz;
-            sc += g * u * u * u;
-        });
-        if (involved) {
-            // c = sigma det(G) m / rho: d c / d G = c G^-T (G is symmetric)
-            const float G[9] = {g0.x, g0.y, g0.z, g1.x, g1.y, g1.z, g2.x, g2.y, g2.z};
-            const float det = G[0] * (G[4] * G[8] - G[5] * G[7]) - G[1] * (G[3] * G[8] - G[5] * G[6]) +
-                              G[2] * (G[3] * G[7] - G[4] * G[6]);
-            if (det != 0.f) {
-                const float k = sc * coef / det;
-                gg[0] += k * (G[4] * G[8] - G[5] * G[7]);
-                gg[1] += k * (G[5] * G[6] - G[3] * G[8]);
-                gg[2] += k * (G[3] * G[7] - G[4] * G[6]);
-                gg[3] += k * (G[2] * G[7] - G[1] * G[8]);
-                gg[4] += k * (G[0] * G[8] - G[2] * G[6]);
-                gg[5] += k * (G[1] * G[6] - G[0] * G[7]);
-                gg[6] += k * (G[1] * G[5] - G[2] * G[4]);
-                gg[7] += k * (G[2] * G[3] - G[0] * G[5]);
-                gg[8] += k * (G[0] * G[4] - G[1] * G[3]);
-            }
-        }
-    }
-    a.gsmooth[j] = make_float4(gxs, gys, gzs, 0.f);
-    a.gG[3ull * j] = make_float4(gg[0], gg[1], gg[2], 0.f);
-    a.gG[3ull * j + 1] = make_float4(gg[3], gg[4], gg[5], 0.f);
-    a.gG[3ull * j + 2] = make_float4(gg[6], gg[7], gg[8], 0.f);
 }
 
 // c = sigma det(G) m / rho: adds (sum dL/dphi (1 - q2)^3) dc/dG = that sum
@@ -695,11 +553,8 @@ void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, c
         fb.gG = a.gG;
         fb.sigma = a.sigma;
         fb.cap = a.cap_band;
-        if (launch_field_aniso_backward_grouped(c, fb, a.ratio, ctr)) {
-            launch_after(k_det_term, nblk(a.n), kT, 0, c.stream, a);
-        } else {
-            launch_after(k_field_backward_aniso, nblk(a.n), kT, 0, c.stream, a);
-        }
+        launch_field_aniso_backward(c, fb, a.ratio, ctr);
+        launch_after(k_det_term, nblk(a.n), kT, 0, c.stream, a);
         // warps may walk the union of their windows when the cull radius stays below 2 cells
         const int smooth_coop = (R * 1.0001f + 1e-4f * cov->sp.cs) < 2.0f * cov->sp.cs * 0.9999f ? 1 : 0;
         auto launch = [&](auto cov_kernel, auto smooth_kernel, uint64_t lanes) {

@@ -32,7 +32,6 @@
 namespace fsr {
 namespace {
 
-constexpr int kBT = 256;            // threads per block
 constexpr int kMaxCells = 125;      // 5 x 5 x 5 window
 
 struct GroupArgs {
@@ -48,7 +47,6 @@ struct GroupArgs {
     float* phi;
     float sigma;
     uint32_t cap;
-    uint32_t vlist_cap;             // capacity of the per-block vertex list
 };
 
 // Shared-memory tables of one group's candidate cells.
@@ -116,69 +114,6 @@ __device__ __forceinline__ bool slab_box(uint32_t part, uint32_t S, int lo[3], i
     return true;
 }
 
-// Lists the candidate cells of the window around cell c (clamped as in the
-// reference, cu:856-864), dropping involved cells whose reach cannot touch
-// the box [b0, b1], and scans their particle counts.  Every thread of the
-// block calls it; returns the number of candidates.
-__device__ uint32_t group_candidates(const Grid& sp, const uint2* __restrict__ ranges,
-                                     const uint8_t* __restrict__ invol, const float* __restrict__ reach,
-                                     const int c[3], const float b0[3], const float b1[3], const CandTables& t,
-                                     uint32_t* s_wsum, uint32_t* s_tot)
-{
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int lx = clampi(c[0] - 2, 0, (int)sp.res[0] - 1), hx = clampi(c[0] + 2, 0, (int)sp.res[0] - 1);
-    const int ly = clampi(c[1] - 2, 0, (int)sp.res[1] - 1), hy = clampi(c[1] + 2, 0, (int)sp.res[1] - 1);
-    const int lz = clampi(c[2] - 2, 0, (int)sp.res[2] - 1), hz = clampi(c[2] + 2, 0, (int)sp.res[2] - 1);
-    uint32_t cnt = 0;
-    if (tid < kMaxCells) {
-        const int dx = tid % 5, dy = (tid / 5) % 5, dz = tid / 25;
-        const int xx = lx + dx, yy = ly + dy, zz = lz + dz;
-        uint32_t st = 0, inv = 0;
-        if (xx <= hx && yy <= hy && zz <= hz) {
-            const uint32_t cell = lin3(xx, yy, zz, sp);
-            const uint2 r = __ldg(&ranges[cell]);
-            if (r.x != kEmpty) {
-                inv = __ldg(&invol[cell]);
-                bool keep = true;
-                if (inv) {
-                    const float cs = sp.cs;
-                    const float cx0 = sp.min[0] + xx * cs, cy0 = sp.min[1] + yy * cs, cz0 = sp.min[2] + zz * cs;
-                    const float gx = fmaxf(0.f, fmaxf(cx0 - b1[0], b0[0] - (cx0 + cs)));
-                    const float gy = fmaxf(0.f, fmaxf(cy0 - b1[1], b0[1] - (cy0 + cs)));
-                    const float gz = fmaxf(0.f, fmaxf(cz0 - b1[2], b0[2] - (cz0 + cs)));
-                    const float cr = cull_radius(__ldg(&reach[cell]), cs);
-                    keep = fmaf(gx, gx, fmaf(gy, gy, gz * gz)) < cr * cr;
-                }
-                if (keep) {
-                    st = r.x;
-                    cnt = r.y - r.x;
-                }
-            }
-        }
-        t.cstart[tid] = st;
-        t.cinv[tid] = inv;
-    }
-    // block-wide exclusive scan of the candidate counts (125 entries, warps 0-3)
-    uint32_t x = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    if (warp < 4 && lane == 31) s_wsum[warp] = x;
-    __syncthreads();
-    if (warp < 4) {
-        uint32_t off = 0;
-        for (int w = 0; w < warp; ++w) off += s_wsum[w];
-        t.cpre[tid + 1] = x + off;
-    }
-    if (tid == 0) t.cpre[0] = 0;
-    __syncthreads();
-    if (tid == 0) *s_tot = t.cpre[kMaxCells];
-    __syncthreads();
-    return *s_tot;
-}
-
 // Candidate j of the group: its sorted particle index and window cell.
 __device__ __forceinline__ uint32_t candidate(uint32_t j, const CandTables& t, int* cell, int ncells = kMaxCells)
 {
@@ -190,27 +125,6 @@ __device__ __forceinline__ uint32_t candidate(uint32_t j, const CandTables& t, i
     }
     *cell = lo;
     return t.cstart[lo] + (j - t.cpre[lo]);
-}
-
-// The 4 float4 field record of particle i: (x~, r2max), G rows with
-// coef = sigma det(G) m / rho in the first row's w; non-involved particles
-// get G = I, support 1 and coef = sigma m / rho.
-__device__ __forceinline__ void load_record(const float4* __restrict__ grec, const float4* __restrict__ smoothed,
-                                            float sigma, uint32_t i, bool involved, float4 r[4])
-{
-    if (involved) {
-        const float4* gsrc = grec + 4ull * i;
-        r[0] = __ldg(gsrc);
-        r[1] = __ldg(gsrc + 1);
-        r[2] = __ldg(gsrc + 2);
-        r[3] = __ldg(gsrc + 3);
-    } else {
-        const float4 s = __ldg(&smoothed[i]);
-        r[0] = make_float4(s.x, s.y, s.z, 1.0f);
-        r[1] = make_float4(1.f, 0.f, 0.f, sigma * s.w);
-        r[2] = make_float4(0.f, 1.f, 0.f, 0.f);
-        r[3] = make_float4(0.f, 0.f, 1.f, 0.f);
-    }
 }
 
 // ---------------------------------------------------------------- forward
@@ -266,12 +180,15 @@ __device__ __forceinline__ int chunk_cell(uint32_t cb, int lane, const uint32_t*
     return cell;
 }
 
-// Warp-level version of group_candidates: the same cells, listed with the
+// Lists the candidate cells of the window around cell c (clamped as in the
+// reference, cu:856-864), dropping involved cells whose reach cannot touch
+// the box [b0, b1]; by the warp: listed with the
 // involved cells first and the other non-empty cells after them (each part
 // in window order); only non-empty kept cells get an entry.
+template <class Slice>
 __device__ uint32_t warp_candidates(const Grid& sp, const uint2* __restrict__ ranges,
                                     const uint8_t* __restrict__ invol, const float* __restrict__ reach,
-                                    const int c[3], const float b0[3], const float b1[3], WarpSlice& w)
+                                    const int c[3], const float b0[3], const float b1[3], Slice& w)
 {
     const int lane = threadIdx.x & 31;
     const int lx = clampi(c[0] - 2, 0, (int)sp.res[0] - 1), hx = clampi(c[0] + 2, 0, (int)sp.res[0] - 1);
@@ -1234,17 +1151,6 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_grouped(IsoFieldArgs a, Ba
 }
 
 // ---------------------------------------------------------------- adjoint
-// dL/dx~ and dL/dG of the anisotropic field, grouped like the forward pass
-// but with the roles swapped: the group's band vertices that carry a
-// non-zero dL/dphi are staged in shared memory (with one bounding box per
-// 32 of them), and each thread takes one candidate particle, walks those
-// vertices and keeps its partial gradient in registers; one float4 atomic
-// per row then adds it to the particle (a particle is a candidate of up to
-// 125 groups).  Per (vertex, particle) pair inside the support:
-//   phi += c (1 - q2)^3, q2 = |G r|^2, r = x~ - v
-//   dL/dx~ += g c (-6 (1 - q2)^2) G^T G r,  dL/dG += g c (-6 (1 - q2)^2) (G r) r^T
-//   and sum g (1 - q2)^3 into the w of the dL/dx~ row (the det(G) term of
-//   c = sigma det(G) m / rho is applied per particle afterwards).
 struct BwdGroupArgs {
     Grid sp, sc;
     BandView band;
@@ -1260,205 +1166,7 @@ struct BwdGroupArgs {
     float4* gG;
     float sigma;
     uint32_t cap;
-    uint32_t vlist_cap;
 };
-
-__device__ __forceinline__ float box_dist2(float x, float y, float z, float4 lo, float4 hi)
-{
-    const float gx = fmaxf(0.f, fmaxf(lo.x - x, x - hi.x));
-    const float gy = fmaxf(0.f, fmaxf(lo.y - y, y - hi.y));
-    const float gz = fmaxf(0.f, fmaxf(lo.z - z, z - hi.z));
-    return fmaf(gx, gx, fmaf(gy, gy, gz * gz));
-}
-
-__global__ void k_field_aniso_backward_grouped(BwdGroupArgs a, uint32_t ratio, const Counters* ctr)
-{
-    after_launch();
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t nch_cap = (a.vlist_cap + 31) / 32;
-    float4* av = reinterpret_cast<float4*>(smem);            // active vertices: (v, dL/dphi)
-    float4* cbox = av + a.vlist_cap;                          // per 32 of them: lo, hi
-    uint32_t* cstart = reinterpret_cast<uint32_t*>(cbox + 2 * nch_cap);
-    uint32_t* cpre = cstart + 128;
-    uint32_t* cinv = cpre + 129;
-    __shared__ uint32_t s_nv, s_tot, s_wsum[4], s_next;
-    __shared__ float4 s_lo, s_hi;
-    const CandTables tabs{cstart, cpre, cinv};
-
-    __shared__ uint32_t s_g;
-    const uint32_t nb = min(ctr->n_band, a.cap);
-    const int tid = threadIdx.x, lane = tid & 31;
-    const uint32_t nlist = a.glist[0];
-
-    // the groups holding gradient vertices, handed out one per block from
-    // the list k_mc_backward built
-    for (;;) {
-        if (tid == 0) s_g = atomicAdd(&a.glist[1], 1u);
-        __syncthreads();
-        const uint32_t k = s_g;
-        __syncthreads();
-        if (k >= nlist) break;
-        const uint32_t g = a.glist[4 + k];
-        int c[3], lo[3], hi[3];
-        if (!group_box(g, a.sp, a.sc, ratio, c, lo, hi)) continue;
-        const int nx = hi[0] - lo[0], ny = hi[1] - lo[1], nz = hi[2] - lo[2];
-        const int nbox = nx * ny * nz;
-
-        // 1. the group's vertices with dL/dphi != 0 (listed in scan order:
-        // brick order, as in the ZB05 adjoint, measured slower here)
-        if (tid == 0) {
-            s_nv = 0;
-            s_next = 0;
-        }
-        __syncthreads();
-        for (int base = 0; base < nbox; base += kBT) {
-            const int i = base + tid;
-            float gv = 0.f;
-            int lx = 0, ly = 0, lz = 0;
-            if (i < nbox) {
-                lx = i % nx;
-                ly = (i / nx) % ny;
-                lz = i / (nx * ny);
-                const uint32_t v = lin3(lo[0] + lx, lo[1] + ly, lo[2] + lz, a.sc);
-                if (band_has(a.band, v)) {
-                    const uint32_t rank = band_rank(a.band, v);
-                    if (rank < nb) gv = __ldg(a.gphi + rank);
-                }
-            }
-            const bool act = gv != 0.f;
-            const uint32_t m = __ballot_sync(0xffffffffu, act);
-            uint32_t off = 0;
-            if (lane == 0 && m) off = atomicAdd(&s_nv, __popc(m));
-            off = __shfl_sync(0xffffffffu, off, 0);
-            if (act) {
-                const uint32_t slot = off + __popc(m & ((1u << lane) - 1u));
-                if (slot < a.vlist_cap)
-                    av[slot] = make_float4(vpos1(lo[0] + lx, a.sc.min[0], a.sc.cs),
-                                           vpos1(lo[1] + ly, a.sc.min[1], a.sc.cs),
-                                           vpos1(lo[2] + lz, a.sc.min[2], a.sc.cs), gv);
-            }
-        }
-        __syncthreads();
-        const uint32_t nv = min(s_nv, a.vlist_cap);
-        if (nv == 0) continue;
-        const uint32_t nch = (nv + 31) / 32;
-        for (uint32_t k = tid; k < nch; k += kBT) {
-            float4 l = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.f), h = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.f);
-            for (uint32_t q = 32 * k; q < min(nv, 32 * k + 32); ++q) {
-                const float4 v = av[q];
-                l.x = fminf(l.x, v.x); l.y = fminf(l.y, v.y); l.z = fminf(l.z, v.z);
-                h.x = fmaxf(h.x, v.x); h.y = fmaxf(h.y, v.y); h.z = fmaxf(h.z, v.z);
-            }
-            cbox[2 * k] = l;
-            cbox[2 * k + 1] = h;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            float4 l = cbox[0], h = cbox[1];
-            for (uint32_t k = 1; k < nch; ++k) {
-                const float4 kl = cbox[2 * k], kh = cbox[2 * k + 1];
-                l.x = fminf(l.x, kl.x); l.y = fminf(l.y, kl.y); l.z = fminf(l.z, kl.z);
-                h.x = fmaxf(h.x, kh.x); h.y = fmaxf(h.y, kh.y); h.z = fmaxf(h.z, kh.z);
-            }
-            s_lo = l;
-            s_hi = h;
-        }
-        __syncthreads();
-        const float4 glo = s_lo, ghi = s_hi;
-
-        // 2. candidate cells whose reach touches the active vertices
-        const float b0[3] = {glo.x, glo.y, glo.z}, b1[3] = {ghi.x, ghi.y, ghi.z};
-        const uint32_t total = group_candidates(a.sp, a.ranges, a.invol, a.reach, c, b0, b1, tabs, s_wsum, &s_tot);
-
-        // 3. one candidate per thread, gradient kept in registers; warps take
-        // the next 32 candidates as they finish, so that the group's slow
-        // candidates do not hold the others at the block's barrier
-        for (;;) {
-            uint32_t cb = 0;
-            if (lane == 0) cb = atomicAdd(&s_next, 32u);
-            cb = __shfl_sync(0xffffffffu, cb, 0);
-            if (cb >= total) break;
-            const uint32_t j = cb + lane;
-            if (j >= total) continue;
-            int cell;
-            const uint32_t i = candidate(j, tabs, &cell);
-            const bool inv = cinv[cell] != 0;
-            float4 r[4];
-            load_record(a.grec, a.smoothed, a.sigma, i, inv, r);
-            const float4 r0 = r[0], g0 = r[1], g1 = r[2], g2 = r[3];
-            if (!(box_dist2(r0.x, r0.y, r0.z, glo, ghi) < r0.w)) continue;
-            const float coef = g0.w;
-            float gxs = 0.f, gys = 0.f, gzs = 0.f, sc = 0.f;
-            if (!inv) {
-                // unscaled kernel (G = I, support 1): d/dx~ (1 - |r|^2)^3 = -6 (1 - |r|^2)^2 r;
-                // no dL/dG.  Candidates come cell by cell, so a warp's threads
-                // mostly take the same branch.
-                for (uint32_t q = 0; q < nv; ++q) {
-                    const float4 v = av[q];
-                    const float rx = r0.x - v.x, ry = r0.y - v.y, rz = r0.z - v.z;
-                    const float q2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                    if (!(q2 < 1.0f)) continue;
-                    const float u = 1.0f - q2;
-                    const float A = -6.0f * v.w * coef * u * u;
-                    gxs = fmaf(A, rx, gxs);
-                    gys = fmaf(A, ry, gys);
-                    gzs = fmaf(A, rz, gzs);
-                }
-                if (gxs != 0.f || gys != 0.f || gzs != 0.f) atomicAdd(a.gsmooth + i, make_float4(gxs, gys, gzs, 0.f));
-                continue;
-            }
-            // per pair, with M = G^T G (the forward's quadratic form) and
-            // B = -3 g c (1 - q2)^2:  dL/dx~ += 2 B M d,  dL/dM += B d d^T
-            // (S, symmetric); dL/dG = 2 G S once per candidate at the end
-            const float4 qa = __ldg(a.qrec + 3ull * i + 1), qb = __ldg(a.qrec + 3ull * i + 2);
-            const float m00 = qa.x, m01 = 0.5f * qa.y, m02 = 0.5f * qa.z;
-            const float m11 = qb.x, m12 = 0.5f * qb.y, m22 = qb.z;
-            float s00 = 0.f, s01 = 0.f, s02 = 0.f, s11 = 0.f, s12 = 0.f, s22 = 0.f;
-            for (uint32_t k = 0; k < nch; ++k) {
-                if (!(box_dist2(r0.x, r0.y, r0.z, cbox[2 * k], cbox[2 * k + 1]) < r0.w)) continue;
-                const uint32_t qe = min(nv, 32 * k + 32);
-                for (uint32_t q = 32 * k; q < qe; ++q) {
-                    const float4 v = av[q];
-                    const float rx = r0.x - v.x, ry = r0.y - v.y, rz = r0.z - v.z;
-                    const float d2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                    if (!(d2 < r0.w)) continue;
-                    const float a0 = fmaf(m00, rx, fmaf(m01, ry, m02 * rz));
-                    const float a1 = fmaf(m01, rx, fmaf(m11, ry, m12 * rz));
-                    const float a2 = fmaf(m02, rx, fmaf(m12, ry, m22 * rz));
-                    const float q2 = fmaf(rx, a0, fmaf(ry, a1, rz * a2));
-                    if (!(q2 < 1.0f)) continue;
-                    const float u = 1.0f - q2;
-                    const float B = -3.0f * v.w * coef * u * u;
-                    const float B2 = B + B;
-                    gxs = fmaf(B2, a0, gxs);
-                    gys = fmaf(B2, a1, gys);
-                    gzs = fmaf(B2, a2, gzs);
-                    const float bx = B * rx, by = B * ry, bz = B * rz;
-                    s00 = fmaf(bx, rx, s00);
-                    s01 = fmaf(bx, ry, s01);
-                    s02 = fmaf(bx, rz, s02);
-                    s11 = fmaf(by, ry, s11);
-                    s12 = fmaf(by, rz, s12);
-                    s22 = fmaf(bz, rz, s22);
-                    sc = fmaf(v.w, u * u * u, sc);
-                }
-            }
-            if (gxs != 0.f || gys != 0.f || gzs != 0.f || sc != 0.f) {
-                atomicAdd(a.gsmooth + i, make_float4(gxs, gys, gzs, sc));
-                // dL/dG = 2 G S
-                auto row = [&](float4 g) {
-                    return make_float4(2.0f * (g.x * s00 + g.y * s01 + g.z * s02),
-                                       2.0f * (g.x * s01 + g.y * s11 + g.z * s12),
-                                       2.0f * (g.x * s02 + g.y * s12 + g.z * s22), 0.f);
-                };
-                atomicAdd(a.gG + 3ull * i, row(g0));
-                atomicAdd(a.gG + 3ull * i + 1, row(g1));
-                atomicAdd(a.gG + 3ull * i + 2, row(g2));
-            }
-        }
-        __syncthreads();
-    }
-}
 
 // Adjoint of the ZB05 / TC01 fields (updateScalarFieldValueZB05 cu:230-289,
 // TC01 cu:178-227), grouped like the forward field with the roles swapped: a
@@ -1665,20 +1373,254 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
     }
 }
 
+// dL/d(smoothed position), dL/dG (without the determinant's term) and the sums
+// that term takes, for the particles of each group holding gradient vertices
+// (cu:938-1031 differentiated).  As the isotropic adjoint above: a warp per group,
+// passes of up to 128 vertices with dL/dphi != 0 in tiles of 32, the candidates
+// staged, those whose support sphere reaches a tile listed, a lane per listed
+// candidate, two vertices per packed operation.  Per pair, with M = G^T G (the
+// forward's quadratic form), q2 = d^T M d, u = 1 - q2 and b = g u^2:
+//   sum b d, sum b d d^T, sum g u^3,
+// from which dL/dx~ = -6 c M (sum b d) and dL/dG = -6 c G (sum b d d^T) follow
+// once per candidate.  Bound by the FP32 pipe.  A block per group with a candidate
+// per thread and the vertices one by one ran 13 of 32 lanes (whole backward: 20k
+// particles 0.25 -> 0.215 ms, 150k 0.49 -> 0.45, 1M 1.44 -> 1.36).  Staged 64 / 96 / 128
+// at a time: 150k 0.47 / 0.45 / 0.46 ms; vertex pairs one, two or four to a step: 20k
+// 0.233 / 0.233 / 0.211.
+constexpr uint32_t kAnisoBwdSeg = 96;  // candidates staged at a time
+constexpr int kBwdSums = 10;
+struct AnisoBwdSlice {
+    float4 vxy[kBwdVerts / 2];  // the pass's vertices two to a pair: (x, x', y, y')
+    float4 vzg[kBwdVerts / 2];  // (z, z', dL/dphi, dL/dphi')
+    uint32_t vloc[kBwdVerts], vrank[kBwdVerts];
+    uint32_t hist[kBwdVerts];
+    float4 box[2 * (kBwdVerts / 32)];
+    float4 c[kAnisoBwdSeg];                // the staged candidates: x, y, z, squared support radius
+    float m[6][kAnisoBwdSeg];              // their quadratic forms: m00, 2 m01, 2 m02, m11, 2 m12, m22
+    float s[kBwdSums][kAnisoBwdSeg];       // their sums: b d, g u^3, b d d^T
+    float coef[kAnisoBwdSeg];              // sigma det(G) m / rho
+    uint32_t cj[kAnisoBwdSeg];             // their sorted index
+    uint32_t list[kAnisoBwdSeg];           // those that reach the tile
+    uint32_t cstart[128], cpre[kMaxCells + 1], cinv[128];
+    uint32_t ncells, total_inv, ninv_cells;
+};
+
+__global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a, uint32_t ratio, const Counters* ctr)
+{
+    after_launch();
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int lane = threadIdx.x & 31;
+    AnisoBwdSlice& w = reinterpret_cast<AnisoBwdSlice*>(smem)[threadIdx.x >> 5];
+    const uint32_t nb = min(ctr->n_band, a.cap);
+    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mc_backward)
+    // Few groups are cut into more work items: fine grids by slabs of vertices,
+    // coarse ones, whose groups hold few vertices, by runs of candidates (backward
+    // by slabs / runs, ms: 10 vertices per cell, 20k particles 0.21 / 0.25, 150k 0.44 / 0.53;
+    // 3 per cell, 20k 0.62 / 0.585).
+    const uint32_t nsub = field_slabs(nlist), nslab = ratio > 4 ? nsub : 1u, nparts = ratio > 4 ? 1u : nsub;
+    const float2 one2 = make_float2(1.0f, 1.0f), mone2 = make_float2(-1.0f, -1.0f);
+
+    for (;;) {
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(&a.glist[1], 1u);
+        k = __shfl_sync(0xffffffffu, k, 0);
+        if (k >= nlist * nsub) break;
+        const uint32_t part = k % nparts;
+        int c[3], lo[3], hi[3];
+        if (!group_box(a.glist[4 + k / nsub], a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi))
+            continue;
+        bool tables = false;
+        uint32_t total = 0;
+
+        auto pass = [&](uint32_t nv) {
+            if (!tables) {
+                const float b0[3] = {vpos1(lo[0], a.sc.min[0], a.sc.cs), vpos1(lo[1], a.sc.min[1], a.sc.cs),
+                                     vpos1(lo[2], a.sc.min[2], a.sc.cs)};
+                const float b1[3] = {vpos1(hi[0] - 1, a.sc.min[0], a.sc.cs), vpos1(hi[1] - 1, a.sc.min[1], a.sc.cs),
+                                     vpos1(hi[2] - 1, a.sc.min[2], a.sc.cs)};
+                total = warp_candidates(a.sp, a.ranges, a.invol, a.reach, c, b0, b1, w);
+                tables = true;
+            }
+            float4 pl, ph;
+            pass_layout<true, kBwdVerts>(w.vloc, w.vrank, lo, a.sc, nullptr, w.hist, w.box, nv, lane, pl, ph);
+            const uint32_t ntiles = (nv + 31) / 32;
+            // the places up to the last tile's end lie far away and have dL/dphi = 0
+            for (uint32_t q = lane; q < 32u * ntiles; q += 32) {
+                float4 vp = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f);
+                if (q < nv) {
+                    vp = vert_pos(w.vloc[q], lo, a.sc);
+                    vp.w = __ldg(a.gphi + w.vrank[q]);
+                }
+                float* d = reinterpret_cast<float*>(w.vxy + (q >> 1)) + (q & 1u);
+                d[0] = vp.x;
+                d[2] = vp.y;
+                d = reinterpret_cast<float*>(w.vzg + (q >> 1)) + (q & 1u);
+                d[0] = vp.z;
+                d[2] = vp.w;
+            }
+            __syncwarp();
+            const uint32_t total_inv = w.total_inv;
+            uint32_t fill = 0;
+            auto tiles = [&]() {
+                for (uint32_t i = lane; i < fill; i += 32)
+#pragma unroll
+                    for (int r = 0; r < kBwdSums; ++r) w.s[r][i] = 0.f;
+                __syncwarp();
+#pragma unroll 1
+                for (uint32_t t = 0; t < ntiles; ++t) {
+                    const float4 tl = w.box[2 * t], th = w.box[2 * t + 1];
+                    uint32_t cnt = 0;
+                    for (uint32_t b = 0; b < fill; b += 32) {
+                        const uint32_t i = b + (uint32_t)lane;
+                        const bool in = i < fill && reaches(w.c[i], tl, th);
+                        const uint32_t m = __ballot_sync(0xffffffffu, in);
+                        if (in) w.list[cnt + __popc(m & ((1u << lane) - 1u))] = i;
+                        cnt += __popc(m);
+                    }
+                    __syncwarp();
+                    const uint32_t pairs = (min(32u, nv - 32u * t) + 1u) >> 1;
+                    for (uint32_t b = lane; b < cnt; b += 32) {
+                        const uint32_t i = w.list[b];
+                        const float4 q = w.c[i];
+                        const float2 qx = make_float2(q.x, q.x), qy = make_float2(q.y, q.y), qz = make_float2(q.z, q.z);
+                        const float2 m0 = make_float2(w.m[0][i], w.m[0][i]), m1 = make_float2(w.m[1][i], w.m[1][i]),
+                                     m2 = make_float2(w.m[2][i], w.m[2][i]), m3 = make_float2(w.m[3][i], w.m[3][i]),
+                                     m4 = make_float2(w.m[4][i], w.m[4][i]), m5 = make_float2(w.m[5][i], w.m[5][i]);
+                        float2 s[kBwdSums];
+#pragma unroll
+                        for (int r = 0; r < kBwdSums; ++r) s[r] = make_float2(0.f, 0.f);
+#pragma unroll 4
+                        for (uint32_t j = 0; j < pairs; ++j) {
+                            const float4 A = w.vxy[16u * t + j], Z = w.vzg[16u * t + j];
+                            const float2 dx = __ffma2_rn(make_float2(A.x, A.y), mone2, qx);
+                            const float2 dy = __ffma2_rn(make_float2(A.z, A.w), mone2, qy);
+                            const float2 dz = __ffma2_rn(make_float2(Z.x, Z.y), mone2, qz);
+                            const float2 t0 = __ffma2_rn(m0, dx, __ffma2_rn(m1, dy, __fmul2_rn(m2, dz)));
+                            const float2 t1 = __ffma2_rn(m3, dy, __fmul2_rn(m4, dz));
+                            const float2 q2 =
+                                __ffma2_rn(dx, t0, __ffma2_rn(dy, t1, __fmul2_rn(__fmul2_rn(m5, dz), dz)));
+                            float2 u = __ffma2_rn(q2, mone2, one2);
+                            u.x = fmaxf(u.x, 0.f);
+                            u.y = fmaxf(u.y, 0.f);
+                            const float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
+                            const float2 bx = __fmul2_rn(bb, dx), by = __fmul2_rn(bb, dy), bz = __fmul2_rn(bb, dz);
+                            s[0] = __fadd2_rn(s[0], bx);
+                            s[1] = __fadd2_rn(s[1], by);
+                            s[2] = __fadd2_rn(s[2], bz);
+                            s[3] = __ffma2_rn(bb, u, s[3]);
+                            s[4] = __ffma2_rn(bx, dx, s[4]);
+                            s[5] = __ffma2_rn(bx, dy, s[5]);
+                            s[6] = __ffma2_rn(bx, dz, s[6]);
+                            s[7] = __ffma2_rn(by, dy, s[7]);
+                            s[8] = __ffma2_rn(by, dz, s[8]);
+                            s[9] = __ffma2_rn(bz, dz, s[9]);
+                        }
+#pragma unroll
+                        for (int r = 0; r < kBwdSums; ++r) w.s[r][i] += s[r].x + s[r].y;
+                    }
+                    __syncwarp();
+                }
+                for (uint32_t i = lane; i < fill; i += 32) {
+                    const float gx = w.s[0][i], gy = w.s[1][i], gz = w.s[2][i], sc = w.s[3][i];
+                    if (gx == 0.f && gy == 0.f && gz == 0.f && sc == 0.f) continue;
+                    const uint32_t id = w.cj[i];
+                    const float f = -6.0f * w.coef[i];
+                    const float m01 = 0.5f * w.m[1][i], m02 = 0.5f * w.m[2][i], m12 = 0.5f * w.m[4][i];
+                    atomicAdd(a.gsmooth + id,
+                              make_float4(f * (w.m[0][i] * gx + m01 * gy + m02 * gz),
+                                          f * (m01 * gx + w.m[3][i] * gy + m12 * gz),
+                                          f * (m02 * gx + m12 * gy + w.m[5][i] * gz), sc));
+                    const float s00 = f * w.s[4][i], s01 = f * w.s[5][i], s02 = f * w.s[6][i];
+                    const float s11 = f * w.s[7][i], s12 = f * w.s[8][i], s22 = f * w.s[9][i];
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) {
+                        const float4 g = __ldg(a.grec + 4ull * id + 1 + r);
+                        atomicAdd(a.gG + 3ull * id + r, make_float4(g.x * s00 + g.y * s01 + g.z * s02,
+                                                                    g.x * s01 + g.y * s11 + g.z * s12,
+                                                                    g.x * s02 + g.y * s12 + g.z * s22, 0.f));
+                    }
+                }
+                __syncwarp();
+                fill = 0;
+            };
+            const CandTables tabs{w.cstart, w.cpre, w.cinv};
+            // the part's candidates: a run of the involved ones, whole 32s
+            const uint32_t n32 = (total_inv + 31) / 32;
+            for (uint32_t cb = 32 * (n32 * part / nparts); cb < 32 * (n32 * (part + 1) / nparts); cb += 32) {
+                const uint32_t j = cb + lane;
+                bool keep = false;
+                uint32_t id = 0;
+                float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0, r2 = r0;
+                if (j < total_inv) {
+                    int cell;
+                    id = candidate(j, tabs, &cell, (int)w.ncells);
+                    const float4* src = a.qrec + 3ull * id;
+                    r0 = __ldg(src);
+                    r1 = __ldg(src + 1);
+                    r2 = __ldg(src + 2);
+                    keep = reaches(r0, pl, ph);
+                }
+                const uint32_t m = __ballot_sync(0xffffffffu, keep);
+                if (keep) {
+                    const uint32_t i = fill + __popc(m & ((1u << lane) - 1u));
+                    w.c[i] = r0;
+                    w.m[0][i] = r1.x;
+                    w.m[1][i] = r1.y;
+                    w.m[2][i] = r1.z;
+                    w.m[3][i] = r2.x;
+                    w.m[4][i] = r2.y;
+                    w.m[5][i] = r2.z;
+                    w.coef[i] = r1.w;
+                    w.cj[i] = id;
+                }
+                fill += __popc(m);
+                if (fill > kAnisoBwdSeg - 32) tiles();
+            }
+            if (fill) tiles();
+            // the others: G = I and support 1, which reaches every vertex; no dL/dG
+            for (uint32_t j = total_inv + 32 * part + lane; j < total; j += 32 * nparts) {
+                int cell;
+                const uint32_t id = candidate(j, tabs, &cell, (int)w.ncells);
+                const float4 q = __ldg(&a.smoothed[id]);
+                const float2 qx = make_float2(q.x, q.x), qy = make_float2(q.y, q.y), qz = make_float2(q.z, q.z);
+                float2 sx = make_float2(0.f, 0.f), sy = sx, sz = sx;
+#pragma unroll 1
+                for (uint32_t v = 0; v < (nv + 1u) >> 1; ++v) {
+                    const float4 A = w.vxy[v], Z = w.vzg[v];
+                    const float2 dx = __ffma2_rn(make_float2(A.x, A.y), mone2, qx);
+                    const float2 dy = __ffma2_rn(make_float2(A.z, A.w), mone2, qy);
+                    const float2 dz = __ffma2_rn(make_float2(Z.x, Z.y), mone2, qz);
+                    const float2 q2 = __ffma2_rn(dx, dx, __ffma2_rn(dy, dy, __fmul2_rn(dz, dz)));
+                    float2 u = __ffma2_rn(q2, mone2, one2);
+                    u.x = fmaxf(u.x, 0.f);
+                    u.y = fmaxf(u.y, 0.f);
+                    const float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
+                    sx = __ffma2_rn(bb, dx, sx);
+                    sy = __ffma2_rn(bb, dy, sy);
+                    sz = __ffma2_rn(bb, dz, sz);
+                }
+                const float f = -6.0f * (a.sigma * q.w);
+                const float4 g = make_float4(f * (sx.x + sx.y), f * (sy.x + sy.y), f * (sz.x + sz.y), 0.f);
+                if (g.x != 0.f || g.y != 0.f || g.z != 0.f) atomicAdd(a.gsmooth + id, g);
+            }
+            __syncwarp();
+        };
+        // the vertices of a row segment with dL/dphi != 0
+        auto with_gradient = [&](uint32_t bits, uint32_t r0) {
+            uint32_t kept = 0;
+            for (uint32_t m = bits, r = r0; m; m &= m - 1u, ++r)
+                if (r < nb && __ldg(a.gphi + r) != 0.f) kept |= m & (0u - m);
+            return kept;
+        };
+        list_band_vertices<kBwdVerts>(a.sc, a.band, lo, hi, w.vloc, w.vrank, lane, with_gradient, pass);
+        __syncwarp();
+    }
+}
+
 }  // namespace
 
-bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs& f, uint32_t ratio,
-                                         const Counters* ctr)
+void launch_field_aniso_backward(const KernelCtx& c, const AnisoBwdArgs& f, uint32_t ratio, const Counters* ctr)
 {
-    const uint32_t vcap = (ratio + 2) * (ratio + 2) * (ratio + 2);
-    const size_t smem = sizeof(float4) * vcap + sizeof(float4) * 2 * ((vcap + 31) / 32) +
-                        sizeof(uint32_t) * (128 + 129 + 128);
-    if (smem > 200 * 1024) return false;
-    static bool configured = false;
-    if (!configured) {
-        cudaFuncSetAttribute(k_field_aniso_backward_grouped, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-        configured = true;
-    }
     BwdGroupArgs a;
     a.sp = f.sp;
     a.sc = f.sc;
@@ -1695,13 +1637,11 @@ bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs&
     a.gG = f.gG;
     a.sigma = f.sigma;
     a.cap = f.cap;
-    a.vlist_cap = vcap;
-    const uint64_t groups = (uint64_t)(f.sp.res[0] + 1) * (f.sp.res[1] + 1) * (f.sp.res[2] + 1);
-    const unsigned grid = (unsigned)std::min<uint64_t>(
-        groups, std::max<uint64_t>(1, (uint64_t)c.num_sms * 8 / std::max(1, c.grid_div)));
-    launch_after(k_field_aniso_backward_grouped, grid, kBT, smem, c.stream, a, ratio, ctr);
+    const size_t smem = sizeof(AnisoBwdSlice) * kFWarps;
+    cudaFuncSetAttribute(k_field_aniso_backward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const unsigned grid = (unsigned)std::max(1, c.num_sms * 4 / std::max(1, c.grid_div));
+    launch_after(k_field_aniso_backward, grid, kFT, smem, c.stream, a, ratio, ctr);
     ++g_launches;
-    return true;
 }
 
 void launch_field_aniso_grouped(const KernelCtx& c, const AnisoFieldArgs& f, const BandView& band, uint32_t ratio,
@@ -1721,7 +1661,6 @@ void launch_field_aniso_grouped(const KernelCtx& c, const AnisoFieldArgs& f, con
     a.phi = f.phi;
     a.sigma = f.sigma;
     a.cap = f.cap;
-    a.vlist_cap = 0;
     const uint64_t groups = (uint64_t)(f.sp.res[0] + 1) * (f.sp.res[1] + 1) * (f.sp.res[2] + 1);
     const unsigned grid = (unsigned)std::min<uint64_t>(
         (groups + kFWarps - 1) / kFWarps, std::max<uint64_t>(1, (uint64_t)c.num_sms * 16 / std::max(1, c.grid_div)));

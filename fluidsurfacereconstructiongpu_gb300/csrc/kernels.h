@@ -134,8 +134,7 @@ void launch_field_aniso_grouped(const KernelCtx& c, const AnisoFieldArgs& a, con
 
 // Adjoint of the anisotropic field, grouped like the forward pass: adds
 // (dL/dx~, sum dL/dphi (1 - q2)^3) to gsmooth and dL/dG rows (without the
-// det(G) term) to gG; both must start at zero.  Returns false (nothing
-// launched) when the grid ratio makes a group too large.
+// det(G) term) to gG; both must start at zero.
 struct AnisoBwdArgs {
     Grid sp, sc;
     BandView band;
@@ -152,8 +151,7 @@ struct AnisoBwdArgs {
     float sigma;
     uint32_t cap;
 };
-bool launch_field_aniso_backward_grouped(const KernelCtx& c, const AnisoBwdArgs& a, uint32_t ratio,
-                                         const Counters* ctr);
+void launch_field_aniso_backward(const KernelCtx& c, const AnisoBwdArgs& a, uint32_t ratio, const Counters* ctr);
 
 // Spatial hashing as a counting sort by cell (cell_sort.cu): sorted particles,
 // their keys and input numbers, cell ranges and occupancy; zeroes cell_rmax (may

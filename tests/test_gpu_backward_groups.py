@@ -83,3 +83,16 @@ def test_gradient_matches_autograd(method, n, h, spread, ratio):
     assert (p.detach() - pos.double()).abs().max() < 1e-4 * h
     want, = torch.autograd.grad((p * g.double()).sum(), x)
     assert (got - want).abs().max() <= 2e-3 * want.abs().max()
+
+
+@pytest.mark.parametrize("ratio", [4, 5])
+def test_anisotropic_adjoint_by_runs_and_by_slabs(ratio):
+    """The anisotropic field's adjoint on both sides of the line between work
+    items by runs of candidates (up to 4 vertices per cell) and by slabs of
+    vertices, at the bar of the finite-difference tests."""
+    from fluidsurfacereconstructiongpu_gb300 import synthetic
+    from tests.test_gpu_backward import ANISO_SETTINGS, _case
+    fr = synthetic.lattice_cube(12, 0.0125, seed=1, origin=(0.3, 0.3, 0.3))
+    rows, err, scale = _case("yu13", fr, **dict(ANISO_SETTINGS["fine"], grid_ratio=ratio))
+    assert scale > 0
+    assert err.max() <= 2e-3 * scale, (err.max() / scale, rows[np.argmax(err)])

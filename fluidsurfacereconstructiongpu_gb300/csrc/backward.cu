@@ -41,12 +41,7 @@ constexpr int kT = 256;
 // without a gradient vertex is found empty there).  Measured with the marking,
 // which was a pass over the band of its own: 500k-particle ZB05 frame (1.1M
 // cubes, with the radius) 151 -> 116 us.
-// kRadius: dL/d(particle radius) of ZB05, minus the sum of dL/dphi over the
-// vertices with weight.  An edge's two terms nearly cancel, -(ga + gb) =
-// dL/df / (phi_b - phi_a), so that difference is summed, in FP64 (the sum of the
-// FP32 gradients was off by 1e-6 to 1e-5, differently in each run).
-template <bool kRadius>
-__global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* ctr, double* radius)
+__global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* ctr)
 {
     after_launch();
     __shared__ float s_val[8 * kT], s_g[8 * kT];  // [corner][thread]
@@ -55,14 +50,12 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
     const uint32_t nq = min(ctr->n_valid, a.cap_valid);
     const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
     const uint32_t kx = a.sp.res[0] + 1, ky = a.sp.res[1] + 1;
-    double rad = 0.0;
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const uint32_t t = a.valid[q];
         const uint32_t info = a.mc[t];
         const uint32_t cs = info >> 8, nv = info & 0xFFu, base = a.vofs[t];
         const uint32_t v = a.sv[t];
         uint32_t r0[4];  // rank of each row's x corner; its x + 1 corner follows
-        uint32_t weighted = 0;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int dy = r & 1, dz = r >> 1;
@@ -71,13 +64,8 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
             val[i0 * kT] = __ldg(a.band.phi + r0[r]);
             val[(i0 + 4) * kT] = __ldg(a.band.phi + r0[r] + 1);
             g[i0 * kT] = g[(i0 + 4) * kT] = 0.f;
-            if (kRadius) {
-                if (__ldg(&a.mv[r0[r]].w) > 0.f) weighted |= 1u << i0;
-                if (__ldg(&a.mv[r0[r] + 1].w) > 0.f) weighted |= 1u << (i0 + 4);
-            }
         }
         const uint64_t tri = a.tri[cs];
-        float cube = 0.f;
         for (uint32_t k = 0; k < nv; ++k) {
             const int e = (int)((tri >> (4u * k)) & 0xFu);
             const int ia = mc::edgeA(e), ib = mc::edgeB(e);
@@ -94,12 +82,7 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
             const float ga = gf * (a.iso - fb) * inv, gb = -gf * (a.iso - fa) * inv;
             g[ia * kT] += ga;
             g[ib * kT] += gb;
-            if (kRadius) {
-                const bool wa = (weighted >> ia) & 1u, wb = (weighted >> ib) & 1u;
-                cube += wa && wb ? gf / d : (wa ? -ga : 0.f) + (wb ? -gb : 0.f);
-            }
         }
-        if (kRadius) rad += (double)cube;
         bool any = false;
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
@@ -129,11 +112,25 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
                         a.glist[4 + atomicAdd(&a.glist[0], 1u)] = key;
                 }
     }
-    if (kRadius) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) rad += __shfl_xor_sync(0xffffffffu, rad, o);
-        if ((threadIdx.x & 31) == 0 && rad != 0.0) atomicAdd(radius, rad);
+}
+
+// dL/d(particle radius) of ZB05: -sum of dL/dphi over vertices with weight.  The
+// weight sums are read only where dL/dphi is not zero (500k-particle frame: 50 ->
+// 35 us).  In FP32, joined per warp: an FP64 sum repeats from run to run, but the
+// field's own roundings put it 0.02 to 3.5e-6 of the result off the FP64 gradient,
+// as far as this one (0 to 8e-6).
+__global__ void __launch_bounds__(kT) k_radius_grad(BwdArgs a, const Counters* ctr, float* out)
+{
+    after_launch();
+    const uint32_t nb = min(ctr->n_band, a.cap_band);
+    float s = 0.f;
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb; t += gridDim.x * blockDim.x) {
+        const float g = a.gphi[t];
+        if (g != 0.f && a.mv[t].w > 0.f) s -= g;
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0 && s != 0.f) atomicAdd(out, s);
 }
 
 // c = sigma det(G) m / rho: adds (sum dL/dphi (1 - q2)^3) dc/dG = that sum
@@ -529,13 +526,18 @@ inline unsigned nblk(uint64_t n) { return (unsigned)std::max<uint64_t>(1, (n + k
 }  // namespace
 
 void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, const Counters* ctr, int method,
-                     float lambda, float R, double* radius_grad_dev, float* out_grad_xyz)
+                     float lambda, float R, float* radius_grad_dev, float* out_grad_xyz)
 {
     const unsigned pb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_valid + kT - 1) / kT,
                                                                           (uint64_t)c.num_sms * 16));
-    if (radius_grad_dev) launch_after(k_mc_backward<true>, pb, kT, 0, c.stream, a, ctr, radius_grad_dev);
-    else launch_after(k_mc_backward<false>, pb, kT, 0, c.stream, a, ctr, nullptr);
+    launch_after(k_mc_backward, pb, kT, 0, c.stream, a, ctr);
     ++g_launches;
+    if (radius_grad_dev) {
+        const unsigned bb = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((a.cap_band + kT - 1) / kT,
+                                                                              (uint64_t)c.num_sms * 16));
+        launch_after(k_radius_grad, bb, kT, 0, c.stream, a, ctr, radius_grad_dev);
+        ++g_launches;
+    }
     if (method == FSR_METHOD_YU13) {
         AnisoBwdArgs fb{};
         fb.sp = a.sp;

@@ -43,6 +43,6 @@ struct BwdArgs {
 void launch_field_iso_backward(const KernelCtx& c, const BwdArgs& a, bool tc01, const Counters* ctr);
 
 void launch_backward(const KernelCtx& c, const BwdArgs& a, const CovArgs* cov, const Counters* ctr, int method,
-                     float lambda, float R, double* radius_grad_dev, float* out_grad_xyz);
+                     float lambda, float R, float* radius_grad_dev, float* out_grad_xyz);
 
 }  // namespace fsr

@@ -152,18 +152,18 @@ extern "C" fsr_status fsr_backward(fsr_handle* h, const float* d_grad_mesh_pos, 
     const uint64_t launches0 = g_launches;
     if (n > 0)
         launch_backward(kc, a, &ca, (const Counters*)h->ctr.ptr, (int)p.method, p.smoothing_lambda, R,
-                        want_radius ? (double*)h->gscalar.ptr : nullptr, d_grad_xyz);
+                        want_radius ? (float*)h->gscalar.ptr : nullptr, d_grad_xyz);
     BCK(cudaGetLastError());
     h->stats.n_backward_launches = (uint32_t)(g_launches - launches0);
     h->stats.device_bytes = 0;
     for (DevBuf* b : h->all_buffers()) h->stats.device_bytes += b->bytes;
     if (grad_particle_radius) {
-        double r = 0.0;
+        float r = 0.f;
         if (want_radius) {
             BCK(cudaMemcpyAsync(&r, h->gscalar.ptr, sizeof(r), cudaMemcpyDeviceToHost, st));
             BCK(cudaStreamSynchronize(st));
         }
-        *grad_particle_radius = (float)r;
+        *grad_particle_radius = r;
     }
     if (prev != h->device) cudaSetDevice(prev);
     return FSR_OK;

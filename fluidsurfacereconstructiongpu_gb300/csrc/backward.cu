@@ -38,9 +38,10 @@ constexpr int kT = 256;
 // up as four rows of two x-neighbours (as in k_mc_classify).  The cube also
 // marks the window centres (keys) its corners fall in; the first mark of a key
 // appends it to the list the grouped adjoints take their groups from (a key
-// without a gradient vertex is found empty there).  Measured with the marking,
-// which was a pass over the band of its own: 500k-particle ZB05 frame (1.1M
-// cubes, with the radius) 151 -> 116 us.
+// without a gradient vertex is found empty there).  Bound by the latency of its
+// scattered reads and atomics (ncu, 256k ZB05: 53 % of the issue slots, 29 % of
+// the DRAM peak).  With the marking and the radius's sum as passes over the band
+// of their own a 500k ZB05 frame took 151 us, now about 125.
 __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* ctr)
 {
     after_launch();

@@ -913,7 +913,9 @@ __global__ void __launch_bounds__(kThreads, FSR_SMOOTH_MIN_BLOCKS) k_smooth(cons
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 uint32_t beg, end;
-                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                int x0 = ulo[0], x1 = uhi[0];
+                if (kSets && !row_reach(box, sp, yy, zz, x0, x1)) continue;
+                row_range(x0, x1, yy, zz, beg, end);
                 for (uint32_t base = beg; base < end; base += 32) {
                     uint32_t nbox;
                     const uint32_t cnt = stage_in_box(sorted, base, end, box, sq, lane, nbox);
@@ -1156,7 +1158,9 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 uint32_t beg, end;
-                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                int x0 = ulo[0], x1 = uhi[0];
+                if (max_span > 3 && !row_reach(mine, sp, yy, zz, x0, x1)) continue;
+                row_range(x0, x1, yy, zz, beg, end);
                 if (own_folds) {
                     own = len = chunk_at = 0;
                     if (mine_in && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
@@ -1370,7 +1374,9 @@ __global__ void __launch_bounds__(kCovThreads, FSR_COV_MIN_BLOCKS) k_cov(CovArgs
         for (int zz = ulo[2]; zz <= uhi[2]; ++zz)
             for (int yy = ulo[1]; yy <= uhi[1]; ++yy) {
                 uint32_t beg, end, own = 0, len = 0;
-                row_range(ulo[0], uhi[0], yy, zz, beg, end);
+                int x0 = ulo[0], x1 = uhi[0];
+                if (kSets && P < 16 && !row_reach(box, a.sp, yy, zz, x0, x1)) continue;
+                row_range(x0, x1, yy, zz, beg, end);
                 if (kSets && in_set && zz >= w.lo[2] && zz <= w.hi[2] && yy >= w.lo[1] && yy <= w.hi[1]) {
                     row_range(w.lo[0], w.hi[0], yy, zz, own, len);
                     len = len > own ? len - own : 0u;

@@ -63,9 +63,9 @@ __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __res
 {
     after_launch();
     const uint32_t stride = gridDim.x * blockDim.x, start = blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint32_t i = start; i < n; i += stride) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
+    for (uint32_t i = start; i < n; i = next_of(i, stride, n)) grouped[__ldg(first + keys[i]) + arrival[i]] = i;
     const uint32_t kx = sp.res[0] + 1, ky = sp.res[1] + 1;
-    for (uint32_t c = start; c < groups; c += stride) {
+    for (uint32_t c = start; c < groups; c = next_of(c, stride, groups)) {
         // (groups beyond the last cell of an axis count as that cell)
         const uint32_t gz = c / (kx * ky), gy = (c - gz * kx * ky) / kx, gx = c - (gz * ky + gy) * kx;
         const uint32_t x1 = sp.res[0] - 1, y1 = sp.res[1] - 1, z1 = sp.res[2] - 1;
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kBigThreads) k_big_cells(const uint32_t* __res
             // digit counts, then their exclusive scan
             if (tid < 256u) base[tid] = 0u;
             __syncthreads();
-            for (uint32_t j = tid; j < m; j += kBigThreads) atomicAdd(&base[(from[j] >> shift) & 255u], 1u);
+            for (uint64_t j = tid; j < m; j += kBigThreads) atomicAdd(&base[(from[j] >> shift) & 255u], 1u);
             __syncthreads();
             if (warp == 0) {
                 uint32_t run = 0;
@@ -158,10 +158,10 @@ __global__ void __launch_bounds__(kBigThreads) k_big_cells(const uint32_t* __res
                     run += __shfl_sync(0xffffffffu, x, 31);
                 }
             }
-            for (uint32_t b = 0; b < m; b += kBigThreads) {
+            for (uint64_t b = 0; b < m; b += kBigThreads) {
                 for (uint32_t k = tid; k < kBigWarps * 256u; k += kBigThreads) whist[k >> 8][k & 255u] = 0u;
                 __syncthreads();
-                const uint32_t j = b + tid;
+                const uint64_t j = b + tid;
                 const bool ok = j < m;
                 const uint32_t v = ok ? from[j] : 0u;
                 const uint32_t digit = (v >> shift) & 255u;
@@ -187,7 +187,7 @@ __global__ void __launch_bounds__(kBigThreads) k_big_cells(const uint32_t* __res
             to = t;
         }
         // an odd number of passes leaves them in out.perm itself
-        for (uint32_t j = tid; j < m; j += kBigThreads) out.put(s + j, key, from[j]);
+        for (uint64_t j = tid; j < m; j += kBigThreads) out.put(s + (uint32_t)j, key, from[j]);
         __syncthreads();
     }
 }

@@ -632,8 +632,8 @@ __global__ void k_band_stamp(const float4* __restrict__ sorted, const uint32_t* 
                              Grid sc, float thr2, uint32_t* __restrict__ bits, Counters* ctr)
 {
     after_launch();
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t t = i / kLanes, plane = i % kLanes;
+    // (kLanes n threads: their number may pass 2^32, the particle's does not)
+    const uint32_t t = blockIdx.x * (blockDim.x / kLanes) + threadIdx.x / kLanes, plane = threadIdx.x % kLanes;
     bool is_s = false;
     if (t < n) is_s = psurf ? psurf[t] != 0 : surf[skeys[t]] != 0;
     warp_count(&ctr->n_surface, is_s && plane == 0);
@@ -1568,10 +1568,12 @@ __global__ void k_mc_classify(McArgs a, const Counters* ctr, uint32_t* tile_sums
     // 9M band vertices 92 us, 80 with runs of 128, 84 with 256; below a million the
     // shorter runs keep more warps busy (a 32k frame 10 / 12).
     const uint32_t span = nb < 1u << 20 ? 32u : 128u;
-    for (uint32_t t0 = span * warp; t0 < nb; t0 += span * nwarps) {
+    const uint32_t step = span * nwarps;
+    for (uint32_t t0 = span * warp; t0 < nb; t0 = next_of(t0, step, nb)) {
         uint32_t sum = 0;
 #pragma unroll 1
-        for (uint32_t t = t0 + lane; t < t0 + span; t += 32u) {
+        for (uint32_t k = lane; k < span; k += 32u) {
+            const uint32_t t = t0 + k;
             const uint32_t v = t < nb ? a.sv[t] : 0xffffffffu;
             uint32_t x, y, z;
             unlin3(v, a.sc, x, y, z);

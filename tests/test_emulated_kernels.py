@@ -1,4 +1,6 @@
 """Kernels run on the host lane by lane (tests/cpp/warp_emul.h)."""
+import pytest
+
 from tests import emulated
 
 
@@ -6,3 +8,12 @@ def test_tile_order_does_not_depend_on_the_order_of_atomics():
     """The two warps of a split work item lay out the same pass each for itself
     and write every second tile: a vertex must have one place."""
     assert emulated.run("tile_order") == "same\n"
+
+
+@pytest.mark.parametrize("what", ["stamp", "group", "classify"])
+def test_counts_above_two_to_the_31(what):
+    """Sizes that frame_plan accepts: no index wraps, every loop ends."""
+    got = emulated.run("big_counts", what, timeout=60)
+    if got == "no address space\n":
+        pytest.skip("cannot reserve the arrays' address space")
+    assert got == "ok\n"

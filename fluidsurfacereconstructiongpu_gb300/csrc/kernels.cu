@@ -1081,7 +1081,11 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
     // The chunk sums end where k_smooth's do, so that both kernels' sums agree
     // bit for bit for radii below a cell (max_span 3): where the whole block is
     // one set, at 32 candidates of its box; else at every 32 of the particle's own
-    // window, row by row (own_folds).
+    // window, row by row (own_folds).  k_smooth's totals also take the 0 of a chunk
+    // that lies beyond R, which can move a compensated total's last bit; after the
+    // first such 0 (s = s - c rounded) the next ones change nothing, so one stands for
+    // all.  (Without it 1 of 12,000 means in rows of 64 and more differed; 3k
+    // particles 302 -> 304 us, 45k 647 -> 648.)
     bool one_set = max_span >= 0;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -1136,6 +1140,7 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
                     const uint32_t c = (S.idx[k] - own) >> 5;
                     if (wt != 0.f && c != chunk_at) {
                         fold();
+                        if (c - chunk_at > 1u) tot.add(0.f);
                         chunk_at = c;
                     }
                     sum(S.q[comp][k], wt);
@@ -1199,6 +1204,7 @@ __global__ void __launch_bounds__(kQuadThreads, 6) k_smooth_quads(const float4* 
                     // the row's full chunks have ended, its rest waits for more
                     if (len >= 32u) {
                         if (chunk_at < (len >> 5)) fold();
+                        if (chunk_at + 1u < (len >> 5)) tot.add(0.f);
                         since = 0;
                     }
                     since += len & 31u;

@@ -17,3 +17,9 @@ def test_counts_above_two_to_the_31(what):
     if got == "no address space\n":
         pytest.skip("cannot reserve the arrays' address space")
     assert got == "ok\n"
+
+
+def test_smoothing_by_four_lanes_joins_its_chunk_sums_like_the_one_lane_kernel():
+    """Also chunks of 32 candidates that all lie beyond the radius, whose sum of
+    0 a compensated total still takes."""
+    assert emulated.run("smooth_sums") == "differing means 0, FP32 means 0, smoothed positions 0\n"

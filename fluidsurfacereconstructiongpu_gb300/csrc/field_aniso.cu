@@ -28,6 +28,7 @@
 #include "backward.h"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace fsr {
 namespace {
@@ -1200,6 +1201,7 @@ struct BwdGroupArgs {
 // (A block per group, whose eight warps met at five barriers per group, spent
 // most of its time waiting there; 500k-particle ZB05 frame: 0.67 -> 0.17 ms.)
 constexpr int kBwdVerts = 128;        // vertices of a pass
+constexpr float kFinite = 3.0e38f;    // larger factors are taken as not finite
 constexpr uint32_t kBwdSeg = 96;      // particles staged at a time
 template <bool TC01>
 struct IsoBwdSlice {
@@ -1215,6 +1217,7 @@ struct IsoBwdSlice {
     float gx[kBwdSeg], gy[kBwdSeg], gz[kBwdSeg];  // their dL/dx
     uint32_t cj[kBwdSeg];                         // their sorted index
     uint32_t list[kBwdSeg];                       // those within h of the tile
+    uint32_t nodd;                                // vertices that are not finite, listed in hist
     uint32_t rb[9], rp[10];
 };
 
@@ -1248,7 +1251,9 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
             pass_layout<true, kBwdVerts>(w.vloc, w.vrank, lo, a.sc, nullptr, w.hist, w.box, nv, lane, pl, ph);
             const uint32_t ntiles = (nv + 31) / 32;
             // the vertices' positions and factors; the places up to the last
-            // tile's end lie beyond h of everything
+            // tile's end lie beyond h of everything.  Vertices whose factors are not
+            // finite are set apart (odd_vertices)
+            uint32_t nodd = 0;
             for (uint32_t q = lane; q < 32u * ntiles; q += 32) {
                 float4 vp = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f);
                 float4 e = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1267,6 +1272,14 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
                         }
                     }
                 }
+                const bool odd = !(fabsf(TC01 ? gv : (e.x + e.y) + (e.z + e.w)) <= kFinite);
+                const uint32_t om = __ballot_sync(0xffffffffu, odd);
+                if (odd) {
+                    w.hist[nodd + __popc(om & ((1u << lane) - 1u))] = q;
+                    gv = 0.f;
+                    e = make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+                nodd += __popc(om);
                 const uint32_t p = q >> 1, s = q & 1u;
                 float* d = reinterpret_cast<float*>(w.vxy + p) + s;
                 d[0] = vp.x;
@@ -1283,8 +1296,42 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
                     d[2] = e.w;
                 }
             }
+            if (lane == 0) w.nodd = nodd;
             __syncwarp();
             uint32_t fill = 0;
+            // The clamp in the pair loop would let a vertex that is not finite reach
+            // every particle of its tile (0 x inf): these take the range test, and reach
+            // the staged particles within h of them only.  (The test in the pair loop
+            // of passes that need it, a second copy of the loop: 500k ZB05 frame's
+            // backward 397 -> 409 us without such a vertex; this way 401 -> 404.)
+            auto odd_vertices = [&]() {
+#pragma unroll 1
+                for (uint32_t o = 0; o < w.nodd; ++o) {
+                    const uint32_t q = w.hist[o], rank = w.vrank[q];
+                    const float4 vp = vert_pos(w.vloc[q], lo, a.sc);
+                    const float gv = __ldg(a.gphi + rank);
+#pragma unroll 1
+                    for (uint32_t i = lane; i < fill; i += 32) {
+                        const float dx = w.cx[i] - vp.x, dy = w.cy[i] - vp.y, dz = w.cz[i] - vp.z;
+                        const float d2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+                        if (!(d2 < h2)) continue;
+                        float sx = 0.f, sy = 0.f, sz = 0.f, k = gv * (d2 * inv_h2 - 1.0f) * inv_h2;
+                        if (!TC01) {
+                            const float4 m = __ldg(a.mv + rank);
+                            const float f = gv / sqrtf(fmaf(m.x, m.x, fmaf(m.y, m.y, m.z * m.z))) / m.w;
+                            const float u = 1.0f - d2 * inv_h2, wt = u * u * u;
+                            sx = wt * (f * m.x);
+                            sy = wt * (f * m.y);
+                            sz = wt * (f * m.z);
+                            k = f * (m.x * (dx - m.x) + m.y * (dy - m.y) + m.z * (dz - m.z)) * (-6.0f * u * u * inv_h2);
+                        }
+                        w.gx[i] += fmaf(k, dx, sx);
+                        w.gy[i] += fmaf(k, dy, sy);
+                        w.gz[i] += fmaf(k, dz, sz);
+                    }
+                }
+                __syncwarp();
+            };
             auto tiles = [&]() {
                 for (uint32_t i = lane; i < fill; i += 32) w.gx[i] = w.gy[i] = w.gz[i] = 0.f;
                 __syncwarp();
@@ -1346,6 +1393,7 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
                     }
                     __syncwarp();
                 }
+                if (w.nodd != 0u) odd_vertices();
                 for (uint32_t i = lane; i < fill; i += 32) {
                     const float4 g = make_float4(w.gx[i], w.gy[i], w.gz[i], 0.f);
                     if (g.x != 0.f || g.y != 0.f || g.z != 0.f) atomicAdd(a.gx + w.cj[i], g);
@@ -1462,11 +1510,13 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
             pass_layout<true, kBwdVerts>(w.vloc, w.vrank, lo, a.sc, nullptr, w.hist, w.box, nv, lane, pl, ph);
             const uint32_t ntiles = (nv + 31) / 32;
             // the places up to the last tile's end lie far away and have dL/dphi = 0
+            float all = 0.f;
             for (uint32_t q = lane; q < 32u * ntiles; q += 32) {
                 float4 vp = make_float4(1.0e18f, 1.0e18f, 1.0e18f, 0.f);
                 if (q < nv) {
                     vp = vert_pos(w.vloc[q], lo, a.sc);
                     vp.w = __ldg(a.gphi + w.vrank[q]);
+                    all += vp.w;
                 }
                 float* d = reinterpret_cast<float*>(w.vxy + (q >> 1)) + (q & 1u);
                 d[0] = vp.x;
@@ -1475,6 +1525,10 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
                 d[0] = vp.z;
                 d[2] = vp.w;
             }
+            // A vertex whose dL/dphi is not finite is not dropped by the clamp of 1 - q2 at
+            // 0 (0 x inf): passes that hold one (or whose lanes' sums overflow) test the
+            // range of each pair, so that it reaches the particles of its support only
+            const bool odd = __any_sync(0xffffffffu, !(fabsf(all) <= kFinite));
             __syncwarp();
             const uint32_t total_inv = w.total_inv;
             uint32_t fill = 0;
@@ -1506,32 +1560,41 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
                         float2 s[kBwdSums];
 #pragma unroll
                         for (int r = 0; r < kBwdSums; ++r) s[r] = make_float2(0.f, 0.f);
+                        auto walk = [&](auto odd_pass) {
+                            constexpr bool kOdd = decltype(odd_pass)::value;
 #pragma unroll 4
-                        for (uint32_t j = 0; j < pairs; ++j) {
-                            const float4 A = w.vxy[16u * t + j], Z = w.vzg[16u * t + j];
-                            const float2 dx = __ffma2_rn(make_float2(A.x, A.y), mone2, qx);
-                            const float2 dy = __ffma2_rn(make_float2(A.z, A.w), mone2, qy);
-                            const float2 dz = __ffma2_rn(make_float2(Z.x, Z.y), mone2, qz);
-                            const float2 t0 = __ffma2_rn(m0, dx, __ffma2_rn(m1, dy, __fmul2_rn(m2, dz)));
-                            const float2 t1 = __ffma2_rn(m3, dy, __fmul2_rn(m4, dz));
-                            const float2 q2 =
-                                __ffma2_rn(dx, t0, __ffma2_rn(dy, t1, __fmul2_rn(__fmul2_rn(m5, dz), dz)));
-                            float2 u = __ffma2_rn(q2, mone2, one2);
-                            u.x = fmaxf(u.x, 0.f);
-                            u.y = fmaxf(u.y, 0.f);
-                            const float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
-                            const float2 bx = __fmul2_rn(bb, dx), by = __fmul2_rn(bb, dy), bz = __fmul2_rn(bb, dz);
-                            s[0] = __fadd2_rn(s[0], bx);
-                            s[1] = __fadd2_rn(s[1], by);
-                            s[2] = __fadd2_rn(s[2], bz);
-                            s[3] = __ffma2_rn(bb, u, s[3]);
-                            s[4] = __ffma2_rn(bx, dx, s[4]);
-                            s[5] = __ffma2_rn(bx, dy, s[5]);
-                            s[6] = __ffma2_rn(bx, dz, s[6]);
-                            s[7] = __ffma2_rn(by, dy, s[7]);
-                            s[8] = __ffma2_rn(by, dz, s[8]);
-                            s[9] = __ffma2_rn(bz, dz, s[9]);
-                        }
+                            for (uint32_t j = 0; j < pairs; ++j) {
+                                const float4 A = w.vxy[16u * t + j], Z = w.vzg[16u * t + j];
+                                const float2 dx = __ffma2_rn(make_float2(A.x, A.y), mone2, qx);
+                                const float2 dy = __ffma2_rn(make_float2(A.z, A.w), mone2, qy);
+                                const float2 dz = __ffma2_rn(make_float2(Z.x, Z.y), mone2, qz);
+                                const float2 t0 = __ffma2_rn(m0, dx, __ffma2_rn(m1, dy, __fmul2_rn(m2, dz)));
+                                const float2 t1 = __ffma2_rn(m3, dy, __fmul2_rn(m4, dz));
+                                const float2 q2 =
+                                    __ffma2_rn(dx, t0, __ffma2_rn(dy, t1, __fmul2_rn(__fmul2_rn(m5, dz), dz)));
+                                float2 u = __ffma2_rn(q2, mone2, one2);
+                                u.x = fmaxf(u.x, 0.f);
+                                u.y = fmaxf(u.y, 0.f);
+                                float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
+                                if (kOdd) {
+                                    if (!(u.x > 0.f)) bb.x = 0.f;
+                                    if (!(u.y > 0.f)) bb.y = 0.f;
+                                }
+                                const float2 bx = __fmul2_rn(bb, dx), by = __fmul2_rn(bb, dy), bz = __fmul2_rn(bb, dz);
+                                s[0] = __fadd2_rn(s[0], bx);
+                                s[1] = __fadd2_rn(s[1], by);
+                                s[2] = __fadd2_rn(s[2], bz);
+                                s[3] = __ffma2_rn(bb, u, s[3]);
+                                s[4] = __ffma2_rn(bx, dx, s[4]);
+                                s[5] = __ffma2_rn(bx, dy, s[5]);
+                                s[6] = __ffma2_rn(bx, dz, s[6]);
+                                s[7] = __ffma2_rn(by, dy, s[7]);
+                                s[8] = __ffma2_rn(by, dz, s[8]);
+                                s[9] = __ffma2_rn(bz, dz, s[9]);
+                            }
+                        };
+                        if (odd) walk(std::true_type());
+                        else walk(std::false_type());
 #pragma unroll
                         for (int r = 0; r < kBwdSums; ++r) w.s[r][i] += s[r].x + s[r].y;
                     }
@@ -1611,7 +1674,11 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
                     float2 u = __ffma2_rn(q2, mone2, one2);
                     u.x = fmaxf(u.x, 0.f);
                     u.y = fmaxf(u.y, 0.f);
-                    const float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
+                    float2 bb = __fmul2_rn(make_float2(Z.z, Z.w), __fmul2_rn(u, u));
+                    if (odd) {
+                        if (!(u.x > 0.f)) bb.x = 0.f;
+                        if (!(u.y > 0.f)) bb.y = 0.f;
+                    }
                     sx = __ffma2_rn(bb, dx, sx);
                     sy = __ffma2_rn(bb, dy, sy);
                     sz = __ffma2_rn(bb, dz, sz);

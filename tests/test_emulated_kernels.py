@@ -23,3 +23,9 @@ def test_smoothing_by_four_lanes_joins_its_chunk_sums_like_the_one_lane_kernel()
     """Also chunks of 32 candidates that all lie beyond the radius, whose sum of
     0 a compensated total still takes."""
     assert emulated.run("smooth_sums") == "differing means 0, FP32 means 0, smoothed positions 0\n"
+
+
+def test_adjoints_of_vertices_that_are_not_finite():
+    """A NaN or infinite dL/dphi reaches the particles in whose support the
+    vertex lies, as a range test has it, and no others."""
+    assert emulated.run("adjoints", "nan") == "ok\n"

@@ -1602,7 +1602,11 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
                 }
                 for (uint32_t i = lane; i < fill; i += 32) {
                     const float gx = w.s[0][i], gy = w.s[1][i], gz = w.s[2][i], sc = w.s[3][i];
-                    if (gx == 0.f && gy == 0.f && gz == 0.f && sc == 0.f) continue;
+                    // (the first moments can cancel where the second ones do not)
+                    bool some = gx != 0.f || gy != 0.f || gz != 0.f || sc != 0.f;
+#pragma unroll
+                    for (int r = 4; r < kBwdSums; ++r) some = some || w.s[r][i] != 0.f;
+                    if (!some) continue;
                     const uint32_t id = w.cj[i];
                     const float f = -6.0f * w.coef[i];
                     const float m01 = 0.5f * w.m[1][i], m02 = 0.5f * w.m[2][i], m12 = 0.5f * w.m[4][i];

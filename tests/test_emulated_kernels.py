@@ -29,3 +29,8 @@ def test_adjoints_of_vertices_that_are_not_finite():
     """A NaN or infinite dL/dphi reaches the particles in whose support the
     vertex lies, as a range test has it, and no others."""
     assert emulated.run("adjoints", "nan") == "ok\n"
+
+
+def test_anisotropic_adjoint_where_the_first_sums_cancel():
+    """dL/dG of a particle whose sums of b d and g u^3 vanish exactly."""
+    assert emulated.run("adjoints", "cancel") == "ok\n"

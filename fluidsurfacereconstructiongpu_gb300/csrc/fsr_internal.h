@@ -17,9 +17,11 @@ namespace fsr {
 // Has the host's page tables hold `bytes` at p before a device copy writes
 // there.  A copy into pages that were never written (a new array) faults them
 // in from the device side: 200 KB 190 us, 66 when they are populated first;
-// 3 MB 300 / 190.  Memory in use (21 and 36 us) is left after one look at the
-// page tables.  Memory that cannot be populated (device, pinned, unmapped)
-// stays as it is; the copy decides.
+// 3 MB 300 / 190.  Anonymous memory in use (21 and 36 us) is left after one look
+// at the page tables; of a file mapping the look tells what the page cache holds,
+// so that cached pages still fault during the copy.  The first refusal ends it
+// (device or unmapped memory, a mapping that may not be written, a kernel before
+// Linux 5.14): the copy decides.
 void populate_host(void* p, size_t bytes);
 
 struct DevBuf {

@@ -153,8 +153,8 @@ void fsr::populate_host(void* p, size_t bytes)
     for (uintptr_t a = (uintptr_t)p & ~(page - 1); a < end; a += page * sizeof(there)) {
         const uintptr_t len = std::min<uintptr_t>(end - a, page * sizeof(there)), pages = (len + page - 1) / page;
         if (mincore((void*)a, len, there) != 0) break;  // not the host's memory
-        if (!std::all_of(there, there + pages, [](unsigned char c) { return c & 1; }))
-            (void)madvise((void*)a, len, kPopulateWrite);
+        if (std::all_of(there, there + pages, [](unsigned char c) { return c & 1; })) continue;
+        if (madvise((void*)a, len, kPopulateWrite) != 0) break;  // an older kernel, or not to be written by the host
     }
     errno = saved;
 #else

@@ -108,8 +108,8 @@ struct fsr_handle {
     cudaEvent_t ev_start = nullptr;
     cudaEvent_t ev[FSR_NUM_STAGES] = {};
 
-    // host mesh arrays that run_frame populates while the device works, and how
-    // much of them (fsr_reconstruct_host: the size of the frame before)
+    // host mesh arrays that run_frame populates while the device works on the first
+    // attempt, and how much of them (fsr_reconstruct_host: the size of the frame before)
     void* host_out[2] = {};
     size_t host_out_bytes = 0;
 

@@ -22,6 +22,7 @@
 #include <cstdio>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/fsr.h"
@@ -611,7 +612,7 @@ fsr_status run_frame(fsr_handle* h, const fsr_frame_header& hdr, const float* d_
     for (int attempt = 0; attempt < 4; ++attempt) {
         if ((s = frame_buffers(h, fp)) != FSR_OK) return s;
         if ((s = frame_enqueue(h, fp, d_xyz, d_den, st, timing)) != FSR_OK) return s;
-        for (void* p : h->host_out) populate_host(p, h->host_out_bytes);
+        for (void*& p : h->host_out) populate_host(std::exchange(p, nullptr), h->host_out_bytes);
         CK(cudaStreamSynchronize(st));
         bool retry = false;
         if ((s = frame_finish(h, fp, timing, &retry)) != FSR_OK || !retry) return s;
@@ -737,7 +738,7 @@ fsr_status fsr_reconstruct_host(fsr_handle* h, const fsr_frame_header* hdr, cons
     h->host_out[1] = out_nrm;
     h->host_out_bytes = 12ull * std::min<uint64_t>(capacity, h->stats.n_mesh_vertices);
     fsr_status s = run_frame(h, *hdr, (const float*)h->in_xyz.ptr, (const float*)h->in_den.ptr, n, st);
-    h->host_out[0] = h->host_out[1] = nullptr;
+    h->host_out[0] = h->host_out[1] = nullptr;  // (left by a frame that failed before its first attempt)
     if (s != FSR_OK) return s;
     const uint64_t nv = h->stats.n_mesh_vertices;
     *n_vertices = nv;

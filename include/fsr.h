@@ -147,7 +147,11 @@ fsr_status fsr_reconstruct(fsr_handle* h, const fsr_frame_header* hdr, const flo
  * device, reconstructs, copies the triangle soup back (positions and
  * normals, 3 floats per mesh vertex, 3 mesh vertices per triangle, in the
  * reference's order).  *n_vertices receives the mesh vertex count; if it
- * exceeds `capacity` nothing is copied and FSR_ERR_CAPACITY is returned. */
+ * exceeds `capacity` nothing is copied and FSR_ERR_CAPACITY is returned.
+ * While the device works, the pages of out_pos and out_nrm may be made
+ * resident for as many vertices as the handle's frame before had (at most
+ * `capacity`), their contents unchanged: also where this frame's mesh turns
+ * out smaller or the call fails. */
 fsr_status fsr_reconstruct_host(fsr_handle* h, const fsr_frame_header* hdr, const float* xyz,
                                 const float* density, uint64_t n, float* out_pos, float* out_nrm,
                                 uint64_t capacity, uint64_t* n_vertices, void* stream);

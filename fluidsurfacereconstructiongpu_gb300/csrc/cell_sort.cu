@@ -202,7 +202,7 @@ bool cell_sort_wanted(uint64_t cells, uint32_t n) { return n > 0 && cells <= 8ul
 cudaError_t launch_cell_sort(const KernelCtx& c, const CellSort& a, Counters* ctr)
 {
     const int threads = 256;
-    const unsigned blocks = (unsigned)((a.n + threads - 1) / threads);
+    const unsigned blocks = (unsigned)(((uint64_t)a.n + threads - 1) / threads);
     const uint32_t cells = a.sp.res[0] * a.sp.res[1] * a.sp.res[2];
     const uint32_t groups = (a.sp.res[0] + 1) * (a.sp.res[1] + 1) * (a.sp.res[2] + 1);
     cudaError_t e = cudaSuccess;

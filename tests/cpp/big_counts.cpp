@@ -1,6 +1,7 @@
 // Kernels at counts above 2^31, in arrays of which only the touched pages exist.
 //   stamp:    a surface particle above 2^31 stamps its band
 //   group:    the grouping loop ends at 2^32 - 2 particles
+//   blocks:   the counting sort's launches cover 2^32 - 2 particles
 //   classify: the classification's loop ends at 2^32 - 2 band vertices
 #include "warp_emul.h"
 
@@ -24,6 +25,9 @@ static T* sparse(uint64_t n)
 }
 
 namespace fsr {
+cudaError_t scan_counts(uint32_t*, uint32_t, uint32_t*, cudaStream_t) { return cudaSuccess; }
+uint32_t bits_for(uint64_t) { return 32; }
+
 static uint32_t stamped(uint32_t n, uint32_t at, std::vector<uint32_t>& bits)
 {
     Grid sp{}, sc{};
@@ -75,6 +79,22 @@ int main(int, char** argv)
         emu::launch(&cfg, k_group, keys, arrival, first, n, sp, 1u, 8u, grouped, nullptr, nullptr, nullptr, nullptr,
                     nullptr, &ctr);
         std::printf(grouped[1] == n - 1 ? "ok\n" : "last particle not grouped\n");
+    } else if (what == "blocks") {
+        CellSort a{};
+        a.n = 0xFFFFFFFEu;
+        a.sp.cs = 1.f;
+        a.sp.res[0] = a.sp.res[1] = a.sp.res[2] = 1;
+        KernelCtx c{};
+        c.num_sms = 1;
+        std::vector<uint64_t> grids;  // of the launches, in blocks
+        emu::wanted_block = [&](unsigned b) {
+            if (b == 0) grids.push_back(0);
+            ++grids.back();
+            return false;
+        };
+        launch_cell_sort(c, a, nullptr);
+        const bool whole = grids.size() == 4 && grids[0] == 1u << 24 && grids[2] == 1u << 24;
+        std::printf(whole ? "ok\n" : "too few blocks\n");
     } else {
         const uint32_t n = 0xFFFFFFFEu;
         McArgs a{};

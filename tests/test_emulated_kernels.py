@@ -10,7 +10,7 @@ def test_tile_order_does_not_depend_on_the_order_of_atomics():
     assert emulated.run("tile_order") == "same\n"
 
 
-@pytest.mark.parametrize("what", ["stamp", "group", "classify"])
+@pytest.mark.parametrize("what", ["stamp", "group", "blocks", "classify"])
 def test_counts_above_two_to_the_31(what):
     """Sizes that frame_plan accepts: no index wraps, every loop ends."""
     got = emulated.run("big_counts", what, timeout=60)

@@ -51,6 +51,7 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
     const uint32_t nq = min(ctr->n_valid, a.cap_valid);
     const uint32_t rx = a.sc.res[0], rxy = a.sc.res[0] * a.sc.res[1];
     const uint32_t kx = a.sp.res[0] + 1, ky = a.sp.res[1] + 1;
+    BwdGroupList groups(a.glist, a.sp);
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nq; q += gridDim.x * blockDim.x) {
         const uint32_t t = a.valid[q];
         const uint32_t info = a.mc[t];
@@ -109,8 +110,9 @@ __global__ void __launch_bounds__(kT) k_mc_backward(BwdArgs a, const Counters* c
             for (uint32_t cy = lo[1]; cy <= hi[1]; ++cy)
                 for (uint32_t cx = lo[0]; cx <= hi[0]; ++cx) {
                     const uint32_t key = (cz * ky + cy) * kx + cx;
-                    if (a.gkey[key] == 0u && atomicExch(&a.gkey[key], 1u) == 0u)
-                        a.glist[4 + atomicAdd(&a.glist[0], 1u)] = key;
+                    if (a.gkey[key] != 0u) continue;
+                    const uint32_t flag = __ldg(a.gflag + key);  // (in flight with the mark)
+                    if (atomicExch(&a.gkey[key], 1u) == 0u) groups.add(key, (flag & kCrowdedGroup) != 0u);
                 }
     }
 }

@@ -18,8 +18,9 @@ struct BwdArgs {
     const float* gmesh;      // dL/d mesh vertex positions, 3 floats each
     float* gphi;             // dL/dphi per band vertex (zeroed)
     uint32_t* gkey;          // per window-centre key: holds a vertex with dL/dphi != 0 (zeroed)
-    uint32_t* glist;         // [0] keys listed, [1] [2] work counters of the grouped adjoints (zeroed),
-                             // [4 ..] the keys with gkey set, in the order k_mc_backward met them
+    uint32_t* glist;         // the keys with gkey set, in the order k_mc_backward met them (BwdGroupList); [1] [2]
+                             // work counters of the grouped adjoints; the first 4 words zeroed
+    const uint32_t* gflag;   // per key: kCrowdedGroup (kernels.h)
     const float4* sorted;
     const uint32_t* skeys;
     const uint32_t* perm;
@@ -36,6 +37,28 @@ struct BwdArgs {
     float4* gx;              // dL/dx in sorted order (zeroed)
     float iso, h, sigma;
     uint32_t cap_band, cap_valid;
+};
+
+// The window groups holding gradient vertices: [0] of them from the list's 5th
+// word on, [3] crowded ones (kCrowdedGroup) from its end.
+struct BwdGroupList {
+    uint32_t* list;
+    uint32_t end;
+#if defined(__CUDACC__)
+    __device__ __forceinline__ BwdGroupList(uint32_t* l, const Grid& sp)
+        : list(l), end(4u + (sp.res[0] + 1) * (sp.res[1] + 1) * (sp.res[2] + 1))
+    {
+    }
+    __device__ __forceinline__ void add(uint32_t key, bool crowded)
+    {
+        if (crowded) list[end - 1u - atomicAdd(&list[3], 1u)] = key;
+        else list[4u + atomicAdd(&list[0], 1u)] = key;
+    }
+    __device__ __forceinline__ uint32_t usual() const { return list[0]; }
+    __device__ __forceinline__ uint32_t crowded() const { return list[3]; }
+    // the k-th, the c crowded ones first
+    __device__ __forceinline__ uint32_t at(uint32_t k, uint32_t c) const { return list[k < c ? end - 1u - k : 4u + (k - c)]; }
+#endif
 };
 
 // Grouped adjoint of the ZB05 / TC01 fields (field_aniso.cu); adds into a.gx

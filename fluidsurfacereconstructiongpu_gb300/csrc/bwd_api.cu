@@ -102,6 +102,7 @@ extern "C" fsr_status fsr_backward(fsr_handle* h, const float* d_grad_mesh_pos, 
     a.gphi = (float*)h->gphi.ptr;
     a.gkey = (uint32_t*)h->gkey.ptr;
     a.glist = (uint32_t*)h->gklist.ptr;
+    a.gflag = (const uint32_t*)h->gflag.ptr;
     a.sorted = (const float4*)h->sorted.ptr;
     a.skeys = h->skeys_ptr;
     a.perm = h->perm_ptr;

@@ -26,6 +26,7 @@ namespace {
 
 constexpr uint32_t kBigCell = 1024;
 constexpr uint32_t kDenseParticles = 16;
+constexpr uint32_t kCrowdedParticles = 7 * 256;  // four times the usual 64 a cell (h = 4 spacings)
 
 __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp, uint32_t* __restrict__ keys,
                              uint32_t* __restrict__ arrival, uint32_t* __restrict__ count, Counters* ctr)
@@ -54,7 +55,8 @@ __global__ void k_hash_count(const float* __restrict__ xyz, uint32_t n, Grid sp,
 // zeros in the cell-sized arrays of later stages (a memset each before).
 // gflag: kDenseGroup for the window groups whose cell and its six neighbours hold
 // enough particles for their field to be a long work item (an isolated
-// particle's groups: one or two), which k_band_list lists first.
+// particle's groups: one or two), which k_band_list lists first; kCrowdedGroup
+// for those whose adjoint several warps share (k_field_iso_backward).
 __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ arrival,
                         const uint32_t* __restrict__ first, uint32_t n, Grid sp, uint32_t cells, uint32_t groups,
                         uint32_t* __restrict__ grouped, uint2* __restrict__ ranges, uint8_t* __restrict__ occ,
@@ -75,7 +77,7 @@ __global__ void k_group(const uint32_t* __restrict__ keys, const uint32_t* __res
         uint32_t sum = held(row + (x ? x - 1 : 0u), row + min(x + 1, x1));  // x-neighbours are one run
         auto one = [&](uint32_t yy, uint32_t zz) { const uint32_t k = lin3(x, yy, zz, sp); return held(k, k); };
         sum += one(y ? y - 1 : 0u, z) + one(min(y + 1, y1), z) + one(y, z ? z - 1 : 0u) + one(y, min(z + 1, z1));
-        gflag[c] = sum >= kDenseParticles ? kDenseGroup : 0u;
+        gflag[c] = (sum >= kDenseParticles ? kDenseGroup : 0u) | (sum >= kCrowdedParticles ? kCrowdedGroup : 0u);
         if (c >= cells) continue;
         const uint32_t s = __ldg(first + c), e = __ldg(first + c + 1);
         ranges[c] = e > s ? make_uint2(s, e) : make_uint2(kEmpty, kEmpty);

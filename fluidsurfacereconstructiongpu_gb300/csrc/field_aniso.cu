@@ -1203,6 +1203,20 @@ struct BwdGroupArgs {
 constexpr int kBwdVerts = 128;        // vertices of a pass
 constexpr float kFinite = 3.0e38f;    // larger factors are taken as not finite
 constexpr uint32_t kBwdSeg = 96;      // particles staged at a time
+// Its work items.  Few groups are cut into more of them: on fine grids by slabs of
+// vertices, on coarse ones (up to 4 vertices per cell: two to five slabs at most) by
+// runs of candidates; crowded groups (kCrowdedGroup) are shared in runs of candidates
+// on all grids, however many groups there are.  Backward, us, block per group / a warp
+// per group or slab / now: default grid, ZB05: 20k-particle block 50 / 66 / 46, 30k at 140
+// a cell 57 / 97 / 47, 1M at 200 a cell 122 / 160 / 118; TC01, 300k at 1000 a cell 82 /
+// 166 / 55; 90k ZB05 particles of which 85k lie in a few cells, default grid 419 / 2380 /
+// 371, fine 2330 / 5990 / 541.  Frames without such groups: 500k fine 907 / 396 / 398.
+constexpr uint32_t kCrowdParts = 64, kPartCandidates = 128;
+__device__ __forceinline__ uint32_t crowd_parts(uint32_t ncrowd)
+{
+    return min(kCrowdParts, (kSlabTarget + ncrowd) / max(ncrowd, 1u));
+}
+
 template <bool TC01>
 struct IsoBwdSlice {
     float4 vxy[kBwdVerts / 2];                // the pass's vertices two to a pair: (x, x', y, y')
@@ -1229,8 +1243,9 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
     const int lane = threadIdx.x & 31;
     IsoBwdSlice<TC01>& w = slices[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap_band);
-    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mc_backward)
-    const uint32_t nslab = field_slabs(nlist);
+    const BwdGroupList groups(a.glist, a.sp);
+    const uint32_t ncrowd = groups.crowded(), cparts = crowd_parts(ncrowd);
+    const uint32_t nusual = groups.usual(), nsub = field_slabs(nusual);
     const float h2 = a.h * a.h, inv_h2 = 1.0f / h2;
     const float cr = cull_radius(a.h, a.sp.cs), cr2 = cr * cr;
     const float2 inv2 = make_float2(inv_h2, inv_h2), ninv2 = make_float2(-inv_h2, -inv_h2);
@@ -1240,11 +1255,21 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
         uint32_t k = 0;
         if (lane == 0) k = atomicAdd(&a.glist[2], 1u);
         k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= nlist * nslab) break;
+        if (k >= ncrowd * cparts + nusual * nsub) break;
+        const bool crowd = k < ncrowd * cparts;
+        const uint32_t item = crowd ? k : k - ncrowd * cparts, cut = crowd ? cparts : nsub;
+        const bool by_slab = !crowd && a.ratio > 4;
         int c[3], lo[3], hi[3];
-        if (!group_box(a.glist[4 + k / nslab], a.sp, a.sc, a.ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi))
+        if (!group_box(groups.at((crowd ? 0u : ncrowd) + item / cut, ncrowd), a.sp, a.sc, a.ratio, c, lo, hi) ||
+            (by_slab && !slab_box(item % cut, cut, lo, hi)))
             continue;
-        const uint32_t total = window_rows(a.sp, a.ranges, c, w.rb, w.rp, lane);
+        uint32_t begin = 0, total = window_rows(a.sp, a.ranges, c, w.rb, w.rp, lane);  // the item's candidates
+        if (!by_slab && cut > 1u) {
+            const uint32_t step = max(kPartCandidates, (total / cut + 32u) & ~31u);
+            begin = (item % cut) * step;
+            if (begin >= total) continue;
+            total = min(total, begin + step);
+        }
 
         auto pass = [&](uint32_t nv) {
             float4 pl, ph;
@@ -1402,7 +1427,7 @@ __global__ void __launch_bounds__(kFT, 6) k_field_iso_backward(BwdArgs a, const 
                 fill = 0;
             };
             int row = 0;
-            for (uint32_t cb = 0; cb < total; cb += 32) {
+            for (uint32_t cb = begin; cb < total; cb += 32) {
                 const uint32_t j = cb + lane;
                 bool keep = false;
                 float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -1477,7 +1502,8 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
     const int lane = threadIdx.x & 31;
     AnisoBwdSlice& w = reinterpret_cast<AnisoBwdSlice*>(smem)[threadIdx.x >> 5];
     const uint32_t nb = min(ctr->n_band, a.cap);
-    const uint32_t nlist = a.glist[0];  // groups holding gradient vertices (k_mc_backward)
+    const BwdGroupList groups(a.glist, a.sp);
+    const uint32_t ncrowd = groups.crowded(), nlist = groups.usual() + ncrowd;  // groups holding gradient vertices
     // Few groups are cut into more work items: fine grids by slabs of vertices,
     // coarse ones, whose groups hold few vertices, by runs of candidates (backward
     // by slabs / runs, ms: 10 vertices per cell, 20k particles 0.21 / 0.25, 150k 0.44 / 0.53;
@@ -1492,7 +1518,7 @@ __global__ void __launch_bounds__(kFT, 4) k_field_aniso_backward(BwdGroupArgs a,
         if (k >= nlist * nsub) break;
         const uint32_t part = k % nparts;
         int c[3], lo[3], hi[3];
-        if (!group_box(a.glist[4 + k / nsub], a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi))
+        if (!group_box(groups.at(k / nsub, ncrowd), a.sp, a.sc, ratio, c, lo, hi) || !slab_box(k % nslab, nslab, lo, hi))
             continue;
         bool tables = false;
         uint32_t total = 0;

@@ -51,8 +51,9 @@ void launch_band_stamp(const KernelCtx& c, const float4* sorted, const uint32_t*
 // The band list, and the list of the window groups (spatial cells of the
 // (res + 1)^3 grid the grouped field kernels walk) that hold band vertices:
 // the ones among many particles from the list's front, the others from its end
-// (GroupList).  gflag: one word per group, starting at 0 or kDenseGroup (cell_sort.cu).
-constexpr uint32_t kMarkedGroup = 1u, kDenseGroup = 2u;
+// (GroupList).  gflag: one word per group, starting at 0 or with kDenseGroup and
+// kCrowdedGroup set (cell_sort.cu).
+constexpr uint32_t kMarkedGroup = 1u, kDenseGroup = 2u, kCrowdedGroup = 4u;
 struct GroupMark {
     Grid sp, sc;
     uint32_t* gflag;

@@ -3,6 +3,8 @@
 //   nan:    one vertex's dL/dphi is not finite: the particles within reach of it
 //           get a gradient that is not finite, the others theirs without it
 //   cancel: dL/dphi whose first sums vanish for a particle, but not its dL/dG
+//   shared: groups whose candidates several warps share, every second one listed as
+//           crowded
 #include "warp_emul.h"
 
 #include "field_aniso.cu"
@@ -244,6 +246,27 @@ int main(int, char** argv)
                 else s.iso(kind == 1);
                 if (!check(s, std::min(kind, 2), "nan")) return 0;
             }
+    } else if (what == "shared") {
+        for (int kind = 0; kind < 3; ++kind) {
+            std::vector<float4> pos;
+            std::vector<float> G;
+            for (int i = 0; i < 900; ++i) {
+                pos.push_back(make_float4(0.75f + uniform(), 0.75f + uniform(), 0.75f + uniform(), 0.5f + uniform()));
+                for (int a = 0; a < 9; ++a) G.push_back(a % 4 == 0 ? 1.75f + 0.5f * uniform() : 0.f);
+            }
+            Scene s(pos, G);
+            for (uint32_t v = 0; v < s.nv; ++v) {
+                if (uniform() < 0.5f) s.gphi[v] = uniform() - 0.5f;
+                s.mv[v] = make_float4(uniform() - 0.5f, uniform() - 0.5f, uniform() - 0.5f, 1.f + uniform());
+            }
+            const uint32_t keys = s.glist[0];
+            s.glist[0] = 0;
+            BwdGroupList list(s.glist.data(), s.sp);
+            for (uint32_t k = 0; k < keys; ++k) list.add(k, k % 2 == 0);
+            if (kind == 2) s.aniso();
+            else s.iso(kind == 1);
+            if (!check(s, kind, "shared")) return 0;
+        }
     } else {
         // at a vertex, G = 1.75 I: +1 a step away along x, -1 along y
         const uint32_t at[3] = {10, 10, 10};

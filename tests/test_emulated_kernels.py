@@ -34,3 +34,8 @@ def test_adjoints_of_vertices_that_are_not_finite():
 def test_anisotropic_adjoint_where_the_first_sums_cancel():
     """dL/dG of a particle whose sums of b d and g u^3 vanish exactly."""
     assert emulated.run("adjoints", "cancel") == "ok\n"
+
+
+def test_adjoints_of_groups_that_warps_share():
+    """Runs of candidates, usual and crowded groups."""
+    assert emulated.run("adjoints", "shared") == "ok\n"

@@ -8,8 +8,9 @@
 //      no particular order inside one;
 //   4. each particle's place inside its cell is the number of smaller particle
 //      numbers there (the sort is stable), which also gathers the particles.
-// Five launches with a scan in one block (seven with a tiled scan) instead of
-// the radix sort's two or three passes of three to five; the radix sort stays
+// Five launches with a scan in one block, six or (beyond kSumTiles tiles) seven
+// with the tiled one, one fewer for at most kBigCell particles, instead of the
+// radix sort's two or three passes of three to five; the radix sort stays
 // for sparse grids, whose scan would cost more than its passes.  Cells of more
 // than kBigCell particles are left to a block each, which sorts their particle
 // numbers by radix (the count in step 4 is quadratic).

@@ -147,7 +147,7 @@ uint32_t grid_for_tiles(uint64_t n_max)
 // 4 x 1024 consecutive elements, each thread four of them, a block scan per
 // tile and a running carry.  One launch instead of three.
 constexpr uint32_t kSingleThreads = 1024;
-constexpr uint32_t kSingleMax = 1u << 14;  // longer arrays take the tiled three-kernel scan (one block is slower from ~64k on)
+constexpr uint32_t kSingleMax = 1u << 14;  // longer arrays take the tiled scan of two or three kernels (one block is slower from ~64k on)
 template <ScanInput M>
 __global__ void __launch_bounds__(kSingleThreads) k_scan_single(const uint32_t* in, uint32_t* out, uint32_t n,
                                                                 uint32_t* total)
